@@ -10,9 +10,9 @@
 // prefilter_bands; here lo16 rounded down to FP16) is a candidate, and only
 // candidates reach the exact check and the register compare of part 2
 // (k_sym_check, kernels_allpairs.cu).  The threshold rides in the MMA as a
-// bias column (row side 1.0, column side -lo16 in the last half, free for
-// S < 64), so a candidate is a product whose sign bit is clear; byte permutes
-// gather the sign bits of 32 products into one mask.
+// bias column (row side 1.0, column side -lo16 in the last half of the last K
+// step in use), so a candidate is a product whose sign bit is clear; one
+// funnel shift a product gathers the sign bits of 32 products into a mask.
 //
 // Work: items (128-row block rb, 256-column tile ct) of the pairs i < j with j
 // in a column window [jlo, jhi) (the whole upper triangle, or the columns of
@@ -22,14 +22,21 @@
 // (the row block's 128 rows once per block into a 2-deep ring, each column
 // tile's 256 rows into a 4-deep ring), warp 1 allocates TMEM (two 256-column
 // accumulators, so an item's MMAs run while the epilogue reads the previous
-// item) and issues 4 MMAs of K = 16 per item, warps 2-17 are the epilogue: a
+// item) and issues the MMAs of K = 16 that hold the S products and the bias per
+// item, warps 2-17 are the epilogue: a
 // thread takes one row and 64 of the tile's columns, keeps the pairs j > i
 // with j in the window and a product of at least lo16 (a contig without
 // abundance has a zero unit row, so it never gets there; part 2 checks the
-// flags), and appends them to its 32-row block's candidate list (entry
-// r << 27 | j, r the row within the block) with one atomic per warp and item.
+// flags).  A warp gathers its entries (r << 27 | j, r the row within the
+// 32-row block) in shared memory and appends 512 at a time to its block's
+// candidate list: with one list atomic per warp and item the warps waited on
+// the atomic's round trip, with a CTA-wide vote per item on one another.
 // A block's list has the capacity the host gave it; the count goes on past it,
 // so a pass that overflows is rerun with exact capacities.
+//
+// Bound by the epilogue's integer issue (ALU 63%, issue 58%; tensor 12% at
+// S = 20).  S = 20, m = 500: 30,000 contigs 175 -> 120 us, 50,000 462 -> 293 us,
+// 200,003 contigs at S = 30 in eight column windows 19.6 -> 11.9 ms.
 //
 // Every mbarrier wait is bounded (2 s of %globaltimer); a wait that runs out
 // records an error code for the host and the CTA stops issuing work, waits
@@ -55,6 +62,7 @@ constexpr int kPN = 256;                       // columns per item (UMMA N)
 constexpr int kPK = 64;                        // halves per padded unit row (128 bytes)
 constexpr int kPStages = 4;                    // column-tile ring
 constexpr int kPEpiWarps = 16;
+constexpr int kPBuf = 512;                     // entries an epilogue warp gathers before it lists them
 constexpr int kPThreads = (2 + kPEpiWarps) * 32;
 constexpr int kABytes = kPM * kPK * 2;         // 16 KB
 constexpr int kBBytes = kPN * kPK * 2;         // 32 KB
@@ -68,6 +76,7 @@ struct PfArgs {
   int jlo, jhi;           // pairs i < j with j in [jlo, jhi) (rows [0, jhi))
   int ct_lo;              // first column tile: jlo / 256
   const int32_t *item0;   // [RB + 1] first item of each 128-row block
+  int ksteps;             // K steps of 16 halves that hold the rows and the bias column
   int RB, NT, items;      // row blocks below jhi, column tiles below jhi, items
   uint32_t *cand;         // block b's entries at cand + coff[b], coff[b + 1] - coff[b] of them
   const int64_t *coff;    // [B32 + 1]
@@ -83,20 +92,6 @@ __device__ __forceinline__ void mma_f16(uint32_t dt, uint64_t ad, uint64_t bd, u
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(dt), "l"(ad), "l"(bd), "r"(kIdescF16), "r"(acc));
-}
-
-// Named barrier 1 of the epilogue warps; returns the OR of every thread's flag.
-__device__ __forceinline__ uint32_t pf_barrier_or(uint32_t flag) {
-  uint32_t out;
-  asm volatile(
-      "{\n\t.reg .pred pi, po;\n\t"
-      "setp.ne.u32 pi, %1, 0;\n\t"
-      "barrier.cta.red.or.pred po, 1, %2, pi;\n\t"
-      "selp.u32 %0, 1, 0, po;\n\t}"
-      : "=r"(out)
-      : "r"(flag), "n"(kPEpiWarps * 32)
-      : "memory");
-  return out;
 }
 
 // Item it -> (row block rb, column tile ct); the next item in order.
@@ -126,7 +121,8 @@ k_sym_prefilter(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
   uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t *sa = base;                                  // [2][kABytes]
   uint8_t *sb = base + 2 * kABytes;                    // [kPStages][kBBytes]
-  uint64_t *bars = (uint64_t *)(sb + kPStages * kBBytes);
+  uint32_t *ebuf = (uint32_t *)(sb + kPStages * kBBytes);   // [kPEpiWarps][kPBuf]
+  uint64_t *bars = (uint64_t *)(ebuf + kPEpiWarps * kPBuf);
   // bars: fullA[2], emptyA[2], full[S], empty[S], tfull[2], tempty[2], mdone
   uint32_t *tmem_slot = (uint32_t *)(bars + 4 + 2 * kPStages + 5);
   int *abort_flag = (int *)(tmem_slot + 4);
@@ -148,7 +144,7 @@ k_sym_prefilter(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
       mbar_init(fullA(i), 1);
       mbar_init(emptyA(i), 1);
       mbar_init(tfull(i), 1);
-      mbar_init(tempty(i), kPEpiWarps * 32);
+      mbar_init(tempty(i), kPEpiWarps);
     }
     for (int s = 0; s < kPStages; ++s) {
       mbar_init(full(s), 1);
@@ -244,7 +240,8 @@ k_sym_prefilter(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
         const uint64_t db = sdesc128(smem_u32(sb + (size_t)s * kBBytes));
 #pragma unroll
         for (int kk = 0; kk < kPK / 16; ++kk)           // K = 16 halves (32 bytes) a step
-          mma_f16(tbase + (uint32_t)(tb * kPN), da + 2 * kk, db + 2 * kk, kk ? 1u : 0u);
+          if (kk < A.ksteps)
+            mma_f16(tbase + (uint32_t)(tb * kPN), da + 2 * kk, db + 2 * kk, kk ? 1u : 0u);
         mma_commit(empty(s));                           // the column tile is free
         mma_commit(tfull(tb));                          // the products are in TMEM
         w.next(A);
@@ -261,18 +258,38 @@ k_sym_prefilter(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
     const int q = warp & 3;                             // TMEM lane quarter of this warp
     const int p = e >> 2;                               // columns [64 p, 64 p + 64)
     const int jlo = A.jlo, jhi = A.jhi;
+    uint32_t *buf = ebuf + e * kPBuf;                   // this warp's entries not yet listed
+    int held = 0;                                       // entries in buf (warp-uniform)
+    int lrb = -1;                                       // row block of buf, off and cap
+    int64_t off = 0, cap = 0;
+    // n entries' slots in the row block's list
+    auto reserve = [&](int n) {
+      int bpos = 0;
+      if (lane == 0) {
+        bpos = atomicAdd(A.ccnt + 4 * lrb + q, n);
+        if ((int64_t)bpos + n > cap) atomicExch(A.overflow, 1);
+      }
+      return (int64_t)__shfl_sync(FULL, bpos, 0);
+    };
+    auto flush = [&]() {
+      if (held == 0) return;
+      __syncwarp();
+      const int64_t pos = reserve(held);
+      for (int i = lane; i < held; i += 32)
+        if (pos + i < cap) A.cand[off + pos + i] = buf[i];
+      __syncwarp();
+      held = 0;
+    };
     ItemWalk w;
     w.start(A, it0);
     unsigned long long npref = 0;
     int k = 0;
     for (int it = it0; it < it1; ++it, ++k, w.next(A)) {
       const int tb = k & 1;
-      uint32_t bad = mbar_wait(tfull(tb), (uint32_t)(k >> 1) & 1u, A.err, 19) ? 0u : 1u;
-      if (*(volatile int *)abort_flag) bad = 1u;
-      if (pf_barrier_or(bad)) {                         // one decision for all epilogue threads
-        *(volatile int *)abort_flag = 1;
-        break;
-      }
+      if (!mbar_wait(tfull(tb), (uint32_t)(k >> 1) & 1u, A.err, 19)) *(volatile int *)abort_flag = 1;
+      // one decision per warp; a warp that leaves stops the issuers through the
+      // flag (or through their own bounded waits for its arrivals)
+      if (__any_sync(FULL, *(volatile int *)abort_flag != 0)) break;
       fence_after();
       uint32_t v0[32], v1[32];
       const uint32_t ta = tbase + ((uint32_t)(q * 32) << 16) + (uint32_t)(tb * kPN + p * 64);
@@ -280,48 +297,46 @@ k_sym_prefilter(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
       tmem_ld32(ta + 32, v1);
       tmem_wait_ld();
       fence_before();
-      mbar_arrive(tempty(tb));                          // the accumulator is free again
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tempty(tb));           // the accumulator is free again
       const int row0w = kPM * w.rb + 32 * q;            // the warp's 32 rows
-      const int row = row0w + lane;
-      // Masks in "gather order": bit 8 q + k stands for column t = 4 k + q of
-      // the 32-column chunk (the order the byte permutes below produce).
-      uint32_t cm[2];
-      int cnt = 0;
+      if (w.rb != lrb) {
+        flush();
+        lrb = w.rb;
+        const bool in = row0w < jhi;                    // blocks past the window have no list
+        off = in ? A.coff[4 * lrb + q] : 0;
+        cap = in ? A.coff[4 * lrb + q + 1] - off : 0;
+      }
+      const int j0 = kPN * w.ct + 64 * p;
+      // The MMA carried the threshold as a bias column (product - lo16): a
+      // candidate's sign bit is clear.  One funnel shift a product moves the
+      // sign into the mask: bit 31 - t stands for column t of the 32.
+      uint32_t s0 = 0, s1 = 0;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t(&v)[32] = h ? v1 : v0;
-        const int j0 = kPN * w.ct + 64 * p + 32 * h;
-        // valid columns: i < j, jlo <= j < jhi (the warp-uniform interior case first)
-        uint32_t valid;
-        if (j0 > row0w + 31 && j0 >= jlo && j0 + 32 <= jhi && row0w + 31 < jhi) {
-          valid = ~0u;
-          npref += 32;
-        } else {
-          const int tl = max(row - j0 + 1, jlo - j0);     // first valid t
-          const int dh = jhi - j0;                        // t < dh
-          uint32_t vt = tl <= 0 ? ~0u : (tl >= 32 ? 0u : (~0u << tl));
-          vt &= dh >= 32 ? ~0u : (dh <= 0 ? 0u : ((1u << dh) - 1u));
+      for (int t = 0; t < 32; ++t) {
+        s0 = __funnelshift_l(v0[t], s0, 1);
+        s1 = __funnelshift_l(v1[t], s1, 1);
+      }
+      uint32_t m0 = ~s0, m1 = ~s1;
+      // valid columns: i < j, jlo <= j < jhi (the warp-uniform interior case first)
+      if (j0 > row0w + 31 && j0 >= jlo && j0 + 64 <= jhi && row0w + 31 < jhi) {
+        npref += 64;
+      } else {
+        const int row = row0w + lane;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int jh = j0 + 32 * h;
+          const int tl = max(row - jh + 1, jlo - jh);   // first valid t
+          const int dh = jhi - jh;                      // t < dh
+          uint32_t vt = tl <= 0 ? ~0u : (tl >= 32 ? 0u : (~0u >> tl));
+          vt &= dh >= 32 ? ~0u : (dh <= 0 ? 0u : ~(~0u >> dh));
           if (row >= jhi) vt = 0u;
           npref += (unsigned)__popc(vt);
-          valid = 0;
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk)                  // t = 4 kk + q -> bit 8 q + kk
-            valid |= ((((vt >> (4 * kk)) & 0xFu) * 0x00204081u) & 0x01010101u) << kk;
+          if (h) m1 &= vt; else m0 &= vt;
         }
-        // The MMA carried the threshold as a bias column (product - lo16): a
-        // candidate's sign bit is clear.  Top bytes of four products per word.
-        uint32_t sg = 0;
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t lo2 = __byte_perm(v[4 * kk], v[4 * kk + 1], 0x0073u);
-          const uint32_t hi2 = __byte_perm(v[4 * kk + 2], v[4 * kk + 3], 0x0073u);
-          const uint32_t g = __byte_perm(lo2, hi2, 0x5410u);
-          sg |= ((g >> 7) & 0x01010101u) << kk;
-        }
-        cm[h] = ~sg & valid;
-        cnt += __popc(cm[h]);
       }
-      // one slot range per warp and item in the 32-row block's list
+      const int cnt = __popc(m0) + __popc(m1);
+      if (!__any_sync(FULL, cnt)) continue;
       int incl = cnt;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
@@ -329,31 +344,38 @@ k_sym_prefilter(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
         if (lane >= d) incl += t;
       }
       const int total = __shfl_sync(FULL, incl, 31);
-      if (total) {
-        const int blk = row0w >> 5;
-        int bpos = 0;
-        if (lane == 0) bpos = atomicAdd(A.ccnt + blk, total);
-        bpos = __shfl_sync(FULL, bpos, 0);
-        const int64_t off = A.coff[blk];
-        const int64_t cap = A.coff[blk + 1] - off;
-        int64_t pos = (int64_t)bpos + incl - cnt;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const uint32_t j0 = (uint32_t)(kPN * w.ct + 64 * p + 32 * h);
-          uint32_t m = cm[h];
-          while (m) {
-            const int bit = __ffs(m) - 1;
-            m &= m - 1;
-            const int t = 4 * (bit & 7) + (bit >> 3);
-            if (pos < cap) A.cand[off + pos] = ((uint32_t)lane << 27) | (j0 + (uint32_t)t);
-            ++pos;
-          }
+      const uint32_t ent = ((uint32_t)lane << 27) | (uint32_t)j0;   // j0 a multiple of 64
+      if (held + total > kPBuf) flush();
+      if (total <= kPBuf) {
+        int at = held + incl - cnt;
+        while (m0) {
+          const int t = __clz(m0);
+          m0 ^= 0x80000000u >> t;
+          buf[at++] = ent | (uint32_t)t;
         }
-        if (lane == 0 && (int64_t)bpos + total > cap) atomicExch(A.overflow, 1);
+        while (m1) {
+          const int t = __clz(m1);
+          m1 ^= 0x80000000u >> t;
+          buf[at++] = ent | (uint32_t)(32 + t);
+        }
+        held += total;
+      } else {                                          // more than the buffer holds: straight out
+        int64_t pos = reserve(total) + incl - cnt;
+        while (m0 | m1) {
+          const int t = m0 ? __clz(m0) : 32 + __clz(m1);
+          if (m0) m0 ^= 0x80000000u >> t;
+          else m1 ^= 0x80000000u >> (t - 32);
+          if (pos < cap) A.cand[off + pos] = ent | (uint32_t)t;
+          ++pos;
+        }
       }
     }
-    npref = __reduce_add_sync(FULL, (unsigned)npref);
-    if (lane == 0 && npref && A.stats) atomicAdd(A.stats, npref);
+    if (lrb >= 0) flush();
+    // lanes hold different counts only in the edge tiles; 64-bit sum in halves
+    const unsigned lo = __reduce_add_sync(FULL, (unsigned)(npref & 0xFFFFFu));
+    const unsigned hi = __reduce_add_sync(FULL, (unsigned)(npref >> 20));
+    if (lane == 0 && (lo | hi) && A.stats)
+      atomicAdd(A.stats, ((unsigned long long)hi << 20) + lo);
   }
   __syncthreads();
   fence_after();
@@ -362,23 +384,23 @@ k_sym_prefilter(const __grid_constant__ CUtensorMap tmapA, const __grid_constant
 }
 
 size_t pf_smem() {
-  return 1024 + 2 * (size_t)kABytes + (size_t)kPStages * kBBytes + (4 + 2 * kPStages + 5) * 8 +
-         16 + 16;
+  return 1024 + 2 * (size_t)kABytes + (size_t)kPStages * kBBytes +
+         (size_t)kPEpiWarps * kPBuf * 4 + (4 + 2 * kPStages + 5) * 8 + 16 + 16;
 }
 
 // unit16 rows (Kp halves) -> two [n][64] copies, zero padded, with the
-// threshold as a bias column in the last half (S < 64 leaves it free): the row
+// threshold as a bias column in half kbias (>= S): the row
 // side (A) holds 1.0 there and the column side (B) -lo16', lo16' the largest
 // FP16 value not above lo16, so each product comes out of the MMA as
 // U_i . U_j - lo16'.
-__global__ void k_pad_unit16(const uint16_t *__restrict__ u, int Kp, int64_t n, float lo16,
-                             uint16_t *__restrict__ outA, uint16_t *__restrict__ outB) {
+__global__ void k_pad_unit16(const uint16_t *__restrict__ u, int Kp, int kbias, int64_t n,
+                             float lo16, uint16_t *__restrict__ outA, uint16_t *__restrict__ outB) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;   // one half each
   if (i >= n * kPK) return;
   const int64_t r = i / kPK;
   const int k = (int)(i - r * kPK);
   uint16_t a = k < Kp ? u[r * Kp + k] : (uint16_t)0, b = a;
-  if (k == kPK - 1) {
+  if (k == kbias) {
     a = __half_as_ushort(__float2half_rn(1.0f));
     b = __half_as_ushort(__hneg(__float2half_rd(lo16)));
   }
@@ -464,11 +486,15 @@ void launch_tc5_items(int64_t cb, int64_t ce, int32_t *item0, cudaStream_t s) {
   k_tc5_items<<<1, 1024, 0, s>>>(RB, NT, (int)(cb / kPN), item0);
 }
 
+// The S products and the bias column (the last half of the last K step) fit
+// these steps; the zero halves after them are not multiplied.
+static int pf_ksteps(int S) { return S / 16 + 1; }
+
 void launch_pad_unit16(const GraphArgs &g, float lo16, uint16_t *u16p, cudaStream_t s) {
   const int64_t nh = g.n * kPK;
   if (nh > 0)
-    k_pad_unit16<<<(unsigned)((nh + 255) / 256), 256, 0, s>>>(g.unit16, g.Kp, g.n, lo16, u16p,
-                                                              u16p + nh);
+    k_pad_unit16<<<(unsigned)((nh + 255) / 256), 256, 0, s>>>(
+        g.unit16, g.Kp, 16 * pf_ksteps(g.S) - 1, g.n, lo16, u16p, u16p + nh);
 }
 
 int launch_sym_prefilter(const GraphArgs &g, const uint16_t *u16p, int64_t cb, int64_t ce,
@@ -507,6 +533,7 @@ int launch_sym_prefilter(const GraphArgs &g, const uint16_t *u16p, int64_t cb, i
   A.jhi = (int)ce;
   A.ct_lo = (int)(cb / kPN);
   A.item0 = item0;
+  A.ksteps = pf_ksteps(g.S);
   A.RB = RB;
   A.NT = NT;
   A.items = items;
