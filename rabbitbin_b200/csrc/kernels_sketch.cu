@@ -95,54 +95,104 @@ __device__ __forceinline__ uint32_t spread16(uint32_t x) {
   return x;
 }
 
-// Warp per contig: histogram of canonical k-mers (k <= 4) and base counts over
-// the packed sequence, then the GC-normalised weights of build_pmh_winners
+// Per contig: histogram of canonical k-mers (k <= 4) and base counts over the
+// packed sequence, then the GC-normalised weights of build_pmh_winners
 // (src/rabbitbin.cpp:1459-1516) and the ascending element list (rank, 1/w).
-// A lane takes one packed word (16 bases) per step, the 3 bases before it come
-// from the previous lane; base counts use popcounts over the 2-bit fields and a
-// shared table maps each k-mer code to its canonical code.
-template <bool GC2>                    // GC-norm mode 2 (dinucleotide model)
-__global__ void k_count(SketchArgs a) {
-  extern __shared__ uint32_t sh_hist[];
+// W warps share a contig (W = 1, or all kCountWarps of the CTA).  A lane takes
+// one packed word (16 bases) per step, the 3 bases before it come from the
+// previous lane; base counts use popcounts over the 2-bit fields.  For k = 4 a
+// word whose 16 windows are all valid adds 8 5-mers ending at its odd bases,
+// each of which stands for two 4-mers (its first and its last four bases):
+// half the shared-memory atomics; the 1,024 5-mer counts are folded into the
+// 4-mer histogram once per contig.
+constexpr int kCountWarps = 8;
+constexpr int kH5 = 1024;               // 5-mer counters of a group
+
+// A group's (the W warps of a contig) shared memory.
+struct CountGroup {
+  uint32_t h5[kH5];
+  uint32_t hist[256];
+  double p[4];                          // base frequencies (mode 2: with pseudocounts)
+  double pc[16];                        // mode 2: P(next | prev)
+  uint32_t bc[4], dn[16];
+  uint32_t tot, pos;
+  unsigned next;
+  uint32_t pad;
+};
+
+template <bool GC2, int W>              // GC2: GC-norm mode 2 (dinucleotide model)
+__global__ void __launch_bounds__(kCountWarps * 32) k_count(SketchArgs a) {
+  extern __shared__ __align__(16) unsigned char sh_count[];
+  __shared__ uint8_t code_of[kMaxElems];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int nb = 1 << (2 * a.k);
-  const int k = a.k;
-  uint32_t *hist = sh_hist + wib * 256;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  // Each warp takes its next contig from a.work (a counter zeroed before the
-  // launch) when the caller gives one, else every warps-th contig: contig
-  // lengths vary by an order of magnitude, and the counter keeps every warp
-  // busy until the last contigs.
-  auto next_contig = [&](int64_t cur) -> int64_t {
-    if (a.work == nullptr) return cur + warps;
-    unsigned t = 0;
-    if (lane == 0) t = atomicAdd(a.work, 1u);
-    return (int64_t)__shfl_sync(0xffffffffu, t, 0);
+  constexpr int kG = kCountWarps / W;   // groups per CTA
+  constexpr int GT = 32 * W;            // threads of a group
+  const int gi = W == 1 ? wib : 0;
+  const int gt = W == 1 ? lane : (int)threadIdx.x;
+  const int wig = W == 1 ? 0 : wib;     // warp within the group
+  CountGroup &G = reinterpret_cast<CountGroup *>(sh_count)[gi];
+  auto gsync = [] {
+    if constexpr (W == 1) __syncwarp();
+    else __syncthreads();
   };
-  const int64_t c_first = a.work ? next_contig(0)
-                                 : (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
-  for (int64_t c = c_first; c < a.n; c = next_contig(c)) {
-  for (int v = lane; v < 256; v += 32) hist[v] = 0;
-  __syncwarp();
-  const int64_t s = a.offsets[c], e = a.offsets[c + 1];
+  const int k = a.k;
+  const int nb = 1 << (2 * k);
   const uint32_t kmask = (uint32_t)nb - 1u;
+  for (int v = threadIdx.x; v < nb; v += blockDim.x) {
+    const int e = a.rank_of_code[v];
+    if (e >= 0) code_of[e] = (uint8_t)v;
+  }
+  for (int v = gt; v < kH5; v += GT) G.h5[v] = 0;
+  __syncthreads();
+  // A group takes its next contig from a.work (a counter zeroed before the
+  // launch) when the caller gives one, else every groups-th contig: contig
+  // lengths vary by an order of magnitude, and the counter keeps every group
+  // busy until the last contigs.
+  const int64_t groups = (int64_t)gridDim.x * kG;
+  auto next_contig = [&](int64_t cur, bool first) -> int64_t {
+    if (a.work == nullptr) return first ? (int64_t)blockIdx.x * kG + gi : cur + groups;
+    if constexpr (W == 1) {
+      unsigned t = 0;
+      if (lane == 0) t = atomicAdd(a.work, 1u);
+      return (int64_t)__shfl_sync(0xffffffffu, t, 0);
+    } else {
+      if (threadIdx.x == 0) G.next = atomicAdd(a.work, 1u);
+      __syncthreads();
+      return (int64_t)G.next;
+    }
+  };
+  for (int64_t c = next_contig(0, true); c < a.n; c = next_contig(c, false)) {
+  for (int v = gt; v < 256; v += GT) G.hist[v] = 0;
+  if (gt < 4) G.bc[gt] = 0;
+  if (gt < 16) G.dn[gt] = 0;
+  if (gt == 0) { G.tot = 0; G.pos = 0; }
+  const int64_t s = a.offsets[c], e = a.offsets[c + 1];
   uint32_t bc0 = 0, bc1 = 0, bc2 = 0, bc3 = 0;
   uint32_t dn[GC2 ? 16 : 1] = {};      // mode 2: dinucleotides (prev, next) = dn[4 prev + next]
+  gsync();
   if (e - s >= k) {
     const int64_t w0 = s >> 4, w1 = (e + 15) >> 4;
-    uint32_t carry_word = 0, carry_bad = 0xFFFFu;     // word before w0: all invalid
-    for (int64_t base = w0; base < w1; base += 32) {
-      const int64_t wi = base + lane;
-      uint32_t cur = 0, bad = 0xFFFFu;
-      if (wi < w1) {
+    // word wi of the contig and the word before the lane group's first one
+    auto fetch = [&](int64_t wi, uint32_t &cur, uint32_t &bad) {
+      cur = 0;
+      bad = 0xFFFFu;
+      if (wi >= w0 && wi < w1) {
         cur = __ldg(a.packed + wi);
         bad = invalid16(a.nmask, wi, s, e);
       }
+    };
+    uint32_t ncur, nbad, npre = 0, nprebad = 0xFFFFu;   // the next step's words
+    int64_t base = w0 + 32 * wig;
+    fetch(base + lane, ncur, nbad);
+    if (lane == 0) fetch(base - 1, npre, nprebad);
+    for (; base < w1; base += 32 * W) {
+      const int64_t wi = base + lane;
+      const uint32_t cur = ncur, bad = nbad;
       uint32_t prev = __shfl_up_sync(0xffffffffu, cur, 1);
       uint32_t prevbad = __shfl_up_sync(0xffffffffu, bad, 1);
-      if (lane == 0) { prev = carry_word; prevbad = carry_bad; }
-      carry_word = __shfl_sync(0xffffffffu, cur, 31);
-      carry_bad = __shfl_sync(0xffffffffu, bad, 31);
+      if (lane == 0) { prev = npre; prevbad = nprebad; }
+      fetch(wi + 32 * W, ncur, nbad);
+      if (lane == 0) fetch(wi + 32 * W - 1, npre, nprebad);
       if (wi < w1) {
         // base counts of the valid bases (base t occupies bits 31-2t .. 30-2t)
         const uint32_t vs = spread16(~bad & 0xFFFFu);
@@ -172,91 +222,104 @@ __global__ void k_count(SketchArgs a) {
         uint32_t kv = ~any & 0xFFFFu;                   // bit 15-t: k-mer ending at t
         const uint64_t win = ((uint64_t)prev << 32) | cur;
         if (kv == 0xFFFFu && k == 4) {
-          // the 16 codes are the bytes of the window shifted by 0, 2, 4 and 6 bits
-          const uint32_t sw[4] = {cur, __funnelshift_r(cur, prev, 2),
-                                  __funnelshift_r(cur, prev, 4), __funnelshift_r(cur, prev, 6)};
+          // bases -3 .. 15 are valid: the 5-mers ending at t = 1, 3, .., 15
 #pragma unroll
-          for (int x = 0; x < 4; ++x)
-#pragma unroll
-            for (int y = 0; y < 4; ++y) atomicAdd(&hist[__byte_perm(sw[x], 0u, 0x4440u + y)], 1u);
+          for (int bp = 14; bp >= 0; bp -= 2)
+            atomicAdd(&G.h5[__funnelshift_r(cur, prev, 2 * bp) & (kH5 - 1)], 1u);
         } else if (kv == 0xFFFFu) {
 #pragma unroll
           for (int bp = 15; bp >= 0; --bp)
-            atomicAdd(&hist[(uint32_t)(win >> (2 * bp)) & kmask], 1u);
+            atomicAdd(&G.hist[(uint32_t)(win >> (2 * bp)) & kmask], 1u);
         } else {
           while (kv) {
             const int bp = __ffs(kv) - 1;               // = 15 - t
             kv &= kv - 1;
-            atomicAdd(&hist[(uint32_t)(win >> (2 * bp)) & kmask], 1u);
+            atomicAdd(&G.hist[(uint32_t)(win >> (2 * bp)) & kmask], 1u);
           }
         }
       }
     }
   }
-  __syncwarp();
-  // fold each reverse-complement code onto its canonical (the smaller) code
-  for (int v = lane; v < nb; v += 32) {
-    uint32_t rev = 0, x = (uint32_t)v;
-    for (int q = 0; q < k; ++q) { rev = (rev << 2) | (3u - (x & 3u)); x >>= 2; }
-    if ((uint32_t)v < rev) {
-      hist[v] += hist[rev];
-      hist[rev] = 0;
-    }
-  }
-  __syncwarp();
-  // totals
-  uint32_t tot = 0;
-  for (int v = lane; v < nb; v += 32) tot += hist[v];
-  tot = __reduce_add_sync(0xffffffffu, tot);
+  // base counts of the group
   bc0 = __reduce_add_sync(0xffffffffu, bc0);
   bc1 = __reduce_add_sync(0xffffffffu, bc1);
   bc2 = __reduce_add_sync(0xffffffffu, bc2);
   bc3 = __reduce_add_sync(0xffffffffu, bc3);
-  int pos = 0;
-  double *ewinv = a.elem_winv + c * a.n_elems;
-  const double inf = __longlong_as_double(0x7FF0000000000000LL);
-  const uint64_t vb = (uint64_t)bc0 + bc1 + bc2 + bc3;
-  double p[4];
-  p[0] = vb > 0 ? (double)bc0 / (double)vb : 0.25;
-  p[1] = vb > 0 ? (double)bc1 / (double)vb : 0.25;
-  p[2] = vb > 0 ? (double)bc2 / (double)vb : 0.25;
-  p[3] = vb > 0 ? (double)bc3 / (double)vb : 0.25;
-  const double inv = tot > 0 ? 1.0 / (double)tot : 0.0;
-  // mode 2 (src/rabbitbin.cpp:1517-1554): base frequencies with pseudocount 1,
-  // P(next | prev) with Laplace pseudocount 1
-  double pm[4], pc[GC2 ? 16 : 1];
+  if (lane < 4) atomicAdd(&G.bc[lane], lane == 0 ? bc0 : lane == 1 ? bc1 : lane == 2 ? bc2 : bc3);
   if constexpr (GC2) {
 #pragma unroll
-    for (int x = 0; x < 16; ++x) dn[x] = __reduce_add_sync(0xffffffffu, dn[x]);
-    const uint32_t bcs[4] = {bc0, bc1, bc2, bc3};
-#pragma unroll
-    for (int b = 0; b < 4; ++b)
-      pm[b] = vb > 0 ? ((double)bcs[b] + 1.0) / ((double)vb + 4.0) : 0.25;
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      double rs = 4.0;
-#pragma unroll
-      for (int y = 0; y < 4; ++y) rs += (double)dn[4 * x + y];
-#pragma unroll
-      for (int y = 0; y < 4; ++y) pc[4 * x + y] = ((double)dn[4 * x + y] + 1.0) / rs;
+    for (int x = 0; x < 16; ++x) {
+      const uint32_t t = __reduce_add_sync(0xffffffffu, dn[x]);
+      if (lane == 0) atomicAdd(&G.dn[x], t);
     }
   }
-  for (int v0 = 0; v0 < nb; v0 += 32) {
-    const int v = v0 + lane;
+  gsync();
+  if (k == 4) {
+    // 5-mer (first four = x, or last four = x) -> 4-mer x
+    for (int x = gt; x < 256; x += GT) {
+      const uint4 f = *reinterpret_cast<const uint4 *>(&G.h5[4 * x]);
+      G.hist[x] += f.x + f.y + f.z + f.w +
+                   G.h5[x] + G.h5[256 + x] + G.h5[512 + x] + G.h5[768 + x];
+    }
+    gsync();
+    for (int v = gt; v < kH5 / 4; v += GT)
+      reinterpret_cast<uint4 *>(G.h5)[v] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  // fold each reverse-complement code onto its canonical (the smaller) code
+  uint32_t tot = 0;
+  for (int v = gt; v < nb; v += GT) {
+    uint32_t rev = 0, x = (uint32_t)v;
+    for (int q = 0; q < k; ++q) { rev = (rev << 2) | (3u - (x & 3u)); x >>= 2; }
+    if ((uint32_t)v > rev) continue;
+    uint32_t cnt = G.hist[v];
+    if ((uint32_t)v < rev) {
+      cnt += G.hist[rev];
+      G.hist[v] = cnt;
+    }
+    tot += cnt;
+  }
+  tot = __reduce_add_sync(0xffffffffu, tot);
+  if (lane == 0) atomicAdd(&G.tot, tot);
+  gsync();
+  tot = G.tot;
+  bc0 = G.bc[0]; bc1 = G.bc[1]; bc2 = G.bc[2]; bc3 = G.bc[3];
+  const uint64_t vb = (uint64_t)bc0 + bc1 + bc2 + bc3;
+  if constexpr (GC2) {
+    // mode 2 (src/rabbitbin.cpp:1517-1554): base frequencies with pseudocount 1,
+    // P(next | prev) with Laplace pseudocount 1
+    if (gt < 4) G.p[gt] = vb > 0 ? ((double)G.bc[gt] + 1.0) / ((double)vb + 4.0) : 0.25;
+    if (gt < 16) {
+      const int x = gt >> 2;
+      double rs = 4.0;
+#pragma unroll
+      for (int y = 0; y < 4; ++y) rs += (double)G.dn[4 * x + y];
+      G.pc[gt] = ((double)G.dn[gt] + 1.0) / rs;
+    }
+  } else {
+    if (gt < 4) G.p[gt] = vb > 0 ? (double)G.bc[gt] / (double)vb : 0.25;
+  }
+  gsync();
+  double *ewinv = a.elem_winv + c * a.n_elems;
+  const double inf = __longlong_as_double(0x7FF0000000000000LL);
+  const double inv = tot > 0 ? 1.0 / (double)tot : 0.0;
+  int pos = 0;
+  for (int el = gt; el < a.n_elems; el += GT) {
+    const uint32_t v = code_of[el];
     double w = 0.0;
-    if (v < nb && tot > 0) {
-      const uint32_t cnt = hist[v];
+    if (tot > 0) {
+      const uint32_t cnt = G.hist[v];
       if (cnt) {
         if (a.gc_norm == 0) {
           w = (double)cnt * inv;
         } else if constexpr (GC2) {
           // bases[i] = (v >> 2i) & 3; forward and reverse-complement chains
-          uint32_t bs[4];
-          for (int q = 0; q < k; ++q) bs[q] = ((uint32_t)v >> (2 * q)) & 3u;
-          double pf = pm[bs[0]];
-          for (int q = 1; q < k; ++q) pf = __dmul_rn(pf, pc[4 * bs[q - 1] + bs[q]]);
-          double pr = pm[3u - bs[k - 1]];
-          for (int q = 1; q < k; ++q) pr = __dmul_rn(pr, pc[4 * (3u - bs[k - q]) + (3u - bs[k - 1 - q])]);
+          double pf = G.p[v & 3u];
+          for (int q = 1; q < k; ++q)
+            pf = __dmul_rn(pf, G.pc[4 * ((v >> (2 * q - 2)) & 3u) + ((v >> (2 * q)) & 3u)]);
+          double pr = G.p[3u - ((v >> (2 * k - 2)) & 3u)];
+          for (int q = 1; q < k; ++q)
+            pr = __dmul_rn(pr, G.pc[4 * (3u - ((v >> (2 * (k - q))) & 3u)) +
+                                    (3u - ((v >> (2 * (k - 1 - q))) & 3u))]);
           const double obs = (double)cnt * inv;
           const double ex = __dadd_rn(pf, pr);
           if (ex > 1e-16) {
@@ -265,11 +328,11 @@ __global__ void k_count(SketchArgs a) {
           }
         } else {
           double pf = 1.0, pr = 1.0;
-          uint32_t code = (uint32_t)v;
+          uint32_t code = v;
           for (int q = 0; q < k; ++q) {
             const uint32_t b = code & 3u;
-            pf = __dmul_rn(pf, p[b]);
-            pr = __dmul_rn(pr, p[3u - b]);
+            pf = __dmul_rn(pf, G.p[b]);
+            pr = __dmul_rn(pr, G.p[3u - b]);
             code >>= 2;
           }
           const double obs = (double)cnt * inv;
@@ -282,12 +345,19 @@ __global__ void k_count(SketchArgs a) {
       }
     }
     const bool take = w > 0.0;
-    pos += __popc(__ballot_sync(0xffffffffu, take));
-    const int e = v < nb ? a.rank_of_code[v] : -1;
-    if (e >= 0) ewinv[e] = take ? 1.0 / w : inf;
+    pos += take;
+    ewinv[el] = take ? 1.0 / w : inf;
   }
-  if (lane == 0) a.elem_cnt[c] = pos;
-  __syncwarp();                        // the next contig clears the histogram
+  pos = (int)__reduce_add_sync(0xffffffffu, (unsigned)pos);
+  if constexpr (W == 1) {
+    if (lane == 0) a.elem_cnt[c] = pos;
+    __syncwarp();                      // the next contig clears the histogram
+  } else {
+    if (lane == 0) atomicAdd(&G.pos, (uint32_t)pos);
+    __syncthreads();
+    if (threadIdx.x == 0) a.elem_cnt[c] = (int32_t)G.pos;
+    __syncthreads();
+  }
   }
 }
 
@@ -442,8 +512,12 @@ __global__ void __launch_bounds__(kMThreads, 3) k_minreduce(SketchArgs a) {
   const double2 *ord = reinterpret_cast<const double2 *>(a.order);
   const double2 *ut = reinterpret_cast<const double2 *>(a.UT);
   const int half = E >> 1;
-  for (int rb = 0; rb < mpad; rb += kMChunk) {
-    const int rn = (m - rb < kMChunk) ? m - rb : kMChunk;
+  // this CTA's registers (gridDim.y ranges of whole 16-column groups)
+  const int groups = mpad >> 4;
+  const int r_lo = 16 * (int)((int64_t)blockIdx.y * groups / gridDim.y);
+  const int r_hi = 16 * (int)((int64_t)(blockIdx.y + 1) * groups / gridDim.y);
+  for (int rb = r_lo; rb < r_hi; rb += kMChunk) {
+    const int rn = min(min(m, r_hi) - rb, kMChunk);
     MinStage st;
     if (warp < rn) min_fetch(st, ord, ut, rb + warp, E, lane);
     for (int rl = warp; rl < rn; rl += kMWarps) {
@@ -480,7 +554,7 @@ __global__ void __launch_bounds__(kMThreads, 3) k_minreduce(SketchArgs a) {
     }
     __syncthreads();
     // code words: columns [rb, rend) of the nc rows; padding columns A = 0, B = 0xFF
-    const int rend = (rb + kMChunk < mpad) ? rb + kMChunk : mpad;
+    const int rend = min(rb + kMChunk, r_hi);
     const int q4 = (rend - rb) >> 2;
     for (int i = threadIdx.x; i < nc * q4; i += kMThreads) {
       const int cc = i / q4, rl = (i - cc * q4) * 4, r4 = rb + rl;
@@ -555,22 +629,40 @@ void launch_codes_b(const uint8_t *codesA, uint8_t *codesB, int64_t bytes, cudaS
                                                           n16);
 }
 
+namespace {
+template <bool GC2, int W>
+void launch_count_w(const SketchArgs &a, int64_t grid, cudaStream_t s) {
+  const size_t smem = (size_t)(kCountWarps / W) * sizeof(CountGroup);
+  smem_cap_max((const void *)k_count<GC2, W>);
+  k_count<GC2, W><<<(unsigned)grid, kCountWarps * 32, smem, s>>>(a);
+}
+}  // namespace
+
+// Contigs up to which a CTA shares each contig (W = 8).  With a warp per contig
+// the longest contig (80 kb) alone takes about 80 us; sharing cuts that to an
+// eighth but pays the per-contig fold and weights with CTA barriers.  Measured
+// (kernel time, warp / CTA per contig): 97 contigs 81 / 17 us, 2,000 142 / 38,
+// 8,000 178 / 98, 16,000 226 / 180, 50,000 450 / 523.
+constexpr int64_t kCountShare = 20000;
+
 void launch_count(const SketchArgs &a, cudaStream_t s) {
   if (a.n == 0) return;
-  const int warps = 8;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // with the contig counter, as many warps as fit (five blocks of 48-register
-  // threads per SM); without it, about eight contigs per warp to even out the
-  // contig lengths
-  const int64_t blocks = (a.n + warps - 1) / warps;
+  const bool share = a.n <= kCountShare;
+  // with the contig counter, as many warps as fit (five blocks per SM);
+  // without it, about eight contigs per group to even out the contig lengths
+  const int64_t blocks = share ? a.n : (a.n + kCountWarps - 1) / kCountWarps;
   const int64_t grid =
       std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)sms * (a.work ? 5 : 4)));
-  if (a.gc_norm == 2)
-    k_count<true><<<(unsigned)grid, warps * 32, warps * 256 * sizeof(uint32_t), s>>>(a);
-  else
-    k_count<false><<<(unsigned)grid, warps * 32, warps * 256 * sizeof(uint32_t), s>>>(a);
+  if (a.gc_norm == 2) {
+    if (share) launch_count_w<true, kCountWarps>(a, grid, s);
+    else launch_count_w<true, 1>(a, grid, s);
+  } else {
+    if (share) launch_count_w<false, kCountWarps>(a, grid, s);
+    else launch_count_w<false, 1>(a, grid, s);
+  }
 }
 
 void smem_cap_max(const void *func) {
@@ -588,12 +680,39 @@ void smem_cap_max(const void *func) {
                        optin - (int)fa.sharedSizeBytes);
 }
 
+// Ranges the registers are split into, one per blockIdx.y.  A CTA costs its
+// set-up (the heavy sets, about as long as three registers of a warp) plus
+// kMWarps registers at a time; few contigs leave SMs idle without a split,
+// many fill them alone.  The smallest cost over the waves of three CTAs per SM
+// (97 contigs: 163 -> 24 us, 2,000: 170 -> 61 us, 16,000: 330 us; from 25,000
+// contigs on unsplit, 50,000: 0.82 ms).
+static int minreduce_split(int64_t gx, int mpad, int sms) {
+  const int groups = mpad / 16;
+  const int64_t slots = 3 * (int64_t)sms;
+  int best = 1;
+  int64_t best_cost = INT64_MAX;
+  for (int y = 1; y <= groups; ++y) {
+    const int64_t waves = (gx * y + slots - 1) / slots;
+    const int64_t regs = 16 * ((groups + y - 1) / y);
+    const int64_t cost = waves * (3 * kMWarps + regs);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = y;
+    }
+  }
+  return best;
+}
+
 void launch_minreduce(const SketchArgs &a, cudaStream_t s) {
   if (a.n == 0) return;
   const size_t smem = minreduce_smem(a.n_elems);
   smem_cap_max((const void *)k_minreduce);
-  const int64_t grid = (a.n + kMC - 1) / kMC;
-  k_minreduce<<<(unsigned)grid, kMThreads, smem, s>>>(a);
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t gx = (a.n + kMC - 1) / kMC;
+  const dim3 grid((unsigned)gx, (unsigned)minreduce_split(gx, a.mpad, sms));
+  k_minreduce<<<grid, kMThreads, smem, s>>>(a);
 }
 
 namespace {
