@@ -193,16 +193,34 @@ __device__ __forceinline__ uint32_t match4(uint32_t a, uint32_t b) {
   return __popc(~t & 0x80808080u);
 }
 
+// Match count of code rows x (A side) and y (B side), mpad bytes each, by the
+// 8 lanes of a pair: 16-byte loads, a row's 128 bytes per step.
+constexpr int kPairLanes = 8;
+__device__ __forceinline__ uint32_t pair_count(const uint8_t *x, const uint8_t *y, int mpad) {
+  const int sub = threadIdx.x & (kPairLanes - 1);
+  const uint4 *a = reinterpret_cast<const uint4 *>(x), *b = reinterpret_cast<const uint4 *>(y);
+  uint32_t c = 0;
+#pragma unroll 4
+  for (int w = sub; w < mpad / 16; w += kPairLanes) {
+    const uint4 p = __ldg(a + w), q = __ldg(b + w);
+    c += match4(p.x, q.x) + match4(p.y, q.y) + match4(p.z, q.z) + match4(p.w, q.w);
+  }
+#pragma unroll
+  for (int d = kPairLanes / 2; d; d >>= 1) c += __shfl_xor_sync(0xffffffffu, c, d);
+  return c;
+}
+
+// The b0 sample's match counts.  30,000 pairs of random rows: a few lanes a
+// pair keep enough row loads in flight to hide the L2 latency (m = 500: 34 us
+// with a thread a pair, 6 us now).
 __global__ void k_pair_counts(const uint8_t *__restrict__ A, const uint8_t *__restrict__ B,
                               int mpad, const int64_t *__restrict__ pairs, int np,
                               uint32_t *__restrict__ out) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= np) return;
-  const uint32_t *a = (const uint32_t *)(A + pairs[2 * p] * (int64_t)mpad);
-  const uint32_t *b = (const uint32_t *)(B + pairs[2 * p + 1] * (int64_t)mpad);
-  uint32_t c = 0;
-  for (int w = 0; w < mpad / 4; ++w) c += match4(__ldg(a + w), __ldg(b + w));
-  out[p] = c;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int p = min(t / kPairLanes, np - 1);            // every lane takes part in the sum
+  const uint32_t c = pair_count(A + pairs[2 * p] * (int64_t)mpad,
+                                B + pairs[2 * p + 1] * (int64_t)mpad, mpad);
+  if (t / kPairLanes < np && (t & (kPairLanes - 1)) == 0) out[p] = c;
 }
 
 // b0 of every assembly of a batch (estimate_pmh_baseline,
@@ -213,15 +231,13 @@ __global__ void k_pair_counts(const uint8_t *__restrict__ A, const uint8_t *__re
 __global__ void k_pair_counts_batch(const BatchAsm *B, const int64_t *pair0s, int nb,
                                     int64_t p_begin, int64_t npairs,
                                     const int32_t *__restrict__ pairs, uint32_t *__restrict__ out) {
-  const int64_t p = p_begin + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= npairs) return;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t p = min(p_begin + t / kPairLanes, npairs - 1);
   const int a = find_asm(pair0s, nb, p);
   const GraphArgs &g = B[a].g;
-  const uint32_t *x = (const uint32_t *)(g.codesA + (int64_t)pairs[2 * p] * g.mpad);
-  const uint32_t *y = (const uint32_t *)(g.codesB + (int64_t)pairs[2 * p + 1] * g.mpad);
-  uint32_t c = 0;
-  for (int w = 0; w < g.mpad / 4; ++w) c += match4(__ldg(x + w), __ldg(y + w));
-  out[p] = c;
+  const uint32_t c = pair_count(g.codesA + (int64_t)pairs[2 * p] * g.mpad,
+                                g.codesB + (int64_t)pairs[2 * p + 1] * g.mpad, g.mpad);
+  if (p_begin + t / kPairLanes < npairs && (t & (kPairLanes - 1)) == 0) out[p] = c;
 }
 
 // b0 = the count at index np/2 of the sorted sample counts (a histogram of
@@ -236,14 +252,28 @@ __device__ __forceinline__ void b0_body(const uint32_t *__restrict__ counts, int
     for (int c = threadIdx.x; c <= m; c += blockDim.x) hist[c] = 0;
     __syncthreads();
     for (int q = threadIdx.x; q < np; q += blockDim.x) atomicAdd(&hist[counts[q]], 1);
+    if (threadIdx.x == 0) med = m;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      int cum = 0, c = 0;
-      for (; c < m; ++c) {
-        cum += hist[c];
-        if (cum > np / 2) break;
+    // the first count whose cumulative total passes np / 2: one warp, each
+    // lane a run of counts (one thread walking m counts took 40 of k_b0's 62 us)
+    if (threadIdx.x < 32) {
+      const int per = (m + 31) / 32, lo = min(m, (int)threadIdx.x * per), hi = min(m, lo + per);
+      int sum = 0;
+      for (int c = lo; c < hi; ++c) sum += hist[c];
+      int incl = sum;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, d);
+        if ((int)threadIdx.x >= d) incl += t;
       }
-      med = c;
+      int cum = incl - sum;
+      if (cum <= np / 2 && incl > np / 2) {            // one lane at most
+        int c = lo;
+        for (; c < hi; ++c) {
+          cum += hist[c];
+          if (cum > np / 2) break;
+        }
+        med = c;
+      }
     }
     __syncthreads();
   }
@@ -616,14 +646,15 @@ void launch_colnorm(const GraphArgs &g, double *acc, cudaStream_t s) {
 
 void launch_b0(const uint32_t *counts, int np, int m, float *b0_out, uint32_t *sv_out,
                cudaStream_t s) {
-  k_b0<<<1, 256, (size_t)(m + 1) * sizeof(int), s>>>(counts, np, m, b0_out, sv_out);
+  k_b0<<<1, 1024, (size_t)(m + 1) * sizeof(int), s>>>(counts, np, m, b0_out, sv_out);
 }
 
 void launch_pair_counts(const uint8_t *A, const uint8_t *B, int mpad, int m,
                         const int64_t *pairs, int np, uint32_t *out, cudaStream_t s) {
   (void)m;
   if (np == 0) return;
-  k_pair_counts<<<(np + 127) / 128, 128, 0, s>>>(A, B, mpad, pairs, np, out);
+  const int per = 128 / kPairLanes;
+  k_pair_counts<<<(np + per - 1) / per, 128, 0, s>>>(A, B, mpad, pairs, np, out);
 }
 
 void launch_sort_rows(const EmitArgs &e, cudaStream_t s) {
@@ -679,9 +710,9 @@ void launch_b0_batch_range(const BatchAsm *B, const int64_t *pair0s, int nb, int
                            int b_begin, int b_end, cudaStream_t s) {
   if (b_end <= b_begin) return;
   if (p_end > p_begin)
-    k_pair_counts_batch<<<(unsigned)((p_end - p_begin + 127) / 128), 128, 0, s>>>(
+    k_pair_counts_batch<<<(unsigned)(((p_end - p_begin) * kPairLanes + 127) / 128), 128, 0, s>>>(
         B, pair0s, nb, p_begin, p_end, pairs, counts);
-  k_b0_batch<<<(unsigned)(b_end - b_begin), 256, (size_t)(max_m + 1) * sizeof(int), s>>>(
+  k_b0_batch<<<(unsigned)(b_end - b_begin), 1024, (size_t)(max_m + 1) * sizeof(int), s>>>(
       B + b_begin, counts);
 }
 

@@ -8,6 +8,7 @@
 // (cuBLASLt, a plain library GEMM).  A warp per row then scans its counts and
 // produces what the dense all-pairs kernel produces: the per-row top-K keys
 // above the admission floor, the row maxima and the compared-pair count.
+#include <algorithm>
 #include <cstdint>
 
 #include "rbg_internal.h"
@@ -51,43 +52,48 @@ __global__ void k_code_presence(const uint8_t *__restrict__ codesA, int64_t n, i
     if (sp[i]) atomicOr(&pres[(int64_t)c0 * 8 + i], sp[i]);
 }
 
-// One block: koff[r] = one-hot columns before register r (koff[m] = K), and
+// koff[r] = one-hot columns before register r (koff[m] = K), and
 // map[r][code] = koff[r] + rank of code among the column's codes (-1 absent).
-__global__ void k_onehot_map(const uint32_t *__restrict__ pres, int m, int32_t *__restrict__ map,
-                             int32_t *__restrict__ koff) {
-  __shared__ int32_t part[1024];
-  const int t = threadIdx.x;
-  const int per = (m + 1023) / 1024;
-  const int a = t * per, b = (a + per < m) ? a + per : m;
+// Latency-bound: a block takes kMapRegs registers (a thread one code of each)
+// and counts the columns before its first one itself, rather than one block
+// walking the m x 256 map (m = 500: 40 us with one block, 7 us now).
+constexpr int kMapRegs = 8;
+__global__ void __launch_bounds__(256) k_onehot_map(const uint32_t *__restrict__ pres, int m,
+                                                    int32_t *__restrict__ map,
+                                                    int32_t *__restrict__ koff) {
+  __shared__ int32_t part[8];
+  __shared__ int32_t cnt[kMapRegs];
+  __shared__ uint32_t bits[kMapRegs * 8];
+  const int t = threadIdx.x, lane = t & 31, wib = t >> 5;
+  const int ra = blockIdx.x * kMapRegs, rb = min(ra + kMapRegs, m);
   int s = 0;
-  for (int r = a; r < b; ++r)
-    for (int w = 0; w < 8; ++w) s += __popc(pres[r * 8 + w]);
-  part[t] = s;
+  for (int w = t; w < ra * 8; w += 256) s += __popc(__ldg(pres + w));
+  s = (int)__reduce_add_sync(FULL, (unsigned)s);
+  if (lane == 0) part[wib] = s;
+  if (t < kMapRegs) cnt[t] = 0;
   __syncthreads();
-  for (int d = 1; d < 1024; d <<= 1) {
-    const int add = (t >= d) ? part[t - d] : 0;
-    __syncthreads();
-    part[t] += add;
-    __syncthreads();
+  if (t < (rb - ra) * 8) {
+    const uint32_t b = __ldg(pres + ra * 8 + t);
+    bits[t] = b;
+    atomicAdd(&cnt[t >> 3], __popc(b));
   }
-  int run = (t > 0) ? part[t - 1] : 0;
-  for (int r = a; r < b; ++r) {
-    koff[r] = run;
-    for (int w = 0; w < 8; ++w) run += __popc(pres[r * 8 + w]);
-  }
-  if (t == 1023) koff[m] = part[1023];
   __syncthreads();
-  for (int64_t e = t; e < (int64_t)m * 256; e += 1024) {
-    const int r = (int)(e >> 8), code = (int)(e & 255);
-    const uint32_t *p = pres + r * 8;
+  int run = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) run += part[q];
+  for (int r = ra; r < rb; ++r) {
+    if (t == 0) koff[r] = run;
+    const uint32_t *p = bits + (r - ra) * 8;             // warp wib holds codes 32 wib ..
     int32_t v = -1;
-    if ((p[code >> 5] >> (code & 31)) & 1u) {
-      int rank = __popc(p[code >> 5] & ((1u << (code & 31)) - 1u));
-      for (int w = 0; w < (code >> 5); ++w) rank += __popc(p[w]);
-      v = koff[r] + rank;
+    if ((p[wib] >> lane) & 1u) {
+      int rank = __popc(p[wib] & ((1u << lane) - 1u));
+      for (int w = 0; w < wib; ++w) rank += __popc(p[w]);
+      v = run + rank;
     }
-    map[e] = v;
+    map[(int64_t)r * 256 + t] = v;
+    run += cnt[r - ra];
   }
+  if (rb == m && t == 0) koff[m] = run;
 }
 
 // X[i][map[r][code_i(r)]] = 1 (X zeroed by the caller; row stride ldx bytes).
@@ -221,14 +227,15 @@ void launch_code_presence(const uint8_t *codesA, int64_t n, int m, int mpad, uin
                           cudaStream_t s) {
   cudaMemsetAsync(pres, 0, (size_t)m * 8 * sizeof(uint32_t), s);
   if (n == 0) return;
-  const int64_t rows_per_block = 64;
+  // 64 rows a block amortise its shared table; fewer while that leaves SMs idle
+  const int64_t rows_per_block = std::max<int64_t>(4, std::min<int64_t>(64, n / 296));
   const dim3 grid((unsigned)((n + rows_per_block - 1) / rows_per_block),
                   (unsigned)((m + kPresCols - 1) / kPresCols));
   k_code_presence<<<grid, 256, 0, s>>>(codesA, n, m, mpad, rows_per_block, pres);
 }
 
 void launch_onehot_map(const uint32_t *pres, int m, int32_t *map, int32_t *koff, cudaStream_t s) {
-  k_onehot_map<<<1, 1024, 0, s>>>(pres, m, map, koff);
+  k_onehot_map<<<(unsigned)((m + kMapRegs - 1) / kMapRegs), 256, 0, s>>>(pres, m, map, koff);
 }
 
 void launch_onehot_fill(const uint8_t *codesA, int64_t n, int m, int mpad, const int32_t *map,
