@@ -262,7 +262,10 @@ void stage_sketch_chunked(rbg_ctx *c, const rbg_params *p, const char *seqcat,
     sym_clear(c, std::max<int64_t>(n, 1));
     CK(cudaStreamWaitEvent(c->stream, c->ev_aux, 0));   // unit rows, anynz
     tc5 = sym_tc5_fits(ga);
-    if (tc5) sym_tc5_setup(c, ga, G);
+    if (tc5) {
+      sym_tc5_clear(c);
+      sym_tc5_setup(c, ga, G);
+    }
   }
   // Packing on the host sends 3/8 of a byte per base instead of the ASCII
   // byte: while chunk g's words copy, the host packs chunk g + 1 into the
@@ -609,12 +612,20 @@ void dense_allpairs_onehot(rbg_ctx *c, const GraphArgs &g) {
 bool sym_tc5_on() { return getenv("RBG_SYM_SINGLE") == nullptr; }
 
 bool sym_tc5_fits(const GraphArgs &g) {
-  // S < 64 leaves the last of the 64 padded halves for the threshold column
-  return sym_tc5_on() && g.S < 64 && g.Kp <= 64 && g.n > 0 && g.n < ((int64_t)1 << 27);
+  // S < 64 leaves the last of the 64 padded halves for the threshold column;
+  // survivor entries hold 26-bit column ids
+  return sym_tc5_on() && g.S < 64 && g.Kp <= 64 && g.n > 0 && g.n <= ((int64_t)1 << 26);
 }
 
-// Buffers, list capacities (for the whole assembly), the padded FP16 rows and
-// cleared flags for the passes over one assembly; `slots` item tables (one per
+// Clears the flags that the passes accumulate (once before the passes whose
+// flags are read back together).
+void sym_tc5_clear(rbg_ctx *c) {
+  c->tc5_flags.ensure(kTc5Flags * sizeof(int));
+  CK(cudaMemsetAsync(c->tc5_flags.p, 0, kTc5Flags * sizeof(int), c->stream));
+}
+
+// Buffers, list capacities (for the whole assembly) and the padded FP16 rows
+// for the passes over one assembly; `slots` item tables (one per
 // pass in flight).  The capacities come from the kept fraction, or exact ones
 // right after a pass whose lists overflowed (the one host copy here, on a
 // rerun only); offsets and item tables are made on the device, so nothing is
@@ -633,25 +644,39 @@ void sym_tc5_setup(rbg_ctx *c, const GraphArgs &g, int slots) {
                        cudaMemcpyHostToDevice, s));
     launch_tc5_coff(n, 0.0, c->tc5_caps.as<int64_t>(), c->tc5_coff.as<int64_t>(), s);
   } else {
-    total = tc5_capacity(n, c->tc5_frac);
-    launch_tc5_coff(n, c->tc5_frac, nullptr, c->tc5_coff.as<int64_t>(), s);
+    total = tc5_capacity(n, c->tc5_frac[g.S]);
+    launch_tc5_coff(n, c->tc5_frac[g.S], nullptr, c->tc5_coff.as<int64_t>(), s);
   }
   c->tc5_exact = false;
   c->tc5_n = n;
   c->tc5_rbmax = RBmax;
   c->tc5_items.ensure((size_t)slots * (RBmax + 1) * sizeof(int32_t));
   c->tc5_cand.ensure((size_t)std::max<int64_t>(total, 1) * sizeof(uint32_t));
-  c->tc5_cnt.ensure((size_t)B32 * sizeof(int32_t));
+  c->tc5_cnt.ensure((size_t)(B32 + 1) * sizeof(int32_t));   // the counts, then the item counter
   c->tc5_u16p.ensure((size_t)n * 256);         // row and column copies
-  c->tc5_flags.ensure(2 * sizeof(int));
-  CK(cudaMemsetAsync(c->tc5_flags.p, 0, 2 * sizeof(int), s));
   launch_pad_unit16(g, prefilter_lo16(g.S, g.prefilter_eps), c->tc5_u16p.as<uint16_t>(), s);
+  const int pg = (g.mpad + 31) / 32;
+  c->planesA.ensure((size_t)n * pg * 32);
+  c->planesB.ensure((size_t)n * pg * 32);
+  c->lowA.ensure((size_t)n * low_plane_words(pg) * 4);
+  c->lowB.ensure((size_t)n * low_plane_words(pg) * 4);
+  c->pflag.ensure((size_t)n);
+  c->tc5_seg.ensure((size_t)(B32 + 2) * sizeof(int32_t));
   c->launches += 2;
 }
 
-// The pass over the pairs i < j with j in [cb, ce) (item table in `slot`).
-void sym_tc5_pass(rbg_ctx *c, const GraphArgs &g, const SymOut &o, int64_t cb, int64_t ce,
+// The pass over the pairs i < j with j in [cb, ce) (item table in `slot`), the
+// rows below cb being in earlier passes' windows; makes the register planes of
+// the rows [cb, ce).
+void sym_tc5_pass(rbg_ctx *c, const GraphArgs &g0, const SymOut &o, int64_t cb, int64_t ce,
                   int slot) {
+  GraphArgs g = g0;
+  g.pg = (g.mpad + 31) / 32;
+  g.planesA = c->planesA.as<uint32_t>();
+  g.planesB = c->planesB.as<uint32_t>();
+  g.lowA = c->lowA.as<uint32_t>();
+  g.lowB = c->lowB.as<uint32_t>();
+  g.pflag = c->pflag.as<uint8_t>();
   int RB = 0, NT = 0;
   const int items = sym_tc5_items(cb, ce, &RB, &NT);
   if (items == 0) return;
@@ -659,7 +684,7 @@ void sym_tc5_pass(rbg_ctx *c, const GraphArgs &g, const SymOut &o, int64_t cb, i
   int32_t *di0 = c->tc5_items.as<int32_t>() + (size_t)slot * (c->tc5_rbmax + 1);
   cudaStream_t s = c->stream;
   launch_tc5_items(cb, ce, di0, s);
-  CK(cudaMemsetAsync(c->tc5_cnt.p, 0, (size_t)blocks * sizeof(int32_t), s));
+  CK(cudaMemsetAsync(c->tc5_cnt.p, 0, (size_t)(blocks + 1) * sizeof(int32_t), s));
   int dev = 0, sms = 148;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -668,47 +693,53 @@ void sym_tc5_pass(rbg_ctx *c, const GraphArgs &g, const SymOut &o, int64_t cb, i
       g, c->tc5_u16p.as<uint16_t>(), cb, ce, di0, RB, NT, items, c->tc5_cand.as<uint32_t>(), c->tc5_coff.as<int64_t>(), c->tc5_cnt.as<int32_t>(),
       c->tc5_flags.as<int>(), c->tc5_flags.as<int>() + 1, sms, s, &why);
   if (rc != RBG_OK) throw Error(rc, std::string("tensor-core prefilter: ") + why);
+  launch_code_planes(g, cb, ce, c->planesA.as<uint32_t>(), c->planesB.as<uint32_t>(),
+                     c->lowA.as<uint32_t>(), c->lowB.as<uint32_t>(), c->pflag.as<uint8_t>(), s);
   launch_sym_check(g, o, c->tc5_cand.as<uint32_t>(), c->tc5_coff.as<int64_t>(),
-                   c->tc5_cnt.as<int32_t>(), blocks, s);
-  c->launches += 3;
+                   c->tc5_cnt.as<int32_t>(), blocks, c->tc5_seg.as<int32_t>(),
+                   (unsigned *)c->tc5_cnt.as<int32_t>() + blocks,
+                   c->tc5_flags.as<float>() + 2 + g.S, sms, s);
+  c->launches += 5;
 }
 
 // After the pass's synchronisation (the flags and counts read back into
 // c->tc5_host): false when a list overflowed (capacities now exact: rerun).
-bool sym_tc5_settle(rbg_ctx *c, int64_t n) {
+bool sym_tc5_settle(rbg_ctx *c, int64_t n, int S) {
   const int64_t B32 = (n + 31) / 32;
+  double &frac_S = c->tc5_frac[S];
   const int *fl = c->tc5_host.as<int>();
-  const int32_t *cnt = fl + 4;
+  const int32_t *cnt = fl + 2;
   if (fl[1] != 0)
     throw Error(RBG_ERR_TIMEOUT, "tensor-core prefilter: a bounded device wait gave up (stage " +
                                      std::to_string(fl[1]) + ")");
   double frac = 0.0;
   for (int64_t b = 0; b < B32; ++b) {
     const double pairs = 32.0 * (double)std::max<int64_t>(n - 32 * b, 0);
-    if (pairs > 0) frac = std::max(frac, cnt[b] / pairs);
+    // past the 256 entries every list has room for
+    if (pairs > 0) frac = std::max(frac, (cnt[b] - 256) / pairs);
   }
   if (fl[0] != 0) {                          // rerun with room for every block's count
     c->tc5_cap.assign((size_t)B32, 0);
     for (int64_t b = 0; b < B32; ++b) {
       const double pairs = 32.0 * (double)std::max<int64_t>(n - 32 * b, 0);
-      const int64_t fc = ((int64_t)(pairs * c->tc5_frac) + 256 + 31) & ~(int64_t)31;
+      const int64_t fc = ((int64_t)(pairs * frac_S) + 256 + 31) & ~(int64_t)31;
       c->tc5_cap[b] = std::max<int64_t>(fc, ((int64_t)cnt[b] + 256 + 31) & ~(int64_t)31);
     }
     c->tc5_exact = true;
-    c->tc5_frac = std::max(c->tc5_frac, frac * 1.25);
+    frac_S = std::max(frac_S, frac * 1.25);
     return false;
   }
-  if (frac * 1.25 > c->tc5_frac) c->tc5_frac = frac * 1.25;   // room to spare next time
+  if (frac * 1.25 > frac_S) frac_S = frac * 1.25;   // room to spare next time
   return true;
 }
 
 // The flags and per-block counts to the host on the stream (read after its sync).
 void sym_tc5_readback(rbg_ctx *c, int64_t n) {
   const int64_t B32 = (n + 31) / 32;
-  c->tc5_host.ensure((size_t)(4 + B32) * sizeof(int32_t));
+  c->tc5_host.ensure((size_t)(2 + B32) * sizeof(int32_t));
   CK(cudaMemcpyAsync(c->tc5_host.p, c->tc5_flags.p, 2 * sizeof(int), cudaMemcpyDeviceToHost,
                      c->stream));
-  CK(cudaMemcpyAsync(c->tc5_host.as<int32_t>() + 4, c->tc5_cnt.p, (size_t)B32 * sizeof(int32_t),
+  CK(cudaMemcpyAsync(c->tc5_host.as<int32_t>() + 2, c->tc5_cnt.p, (size_t)B32 * sizeof(int32_t),
                      cudaMemcpyDeviceToHost, c->stream));
 }
 
@@ -892,6 +923,7 @@ void run_graph(rbg_ctx *c, const rbg_params *p, const ShardCtx *sc = nullptr) {
       } else {
         sym_clear(c, n1);
         if (tc5) {
+          sym_tc5_clear(c);
           sym_tc5_setup(c, g, 1);
           sym_tc5_pass(c, g, o, 0, n, 0);
           sym_tc5_readback(c, n);
@@ -922,12 +954,12 @@ void run_graph(rbg_ctx *c, const rbg_params *p, const ShardCtx *sc = nullptr) {
                                        "(stage " + std::to_string(fl[1]) + ")");
         if (fl[0] != 0) {                            // a window's list overflowed: rescore
           CK(cudaStreamSynchronize(c->stream));
-          c->tc5_frac *= 2.0;
+          c->tc5_frac[S] *= 2.0;
           streamed = false;
           continue;
         }
       }
-      if (tc5 && !sym_tc5_settle(c, n)) {           // a candidate list overflowed: rerun
+      if (tc5 && !sym_tc5_settle(c, n, S)) {           // a candidate list overflowed: rerun
         CK(cudaStreamSynchronize(c->stream));
         continue;
       }
@@ -1443,7 +1475,8 @@ int rbg_destroy(rbg_ctx *c) {
                   &c->shard_send, &c->shard_recv, &c->oh_pres, &c->oh_map, &c->oh_koff,
                   &c->oh_X, &c->oh_cand, &c->oh_cnt, &c->oh_tab, &c->oh_err, &c->kept, &c->b0dev,
                   &c->count_work, &c->tc5_u16p, &c->tc5_cand, &c->tc5_cnt, &c->tc5_items,
-                  &c->tc5_coff, &c->tc5_caps, &c->tc5_flags,
+                  &c->tc5_coff, &c->tc5_caps, &c->tc5_flags, &c->planesA, &c->planesB, &c->lowA,
+                  &c->lowB, &c->pflag, &c->tc5_seg,
                   &c->qa, &c->qb, &c->qo, &c->qt, &c->ix_keys, &c->ix_sorted,
                   &c->ix_contig, &c->ix_post, &c->ix_ukeys, &c->ix_count, &c->ix_off,
                   &c->ix_nk, &c->ix_scratch};

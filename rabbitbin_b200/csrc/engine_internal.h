@@ -136,10 +136,14 @@ void check_onehot_status(rbg_ctx *c);
 // after the sync, false when a list overflowed (the caller reruns).
 bool sym_tc5_fits(const GraphArgs &g);
 void sym_tc5_setup(rbg_ctx *c, const GraphArgs &g, int slots);
+void sym_tc5_clear(rbg_ctx *c);
+// Flags read back: [0] a list overflowed, [1] wait error, [2 + S] float bits of
+// the largest kept fraction of the passes at S samples.
+constexpr int kTc5Flags = 2 + 65;
 void sym_tc5_pass(rbg_ctx *c, const GraphArgs &g, const SymOut &o, int64_t cb, int64_t ce,
                   int slot);
 void sym_tc5_readback(rbg_ctx *c, int64_t n);
-bool sym_tc5_settle(rbg_ctx *c, int64_t n);
+bool sym_tc5_settle(rbg_ctx *c, int64_t n, int S);
 // The dense regime runs on the one-hot tensor-core kernel unless RBG_DENSE_ALU
 // is set (then the integer-ALU register compare, kept for the measured
 // comparison).
@@ -360,12 +364,13 @@ struct rbg_ctx {
   rbg::DBuf oh_pres, oh_map, oh_koff, oh_X, oh_cand, oh_cnt, oh_tab, oh_err;
   rbg::DBuf count_work;                 // contig counter of the k-mer count kernel
   // symmetric pass on the tensor-core prefilter: candidate lists per 32-row
-  // block (capacities tc5_cap, sized from the kept fraction tc5_frac)
+  // block (capacities tc5_cap, sized from the kept fractions tc5_frac)
   rbg::DBuf tc5_u16p, tc5_cand, tc5_cnt, tc5_items, tc5_coff, tc5_caps, tc5_flags;
+  rbg::DBuf planesA, planesB, lowA, lowB, pflag, tc5_seg;   // register planes, check items
   rbg::HBuf tc5_pin, tc5_host;
   std::vector<int64_t> tc5_cap;
   int64_t tc5_n = -1;
-  double tc5_frac = 0.03;
+  std::vector<double> tc5_frac = std::vector<double>(65, 0.03);   // by S
   bool tc5_exact = false;               // tc5_cap holds exact capacities for the next setup
   int64_t tc5_rbmax = 0;                // item-table slot length - 1
   bool streamed_tc5 = false;            // the pairs behind the copy went through that pass

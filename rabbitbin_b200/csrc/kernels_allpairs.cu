@@ -111,6 +111,13 @@ __device__ __forceinline__ void cp16(void *dst, const void *src) {
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
+// Survivor entries of k_sym_check: row of the block << 27 | kHiBit when both
+// rows hold codes above kLowCodes | column (below 2^26).
+constexpr unsigned kHiBit = 1u << 26, kIdMask = kHiBit - 1u;
+constexpr unsigned kLowCodes = 62;
+// words of a row's low planes: four planes of every group, then the other two
+__host__ __device__ __forceinline__ int low_stride(int pg) { return (6 * pg + 3) & ~3; }
+
 struct Warp {
   uint64_t *gbuf;     // [32 rows][cap] candidate keys of this warp's rows
   int *cnt;           // smem [32]
@@ -188,19 +195,63 @@ __device__ __forceinline__ void count_batch_coop(const GraphArgs &g, Warp &w, co
   compact_full_rows(w, w.cap - 32);
 }
 
-// Symmetric form of count_batch_coop: the same counts, then each survivor
-// (i = row0 + r, j) raises both rows' maxima (row i through the warp's own
-// state, row j by an atomic) and, when its similarity passes the admission
-// floor, is appended once to the pair list with both rows' counts raised.
-// grow0: the assembly's first row in the row space of the pair list.
-template <int NF = 4>
+// Up to 32 survivors (i = row0 + r, j) with their match counts (lane p:
+// survivor p's count `mine`): each raises both rows' maxima (row i through the
+// warp's own state, row j by an atomic) and, when its similarity passes the
+// admission floor, is appended once to the pair list with both rows' counts
+// raised.  grow0: the assembly's first row in the row space of the pair list;
+// rc: the block's own rows' counts in shared memory (null: straight to o.rowcnt).
+__device__ __forceinline__ void admit_sym(const GraphArgs &g, const SymOut &o, uint32_t *mxc,
+                                          int64_t row0, int64_t grow0, const unsigned *q, int nq,
+                                          uint32_t mine, unsigned id_mask, int *rc) {
+  const int lane = threadIdx.x & 31;
+  bool adm = false;
+  int r = 0;
+  uint32_t j = 0, svb = 0;
+  if (lane < nq) {
+    const unsigned e = q[lane];
+    r = (int)(e >> 27);
+    j = e & id_mask;
+    // shared-memory atomics: they serialise only the survivors of one row
+    // (grouping the lanes by row runs one step per row of the batch)
+    atomicMax(mxc + r, mine);
+    if (mine) atomicMax(g.maxcnt_cand + j, mine);
+    if (o.defer) {
+      svb = mine;                        // converted once the similarity table exists
+      adm = mine > 0;
+    } else {
+      svb = __ldg(g.sv_bits + mine);
+      adm = svb > (uint32_t)(g.key_floor >> 32);
+    }
+  }
+  const unsigned am = __ballot_sync(FULL, adm);
+  if (am) {
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(o.npairs, (unsigned long long)__popc(am));
+    base = __shfl_sync(FULL, base, 0);
+    if (adm) {
+      const unsigned long long pos = base + (unsigned)__popc(am & ((1u << lane) - 1u));
+      if (pos < o.cap) {
+        const uint32_t gi = (uint32_t)(grow0 + row0 + r), gj = (uint32_t)(grow0 + j);
+        o.pairs[pos] = make_uint4(gi, gj, svb, (uint32_t)grow0);
+        if (rc) atomicAdd(rc + r, 1);
+        else atomicAdd(o.rowcnt + gi, 1);
+        atomicAdd(o.rowcnt + gj, 1);
+      }
+    }
+  }
+  __syncwarp();
+}
+
+// Symmetric form of count_batch_coop: the same counts, then admit_sym.
 __device__ __forceinline__ void count_batch_sym(const GraphArgs &g, const SymOut &o, uint32_t *mxc,
                                                 int64_t row0, int64_t grow0, const int *q, int nq,
                                                 const unsigned char *sA) {
+  constexpr int NF = 4;                            // survivors' column codes in flight
   const int lane = threadIdx.x & 31;
   const int m16 = g.mpad >> 4;
   uint32_t mine = 0;
-  for (int p = 0; p < nq; p += NF) {               // NF survivors' column codes in flight
+  for (int p = 0; p < nq; p += NF) {
     const uint4 *ra[NF], *cb[NF];
 #pragma unroll
     for (int u = 0; u < NF; ++u) {
@@ -224,43 +275,87 @@ __device__ __forceinline__ void count_batch_sym(const GraphArgs &g, const SymOut
       if (lane == p + u) mine = c;
     }
   }
-  const unsigned act = __ballot_sync(FULL, lane < nq);
-  bool adm = false;
-  int r = 0;
-  uint32_t j = 0, svb = 0;
-  if (lane < nq) {
-    const unsigned e = (unsigned)q[lane];
-    r = (int)(e >> 27);
-    j = e & 0x07FFFFFFu;
-    const unsigned grp = __match_any_sync(act, r);
-    const uint32_t mx = __reduce_max_sync(grp, mine);
-    if (lane == __ffs(grp) - 1 && mx > mxc[r]) mxc[r] = mx;
-    if (mine) atomicMax(g.maxcnt_cand + j, mine);
-    if (o.defer) {
-      svb = mine;                        // converted once the similarity table exists
-      adm = mine > 0;
-    } else {
-      svb = __ldg(g.sv_bits + mine);
-      adm = svb > (uint32_t)(g.key_floor >> 32);
+  admit_sym(g, o, mxc, row0, grow0, (const unsigned *)q, nq, mine, 0x07FFFFFFu, nullptr);
+}
+
+// The same counts on bit planes (launch_code_planes).  A group of 32 registers
+// is six words, word p holding bit p of the registers' low codes (the codes up
+// to 62, which name the winners of all but a few registers in a million; a register with
+// another code or none matches nothing here): the registers that differ are the
+// OR over the planes of the two sides' XORs, six three-input logic operations
+// and one population count for 32 registers, where bytes take five operations
+// for every 4 codes.  A pair whose rows both hold codes above 62 (kHiBit of its
+// entry) is counted on the eight planes of the whole codes instead.  LP lanes
+// take one survivor (a group each; LP < 32 only when the row's groups fit and a
+// count fits LP bits), 32 / LP survivors a step, four steps' column planes in
+// flight.  sP: the block's low row planes.
+template <int LP>
+__device__ __forceinline__ void count_batch_planes(const GraphArgs &g, const SymOut &o,
+                                                   uint32_t *mxc, int *rc, int64_t row0,
+                                                   const unsigned *q, int nq,
+                                                   const uint32_t *sP) {
+  constexpr int PER = 32 / LP, U = 4;
+  const int lane = threadIdx.x & 31, sub = lane & (LP - 1), which = lane / LP;
+  const int pg = g.pg, ls = low_stride(pg);
+  uint32_t mine = 0;
+  for (int p = 0; p < nq; p += PER * U) {
+    unsigned e[U];
+    uint32_t cnt[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      e[u] = q[min(p + u * PER + which, nq - 1)];
+      cnt[u] = 0;
     }
-  }
-  const unsigned am = __ballot_sync(FULL, adm);
-  if (am) {
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(o.npairs, (unsigned long long)__popc(am));
-    base = __shfl_sync(FULL, base, 0);
-    if (adm) {
-      const unsigned long long pos = base + (unsigned)__popc(am & ((1u << lane) - 1u));
-      if (pos < o.cap) {
-        const uint32_t gi = (uint32_t)(grow0 + row0 + r), gj = (uint32_t)(grow0 + j);
-        o.pairs[pos] = make_uint4(gi, gj, svb, (uint32_t)grow0);
-        atomicAdd(o.rowcnt + gi, 1);
-        atomicAdd(o.rowcnt + gj, 1);
+    for (int t = sub; t < pg; t += LP) {           // one round when LP >= pg
+      uint4 b[U];
+      uint2 b4[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t *c = g.lowB + (int64_t)(e[u] & kIdMask) * ls;
+        b[u] = __ldg(reinterpret_cast<const uint4 *>(c) + t);
+        b4[u] = __ldg(reinterpret_cast<const uint2 *>(c + 4 * pg) + t);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t *r = sP + (e[u] >> 27) * ls;
+        const uint4 a = lds128(reinterpret_cast<const uint4 *>(r) + t);
+        uint32_t d = a.x ^ b[u].x;
+        d |= a.y ^ b[u].y;
+        d |= a.z ^ b[u].z;
+        d |= a.w ^ b[u].w;
+        const uint2 a4 = reinterpret_cast<const uint2 *>(r + 4 * pg)[t];
+        d |= a4.x ^ b4[u].x;
+        d |= a4.y ^ b4[u].y;
+        cnt[u] += __popc(~d);
       }
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (__any_sync(FULL, e[u] & kHiBit)) {
+        if (e[u] & kHiBit) {
+          const int64_t i = row0 + (e[u] >> 27), j = e[u] & kIdMask;
+          uint32_t c = 0;
+          for (int t = sub; t < pg; t += LP) {
+            const uint4 *x = reinterpret_cast<const uint4 *>(g.planesA) + i * (2 * pg) + t;
+            const uint4 *y = reinterpret_cast<const uint4 *>(g.planesB) + j * (2 * pg) + t;
+            const uint4 x0 = __ldg(x), x1 = __ldg(x + pg), y0 = __ldg(y), y1 = __ldg(y + pg);
+            c += __popc(~((x0.x ^ y0.x) | (x0.y ^ y0.y) | (x0.z ^ y0.z) | (x0.w ^ y0.w) |
+                          (x1.x ^ y1.x) | (x1.y ^ y1.y) | (x1.z ^ y1.z) | (x1.w ^ y1.w)));
+          }
+          cnt[u] = c;
+        }
+        __syncwarp();
+      }
+      // the PER survivors' sums side by side in one word, LP bits each
+      const uint32_t c = __reduce_add_sync(FULL, cnt[u] << ((LP & 31) * which));
+      const unsigned rel = (unsigned)(lane - (p + u * PER));
+      if (rel < (unsigned)PER)
+        mine = LP == 32 ? c : (c >> ((LP & 31) * rel)) & ((1u << (LP & 31)) - 1u);
+    }
   }
-  __syncwarp();
+  admit_sym(g, o, mxc, row0, o.row_base, q, nq, mine, kIdMask, rc);
 }
+
 
 // Dense regime: one work item = 32 rows (row block bx) x the column slices
 // kWarps*by .. kWarps*by+3, one warp per slice.
@@ -391,6 +486,7 @@ constexpr int kTCT = 16;          // columns per staged tile
 // (32 rows x 8 columns) of one step; not a power of two, indexed modulo
 constexpr int kCQ = 320;
 constexpr int kTcWs = 768;        // per-warp workspace: thresholds, counts, maxima, survivors
+constexpr int kScWs = 512;        // the same in k_sym_check: maxima, counts, survivors
 
 __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
                                          uint32_t b1) {
@@ -414,10 +510,36 @@ __device__ __forceinline__ void ldsm_x2(uint32_t &r0, uint32_t &r1, const void *
                : "r"(a));
 }
 
-// Exact prune decision for up to 32 queued candidates (lane = candidate),
-// survivors appended to the counting queue.  RING: candidates in the check
-// ring at head (modulo kCQ); otherwise a plain list from cq + head.
-template <int SMAX, bool SYM, bool RING = true>
+// Exact prune decision of one candidate (row r of the block, column j) per
+// lane: the FP32 chain, the AVX-512 order inside its band.
+template <int SMAX>
+__device__ __forceinline__ bool prune_pass(const GraphArgs &g, int r, int64_t j, float lo,
+                                           float hi, const float *sU, int SuP) {
+  const int Su = g.Su;
+  const float4 *ua = (const float4 *)(sU + r * SuP);
+  const float4 *ub = (const float4 *)(g.unit + j * Su);
+  float ur[SMAX];
+  float c1 = 0.f;
+#pragma unroll
+  for (int t4 = 0; t4 < SMAX; t4 += 4) {
+    if (t4 < Su) {
+      const float4 x = ua[t4 >> 2], y = __ldg(ub + (t4 >> 2));
+      ur[t4] = x.x; ur[t4 + 1] = x.y; ur[t4 + 2] = x.z; ur[t4 + 3] = x.w;
+      c1 = __fmaf_rn(x.x, y.x, c1);
+      c1 = __fmaf_rn(x.y, y.y, c1);
+      c1 = __fmaf_rn(x.z, y.z, c1);
+      c1 = __fmaf_rn(x.w, y.w, c1);
+    } else {
+      ur[t4] = ur[t4 + 1] = ur[t4 + 2] = ur[t4 + 3] = 0.f;
+    }
+  }
+  if (c1 >= hi) return true;
+  return c1 >= lo && !(dot_avx512<SMAX>(ur, g.unit + j * Su, g.S) < g.prefilter_eps);
+}
+
+// prune_pass of up to 32 candidates of the check ring (at head, modulo kCQ),
+// survivors appended to the counting queue.
+template <int SMAX, bool SYM>
 __device__ __forceinline__ void check_batch(const GraphArgs &g, Warp &w, const SymOut &o,
                                             int64_t grow0, const int *cq, unsigned head, int nq,
                                             int64_t row0, int *q, int &qn, float lo, float hi,
@@ -425,39 +547,17 @@ __device__ __forceinline__ void check_batch(const GraphArgs &g, Warp &w, const S
                                             int SuP, const unsigned char *sA) {
   const int lane = threadIdx.x & 31;
   const bool act = lane < nq;
-  const unsigned e = act ? (unsigned)cq[RING ? (head + lane) % kCQ : head + lane] : 0u;
+  const unsigned e = act ? (unsigned)cq[(head + lane) % kCQ] : 0u;
   const int r = (int)(e >> 27);
-  const int64_t j = e & 0x07FFFFFFu;
-  const int64_t row = row0 + r;
-  bool pass = false;
-  if (act && j != row && (__ldg(g.anynz + row) | __ldg(g.anynz + j))) {
-    const int Su = g.Su;
-    const float4 *ua = (const float4 *)(sU + r * SuP);
-    const float4 *ub = (const float4 *)(g.unit + j * Su);
-    float ur[SMAX];
-    float c1 = 0.f;
-#pragma unroll
-    for (int t4 = 0; t4 < SMAX; t4 += 4) {
-      if (t4 < Su) {
-        const float4 x = ua[t4 >> 2], y = __ldg(ub + (t4 >> 2));
-        ur[t4] = x.x; ur[t4 + 1] = x.y; ur[t4 + 2] = x.z; ur[t4 + 3] = x.w;
-        c1 = __fmaf_rn(x.x, y.x, c1);
-        c1 = __fmaf_rn(x.y, y.y, c1);
-        c1 = __fmaf_rn(x.z, y.z, c1);
-        c1 = __fmaf_rn(x.w, y.w, c1);
-      } else {
-        ur[t4] = ur[t4 + 1] = ur[t4 + 2] = ur[t4 + 3] = 0.f;
-      }
-    }
-    if (c1 >= hi) pass = true;
-    else if (c1 >= lo) pass = !(dot_avx512<SMAX>(ur, g.unit + j * Su, g.S) < g.prefilter_eps);
-  }
+  const int64_t j = e & 0x07FFFFFFu, row = row0 + r;
+  const bool pass = act && j != row && (__ldg(g.anynz + row) | __ldg(g.anynz + j)) &&
+                    prune_pass<SMAX>(g, r, j, lo, hi, sU, SuP);
   const unsigned m = __ballot_sync(FULL, pass);
-  if (pass) q[qn + __popc(m & ((1u << lane) - 1u))] = (int)(((unsigned)r << 27) | (unsigned)j);
+  if (pass) q[qn + __popc(m & ((1u << lane) - 1u))] = (int)e;
   qn += __popc(m);
   __syncwarp();
   if (qn >= 32) {
-    if constexpr (SYM) count_batch_sym<RING ? 4 : 8>(g, o, w.mxc, row0, grow0, q, 32, sA);
+    if constexpr (SYM) count_batch_sym(g, o, w.mxc, row0, grow0, q, 32, sA);
     else count_batch_coop(g, w, q, 32, sA);
     n_cmp += 1;
     if (lane + 32 < qn) q[lane] = q[lane + 32];
@@ -698,80 +798,270 @@ k_allpairs_tc_win(GraphArgs g, int P, float lo, float hi, float lo16, SymOut o, 
                           0, cb, ce);
 }
 
-// Symmetric pass, part 2 (after k_sym_prefilter, kernels_sym_tc5.cu): a CTA
-// takes 32-row block x and block B-1-x of the B blocks in play (as
-// k_allpairs_tc_sym pairs them; gridDim.y CTAs share a pair's lists), with
-// the block's register codes and unit rows in shared memory, and its warps work
-// through the block's candidate list 32 entries at a time: the exact prune
-// decision (check_batch), then the survivors' register compares and pair
-// records (count_batch_sym), exactly as in the single-kernel pass.
-template <int SMAX>
-__device__ __forceinline__ void sym_check_block(const GraphArgs &g, const SymOut &o, float lo,
-                                                float hi, const uint32_t *cand,
-                                                const int64_t *coff, const int32_t *ccnt,
-                                                int64_t bx, unsigned char *smem) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t n = g.n, row0 = bx * 32;
-  unsigned char *ws = smem + (size_t)warp * kTcWs;
-  uint64_t *thr = (uint64_t *)ws;
-  int *cntw = (int *)(thr + 32);
-  uint32_t *mxc = (uint32_t *)(cntw + 32);
-  int *q = (int *)(mxc + 32);                      // [64] survivors to count
-  unsigned char *sA = smem + (size_t)kWarps * kTcWs;
-  float *sU = (float *)(sA + (size_t)32 * g.mpad);
-  const int SuP = su_stride(g.Su);
-  {
-    const int m16 = g.mpad >> 4, s4 = g.Su >> 2;
-    for (int i = threadIdx.x; i < 32 * m16; i += blockDim.x) {
-      const int r = i / m16, t = i - r * m16;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (row0 + r < n) v = __ldg((const uint4 *)(g.codesA + (row0 + r) * g.mpad) + t);
-      *((uint4 *)(sA + (size_t)r * g.mpad) + t) = v;
-    }
-    for (int i = threadIdx.x; i < 32 * s4; i += blockDim.x) {
-      const int r = i / s4, t = i - r * s4;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (row0 + r < n) v = __ldg((const float4 *)(g.unit + (row0 + r) * g.Su) + t);
-      *((float4 *)(sU + (size_t)r * SuP) + t) = v;
-    }
-  }
-  mxc[lane] = 0;
+// Work items of k_sym_check: segments of the blocks' candidate lists.  seg[0 ..
+// B] = first item of each block, seg[B + 1] = entries of a segment: about six
+// items a CTA slot, so that the last ones leave few SMs idle (with a block
+// pair's whole lists per CTA, 30% of the kernel's time was its tail).
+__global__ void __launch_bounds__(1024) k_check_items(const int64_t *coff, const int32_t *ccnt,
+                                                      int64_t B, int64_t n, int slots,
+                                                      int32_t *seg, float *need) {
+  __shared__ int part[1024];
+  __shared__ unsigned long long all;
+  const int t = threadIdx.x;
+  auto listed = [&](int64_t b) { return (int)min((int64_t)ccnt[b], coff[b + 1] - coff[b]); };
+  if (t == 0) all = 0;
   __syncthreads();
-  Warp w{nullptr, cntw, thr, mxc, 0, g.K};
+  const int64_t per = (B + 1023) / 1024;
+  const int64_t lo = min(B, t * per), hi = min(B, lo + per);
+  unsigned long long sum = 0;
+  float kept = 0.f;                    // a block's pairs: 32 rows against the columns from its first on
+  for (int64_t b = lo; b < hi; ++b) {
+    sum += (unsigned)listed(b);
+    // (past the 256 entries every list has room for)
+    kept = fmaxf(kept, (float)(ccnt[b] - 256) / (32.f * (float)(n - 32 * b)));
+  }
+  // non-negative floats order as their bits
+  kept = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(kept)));
+  if ((t & 31) == 0) atomicMax((int *)need, __float_as_int(kept));
+#pragma unroll
+  for (int d = 16; d; d >>= 1) sum += __shfl_xor_sync(FULL, sum, d);
+  if ((t & 31) == 0) atomicAdd(&all, sum);
+  __syncthreads();
+  const int len = (int)(min(4096ull, max(256ull, all / (6ull * slots))) + 127) & ~127;
+  int s = 0;
+  for (int64_t b = lo; b < hi; ++b) s += (listed(b) + len - 1) / len;
+  part[t] = s;
+  __syncthreads();
+  for (int d = 1; d < 1024; d <<= 1) {
+    const int add = t >= d ? part[t - d] : 0;
+    __syncthreads();
+    part[t] += add;
+    __syncthreads();
+  }
+  int run = t ? part[t - 1] : 0;
+  for (int64_t b = lo; b < hi; ++b) {
+    seg[b] = run;
+    run += (listed(b) + len - 1) / len;
+  }
+  if (t == 1023) {
+    seg[B] = part[1023];
+    seg[B + 1] = len;
+  }
+}
+
+// Symmetric pass, part 2 (after k_sym_prefilter, kernels_sym_tc5.cu).  CTAs
+// pull segments of the 32-row blocks' candidate lists from a counter; with the
+// block's low register planes and unit rows in shared memory, the warps work
+// through the segment 32 entries at a time: the exact prune decision
+// (prune_pass), then the survivors' register compares (count_batch_planes) and
+// pair records (admit_sym).  Bound by the L1 data path: per survivor its column
+// planes (24 bytes a group of 32 registers), the candidate's unit row, and the
+// atomics of the later row's maximum and count (70% of its wavefronts; issue
+// 52%).  m = 500: 30,000 contigs 722 us on bytes -> 515 us (S = 20, 7.0 M
+// survivors), 4.25 -> 3.04 ms (S = 5, 51 M).
+template <int SMAX, int LP>
+__global__ void __launch_bounds__(kWarps * 32, SMAX <= 32 ? 6 : 1)
+k_sym_check(GraphArgs g, float lo, float hi, SymOut o, const uint32_t *cand,
+            const int64_t *coff, const int32_t *ccnt, int B, const int32_t *seg, unsigned *next) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int s_block, s_first;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t n = g.n;
+  unsigned char *ws = smem + (size_t)warp * kScWs;
+  uint32_t *mxc = (uint32_t *)ws;
+  int *rc = (int *)(mxc + 32);                     // pairs listed of the block's rows
+  unsigned *q = (unsigned *)(rc + 32);             // [64] survivors to count
+  const int ls = low_stride(g.pg);
+  uint32_t *sP = (uint32_t *)(smem + (size_t)kWarps * kScWs);
+  float *sU = (float *)(sP + (size_t)32 * ls);
+  const int SuP = su_stride(g.Su);
+  const int len = seg[B + 1], items = seg[B];
   unsigned long long n_cmp = 0;
-  int qn = 0;
-  const int64_t off = coff[bx];
-  const int cnt = (int)min((int64_t)ccnt[bx], coff[bx + 1] - off);
-  const int *list = (const int *)(cand + off);
-  // the gridDim.y CTAs of a block pair share its list
-  for (int i0 = ((int)blockIdx.y * kWarps + warp) * 32; i0 < cnt;
-       i0 += (int)gridDim.y * kWarps * 32)
-    check_batch<SMAX, true, false>(g, w, o, 0, list, (unsigned)i0, min(32, cnt - i0), row0, q,
-                                   qn, lo, hi, n_cmp, sU, SuP, sA);
-  if (qn > 0) {
-    n_cmp += lane < qn;
-    count_batch_sym<8>(g, o, mxc, row0, 0, q, qn, sA);
+  for (;;) {
+    if (warp == 0) {
+      // the next item and its block: the last b with seg[b] <= item, by 32-ary search
+      unsigned it = 0;
+      if (lane == 0) it = atomicAdd(next, 1u);
+      it = __shfl_sync(FULL, it, 0);
+      int b0 = 0, span = B;                        // the block is in [b0, b0 + span)
+      if (it < (unsigned)items) {
+        while (span > 1) {
+          const int step = (span + 31) / 32;
+          const int b = b0 + lane * step;
+          const bool le = lane * step < span && __ldg(seg + b) <= (int)it;
+          const int k = 31 - __clz((int)__ballot_sync(FULL, le));   // lane 0 always holds
+          const int left = span - k * step;
+          b0 += k * step;
+          span = left < step ? left : step;
+        }
+      } else {
+        b0 = -1;
+      }
+      if (lane == 0) {
+        s_block = b0;
+        s_first = b0 < 0 ? 0 : ((int)it - __ldg(seg + b0)) * len;
+      }
+    }
+    __syncthreads();
+    const int bx = s_block;
+    if (bx < 0) break;
+    const int64_t row0 = (int64_t)bx * 32;
+    {
+      const int p16 = ls >> 2, s4 = g.Su >> 2;
+      const uint4 *rows = reinterpret_cast<const uint4 *>(g.lowA) + row0 * p16;
+      const int lim = (int)min((int64_t)32, n - row0) * p16;
+      for (int i = threadIdx.x; i < 32 * p16; i += blockDim.x)
+        ((uint4 *)sP)[i] = i < lim ? __ldg(rows + i) : make_uint4(0u, 0u, 0u, 0u);
+      for (int i = threadIdx.x; i < 32 * s4; i += blockDim.x) {
+        const int r = i / s4, t = i - r * s4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row0 + r < n) v = __ldg((const float4 *)(g.unit + (row0 + r) * g.Su) + t);
+        *((float4 *)(sU + (size_t)r * SuP) + t) = v;
+      }
+    }
+    mxc[lane] = 0;
+    rc[lane] = 0;
+    const int64_t off = coff[bx];
+    const int cnt = min((int)min((int64_t)ccnt[bx], coff[bx + 1] - off), s_first + len);
+    const uint32_t *list = cand + off;
+    const uint32_t rflag = row0 + lane < n ? __ldg(g.pflag + row0 + lane) : 0u;
+    const unsigned rhi = __ballot_sync(FULL, rflag & 1u);   // rows with codes above kLowCodes
+    const unsigned rnz = __ballot_sync(FULL, rflag & 2u);   // rows with abundance
+    int i0 = s_first + warp * 32;
+    __syncthreads();
+    int qn = 0;
+    unsigned enext = i0 + lane < cnt ? list[i0 + lane] : 0u;
+    for (; i0 < cnt; i0 += kWarps * 32) {
+      const bool act = i0 + lane < cnt;
+      unsigned e = enext;
+      const int inext = i0 + kWarps * 32 + lane;     // the next entries load meanwhile
+      enext = inext < cnt ? list[inext] : 0u;
+      const int r = (int)(e >> 27);
+      const int64_t j = e & 0x07FFFFFFu;
+      // flag and unit row load together (an idle lane reads column 0)
+      const unsigned jf = __ldg(g.pflag + j);
+      const bool dot = prune_pass<SMAX>(g, r, j, lo, hi, sU, SuP);
+      const bool pass = act && dot && (((rnz >> r) & 1u) | (jf & 2u));
+      const unsigned m = __ballot_sync(FULL, pass);
+      if (pass) {
+        if ((rhi >> r) & jf & 1u) e |= kHiBit;
+        q[qn + __popc(m & ((1u << lane) - 1u))] = e;
+      }
+      qn += __popc(m);
+      __syncwarp();
+      if (qn >= 32) {
+        count_batch_planes<LP>(g, o, mxc, rc, row0, q, 32, sP);
+        n_cmp += 1;
+        if (lane + 32 < qn) q[lane] = q[lane + 32];
+        __syncwarp();
+        qn -= 32;
+      }
+    }
+    if (qn > 0) {
+      n_cmp += lane < qn;
+      count_batch_planes<LP>(g, o, mxc, rc, row0, q, qn, sP);
+    }
+    __syncwarp();
+    const int64_t row = row0 + lane;
+    if (row < n && mxc[lane]) atomicMax(g.maxcnt_cand + row, mxc[lane]);
+    if (rc[lane]) atomicAdd(o.rowcnt + o.row_base + row, rc[lane]);
+    __syncthreads();                               // shared rows and the item are done with
   }
   if (g.stats) {
     const unsigned b = __reduce_add_sync(FULL, (unsigned)n_cmp);
     if (lane == 0 && b) atomicAdd(g.stats + 1, (unsigned long long)b);
   }
-  __syncwarp();
-  const int64_t row = row0 + lane;
-  if (row < n && mxc[lane]) atomicMax(g.maxcnt_cand + row, mxc[lane]);
 }
 
-template <int SMAX>
-__global__ void __launch_bounds__(kWarps * 32, SMAX == 32 ? 6 : 1)
-k_sym_check(GraphArgs g, float lo, float hi, SymOut o, const uint32_t *cand,
-            const int64_t *coff, const int32_t *ccnt, int64_t B) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int64_t b1 = blockIdx.x, b2 = B - 1 - b1;
-  sym_check_block<SMAX>(g, o, lo, hi, cand, coff, ccnt, b1, smem);
-  if (b2 > b1) {
-    __syncthreads();
-    sym_check_block<SMAX>(g, o, lo, hi, cand, coff, ccnt, b2, smem);
+// Bits of 8 codes (bytes of x, then y) as 8 bytes: byte p of (x, y) gets one
+// bit of each code, the same bit of every code for one p (an 8 x 8 bit
+// transpose by three rounds of block swaps).
+__device__ __forceinline__ void transpose8(uint32_t &x, uint32_t &y) {
+  uint32_t t = (x ^ (x >> 7)) & 0x00AA00AAu;
+  x ^= t ^ (t << 7);
+  t = (y ^ (y >> 7)) & 0x00AA00AAu;
+  y ^= t ^ (t << 7);
+  t = (x ^ (x >> 14)) & 0x0000CCCCu;
+  x ^= t ^ (t << 14);
+  t = (y ^ (y >> 14)) & 0x0000CCCCu;
+  y ^= t ^ (t << 14);
+  t = (y & 0x0F0F0F0Fu) << 4 | (x & 0x0F0F0F0Fu);
+  y = (x >> 4 & 0x0F0F0F0Fu) | (y & 0xF0F0F0F0u);
+  x = t;
+}
+
+// Eight plane words of 32 codes (word p: bit p of each).
+__device__ __forceinline__ void planes32(const uint4 v0, const uint4 v1, uint32_t (&w)[8]) {
+  uint32_t x[4] = {v0.x, v0.z, v1.x, v1.z}, y[4] = {v0.y, v0.w, v1.y, v1.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) transpose8(x[k], y[k]);
+  // word p of the group: byte p of the four 8-code transposes
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t(&z)[4] = h ? y : x;
+    const uint32_t l01 = __byte_perm(z[0], z[1], 0x5140u), h01 = __byte_perm(z[0], z[1], 0x7362u);
+    const uint32_t l23 = __byte_perm(z[2], z[3], 0x5140u), h23 = __byte_perm(z[2], z[3], 0x7362u);
+    w[4 * h] = __byte_perm(l01, l23, 0x5410u);
+    w[4 * h + 1] = __byte_perm(l01, l23, 0x7632u);
+    w[4 * h + 2] = __byte_perm(h01, h23, 0x5410u);
+    w[4 * h + 3] = __byte_perm(h01, h23, 0x7632u);
   }
+}
+
+// 0xFF in the bytes of x above kLowCodes.
+__device__ __forceinline__ uint32_t above_low(uint32_t x) {
+  const uint32_t hi = (x & 0x80808080u) |
+                      ((x & 0x7F7F7F7Fu) + (0x7Fu - kLowCodes) * 0x01010101u & 0x80808080u);
+  return (hi >> 7) * 0xFFu;
+}
+
+// Register planes of rows [r_lo, r_hi), both sides (blockIdx.y): thread = (row,
+// group of 32 registers), rows_per rows a block.  Registers past mpad count as
+// unset (A 0, B 0xFF).  Whole codes: [row][2][pg] of four planes; low codes (see
+// count_batch_planes): [row] low_stride words, 0 (A) or 63 (B) where a register
+// has no code up to kLowCodes; pflag[row]: bit 0 some code is above it, bit 1 anynz.
+__global__ void __launch_bounds__(256) k_code_planes(const uint4 *__restrict__ A,
+                                                     const uint4 *__restrict__ B, int64_t r_lo,
+                                                     int64_t r_hi, int m16, int pg, int rows_per,
+                                                     uint4 *__restrict__ pA, uint4 *__restrict__ pB,
+                                                     uint32_t *__restrict__ lA,
+                                                     uint32_t *__restrict__ lB,
+                                                     const uint8_t *__restrict__ anynz,
+                                                     uint8_t *__restrict__ pflag) {
+  __shared__ int any[256];
+  const int rl = threadIdx.x / pg, t = threadIdx.x - rl * pg;
+  const int64_t row = r_lo + (int64_t)blockIdx.x * rows_per + rl;
+  const bool side = blockIdx.y != 0;
+  if (threadIdx.x < rows_per) any[threadIdx.x] = 0;
+  __syncthreads();
+  if (rl < rows_per && row < r_hi) {
+    const uint4 *src = (side ? B : A) + row * m16;
+    const uint32_t fill = side ? 0xFFFFFFFFu : 0u;
+    uint4 v0 = __ldg(src + 2 * t);
+    uint4 v1 = 2 * t + 1 < m16 ? __ldg(src + 2 * t + 1) : make_uint4(fill, fill, fill, fill);
+    uint32_t w[8];
+    planes32(v0, v1, w);
+    uint4 *dst = (side ? pB : pA) + row * (2 * pg) + t;
+    dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    dst[pg] = make_uint4(w[4], w[5], w[6], w[7]);
+    const uint32_t none = side ? 0x3F3F3F3Fu : 0u;
+    uint32_t seen = 0;
+    auto low = [&](uint32_t x) {
+      const uint32_t h = above_low(x);
+      seen |= h;
+      return (x & ~h) | (h & none);
+    };
+    v0 = make_uint4(low(v0.x), low(v0.y), low(v0.z), low(v0.w));
+    v1 = make_uint4(low(v1.x), low(v1.y), low(v1.z), low(v1.w));
+    planes32(v0, v1, w);
+    uint32_t *l = (side ? lB : lA) + row * low_stride(pg);
+    reinterpret_cast<uint4 *>(l)[t] = make_uint4(w[0], w[1], w[2], w[3]);
+    reinterpret_cast<uint2 *>(l + 4 * pg)[t] = make_uint2(w[4], w[5]);
+    if (!side && seen) any[rl] = 1;                // A: unset registers are 0
+  }
+  if (side) return;
+  __syncthreads();
+  if (rl < rows_per && row < r_hi && t == 0) pflag[row] = (uint8_t)(any[rl] | (anynz[row] ? 2 : 0));
 }
 
 // Persistent form over a batch: CTAs pull (assembly, row block, slice group)
@@ -1093,27 +1383,51 @@ void launch_merge_topk(const GraphArgs &g, const uint64_t *gbuf, const int32_t *
       g, gbuf, gcnt, cap, P);
 }
 
+size_t low_plane_words(int pg) { return (size_t)low_stride(pg); }
+
+void launch_code_planes(const GraphArgs &g, int64_t r_lo, int64_t r_hi, uint32_t *planesA,
+                        uint32_t *planesB, uint32_t *lowA, uint32_t *lowB, uint8_t *pflag,
+                        cudaStream_t s) {
+  if (r_hi <= r_lo) return;
+  const int rows_per = 256 / g.pg;                 // pg <= 128
+  const int64_t blocks = (r_hi - r_lo + rows_per - 1) / rows_per;
+  k_code_planes<<<dim3((unsigned)blocks, 2), 256, 0, s>>>(
+      (const uint4 *)g.codesA, (const uint4 *)g.codesB, r_lo, r_hi, g.mpad / 16, g.pg, rows_per,
+      (uint4 *)planesA, (uint4 *)planesB, lowA, lowB, g.anynz, pflag);
+}
+
 void launch_sym_check(const GraphArgs &g, const SymOut &o, const uint32_t *cand,
-                      const int64_t *coff, const int32_t *ccnt, int64_t B, cudaStream_t s) {
+                      const int64_t *coff, const int32_t *ccnt, int64_t B, int32_t *seg,
+                      unsigned *next, float *need, int sms, cudaStream_t s) {
   if (g.n == 0 || B <= 0) return;
   float lo, hi, lo16;
   prefilter_bands(g.S, g.prefilter_eps, &lo, &hi, &lo16);
   const int v = allpairs_variant(g);
-  const size_t smem = (size_t)kWarps * kTcWs + (size_t)32 * g.mpad +
+  const size_t smem = (size_t)kWarps * kScWs + (size_t)32 * low_stride(g.pg) * 4 +
                       (size_t)32 * su_stride(g.Su) * 4;
-  // enough CTAs for six per SM: a block pair's list is split over gridDim.y CTAs
-  const int64_t pairs = (B + 1) / 2;
-  const unsigned gy =
-      (unsigned)std::min<int64_t>(4, std::max<int64_t>(1, (6 * 148 + pairs - 1) / pairs));
-  const dim3 grid((unsigned)pairs, gy);
-#define RBG_SC(SM)                                                                        \
-  do {                                                                                    \
-    smem_cap_max((const void *)k_sym_check<SM>);                                          \
-    k_sym_check<SM><<<grid, kWarps * 32, smem, s>>>(g, lo, hi, o, cand, coff, ccnt, B);   \
+  // lanes a survivor: its groups, while a count fits as many bits
+  const int lp = g.pg <= 8 && g.m <= 255 ? 8 : (g.pg <= 16 ? 16 : 32);
+#define RBG_SC(SM, LP)                                                                        \
+  do {                                                                                        \
+    smem_cap_max((const void *)k_sym_check<SM, LP>);                                          \
+    int per_sm = 1;                                                                           \
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sym_check<SM, LP>, kWarps * 32,  \
+                                                  smem);                                      \
+    const int grid = std::max(per_sm, 1) * sms;                                               \
+    k_check_items<<<1, 1024, 0, s>>>(coff, ccnt, B, g.n, grid, seg, need);                    \
+    k_sym_check<SM, LP><<<grid, kWarps * 32, smem, s>>>(g, lo, hi, o, cand, coff, ccnt,       \
+                                                        (int)B, seg, next);                   \
   } while (0)
-  if (v == 1) RBG_SC(16);
-  else if (v == 2) RBG_SC(32);
-  else RBG_SC(64);
+#define RBG_SCL(SM)                                                                           \
+  do {                                                                                        \
+    if (lp == 8) RBG_SC(SM, 8);                                                               \
+    else if (lp == 16) RBG_SC(SM, 16);                                                        \
+    else RBG_SC(SM, 32);                                                                      \
+  } while (0)
+  if (v == 1) RBG_SCL(16);
+  else if (v == 2) RBG_SCL(32);
+  else RBG_SCL(64);
+#undef RBG_SCL
 #undef RBG_SC
 }
 

@@ -123,6 +123,10 @@ struct GraphArgs {
   int m = 500, mpad = 512, S = 0, K = 200;
   int Su = 4;                          // row stride of `unit` (S rounded up to 4)
   const uint8_t *codesA = nullptr, *codesB = nullptr;
+  const uint32_t *planesA = nullptr, *planesB = nullptr;   // register planes [n][2][pg][4]
+  const uint32_t *lowA = nullptr, *lowB = nullptr;     // low-code planes [n][low_plane_words(pg)]
+  const uint8_t *pflag = nullptr;      // [n]: the row holds codes above the low ones
+  int pg = 0;                          // groups of 32 registers: (mpad + 31) / 32
   const float *depth_raw = nullptr;    // [n][S]
   float *unit = nullptr;               // [n][Su] centred + L2-normalised ranks, 0-padded
   uint16_t *unit16 = nullptr;          // [n][Kp] the same rows rounded to FP16 (tensor-core prefilter)
@@ -231,6 +235,7 @@ struct SymOut {
   // similarity bits; launch_rows_topk converts it.  The top-K of all keys cut
   // at the calibrated cutoff equals the top-K of the admitted keys cut there.
   int defer = 0;
+  uint32_t row_base = 0;                // the assembly's first row in the row space (launch_sym_check)
 };
 // Symmetric pass of the abundance-pruned (tensor-core) regime: row maxima into
 // g.maxcnt_cand, admitted pairs into o.  Requires allpairs_variant(g) != 0.
@@ -258,8 +263,18 @@ int launch_sym_prefilter(const GraphArgs &g, const uint16_t *u16p, int64_t cb, i
                          const int32_t *item0, int RB, int NT, int items, uint32_t *cand,
                          const int64_t *coff, int32_t *ccnt, int *overflow, int *err, int sms,
                          cudaStream_t s, const char **why);
+// Register planes of rows [r_lo, r_hi) from g.codesA / codesB (g.pg groups of
+// 32 registers a row): the operands of launch_sym_check.
+size_t low_plane_words(int pg);
+void launch_code_planes(const GraphArgs &g, int64_t r_lo, int64_t r_hi, uint32_t *planesA,
+                        uint32_t *planesB, uint32_t *lowA, uint32_t *lowB, uint8_t *pflag,
+                        cudaStream_t s);
+// Exact check and register compare of the candidate lists of blocks [0, B)
+// (seg: B + 2 words of scratch; next: a counter zeroed before the launch).
+// need: raised to the largest fraction of a block's pairs that were candidates.
 void launch_sym_check(const GraphArgs &g, const SymOut &o, const uint32_t *cand,
-                      const int64_t *coff, const int32_t *ccnt, int64_t blocks, cudaStream_t s);
+                      const int64_t *coff, const int32_t *ccnt, int64_t B, int32_t *seg,
+                      unsigned *next, float *need, int sms, cudaStream_t s);
 float prefilter_lo16(int S, float eps);
 
 // A pair list gathered from several ranks: its per-row key counts (rowcnt

@@ -28,3 +28,34 @@ def test_prefilter_graph(gpu_ctx, orc, G, N, S):
         assert got["b0"] == want["b0"] and got["sim_cutoff"] == want["sim_cutoff"]
         assert np.array_equal(got["src"], ws) and np.array_equal(got["dst"], wd)
         assert np.array_equal(got["scomp"], wsc) and np.array_equal(got["score"], wsw)
+
+
+@pytest.mark.parametrize("m", [17, 250, 255, 256, 500, 700, 1030])
+def test_register_planes(gpu_ctx, orc, m):
+    """Register compares on bit planes: short repeats leave few elements in a
+    contig, so many registers are won by elements of large U (codes above the
+    low planes'); m around the lanes a survivor takes (8, 16, 32) and above
+    32 groups of 32 registers."""
+    rng = np.random.default_rng(m)
+    N = 2600
+    seqs = []
+    for i in range(N):
+        if i % 3 == 0:
+            unit = bytes(rng.choice(list(b"ACGT"), size=1 + i % 7))
+            seqs.append((unit * 400)[:400])
+        else:
+            seqs.append(bytes(rng.choice(list(b"ACGT"), size=300 + i % 200)))
+        if i % 501 == 0:
+            seqs[-1] = b"NN"                      # no registers at all
+    offs = np.zeros(N + 1, np.int64)
+    offs[1:] = np.cumsum([len(s) for s in seqs])
+    buf = b"".join(seqs)
+    depth = rng.poisson(np.exp(rng.normal(2.0, 1.0, size=(4, 10)))[rng.integers(0, 4, N)])
+    depth = depth.astype(np.float32)
+    w = orc.build_winners(buf, offs, m=m)
+    want = orc.run_graph(oracle.default_params(N, m, 10, force_path=2), w, depth)
+    ws, wd, wsc, wsw = oracle.sorted_edges(want)
+    got = gpu_ctx.bin_graph(buf, offs, depth, api.default_params(m=m, force_path=2))
+    assert got["b0"] == want["b0"] and got["sim_cutoff"] == want["sim_cutoff"]
+    assert np.array_equal(got["src"], ws) and np.array_equal(got["dst"], wd)
+    assert np.array_equal(got["scomp"], wsc) and np.array_equal(got["score"], wsw)
