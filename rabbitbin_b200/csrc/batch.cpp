@@ -38,6 +38,10 @@ constexpr int kVariants[4] = {0, 1, 2, 4};
 
 inline int vslot(int v) { return v == 0 ? 0 : (v == 1 ? 1 : (v == 2 ? 2 : 3)); }
 
+// Tuning choice of a pruned assembly: the two-kernel symmetric pass instead of
+// the queue (any other choice is the queue with that pairs-per-item multiplier).
+constexpr double kTwoKernels = 0.0;
+
 struct AsmPlan {
   int orig = 0;
   const rbg_params *p = nullptr;
@@ -46,6 +50,7 @@ struct AsmPlan {
   int S = 0, Su = 4, Kp = 16, m = 500, mpad = 512, K = 200, E = 136;
   bool fused = false, abdfirst = false;
   bool gemm = false;                   // dense regime on the one-hot GEMM (not in the queue)
+  bool tc5 = false;                    // pruned regime on the two-kernel pass (not in the queue)
   double w_comp = 0.0;
   int variant = 0, P = 4, cap = 288;
   // offsets into the batch buffers (elements of each buffer's type)
@@ -252,7 +257,10 @@ void plan_batch(const rbg_params *defaults, const rbg_assembly *asms, int nb, Ba
       const auto it = tune->find(tune_key(a));
       if (it != tune->end()) mult = it->second;
     }
-    a.P = batch_slices(a.n, a.K, a.variant, mult);
+    GraphArgs fit;
+    fit.n = a.n; fit.S = a.S; fit.Kp = a.Kp;
+    a.tc5 = mult == kTwoKernels && a.abdfirst && sym_tc5_fits(fit);
+    a.P = batch_slices(a.n, a.K, a.variant, mult == kTwoKernels ? 1.0 : mult);
     a.cap = allpairs_cap(a.K);
   }
   // group order: equal count configuration, then equal sketch tables
@@ -505,9 +513,25 @@ int launch_sketch_groups(rbg_ctx *c, BatchBufs &B, const BatchPlan &L,
   return launches;
 }
 
+// The two-kernel symmetric pass of the pruned assemblies of positions [bb, be)
+// (of one variant, or all with variant < 0), one after the other on shared
+// scratch (pair records and row counts in the batch's row space).
+int launch_tc5_range(rbg_ctx *c, const BatchPlan &L, const std::vector<BatchAsm> &D, SymOut o,
+                     int bb, int be, int variant = -1) {
+  const int before = c->launches;
+  for (int b = bb; b < be; ++b) {
+    const AsmPlan &a = L.at(b);
+    if (!a.tc5 || (variant >= 0 && a.variant != variant)) continue;
+    o.row_base = (uint32_t)a.row0;
+    sym_tc5_setup(c, D[b].g, 1);
+    sym_tc5_pass(c, D[b].g, o, 0, a.n, 0);
+  }
+  return c->launches - before;
+}
+
 // Depth rows, b0, all-pairs and merge for the whole batch.
-int launch_graph_stage(rbg_ctx *c, BatchBufs &B, const BatchPlan &L, const Lists &W, int nb,
-                       bool timed = false) {
+int launch_graph_stage(rbg_ctx *c, BatchBufs &B, const BatchPlan &L, const Lists &W,
+                       const std::vector<BatchAsm> &D, int nb, bool timed = false) {
   const BatchAsm *dD = B.desc.as<BatchAsm>();
   const int64_t rows1 = std::max<int64_t>(L.rows, 1);
   int launches = 0;
@@ -526,15 +550,18 @@ int launch_graph_stage(rbg_ctx *c, BatchBufs &B, const BatchPlan &L, const Lists
     CK(cudaMemsetAsync(B.sym_rowcnt.p, 0, rows1 * sizeof(int32_t), c->stream));
     CK(cudaMemsetAsync(B.sym_np.p, 0, sizeof(unsigned long long), c->stream));
   }
+  if (L.sym_rows > 0) sym_tc5_clear(c);
   for (int v = 0; v < 4; ++v) {
-    if (W.list[v].empty()) continue;
     if (timed) CK(cudaEventRecord(B.tev[2 * v], c->stream));
-    launch_allpairs_batch(dD, kVariants[v], B.lists.as<int32_t>() + v * (nb + 1),
-                          B.item0s.as<int64_t>() + v * (nb + 1), (int)W.list[v].size(),
-                          W.item0[v].back(), W.smem[v], B.queues.as<unsigned long long>() + v,
-                          o, c->stream);
+    if (!W.list[v].empty()) {
+      launch_allpairs_batch(dD, kVariants[v], B.lists.as<int32_t>() + v * (nb + 1),
+                            B.item0s.as<int64_t>() + v * (nb + 1), (int)W.list[v].size(),
+                            W.item0[v].back(), W.smem[v], B.queues.as<unsigned long long>() + v,
+                            o, c->stream);
+      ++launches;
+    }
+    if (v > 0) launches += launch_tc5_range(c, L, D, o, 0, nb, kVariants[v]);
     if (timed) CK(cudaEventRecord(B.tev[2 * v + 1], c->stream));
-    ++launches;
   }
   if (!W.list[0].empty()) {
     launch_merge_batch(dD, B.row0s.as<int64_t>(), nb, L.rows, c->stream);
@@ -597,6 +624,21 @@ Lists sub_lists(const Lists &W, int bb, int be) {
   return R;
 }
 
+// The passes' flags after their synchronisation: a kept fraction per S with room
+// to spare for the next lists; false when a list overflowed.
+bool tc5_batch_settle(rbg_ctx *c) {
+  const int *fl = c->tc5_host.as<int>();
+  if (fl[1] != 0)
+    throw Error(RBG_ERR_TIMEOUT, "tensor-core prefilter: a bounded device wait gave up (stage " +
+                                     std::to_string(fl[1]) + ")");
+  for (size_t S = 0; S < c->tc5_frac.size(); ++S) {
+    float need;
+    std::memcpy(&need, fl + 2 + S, sizeof(need));
+    c->tc5_frac[S] = std::max(c->tc5_frac[S], 1.25 * (double)need);
+  }
+  return fl[0] == 0;
+}
+
 // Device descriptors of the batch positions and the per-variant work lists.
 void build_items(BatchBufs &B, const BatchPlan &L, int nb, std::vector<BatchAsm> &D, Lists &W) {
   D.assign(nb, BatchAsm());
@@ -604,7 +646,7 @@ void build_items(BatchBufs &B, const BatchPlan &L, int nb, std::vector<BatchAsm>
   for (int b = 0; b < nb; ++b) {
     const AsmPlan &a = L.at(b);
     D[b] = describe(B, a, b);
-    if (a.n > 0 && !a.gemm) {
+    if (a.n > 0 && !a.gemm && !a.tc5) {
       const int vs = vslot(a.variant);
       if (W.item0[vs].empty()) W.item0[vs].push_back(0);
       W.list[vs].push_back(b);
@@ -615,9 +657,10 @@ void build_items(BatchBufs &B, const BatchPlan &L, int nb, std::vector<BatchAsm>
 }
 
 // Autotuner.  For keys (variant, m, log2 n) of this batch it has no choice for,
-// the graph stage runs again with the pairs-per-item target at 1x, 1/4 and 4x
-// the rule's (outside the CUDA graphs), each variant's persistent launch timed
-// by events; the fastest multiplier per variant becomes the choice for
+// the graph stage runs again (outside the CUDA graphs) with the two-kernel pass
+// of the pruned assemblies, then with the queue at 1x, 1/4 and 4x the rule's
+// pairs per item, each variant's part timed by events; the fastest choice per
+// variant becomes the choice for
 // the batch's untuned keys of that variant.  The runs recompute the same
 // values (top-K sets and maxima do not depend on the tiling).
 int autotune_batch(rbg_ctx *c, BatchBufs &B, const rbg_params *defaults,
@@ -631,11 +674,11 @@ int autotune_batch(rbg_ctx *c, BatchBufs &B, const rbg_params *defaults,
     if (std::find(fresh.begin(), fresh.end(), k) == fresh.end()) fresh.push_back(k);
   }
   if (fresh.empty()) return 0;
-  const double mults[3] = {1.0, 0.25, 4.0};
-  float t[3][4];
+  const double mults[4] = {kTwoKernels, 1.0, 0.25, 4.0};
+  float t[4][4];
   for (auto &e : B.tev)
     if (!e) CK(cudaEventCreate(&e));
-  for (int ci = 0; ci < 3; ++ci) {
+  for (int ci = 0; ci < 4; ++ci) {
     BatchPlan L;
     plan_batch(defaults, asms, nb, L, &B.tune, mults[ci]);
     ensure_buffers(B, L, nb);
@@ -654,17 +697,16 @@ int autotune_batch(rbg_ctx *c, BatchBufs &B, const rbg_params *defaults,
                        cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(B.item0s.p, item0s.data(), item0s.size() * sizeof(int64_t),
                        cudaMemcpyHostToDevice, c->stream));
-    launch_graph_stage(c, B, L, W, nb, true);
+    launch_graph_stage(c, B, L, W, D, nb, true);
     CK(cudaStreamSynchronize(c->stream));
     for (int v = 0; v < 4; ++v) {
-      t[ci][v] = 0.f;
-      if (!W.list[v].empty()) CK(cudaEventElapsedTime(&t[ci][v], B.tev[2 * v], B.tev[2 * v + 1]));
+      CK(cudaEventElapsedTime(&t[ci][v], B.tev[2 * v], B.tev[2 * v + 1]));
     }
   }
   double best[4];
   for (int v = 0; v < 4; ++v) {
     int bi = 0;
-    for (int ci = 1; ci < 3; ++ci)
+    for (int ci = 1; ci < 4; ++ci)
       if (t[ci][v] < t[bi][v]) bi = ci;
     best[v] = mults[bi];
   }
@@ -691,7 +733,7 @@ void run_batch(rbg_ctx *c, const rbg_params *defaults, const rbg_assembly *asms,
   const bool use_graph = getenv("RBG_NO_GRAPHS") == nullptr;
 
   BatchPlan L;
-  plan_batch(defaults, asms, nb, L, &B.tune, 1.0);
+  plan_batch(defaults, asms, nb, L, &B.tune, kTwoKernels);
   const int64_t rows = L.rows, rows1 = std::max<int64_t>(rows, 1);
   stats.rows = rows;
   stats.pairs = L.pairs_scored;
@@ -786,6 +828,12 @@ void run_batch(rbg_ctx *c, const rbg_params *defaults, const rbg_assembly *asms,
     CK(cudaMemsetAsync(B.sym_rowcnt.p, 0, rows1 * sizeof(int32_t), c->stream));
     CK(cudaMemsetAsync(B.sym_np.p, 0, sizeof(unsigned long long), c->stream));
   }
+  bool any_tc5 = false;
+  for (int b = 0; b < nb; ++b) any_tc5 |= L.at(b).tc5;
+  if (any_tc5) {
+    sym_tc5_clear(c);
+    c->tc5_host.ensure(kTc5Flags * sizeof(int));
+  }
   int launches = 0;
   {
     CK(cudaEventRecord(c->ev_cin, c->stream));             // earlier work on the buffers is done
@@ -820,8 +868,10 @@ void run_batch(rbg_ctx *c, const rbg_params *defaults, const rbg_assembly *asms,
       launches += launch_graph_run(c, B, L, Wr[r], nb, runcut[r], runcut[r + 1],
                                    B.lists.as<int32_t>() + base, B.item0s.as<int64_t>() + base,
                                    B.queues.as<unsigned long long>() + (size_t)(r + 1) * 4);
-      // dense assemblies of the run: one-hot GEMM and row scan each, on the
-      // b0 and similarity tables just computed
+      // pruned assemblies of the run: the two-kernel symmetric pass each; dense
+      // ones: one-hot GEMM and row scan each, on the b0 and similarity tables
+      // just computed
+      if (any_tc5) launches += launch_tc5_range(c, L, D, sym_out(B), runcut[r], runcut[r + 1]);
       for (int b = runcut[r]; b < runcut[r + 1]; ++b)
         if (L.at(b).gemm && L.at(b).n > 0) {
           dense_allpairs_onehot(c, D[b].g);
@@ -848,7 +898,7 @@ void run_batch(rbg_ctx *c, const rbg_params *defaults, const rbg_assembly *asms,
     reran = !first;
     captured(c, 0, use_graph && first, stats.graph_launches, [&] {
       if (!first) {
-        launches += launch_graph_stage(c, B, L, W, nb);
+        launches += launch_graph_stage(c, B, L, W, D, nb);
       } else if (L.sym_rows > 0) {
         launch_rows_topk_batch(B.desc.as<BatchAsm>(), B.row0s.as<int64_t>(), nb, rows, sym_out(B),
                                B.sym_rowoff.as<int64_t>(), B.sym_keys.as<uint64_t>(), c->stream);
@@ -864,11 +914,16 @@ void run_batch(rbg_ctx *c, const rbg_params *defaults, const rbg_assembly *asms,
       if (L.sym_rows > 0)
         CK(cudaMemcpyAsync(h_np, B.sym_np.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                            c->stream));
+      if (any_tc5)
+        CK(cudaMemcpyAsync(c->tc5_host.p, c->tc5_flags.p, kTc5Flags * sizeof(int),
+                           cudaMemcpyDeviceToHost, c->stream));
     });
     CK(cudaEventRecord(ev2, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     check_onehot_status(c);
-    if (L.sym_rows == 0 || *h_np <= B.sym_cap) break;
+    const bool lists_ok = !any_tc5 || tc5_batch_settle(c);
+    if (lists_ok && (L.sym_rows == 0 || *h_np <= B.sym_cap)) break;
+    if (*h_np <= B.sym_cap) continue;
     B.sym_cap = *h_np + *h_np / 4;
     B.sym_pairs.ensure(B.sym_cap * sizeof(uint4));
     B.sym_keys.ensure(2 * B.sym_cap * sizeof(uint64_t));
