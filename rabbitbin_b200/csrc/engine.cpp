@@ -237,20 +237,24 @@ void sym_clear(rbg_ctx *c, int64_t n1);
 // in [c0, c1) are scored (rows [0, c1)), with admission deferred until b0 is
 // known (run_graph finishes the selection).
 void stage_sketch_chunked(rbg_ctx *c, const rbg_params *p, const char *seqcat,
-                          const int64_t *offsets, int64_t n, const float *depth, int S) {
+                          const int64_t *offsets, int64_t n, const float *depth, int S,
+                          bool want_winners = false) {
   stage_meta(c, seqcat, offsets, n, depth, S);
-  const SketchArgs all = sketch_setup(c, p, false);
+  const SketchArgs all = sketch_setup(c, p, want_winners);
   const int64_t nb = c->nbases, nwords = (nb + 15) / 16;
   const int E = all.n_elems, mpad = all.mpad;
   CK(cudaEventRecord(c->ev[0], c->stream));
   prep_depth(c, p);
   CK(cudaEventRecord(c->ev_cin, c->stream));             // the buffers are free to overwrite
   CK(cudaStreamWaitEvent(c->copy, c->ev_cin, 0));
-  const int G = nwords >= ((int64_t)kChunks << 16) ? kChunks : 1;
+  // Chunks of at least 4 MB: a chunk's kernels take about 60 us however small it
+  // is, which 4 MB on the bus (75 us) just hide (16.7 MB in eight chunks: 1.04 ms
+  // a call, in four 0.88 ms).
+  const int G = (int)std::max<int64_t>(1, std::min<int64_t>(kChunks, nb >> 22));
   // Streaming keeps every survivor of the prune until b0 is known; with few
   // samples the prune passes a large share of the pairs, so it streams from
   // S >= 10, and never again at an S whose survivors outgrew the list.
-  const bool stream_pairs = G > 1 && S >= 10 && sym_regime(p, n, S) &&
+  const bool stream_pairs = G > 1 && S >= 10 && !want_winners && sym_regime(p, n, S) &&
                             !((c->no_stream_S >> (S & 63)) & 1u);
   GraphArgs ga;
   SymOut o;
