@@ -412,6 +412,13 @@ int rbg_fetch_graph(rbg_ctx *ctx, rbg_graph *out);
 
 int rbg_free_graph(rbg_graph *g);
 
+/* Pinned host memory for results, from the pool that the graphs' arrays come
+ * from: a call that writes its output there skips the driver's staging of
+ * pageable memory and a fresh array's page faults.  NULL when it cannot be had
+ * (use any memory then); release with rbg_result_free. */
+void *rbg_result_alloc(size_t bytes);
+void rbg_result_free(void *p);
+
 /* rbg_build_pmh_winners for callers that cannot allocate device memory (a host
  * framework that owns the device heap through its own pool, a plugin inside
  * another process's CUDA context with a fixed budget, a caller that must not

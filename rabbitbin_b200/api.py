@@ -304,6 +304,8 @@ def lib():
         "rbg_run_resident": ([vp, P(Params), P(Timing)], C.c_int),
         "rbg_fetch_graph": ([vp, P(Graph)], C.c_int),
         "rbg_free_graph": ([P(Graph)], C.c_int),
+        "rbg_result_alloc": ([C.c_size_t], vp),
+        "rbg_result_free": ([vp], None),
         "rbg_pmh_stream_tables": ([C.c_int32, C.c_int32, C.c_uint64, C.c_int32,
                                    P(C.c_int32), P(C.c_int32), P(C.c_double),
                                    P(C.c_uint32)], C.c_int),
@@ -417,6 +419,33 @@ class _View:
                                     "data": (addr, False), "version": 3}
 
 
+class _ResultMem:
+    """Owns one block of rbg_result_alloc and describes it as an array."""
+
+    def __init__(self, L, addr, shape, typestr):
+        self._L, self._addr = L, addr
+        self.__array_interface__ = {"shape": shape, "typestr": typestr,
+                                    "data": (addr, False), "version": 3}
+
+    def __del__(self):
+        try:
+            self._L.rbg_result_free(self._addr)
+        except Exception:
+            pass
+
+
+def _result(L, shape, dtype):
+    """An output array that the call fills completely: pinned memory of the
+    library's pool from 1 MB on (the device writes it at bus speed)."""
+    dt = np.dtype(dtype)
+    nbytes = int(np.prod(shape, dtype=np.int64)) * dt.itemsize
+    if nbytes >= 1 << 20:
+        addr = L.rbg_result_alloc(nbytes)
+        if addr:
+            return np.asarray(_ResultMem(L, addr, tuple(shape), dt.str))
+    return np.zeros(shape, dt)
+
+
 def _graph_dict(L, g):
     """The graph's arrays as numpy views of the library's buffers (no copy);
     the buffers are released with rbg_free_graph when the views are gone."""
@@ -468,7 +497,7 @@ class Context:
         p = params or default_params()
         offs = np.ascontiguousarray(offsets, np.int64)
         n = len(offs) - 1
-        out = np.zeros((n, p.m), np.uint32)
+        out = _result(self._L, (n, p.m), np.uint32)
         self._check(self._L.rbg_build_pmh_winners(self._h, C.byref(p), seqcat, _p(offs, C.c_int64),
                                                   n, _p(out, C.c_uint32)), "build_pmh_winners")
         return out
@@ -479,8 +508,8 @@ class Context:
         p = params or default_params()
         offs = np.ascontiguousarray(offsets, np.int64)
         n = len(offs) - 1
-        w = np.zeros((n, p.m), np.uint64)
-        r = np.zeros((n, p.m), np.float64)
+        w = _result(self._L, (n, p.m), np.uint64)
+        r = _result(self._L, (n, p.m), np.float64)
         self._check(self._L.rbg_build_pmh_sketches(self._h, C.byref(p), seqcat,
                                                    _p(offs, C.c_int64), n, _p(w, C.c_uint64),
                                                    _p(r, C.c_double)), "build_pmh_sketches")
@@ -495,7 +524,7 @@ class Context:
         dt = np.uint64 if code == 0 else np.float64
         A = np.ascontiguousarray(A, dt)
         B = np.ascontiguousarray(B, dt)
-        out = np.zeros((A.shape[0], B.shape[0]), np.float64)
+        out = _result(self._L, (A.shape[0], B.shape[0]), np.float64)
         self._check(self._L.rbg_pmh_compare(self._h, code, A.shape[1], kmer_size,
                                             A.ctypes.data, A.shape[0], B.ctypes.data,
                                             B.shape[0], _p(out, C.c_double)), "pmh_compare")
@@ -504,7 +533,7 @@ class Context:
     def pmh_merge_registers(self, A, B):
         A = np.ascontiguousarray(A, np.float64)
         B = np.ascontiguousarray(B, np.float64)
-        out = np.zeros_like(A)
+        out = _result(self._L, A.shape, np.float64)
         self._check(self._L.rbg_pmh_merge_registers(self._h, _p(A, C.c_double), _p(B, C.c_double),
                                                     A.shape[0], A.shape[1], _p(out, C.c_double)),
                     "pmh_merge_registers")

@@ -317,6 +317,7 @@ void stage_sketch_chunked(rbg_ctx *c, const rbg_params *p, const char *seqcat,
       if (a.elem_cnt) a.elem_cnt += c0;
       a.codesA += c0 * mpad;
       a.codesB += c0 * mpad;
+      if (a.winners32) a.winners32 += c0 * all.m;
       sketch_contigs(c, p, a, nullptr);
       if (stream_pairs) {
         if (tc5) {
@@ -1191,6 +1192,51 @@ PinnedPool &pinned_pool() {
 
 namespace rbg {
 
+namespace {
+constexpr size_t kBounce = (size_t)8 << 20;
+
+// Whether a copy of `bytes` at p goes through the pinned slots.
+bool bounced(const void *p, size_t bytes) {
+  if (bytes < ((size_t)1 << 20)) return false;
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeUnregistered;
+}
+
+// Slot k, its last copy done.
+char *bounce_slot(rbg_ctx *c, int k) {
+  c->bounce[k].ensure(kBounce);
+  if (!c->ev_bounce[k]) CK(cudaEventCreateWithFlags(&c->ev_bounce[k], cudaEventDisableTiming));
+  else CK(cudaEventSynchronize(c->ev_bounce[k]));
+  return c->bounce[k].as<char>();
+}
+}  // namespace
+
+void copy_out(rbg_ctx *c, void *dst, const void *src, size_t bytes, cudaStream_t s) {
+  if (bytes == 0) return;
+  if (!bounced(dst, bytes)) {
+    CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    return;
+  }
+  const size_t pieces = (bytes + kBounce - 1) / kBounce;
+  for (size_t i = 0; i <= pieces; ++i) {
+    if (i < pieces) {                       // piece i into its slot, emptied two pieces ago
+      const size_t at = i * kBounce, len = std::min(kBounce, bytes - at);
+      char *slot = bounce_slot(c, (int)(i & 1));
+      CK(cudaMemcpyAsync(slot, (const char *)src + at, len, cudaMemcpyDeviceToHost, s));
+      CK(cudaEventRecord(c->ev_bounce[i & 1], s));
+    }
+    if (i > 0) {                            // piece i - 1 out
+      const size_t at = (i - 1) * kBounce, len = std::min(kBounce, bytes - at);
+      host_copy((char *)dst + at, bounce_slot(c, (int)((i - 1) & 1)), len);
+    }
+  }
+}
+
 void *pinned_take(size_t bytes) { return pinned_pool().take(bytes); }
 void pinned_share(void *blk, const std::vector<void *> &firsts) {
   pinned_pool().share(blk, firsts);
@@ -1394,6 +1440,21 @@ void bin_graph_one(rbg_ctx *c, const rbg_params *p, const rbg_assembly &x, rbg_g
 
 extern "C" {
 
+void *rbg_result_alloc(size_t bytes) {
+  try {
+    return bytes ? pinned_pool().take(bytes) : nullptr;
+  } catch (...) {
+    return nullptr;
+  }
+}
+
+void rbg_result_free(void *p) {
+  try {
+    if (p) pinned_pool().give(p);
+  } catch (...) {
+  }
+}
+
 int rbg_default_params(rbg_params *p) {
   if (!p) return RBG_ERR_ARG;
   std::memset(p, 0, sizeof(*p));
@@ -1500,6 +1561,10 @@ int rbg_destroy(rbg_ctx *c) {
   for (cudaEvent_t e : {c->ev_in, c->ev_aux, c->ev_a0, c->ev_a1, c->ev_cin}) cudaEventDestroy(e);
   for (auto &e : c->ev_chunk) cudaEventDestroy(e);
   for (auto &e : c->ev_slot) cudaEventDestroy(e);
+  c->bounce[0].release();
+  c->bounce[1].release();
+  for (auto &e : c->ev_bounce)
+    if (e) cudaEventDestroy(e);
   c->pack_pin[0].release();
   c->pack_pin[1].release();
   c->tc5_pin.release();
@@ -1520,10 +1585,10 @@ int rbg_build_pmh_winners(rbg_ctx *c, const rbg_params *p, const char *seqcat,
   return guarded(c, [&] {
     validate(p);
     if (!out && n > 0) throw Error(RBG_ERR_ARG, "null output");
-    stage(c, seqcat, offsets, n, nullptr, 0);
-    run_sketch(c, p, true);
+    stage_sketch_chunked(c, p, seqcat, offsets, n, nullptr, 0, true);
     c->prep_done = false;
-    if (n) CK(cudaMemcpyAsync(out, c->winners32.p, (size_t)n * p->m * 4, cudaMemcpyDeviceToHost, c->stream));
+    copy_out(c, out, c->winners32.p, (size_t)n * p->m * 4, c->stream);
+    CK(cudaStreamSynchronize(c->copy));
     CK(cudaStreamSynchronize(c->stream));
   });
 }
@@ -1742,8 +1807,8 @@ int rbg_build_pmh_sketches(rbg_ctx *c, const rbg_params *p, const char *seqcat,
       launch_pmh_rows(c->tmp.as<uint8_t>(), c->elem_winv.as<double>(), n, m, T.t->n_elems,
                       T.W64.as<uint64_t>(), T.U.as<double>(), dw, dr, c->stream);
       CK(cudaGetLastError());
-      if (dw) CK(cudaMemcpyAsync(out_winners64, dw, cells * 8, cudaMemcpyDeviceToHost, c->stream));
-      if (dr) CK(cudaMemcpyAsync(out_registers, dr, cells * 8, cudaMemcpyDeviceToHost, c->stream));
+      if (dw) copy_out(c, out_winners64, dw, cells * 8, c->stream);
+      if (dr) copy_out(c, out_registers, dr, cells * 8, c->stream);
     }
     CK(cudaStreamSynchronize(c->stream));
   });
@@ -1799,9 +1864,7 @@ int rbg_pmh_compare(rbg_ctx *c, int32_t metric, int32_t m, int32_t kmer_size, co
       launch_pmh_compare(c->qa.as<uint64_t>(), ra, c->qb.as<uint64_t>(), nb, m, regs,
                          c->qt.as<double>(), c->qo.as<double>(), c->stream);
       CK(cudaGetLastError());
-      CK(cudaMemcpyAsync(out + (size_t)a0 * nb, c->qo.p, (size_t)ra * nb * sizeof(double),
-                         cudaMemcpyDeviceToHost, c->stream));
-      CK(cudaStreamSynchronize(c->stream));
+      copy_out(c, out + (size_t)a0 * nb, c->qo.p, (size_t)ra * nb * sizeof(double), c->stream);
     }
   });
 }
@@ -1821,8 +1884,7 @@ int rbg_pmh_merge_registers(rbg_ctx *c, const double *A, const double *B, int64_
     launch_pmh_merge(c->qa.as<double>(), c->qb.as<double>(), (int64_t)n * m, c->qo.as<double>(),
                      c->stream);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(out, c->qo.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    copy_out(c, out, c->qo.p, bytes, c->stream);
   });
 }
 

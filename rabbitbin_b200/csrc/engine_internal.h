@@ -87,6 +87,19 @@ struct HBuf {
   }
 };
 
+// memcpy split over the library's host threads.
+void host_copy(void *dst, const void *src, size_t bytes);
+
+// Copy of a device result to the caller's memory on stream s, complete on
+// return.  Pinned (or small) memory directly.  The driver moves a pageable
+// destination through a staging buffer on one thread, which also takes a fresh
+// destination's page faults (40 MB: 8.2 ms with huge pages, 18 ms without);
+// here 8 MB pieces land in the context's two pinned slots and the host threads
+// empty one while the other is on the bus (3.0 ms).  The other direction stays
+// with the driver: the bus reads a slot that many cores have just written at
+// 5 GB/s, the driver's own staging at 20.
+void copy_out(rbg_ctx *c, void *dst, const void *src, size_t bytes, cudaStream_t s);
+
 inline int mpad_of(int m) { return (m + 15) & ~15; }
 
 // Chunks of the host-to-device copy that rbg_bin_graph overlaps with the sketch.
@@ -366,6 +379,8 @@ struct rbg_ctx {
   // symmetric pass on the tensor-core prefilter: candidate lists per 32-row
   // block (capacities tc5_cap, sized from the kept fractions tc5_frac)
   rbg::DBuf tc5_u16p, tc5_cand, tc5_cnt, tc5_items, tc5_coff, tc5_caps, tc5_flags;
+  rbg::HBuf bounce[2];                  // pinned slots of copy_out
+  cudaEvent_t ev_bounce[2] = {nullptr, nullptr};
   rbg::DBuf planesA, planesB, lowA, lowB, pflag, tc5_seg;   // register planes, check items
   rbg::HBuf tc5_pin, tc5_host;
   std::vector<int64_t> tc5_cap;

@@ -167,6 +167,22 @@ Pool &pool() {
 
 int host_pack_threads() { return pool().size(); }
 
+void host_copy(void *dst, const void *src, size_t bytes) {
+  // about 256 KB a part: shorter ones cost more in waking threads than they move
+  const int parts = (int)std::min<size_t>(pool().size(), std::max<size_t>(1, bytes >> 18));
+  if (parts == 1) {
+    std::memcpy(dst, src, bytes);
+    return;
+  }
+  pool().run(
+      [&](int part) {
+        const size_t a = bytes * part / parts & ~(size_t)63;
+        const size_t b = part + 1 == parts ? bytes : bytes * (part + 1) / parts & ~(size_t)63;
+        std::memcpy((char *)dst + a, (const char *)src + a, b - a);
+      },
+      parts);
+}
+
 void host_pack_words(const char *ascii, int64_t nbases, int64_t w0, int64_t w1,
                      uint32_t *packed, uint32_t *mask) {
   // word pairs [w0, w1) rounded up to an even count; w0 is even
