@@ -14,9 +14,9 @@
 // given in the same round.  Here every warp claims the next position of the
 // order (one atomic counter, so positions are claimed in order by running
 // warps), waits until each neighbour that comes earlier in the order has been
-// visited in this round (a per-node round stamp, published with release
-// semantics after the node's writes), and then decides exactly as the
-// sequential loop would: the labels of earlier neighbours are final for the
+// visited in this round (a per-node round stamp in one 64-bit word with the
+// label: one load an arc gives both, and no fence orders them), and then
+// decides exactly as the sequential loop would: the labels of earlier neighbours are final for the
 // round, those of later neighbours still hold the previous round's value
 // (a later neighbour waits for this node before it writes).  Waiting only on
 // positions that were claimed before cannot deadlock: the earliest unfinished
@@ -58,8 +58,8 @@ constexpr int kLpaWarps = 8;                  // warps per CTA of the sweep kern
 constexpr int kTabSlots = 512;                // shared hash slots per warp
 constexpr int kTabMaxDeg = 256;               // arcs above which a node takes the general path
 // per-warp shared region: scores, keys, counts, first-appearance list, then the
-// arc stage (neighbour / label and quantity per arc, later the label score
-// intervals), then a 32-float exchange buffer of the general path
+// arc stage (neighbour / label, and quantity as a double, per arc, later the label
+// score intervals), then a 32-float exchange buffer of the general path
 constexpr int kWarpSmem = kTabSlots * 16 + kTabMaxDeg * 4 + kTabMaxDeg * 16 + 32 * 4;
 constexpr int kVisitPer = 14;                 // labels per visited-set block
 constexpr uint64_t kWaitNs = 5000000000ull;   // bound of one wait
@@ -69,11 +69,6 @@ __device__ __forceinline__ uint64_t now_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t *p) {
   uint32_t v;
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -82,10 +77,14 @@ __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t *p) {
 __device__ __forceinline__ void st_relaxed(uint32_t *p, uint32_t v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ void st_release(uint32_t *p, uint32_t v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ uint64_t ld_relaxed64(const uint64_t *p) {
+  uint64_t v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
 }
-__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ void st_relaxed64(uint64_t *p, uint64_t v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 // State that other launches wrote (labels, flags, visited sets, proposals) is
 // read at the L2, never from a line an SM's L1 may still hold from an earlier
 // round: ld.global.cg.
@@ -120,11 +119,11 @@ __device__ double lpa_combine(int rule, int m, double acc) {
     default: return acc;                                  // sum, max
   }
 }
-__device__ __forceinline__ void lpa_accumulate(int rule, double &dst, float x) {
+__device__ __forceinline__ void lpa_accumulate(int rule, double &dst, double x) {
   if (rule == RBG_LPA_MAX) {
-    if ((double)x > dst) dst = (double)x;
+    if (x > dst) dst = x;
   } else {
-    dst = dd::add(dst, (double)x);
+    dst = dd::add(dst, x);
   }
 }
 
@@ -321,7 +320,7 @@ __global__ void __launch_bounds__(256) k_lpa_sort(const int64_t *__restrict__ of
 __global__ void k_lpa_init(const uint32_t *__restrict__ order, int64_t n, uint32_t *__restrict__ pos,
                            uint32_t *__restrict__ label, uint8_t *__restrict__ active,
                            uint8_t *__restrict__ next_active, uint8_t *__restrict__ frozen,
-                           uint32_t *__restrict__ done, uint32_t *__restrict__ vcnt,
+                           uint64_t *__restrict__ state, uint32_t *__restrict__ vcnt,
                            uint32_t *__restrict__ vnext) {
   for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n;
        p += (int64_t)gridDim.x * blockDim.x) {
@@ -330,10 +329,18 @@ __global__ void k_lpa_init(const uint32_t *__restrict__ order, int64_t n, uint32
     active[p] = 1;
     next_active[p] = 0;
     frozen[p] = 0;
-    done[p] = 0;
+    state[p] = (uint64_t)p;
     vcnt[p] = 0;
     vnext[p] = kEmpty;
   }
+}
+
+// Labels of the Gauss-Seidel state words.
+__global__ void k_lpa_labels(const uint64_t *__restrict__ state, int64_t n,
+                             uint32_t *__restrict__ label) {
+  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
+       v += (int64_t)gridDim.x * blockDim.x)
+    label[v] = (uint32_t)state[v];
 }
 
 // Per arc: does the neighbour come earlier in the node order than the node?
@@ -363,7 +370,9 @@ struct Sweep {
   const uint4 *rec;               // per position: node, degree, first arc (low, high)
   uint32_t *label;
   uint8_t *active, *next_active, *frozen;
-  uint32_t *done;                 // round of a node's last visit (Gauss-Seidel)
+  // Gauss-Seidel: stamp of the node's last visit << 32 | its label, written as
+  // one word, so that a reader that sees the stamp has the label with it
+  uint64_t *state;
   uint32_t *prop;                 // proposals (synchronous)
   // visited sets: block v belongs to node v; vcnt[v] labels, spill blocks
   // chained from vnext[v] (kEmpty: none) out of the pool above n
@@ -418,8 +427,8 @@ __device__ __forceinline__ int table_find(Table &T, uint32_t L, bool *fresh) {
 
 // Label scores of v's arcs [a0, a1) and the decision of rb_cluster.cpp:532-553:
 // returns the chosen label (cur when the list is empty, *touched false then).
-__device__ uint32_t decide(const Sweep &S, Table &T, float *wb, uint32_t v, int64_t a0,
-                           int64_t a1, uint32_t cur, bool *touched) {
+__device__ uint32_t decide(const Sweep &S, Table &T, float *wb, int64_t a0, int64_t a1,
+                           uint32_t cur, bool sequential, bool *touched) {
   const int lane = threadIdx.x & 31;
   int nlist = 0;
   for (int64_t c = a0; c < a1; c += 32) {
@@ -427,7 +436,8 @@ __device__ uint32_t decide(const Sweep &S, Table &T, float *wb, uint32_t v, int6
     const bool valid = a < a1;
     uint32_t L = kEmpty;
     if (valid) {
-      L = ld_relaxed(S.label + __ldg(S.nbr + a));
+      const uint32_t u = __ldg(S.nbr + a);
+      L = sequential ? (uint32_t)ld_relaxed64(S.state + u) : ld_relaxed(S.label + u);
       wb[lane] = __ldg(S.w + a);
     }
     __syncwarp();
@@ -438,7 +448,7 @@ __device__ uint32_t decide(const Sweep &S, Table &T, float *wb, uint32_t v, int6
     if (lead) {
       slot = table_find(T, L, &fresh);
       double s = T.score[slot];
-      for (uint32_t g = grp; g; g &= g - 1) lpa_accumulate(S.rule, s, wb[__ffs(g) - 1]);
+      for (uint32_t g = grp; g; g &= g - 1) lpa_accumulate(S.rule, s, (double)wb[__ffs(g) - 1]);
       T.score[slot] = s;
       T.cnt[slot] += __popc(grp);
     }
@@ -489,12 +499,14 @@ __device__ uint32_t decide(const Sweep &S, Table &T, float *wb, uint32_t v, int6
 }
 
 // Applies a change of v from kprev to best (rb_cluster.cpp:565-582 and
-// :685-708): label, counters, neighbours' activation marks, visited set and
-// freeze.  Called by the whole warp.
-// Marks go to next_active, which no one reads before the next round: in the
-// synchronous sweep every neighbour, in the sequential one only the neighbours
-// already visited in this round (and the node itself on a self-loop) -- the
-// later ones learn of the change from the stamp within this round.
+// :685-708): label (the sequential sweep has published it already), counters,
+// neighbours' activation marks, visited set and freeze.  Called by the whole
+// warp.  Nothing written here is read before the next round: marks go to
+// next_active, and the visited set and freeze flag are read at v's next visit.
+// In the synchronous sweep every neighbour is marked, in the sequential one only
+// the neighbours already visited in this round (and the node itself on a
+// self-loop) -- the later ones learn of the change from the stamp within this
+// round.
 __device__ void commit(const Sweep &S, uint32_t v, uint32_t kprev, uint32_t best, int64_t a0,
                        int64_t a1, bool sequential) {
   const int lane = threadIdx.x & 31;
@@ -503,43 +515,46 @@ __device__ void commit(const Sweep &S, uint32_t v, uint32_t kprev, uint32_t best
     if (!sequential || __ldg(S.early + a) || u == v) S.next_active[u] = 1;
   }
   if (lane == 0) {
-    st_relaxed(S.label + v, best);
+    if (!sequential) st_relaxed(S.label + v, best);
     atomicAdd(S.counts, 1ull);
-    // visited set: {kprev} on the first change, then best; a label seen before freezes v
-    uint32_t *blk = S.vlab + (size_t)v * kVisitPer;
-    uint32_t *cntp = S.vcnt + v, *nextp = S.vnext + v;
-    if (ld_cg(S.vcnt + v) == 0) {
-      blk[0] = kprev;
-      S.vcnt[v] = 1;
-    }
-    bool seen = false;
-    uint32_t c = 0;
-    for (;;) {
-      c = ld_cg(cntp);
-      for (uint32_t i = 0; i < c && !seen; ++i) seen = ld_cg(blk + i) == best;
-      const uint32_t b = ld_cg(nextp);
-      if (seen || b == kEmpty) break;
-      blk = S.vlab + (size_t)b * kVisitPer;
-      cntp = S.vcnt + b;
-      nextp = S.vnext + b;
-    }
-    if (seen) {
-      S.frozen[v] = 1;
-      atomicAdd(S.counts + 1, 1ull);
-    } else if (c < (uint32_t)kVisitPer) {
-      blk[c] = best;
-      *cntp = c + 1;
+  }
+  // visited set: {kprev, best} on the first change, then best; a label seen
+  // before freezes v
+  uint32_t *blk = S.vlab + (size_t)v * kVisitPer;
+  uint32_t *cntp = S.vcnt + v, *nextp = S.vnext + v;
+  uint32_t c = ld_cg(cntp);
+  if (c == 0) {
+    if (lane < 2) blk[lane] = lane ? best : kprev;
+    if (lane == 0) *cntp = 2;
+    return;
+  }
+  bool seen = false;
+  for (;;) {
+    const uint32_t nx = ld_cg(nextp);
+    seen = __any_sync(FULL, lane < (int)c && ld_cg(blk + lane) == best);
+    if (seen || nx == kEmpty) break;
+    blk = S.vlab + (size_t)nx * kVisitPer;
+    cntp = S.vcnt + nx;
+    nextp = S.vnext + nx;
+    c = ld_cg(cntp);
+  }
+  if (lane != 0) return;
+  if (seen) {
+    S.frozen[v] = 1;
+    atomicAdd(S.counts + 1, 1ull);
+  } else if (c < (uint32_t)kVisitPer) {
+    blk[c] = best;
+    *cntp = c + 1;
+  } else {
+    const uint32_t b = atomicAdd(S.vpool_used, 1u);
+    if (b >= S.vpool_cap) {
+      atomicCAS(S.err, 0, RBG_ERR_NOMEM);                 // pool too small: the host reruns bigger
     } else {
-      const uint32_t b = atomicAdd(S.vpool_used, 1u);
-      if (b >= S.vpool_cap) {
-        atomicCAS(S.err, 0, RBG_ERR_NOMEM);               // pool too small: the host reruns bigger
-      } else {
-        const uint32_t id = (uint32_t)S.n + b;
-        S.vlab[(size_t)id * kVisitPer] = best;
-        S.vcnt[id] = 1;
-        S.vnext[id] = kEmpty;
-        *nextp = id;
-      }
+      const uint32_t id = (uint32_t)S.n + b;
+      S.vlab[(size_t)id * kVisitPer] = best;
+      S.vcnt[id] = 1;
+      S.vnext[id] = kEmpty;
+      *nextp = id;
     }
   }
 }
@@ -551,8 +566,8 @@ __device__ __forceinline__ unsigned char *warp_region(unsigned char *smem) {
 __device__ __forceinline__ uint32_t *warp_stage_u(unsigned char *smem) {
   return (uint32_t *)(warp_region(smem) + kTabSlots * 16 + kTabMaxDeg * 4);
 }
-__device__ __forceinline__ float *warp_stage_w(unsigned char *smem) {
-  return (float *)(warp_stage_u(smem) + kTabMaxDeg);
+__device__ __forceinline__ double *warp_stage_w(unsigned char *smem) {   // quantities, exact
+  return (double *)(warp_stage_u(smem) + kTabMaxDeg);
 }
 __device__ __forceinline__ double *warp_stage_d(unsigned char *smem) {   // lo, hi intervals
   return (double *)warp_stage_u(smem);
@@ -606,19 +621,18 @@ __device__ void clear_tables(const Sweep &S, unsigned char *smem, int gwarp) {
   __syncthreads();
 }
 
-// Visit stamps: a node visited in round r holds 2r + 1 when its label
-// changed, 2r otherwise, published after its writes.  Bounded wait (relaxed
-// polls; the caller fences before it reads what the node wrote) until u was
-// visited in this round; returns its stamp, or 0 after giving up.
-__device__ __forceinline__ uint32_t wait_visited(const Sweep &S, uint32_t u) {
+// Visit stamps: a node visited in round r holds 2r + 1 when its label changed,
+// 2r otherwise.  Bounded wait until u was visited in this round; returns its
+// state word, or 0 after giving up.
+__device__ __forceinline__ uint64_t wait_visited(const Sweep &S, uint32_t u) {
   const uint32_t want = 2u * S.round;
-  uint32_t st = ld_relaxed(S.done + u);
-  if (st >= want) return st;
+  uint64_t st = ld_relaxed64(S.state + u);
+  if ((uint32_t)(st >> 32) >= want) return st;
   const uint64_t t0 = now_ns();
   for (int it = 1;; ++it) {
     __nanosleep(it < 16 ? 20 : 200);
-    st = ld_relaxed(S.done + u);
-    if (st >= want) return st;
+    st = ld_relaxed64(S.state + u);
+    if ((uint32_t)(st >> 32) >= want) return st;
     if ((it & 15) == 0) {
       if (*(volatile int *)S.err != 0) return 0;
       if (now_ns() - t0 > kWaitNs) {
@@ -636,10 +650,18 @@ __device__ __forceinline__ uint32_t wait_visited(const Sweep &S, uint32_t u) {
 // the best (upper end at or above the largest lower end) when more than one
 // can, and the current label against the best when the 1e-12 rule is not
 // settled by the intervals.  Same result as decide().
-__device__ uint32_t decide_staged(const Sweep &S, Table &T, const uint32_t *su, const float *sw,
+__device__ uint32_t decide_staged(const Sweep &S, Table &T, const uint32_t *su, const double *sw,
                                   double *dlo, const double *inv, int d, uint32_t cur,
                                   bool *touched) {
   const int lane = threadIdx.x & 31;
+  // one label on every arc: it is the best whatever its score
+  const uint32_t first_label = d ? su[0] : cur;
+  bool same = true;
+  for (int i = lane; i < d; i += 32) same &= su[i] == first_label;
+  if (__all_sync(FULL, same)) {
+    *touched = d > 0;
+    return first_label;
+  }
   int nlist = 0;
   for (int c = 0; c < d; c += 32) {
     const int i = c + lane;
@@ -739,55 +761,6 @@ __device__ uint32_t decide_staged(const Sweep &S, Table &T, const uint32_t *su, 
   return bk;
 }
 
-// Stages v's arcs (neighbour ids into su, quantities into sw) and, in the
-// Gauss-Seidel sweep, waits (bounded) until every earlier neighbour has been
-// visited in this round, polling all their stamps at once.  *chg: some earlier
-// neighbour of this lane's arcs changed its label in this round.  Returns
-// false after a wait gave up.  The caller fences before reading labels.
-__device__ bool stage_and_wait(const Sweep &S, uint32_t *su, float *sw, int64_t a0, int d,
-                               bool wait, bool *chg) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t want = 2u * S.round;
-  uint32_t pend = 0;
-  *chg = false;
-#pragma unroll
-  for (int j = 0; j < kTabMaxDeg / 32; ++j) {
-    const int i = lane + 32 * j;
-    if (i < d) {
-      const uint32_t u = __ldg(S.nbr + a0 + i);
-      su[i] = u;
-      sw[i] = __ldg(S.w + a0 + i);
-      if (wait && __ldg(S.early + a0 + i)) pend |= 1u << j;
-    }
-  }
-  if (!wait || __reduce_or_sync(FULL, pend) == 0) return true;
-  uint64_t t0 = 0;
-  bool changed = false;
-  for (int it = 0; pend; ++it) {
-#pragma unroll
-    for (int j = 0; j < kTabMaxDeg / 32; ++j)
-      if ((pend >> j) & 1u) {
-        const uint32_t st = ld_relaxed(S.done + su[lane + 32 * j]);
-        if (st >= want) {
-          pend &= ~(1u << j);
-          changed |= st == want + 1u;
-        }
-      }
-    if (!pend) break;
-    if (it == 0) t0 = now_ns();
-    __nanosleep(it < 16 ? 20 : 200);
-    if ((it & 15) == 15) {
-      if (*(volatile int *)S.err != 0) return false;
-      if (now_ns() - t0 > kWaitNs) {
-        atomicCAS(S.err, 0, RBG_ERR_TIMEOUT);
-        return false;
-      }
-    }
-  }
-  *chg = changed;
-  return true;
-}
-
 // One Gauss-Seidel round (rb_cluster.cpp:611-714).
 //
 // Activity.  In the reference a node is active when a neighbour changed since
@@ -797,6 +770,11 @@ __device__ bool stage_and_wait(const Sweep &S, uint32_t *su, float *sw, int64_t 
 // and changes of earlier neighbours in this round are the change bits of their
 // stamps.  No flag is written while it can be read, so nothing races.
 // An inactive node writes nothing; it only publishes its stamp.
+//
+// Bound by the chains of dependent visits: what counts is the time from an
+// earlier neighbour's store to this node's.  That is one L2 round trip of the
+// poll, the decision, and one store of the state word; the marks and the visited
+// set follow after it.
 __global__ void __launch_bounds__(kLpaWarps * 32) k_lpa_gs_round(const Sweep S) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
@@ -804,7 +782,7 @@ __global__ void __launch_bounds__(kLpaWarps * 32) k_lpa_gs_round(const Sweep S) 
   clear_tables(S, smem, gwarp);
   float *wb = warp_wbuf(smem);
   uint32_t *su = warp_stage_u(smem);
-  float *sw = warp_stage_w(smem);
+  double *sw = warp_stage_w(smem);
   double *sd = warp_stage_d(smem);
   const double *inv = cta_inv(smem);
   const uint32_t want = 2u * S.round;
@@ -818,48 +796,59 @@ __global__ void __launch_bounds__(kLpaWarps * 32) k_lpa_gs_round(const Sweep S) 
     const uint32_t v = r.x;
     const int64_t d = r.y, a0 = (int64_t)r.z | ((int64_t)r.w << 32), a1 = a0 + d;
     const bool marked = ld_cg8(S.active + v) != 0;          // written in the previous round
-    bool ok = true, chg = false, changed = false;
-    const uint32_t cur = ld_cg(S.label + v);
+    const bool frozen = ld_cg8(S.frozen + v) != 0;
+    const uint32_t cur = (uint32_t)ld_relaxed64(S.state + v);
+    bool ok = true, chg = false;
+    bool touched = false;
+    uint32_t best = cur;
+    Table T = warp_table(S, smem, d, gwarp);
     if (d <= kTabMaxDeg) {
-      // stage the arcs and poll the earlier neighbours once
-      uint32_t uid[J];
+      // each arc's neighbour: stamp and label in one load; the earlier
+      // neighbours not yet visited in this round are polled (bounded)
+      uint32_t uid[J], lab[J];
       uint32_t pend = 0;
 #pragma unroll
       for (int j = 0; j < J; ++j) {
         const int i = lane + 32 * j;
         uid[j] = 0;
+        lab[j] = 0;
         if (i < d) {
           uid[j] = __ldg(S.nbr + a0 + i);
-          sw[i] = __ldg(S.w + a0 + i);
           if (__ldg(S.early + a0 + i)) pend |= 1u << j;
+        }
+      }
+      uint32_t early = pend;
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const int i = lane + 32 * j;
+        if (i < d) {
+          const uint64_t st = ld_relaxed64(S.state + uid[j]);
+          const uint32_t stamp = (uint32_t)(st >> 32);
+          lab[j] = (uint32_t)st;
+          if ((early >> j) & 1u) {
+            if (stamp >= want) pend &= ~(1u << j);
+            chg |= stamp == want + 1u;
+          }
         }
       }
 #pragma unroll
       for (int j = 0; j < J; ++j) {
         const int i = lane + 32 * j;
-        if ((pend >> j) & 1u) {
-          const uint32_t st = ld_relaxed(S.done + uid[j]);
-          if (st >= want) {
-            pend &= ~(1u << j);
-            chg |= st == want + 1u;
-          }
-        }
+        if (i < d) sw[i] = (double)__ldg(S.w + a0 + i);
       }
-      bool touched = false;
-      uint32_t best = cur;
-      Table T = warp_table(S, smem, d, gwarp);
-      // the remaining waits (bounded)
       uint64_t t0 = 0;
       for (int it = 0; pend && ok; ++it) {
         if (it == 0) t0 = now_ns();
-        __nanosleep(it < 16 ? 20 : 200);
+        else if (it >= 8) __nanosleep(it < 64 ? 20 : 200);
 #pragma unroll
         for (int j = 0; j < J; ++j)
           if ((pend >> j) & 1u) {
-            const uint32_t st = ld_relaxed(S.done + uid[j]);
-            if (st >= want) {
+            const uint64_t st = ld_relaxed64(S.state + uid[j]);
+            const uint32_t stamp = (uint32_t)(st >> 32);
+            if (stamp >= want) {
               pend &= ~(1u << j);
-              chg |= st == want + 1u;
+              lab[j] = (uint32_t)st;
+              chg |= stamp == want + 1u;
             }
           }
         if (pend && (it & 15) == 15) {
@@ -870,61 +859,35 @@ __global__ void __launch_bounds__(kLpaWarps * 32) k_lpa_gs_round(const Sweep S) 
           }
         }
       }
-      if (!__all_sync(FULL, ok)) {
-        if (lane == 0) st_release(S.done + v, want);
-        break;
-      }
-      const bool anychg = __any_sync(FULL, chg);
-      if ((marked || anychg) && d > 0) {
-        // the labels after the waits: an earlier neighbour that changed wrote its
-        // label before its stamp (acquired by the fence); the others did not move
-        if (anychg) fence_acq_rel();
+      if (__all_sync(FULL, ok) && __any_sync(FULL, marked || chg) && d > 0) {
 #pragma unroll
         for (int j = 0; j < J; ++j) {
           const int i = lane + 32 * j;
-          if (i < d) su[i] = ld_relaxed(S.label + uid[j]);
+          if (i < d) su[i] = lab[j];
         }
         __syncwarp();
         best = decide_staged(S, T, su, sw, sd, inv, (int)d, cur, &touched);
-        if (touched && best != cur && !ld_cg8(S.frozen + v)) {
-          commit(S, v, cur, best, a0, a1, true);
-          changed = true;
+      }
+    } else {
+      // general path (more arcs than the stage holds): wait, then decide (the
+      // same lane reads an arc's word again, so it sees this round's)
+      for (int64_t a = a0 + lane; a < a1 && ok; a += 32)
+        if (__ldg(S.early + a)) {
+          const uint64_t st = wait_visited(S, __ldg(S.nbr + a));
+          ok = st != 0;
+          chg |= (uint32_t)(st >> 32) == want + 1u;
         }
-      }
-      __syncwarp();
-      if (lane == 0) {
-        if (marked || anychg) st_release(S.done + v, want + (changed ? 1u : 0u));
-        else st_relaxed(S.done + v, want);
-      }
-      continue;
+      if (__all_sync(FULL, ok) && __any_sync(FULL, marked || chg))
+        best = decide(S, T, wb, a0, a1, cur, true, &touched);
     }
-    // general path (more arcs than the stage holds): wait, then decide
-    for (int64_t a = a0 + lane; a < a1 && ok; a += 32)
-      if (__ldg(S.early + a)) {
-        const uint32_t st = wait_visited(S, __ldg(S.nbr + a));
-        ok = st != 0;
-        chg |= st == want + 1u;
-      }
-    if (!__all_sync(FULL, ok)) {
-      if (lane == 0) st_release(S.done + v, want);
-      break;
-    }
-    const bool act = __any_sync(FULL, marked || chg);
-    if (act) {
-      fence_acq_rel();
-      Table T = warp_table(S, smem, d, gwarp);
-      bool touched = false;
-      const uint32_t best = decide(S, T, wb, v, a0, a1, cur, &touched);
-      if (touched && best != cur && !ld_cg8(S.frozen + v)) {
-        commit(S, v, cur, best, a0, a1, true);
-        changed = true;
-      }
-    }
+    const bool good = __all_sync(FULL, ok);
+    const bool changed = good && touched && best != cur && !frozen;
+    if (lane == 0)
+      st_relaxed64(S.state + v, ((uint64_t)(want + (changed ? 1u : 0u)) << 32) |
+                                    (changed ? best : cur));
+    if (!good) break;
+    if (changed) commit(S, v, cur, best, a0, a1, true);
     __syncwarp();
-    if (lane == 0) {
-      if (act) st_release(S.done + v, want + (changed ? 1u : 0u));
-      else st_relaxed(S.done + v, want);
-    }
   }
 }
 
@@ -936,7 +899,7 @@ __global__ void __launch_bounds__(kLpaWarps * 32) k_lpa_sync_propose(const Sweep
   clear_tables(S, smem, gwarp);
   float *wb = warp_wbuf(smem);
   uint32_t *su = warp_stage_u(smem);
-  float *sw = warp_stage_w(smem);
+  double *sw = warp_stage_w(smem);
   const double *inv = cta_inv(smem);
   const int64_t nw = (int64_t)gridDim.x * kLpaWarps;
   for (int64_t v = gwarp; v < S.n; v += nw) {
@@ -949,17 +912,24 @@ __global__ void __launch_bounds__(kLpaWarps * 32) k_lpa_sync_propose(const Sweep
       uint32_t best;
       if (a1 - a0 <= kTabMaxDeg) {
         const int d = (int)(a1 - a0);
-        bool chg = false;
-        stage_and_wait(S, su, sw, a0, d, false, &chg);
+        uint32_t uid[kTabMaxDeg / 32];
 #pragma unroll
         for (int j = 0; j < kTabMaxDeg / 32; ++j) {
           const int i = lane + 32 * j;
-          if (i < d) su[i] = ld_cg(S.label + su[i]);
+          uid[j] = i < d ? __ldg(S.nbr + a0 + i) : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < kTabMaxDeg / 32; ++j) {
+          const int i = lane + 32 * j;
+          if (i < d) {
+            su[i] = ld_cg(S.label + uid[j]);
+            sw[i] = (double)__ldg(S.w + a0 + i);
+          }
         }
         __syncwarp();
         best = decide_staged(S, T, su, sw, warp_stage_d(smem), inv, d, cur, &touched);
       } else {
-        best = decide(S, T, wb, (uint32_t)v, a0, a1, cur, &touched);
+        best = decide(S, T, wb, a0, a1, cur, false, &touched);
       }
       if (touched) prop = best;
     }
@@ -1014,12 +984,12 @@ void launch_lpa_sort(const int64_t *off, int64_t n, uint64_t *key, const float *
 }
 
 void launch_lpa_init(const uint32_t *order, int64_t n, uint32_t *pos, uint32_t *label,
-                     uint8_t *active, uint8_t *next_active, uint8_t *frozen, uint32_t *done,
+                     uint8_t *active, uint8_t *next_active, uint8_t *frozen, uint64_t *state,
                      uint32_t *vcnt, uint32_t *vnext, cudaStream_t s) {
   if (n == 0) return;
   const int64_t blocks = std::min<int64_t>((n + 255) / 256, 148 * 16);
   k_lpa_init<<<(unsigned)blocks, 256, 0, s>>>(order, n, pos, label, active, next_active, frozen,
-                                              done, vcnt, vnext);
+                                              state, vcnt, vnext);
 }
 
 void launch_lpa_early(const int64_t *off, const uint32_t *nbr, const uint32_t *pos, int64_t n,
@@ -1043,6 +1013,12 @@ int lpa_sweep_warps(int sms) {
   return sms * occ * kLpaWarps;
 }
 
+void launch_lpa_labels(const uint64_t *state, int64_t n, uint32_t *label, cudaStream_t s) {
+  if (n == 0) return;
+  const int64_t blocks = std::min<int64_t>((n + 255) / 256, 148 * 16);
+  k_lpa_labels<<<(unsigned)blocks, 256, 0, s>>>(state, n, label);
+}
+
 int lpa_table_max_deg() { return kTabMaxDeg; }
 int lpa_visit_block() { return kVisitPer; }
 
@@ -1060,7 +1036,7 @@ void launch_lpa_round(const LpaSweepArgs &a, int sync, int warps, cudaStream_t s
   S.active = a.active;
   S.next_active = a.next_active;
   S.frozen = a.frozen;
-  S.done = a.done;
+  S.state = a.state;
   S.prop = a.prop;
   S.vlab = a.vlab;
   S.vcnt = a.vcnt;

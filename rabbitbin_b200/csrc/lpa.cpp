@@ -130,7 +130,7 @@ void propagate(rbg_ctx *c, const rbg_lpa_params *lp, int64_t n, const EdgeView &
   B.act0.ensure(n1);
   B.act1.ensure(n1);
   B.frozen.ensure(n1);
-  B.done.ensure(n1 * 4);
+  B.done.ensure(n1 * 8);
   B.prop.ensure(n1 * 4);
   int dev = 0, sms = 148;
   CK(cudaGetDevice(&dev));
@@ -158,7 +158,7 @@ void propagate(rbg_ctx *c, const rbg_lpa_params *lp, int64_t n, const EdgeView &
   a.pos = B.pos.as<uint32_t>();
   a.label = B.label.as<uint32_t>();
   a.frozen = B.frozen.as<uint8_t>();
-  a.done = B.done.as<uint32_t>();
+  a.state = B.done.as<uint64_t>();
   a.prop = B.prop.as<uint32_t>();
   a.vpool_used = (uint32_t *)(misc + 5);
   a.claim = (uint32_t *)(misc + 4);
@@ -180,7 +180,7 @@ void propagate(rbg_ctx *c, const rbg_lpa_params *lp, int64_t n, const EdgeView &
     uint8_t *act = B.act0.as<uint8_t>(), *nxt = B.act1.as<uint8_t>();
     CK(cudaMemsetAsync(misc + 1, 0, 4, s));
     CK(cudaMemsetAsync(misc + 5, 0, 4, s));
-    launch_lpa_init(a.order, n, B.pos.as<uint32_t>(), a.label, act, nxt, a.frozen, a.done, a.vcnt,
+    launch_lpa_init(a.order, n, B.pos.as<uint32_t>(), a.label, act, nxt, a.frozen, a.state, a.vcnt,
                     a.vnext, s);
     if (attempt == 0) {
       B.early.ensure(a1);
@@ -234,6 +234,7 @@ void propagate(rbg_ctx *c, const rbg_lpa_params *lp, int64_t n, const EdgeView &
     if (attempt >= 4) throw Error(RBG_ERR_NOMEM, "label propagation: visited sets outgrew their pool");
     vcap *= 4;
   }
+  if (!lp->synchronous) launch_lpa_labels(a.state, n, a.label, s);
   CK(cudaEventRecord(e2, s));
   CK(cudaMemcpyAsync(membership, a.label, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));

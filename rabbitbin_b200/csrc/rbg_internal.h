@@ -478,7 +478,7 @@ void launch_lpa_scatter(const uint32_t *from, const uint32_t *to, const float *s
 void launch_lpa_sort(const int64_t *off, int64_t n, uint64_t *key, const float *q, uint32_t *nbr,
                      float *w, cudaStream_t s);
 void launch_lpa_init(const uint32_t *order, int64_t n, uint32_t *pos, uint32_t *label,
-                     uint8_t *active, uint8_t *next_active, uint8_t *frozen, uint32_t *done,
+                     uint8_t *active, uint8_t *next_active, uint8_t *frozen, uint64_t *state,
                      uint32_t *vcnt, uint32_t *vnext, cudaStream_t s);
 // State of the sweeps (see kernels_lpa.cu); vlab holds lpa_visit_block()
 // labels per visited-set block, blocks 0..n-1 owned by the nodes, vpool_cap
@@ -494,7 +494,8 @@ struct LpaSweepArgs {
   const uint4 *rec = nullptr;             // per position: node, degree, first arc
   uint32_t *label = nullptr;
   uint8_t *active = nullptr, *next_active = nullptr, *frozen = nullptr;
-  uint32_t *done = nullptr, *prop = nullptr;
+  uint64_t *state = nullptr;              // sequential sweep: visit stamp << 32 | label
+  uint32_t *prop = nullptr;
   uint32_t *vlab = nullptr, *vcnt = nullptr, *vnext = nullptr, *vpool_used = nullptr;
   uint32_t vpool_cap = 0;
   uint32_t *claim = nullptr;
@@ -511,6 +512,8 @@ void launch_lpa_early(const int64_t *off, const uint32_t *nbr, const uint32_t *p
                       uint8_t *early, uint4 *rec, cudaStream_t s);
 // Warps of one sweep launch (a multiple of the CTA's 8).
 int lpa_sweep_warps(int sms);
+// Labels of the sequential sweep's state words.
+void launch_lpa_labels(const uint64_t *state, int64_t n, uint32_t *label, cudaStream_t s);
 int lpa_table_max_deg();
 int lpa_visit_block();
 void launch_lpa_round(const LpaSweepArgs &a, int sync, int warps, cudaStream_t s);
