@@ -340,6 +340,7 @@ void ensure_buffers(BatchBufs &B, const BatchPlan &L, int nb) {
   B.nbr_sv.ensure(std::max<int64_t>(L.topk, 1) * sizeof(float));
   B.nbr_cnt.ensure(rows1 * sizeof(int32_t));
   B.row_edges.ensure((L.rows + 1) * sizeof(int32_t));
+  B.row_cnt.ensure(rows1 * sizeof(int32_t));
   B.edge0s.ensure((nb + 1) * sizeof(int64_t));
   B.desc.ensure(nb * sizeof(BatchAsm));
   B.row0s.ensure((nb + 1) * sizeof(int64_t));
@@ -423,6 +424,7 @@ BatchAsm describe(BatchBufs &B, const AsmPlan &a, int b) {
   e.nbr_sv = dptr<float>(B.nbr_sv, a.topk0);
   e.nbr_cnt = dptr<int32_t>(B.nbr_cnt, a.row0);
   e.row_edges = dptr<int32_t>(B.row_edges, a.row0);
+  e.row_cnt = dptr<int32_t>(B.row_cnt, a.row0);
   WeightArgs &w = d.w;
   w.S = a.S;
   w.unit = g.unit;
@@ -987,7 +989,8 @@ void run_batch(rbg_ctx *c, const rbg_params *defaults, const rbg_assembly *asms,
   const BatchAsm *dD = B.desc.as<BatchAsm>();
   captured(c, 1, use_graph, stats.graph_launches, [&] {
     CK(cudaMemcpyAsync(B.desc.p, h_desc, desc_bytes, cudaMemcpyHostToDevice, c->stream));
-    launch_emit_batch(dD, B.row0s.as<int64_t>(), nb, rows, L.max_k, B.row_edges.as<int32_t>(),
+    launch_emit_batch(dD, B.row0s.as<int64_t>(), nb, rows, L.max_k, B.row_cnt.as<int32_t>(),
+                      B.row_edges.as<int32_t>(),
                       B.edge0s.as<int64_t>(), c->stream);
     launches += (rows ? 2 : 0) + 2;
     CK(cudaMemcpyAsync(h_edge0s, B.edge0s.p, (nb + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,

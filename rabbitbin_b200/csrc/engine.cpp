@@ -1030,6 +1030,7 @@ void run_graph(rbg_ctx *c, const rbg_params *p, const ShardCtx *sc = nullptr) {
   c->nbr_sv.ensure(n1 * K * sizeof(float));
   c->nbr_cnt.ensure(n1 * sizeof(int32_t));
   c->row_edges.ensure((n1 + 1) * sizeof(int32_t));
+  c->row_cnt.ensure(n1 * sizeof(int32_t));
   EmitArgs e;
   e.n = n; e.K = K; e.mutual = p->mutual; e.small_path = fused ? 0 : 1;
   e.topk = g.topk; e.topk_cnt = g.topk_cnt;
@@ -1038,6 +1039,7 @@ void run_graph(rbg_ctx *c, const rbg_params *p, const ShardCtx *sc = nullptr) {
   e.nbr_sv = c->nbr_sv.as<float>();
   e.nbr_cnt = c->nbr_cnt.as<int32_t>();
   e.row_edges = c->row_edges.as<int32_t>();
+  e.row_cnt = c->row_cnt.as<int32_t>();
   c->kept.ensure(n1 * ((K + 31) / 32) * sizeof(uint32_t));
   e.kept = c->kept.as<uint32_t>();
   if (sc && !sym_shard) {
@@ -1534,7 +1536,7 @@ int rbg_destroy(rbg_ctx *c) {
                   &c->elem_winv, &c->elem_cnt, &c->codesA, &c->codesB, &c->winners32, &c->unit,
                   &c->anynz, &c->colnorm, &c->svbits, &c->topk, &c->topk_cnt, &c->maxc_cand,
                   &c->maxc_all, &c->stats, &c->pairs, &c->pair_out, &c->nbr, &c->nbr_sv,
-                  &c->nbr_cnt, &c->row_edges, &c->e_from, &c->e_to, &c->e_scomp, &c->e_score,
+                  &c->nbr_cnt, &c->row_edges, &c->row_cnt, &c->e_from, &c->e_to, &c->e_scomp, &c->e_score,
                   &c->badflag, &c->tmp, &c->cand_buf, &c->cand_cnt, &c->colacc, &c->unit16,
                   &c->sym_pairs, &c->sym_np, &c->sym_rowcnt, &c->sym_rowoff, &c->sym_keys,
                   &c->shard_send, &c->shard_recv, &c->oh_pres, &c->oh_map, &c->oh_koff,

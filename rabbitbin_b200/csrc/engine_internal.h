@@ -188,7 +188,7 @@ struct BatchBufs {
   DBuf ascii, offsets, depth, packed, nmask, winv, ecnt, codesA, codesB;
   DBuf unit, unit16, anynz, colnorm, colacc, svbits, topk, topk_cnt, maxc_cand, maxc_all, stats;
   DBuf gbuf, gcnt, pairs, pair_cnt, b0;
-  DBuf nbr, nbr_sv, nbr_cnt, row_edges, edge0s;
+  DBuf nbr, nbr_sv, nbr_cnt, row_edges, row_cnt, edge0s;
   DBuf e_from, e_to, e_scomp, e_score;
   DBuf desc, row0s, lists, item0s, queues, pair0s;
   // symmetric all-pairs pass of the tensor-core assemblies (row space of the batch)
@@ -205,7 +205,7 @@ struct BatchBufs {
     DBuf *all[] = {&ascii, &offsets, &depth, &packed, &nmask, &winv, &ecnt, &codesA, &codesB,
                    &unit, &unit16, &anynz, &colnorm, &colacc, &svbits, &topk, &topk_cnt,
                    &maxc_cand, &maxc_all, &stats, &gbuf, &gcnt, &pairs, &pair_cnt, &b0, &nbr,
-                   &nbr_sv, &nbr_cnt, &row_edges, &edge0s, &e_from, &e_to, &e_scomp, &e_score,
+                   &nbr_sv, &nbr_cnt, &row_edges, &row_cnt, &edge0s, &e_from, &e_to, &e_scomp, &e_score,
                    &desc, &row0s, &lists, &item0s, &queues, &pair0s, &sym_pairs, &sym_np,
                    &sym_rowcnt, &sym_rowoff, &sym_keys};
     for (DBuf *b : all) b->release();
@@ -361,7 +361,7 @@ struct rbg_ctx {
   rbg::DBuf packed, nmask, elem_idx, elem_winv, elem_cnt, codesA, codesB, winners32;
   // graph state
   rbg::DBuf unit, unit16, anynz, colnorm, svbits, topk, topk_cnt, maxc_cand, maxc_all, stats;
-  rbg::DBuf pairs, pair_out, nbr, nbr_sv, nbr_cnt, row_edges, cand_buf, cand_cnt;
+  rbg::DBuf pairs, pair_out, nbr, nbr_sv, nbr_cnt, row_edges, row_cnt, cand_buf, cand_cnt;
   rbg::DBuf e_from, e_to, e_scomp, e_score, badflag, tmp, colacc;
   rbg::DBuf kept;                        // kept-neighbour masks of the edge count
   rbg::DBuf b0dev;                       // b0 as made on the device (float)

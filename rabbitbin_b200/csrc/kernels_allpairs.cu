@@ -27,6 +27,7 @@
 #include <cuda_fp16.h>
 
 #include "rbg_internal.h"
+#include "scan.cuh"
 #include "select_topk.cuh"
 
 namespace rbg {
@@ -1182,27 +1183,6 @@ __global__ void k_max_blocks(const uint32_t *__restrict__ blocks, int W, int64_t
   }
 }
 
-// Row offsets of the admitted keys: exclusive scan of the per-row counts, one CTA.
-__global__ void k_rows_scan(const int32_t *cnt, int64_t *off, int64_t n) {
-  __shared__ int64_t part[1024];
-  const int t = threadIdx.x;
-  const int64_t per = (n + 1023) / 1024;
-  const int64_t a = t * per, b = (a + per < n) ? a + per : n;
-  int64_t s = 0;
-  for (int64_t q = a; q < b; ++q) s += cnt[q];
-  part[t] = s;
-  __syncthreads();
-  for (int d = 1; d < 1024; d <<= 1) {
-    const int64_t add = (t >= d) ? part[t - d] : 0;
-    __syncthreads();
-    part[t] += add;
-    __syncthreads();
-  }
-  int64_t run = (t > 0) ? part[t - 1] : 0;
-  for (int64_t q = a; q < b; ++q) { off[q] = run; run += cnt[q]; }
-  if (t == 1023) off[n] = part[1023];
-}
-
 // Both keys of every admitted pair into their rows' segments (grid-stride over
 // the pairs written).  Positions count down from each row's end, so the row
 // counts return to zero.
@@ -1220,45 +1200,127 @@ __global__ void k_scatter_pairs(SymOut o, const int64_t *off, uint64_t *keys,
   }
 }
 
+// Keys of a row ranked by a histogram of their similarity.  Bins of 2^15 steps of
+// the similarity's float bits above 1/32 (admitted similarities lie in
+// (0.039, 1)): one register count a bin at m = 500, finer below 0.5.
+constexpr uint32_t kBinBase = 0x3D000000u;          // 0.03125f
+constexpr int kBins = 1280;                         // through 1.0f
+constexpr int kBinShift = 15;
+constexpr int kSelWords = kBins;                    // 32-bit words of a warp's buffer
+static_assert(kMergeBuf * 2 <= kSelWords, "the tie buffer lies over the histogram");
+
+__device__ __forceinline__ int key_bin(uint64_t key) {
+  const uint32_t b = ((uint32_t)(key >> 32) - kBinBase) >> kBinShift;
+  return (int)(b < (uint32_t)kBins ? b : 0u);       // below the base: the lowest bin
+}
+
+// Keeps the R largest of the cnt unique keys in buf, in place.  Up to 96 keys by
+// their ranks (each lane counts the keys above its own), else by select_topk.
+__device__ __forceinline__ void keep_largest(uint64_t *buf, int cnt, int R) {
+  const int lane = threadIdx.x & 31;
+  if (cnt > 96) {
+    select_topk(buf, cnt, R);
+    return;
+  }
+  uint64_t v[3];
+  int rank[3] = {0, 0, 0};
+#pragma unroll
+  for (int t = 0; t < 3; ++t) v[t] = t * 32 + lane < cnt ? buf[t * 32 + lane] : 0ull;
+  for (int i = 0; i < cnt; ++i) {
+    const uint64_t x = buf[i];
+#pragma unroll
+    for (int t = 0; t < 3; ++t) rank[t] += x > v[t];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < 3; ++t)
+    if (t * 32 + lane < cnt && rank[t] < R) buf[rank[t]] = v[t];
+  __syncwarp();
+}
+
 // Warp per row: the K best keys of the row's segment (row space index gr,
-// assembly row `row`), streamed through a 512-key shared buffer (the register
-// radix select keeps the K best whenever it fills).
+// assembly row `row`).  Two passes over the segment: a histogram gives the bin
+// that holds the K-th key; keys above it are kept as they stream by, keys in it
+// are gathered (in a 512-key buffer over the histogram, cut when it fills) and
+// the largest of them fill up.  A segment read twice against a bit-by-bit search
+// over every 512 keys: 50,000 rows (470 keys each) 0.31 -> 0.13 ms, 30,011 rows
+// at S = 5 (3,400 keys) 0.72 -> 0.23 ms.
 __device__ __forceinline__ void select_row(const GraphArgs &g, int64_t row, int64_t gr,
                                            const int64_t *off, const uint64_t *keys,
-                                           uint64_t *buf) {
+                                           uint32_t *words) {
   const int lane = threadIdx.x & 31;
   const int K = g.K;
   const int64_t s0 = off[gr];
   const int64_t c = off[gr + 1] - s0;
   const uint64_t *src = keys + s0;
+  uint64_t *top = g.topk + row * K;
   if (c <= K) {
-    for (int64_t i = lane; i < c; i += 32) g.topk[row * K + i] = src[i];
+    for (int64_t i = lane; i < c; i += 32) top[i] = src[i];
     if (lane == 0) g.topk_cnt[row] = (int32_t)c;
     return;
   }
-  int fill = 0;
-  for (int64_t i0 = 0; i0 < c;) {
-    const int take = (int)(c - i0 < (int64_t)(kMergeBuf - fill) ? c - i0 : (int64_t)(kMergeBuf - fill));
-    for (int i = lane; i < take; i += 32) buf[fill + i] = src[i0 + i];
-    fill += take;
-    i0 += take;
-    __syncwarp();
-    if (fill == kMergeBuf) {
-      select_topk(buf, fill, K);
-      fill = K;
+  for (int i = lane; i < kBins / 4; i += 32)
+    reinterpret_cast<uint4 *>(words)[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncwarp();
+  for (int64_t i = lane; i < c; i += 32) atomicAdd(words + key_bin(src[i]), 1u);
+  __syncwarp();
+  // bins from the top: lane l owns the 40 bins below kBins - 40 l
+  constexpr int kPer = kBins / 32;
+  const uint32_t *mine = words + kBins - kPer * (lane + 1);
+  uint32_t sum = 0;
+#pragma unroll
+  for (int i = 0; i < kPer; i += 4) {
+    const uint4 x = *reinterpret_cast<const uint4 *>(mine + i);
+    sum += x.x + x.y + x.z + x.w;
+  }
+  uint32_t incl = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(FULL, incl, d);
+    if (lane >= d) incl += t;
+  }
+  int bin = 0, above = 0;                            // the K-th key's bin, keys above it
+  const unsigned own = __ballot_sync(FULL, incl >= (uint32_t)K);
+  const int who = __ffs(own) - 1;                    // c > K: some lane reaches K
+  if (lane == who) {
+    uint32_t at = incl - sum;
+    int i = kPer - 1;
+    for (; i > 0 && at + mine[i] < (uint32_t)K; --i) at += mine[i];
+    bin = kBins - kPer * (lane + 1) + i;
+    above = (int)at;
+  }
+  bin = __shfl_sync(FULL, bin, who);
+  above = __shfl_sync(FULL, above, who);
+  __syncwarp();                                      // the histogram is done with
+  uint64_t *buf = reinterpret_cast<uint64_t *>(words);
+  const int need = K - above;                        // keys taken from the bin
+  int out = 0, fill = 0;
+  for (int64_t i0 = 0; i0 < c; i0 += 32) {
+    const int64_t i = i0 + lane;
+    const uint64_t key = i < c ? src[i] : 0ull;
+    const int b = i < c ? key_bin(key) : -1;
+    const unsigned hi = __ballot_sync(FULL, b > bin), eq = __ballot_sync(FULL, b == bin);
+    const unsigned below = (1u << lane) - 1u;
+    if (b > bin) top[out + __popc(hi & below)] = key;
+    out += __popc(hi);
+    if (eq) {
+      if (fill + __popc(eq) > kMergeBuf) {
+        select_topk(buf, fill, need);
+        fill = need;
+      }
+      if (b == bin) buf[fill + __popc(eq & below)] = key;
+      fill += __popc(eq);
+      __syncwarp();
     }
   }
-  if (fill > K) {
-    select_topk(buf, fill, K);
-    fill = K;
-  }
-  for (int i = lane; i < fill; i += 32) g.topk[row * K + i] = buf[i];
-  if (lane == 0) g.topk_cnt[row] = fill;
+  if (fill > need) keep_largest(buf, fill, need);
+  for (int i = lane; i < need; i += 32) top[above + i] = buf[i];
+  if (lane == 0) g.topk_cnt[row] = K;
 }
 
 __global__ void __launch_bounds__(kMergeWarps * 32)
 k_select_rows(GraphArgs g, const int64_t *off, const uint64_t *keys) {
-  __shared__ uint64_t mk[kMergeWarps][kMergeBuf];
+  __shared__ __align__(16) uint32_t mk[kMergeWarps][kSelWords];
   const int wib = threadIdx.x >> 5;
   const int64_t row = (int64_t)blockIdx.x * kMergeWarps + wib;
   if (row < g.n) select_row(g, row, row, off, keys, mk[wib]);
@@ -1267,7 +1329,7 @@ k_select_rows(GraphArgs g, const int64_t *off, const uint64_t *keys) {
 __global__ void __launch_bounds__(kMergeWarps * 32)
 k_select_rows_batch(const BatchAsm *B, const int64_t *row0s, int nb, int64_t rows,
                     const int64_t *off, const uint64_t *keys) {
-  __shared__ uint64_t mk[kMergeWarps][kMergeBuf];
+  __shared__ __align__(16) uint32_t mk[kMergeWarps][kSelWords];
   const int wib = threadIdx.x >> 5;
   const int64_t r = (int64_t)blockIdx.x * kMergeWarps + wib;
   if (r >= rows) return;
@@ -1486,7 +1548,7 @@ void launch_allpairs_sym_window(const GraphArgs &g, const SymOut &o, int64_t cb,
 void launch_rows_topk_counts(const GraphArgs &g, const SymOut &o, const uint32_t *svtab,
                              int64_t *rowoff, uint64_t *keys, cudaStream_t s) {
   if (g.n == 0) return;
-  k_rows_scan<<<1, 1024, 0, s>>>(o.rowcnt, rowoff, g.n);
+  launch_exclusive_scan(o.rowcnt, rowoff, g.n, s);
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1498,7 +1560,7 @@ void launch_rows_topk_counts(const GraphArgs &g, const SymOut &o, const uint32_t
 void launch_rows_topk(const GraphArgs &g, const SymOut &o, int64_t *rowoff, uint64_t *keys,
                       cudaStream_t s) {
   if (g.n == 0) return;
-  k_rows_scan<<<1, 1024, 0, s>>>(o.rowcnt, rowoff, g.n);
+  launch_exclusive_scan(o.rowcnt, rowoff, g.n, s);
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1510,7 +1572,7 @@ void launch_rows_topk(const GraphArgs &g, const SymOut &o, int64_t *rowoff, uint
 void launch_rows_topk_batch(const BatchAsm *B, const int64_t *row0s, int nb, int64_t rows,
                             const SymOut &o, int64_t *rowoff, uint64_t *keys, cudaStream_t s) {
   if (rows == 0) return;
-  k_rows_scan<<<1, 1024, 0, s>>>(o.rowcnt, rowoff, rows);
+  launch_exclusive_scan(o.rowcnt, rowoff, rows, s);
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

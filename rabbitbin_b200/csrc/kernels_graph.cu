@@ -10,6 +10,7 @@
 #include <cuda_fp16.h>
 
 #include "rbg_internal.h"
+#include "scan.cuh"
 
 namespace rbg {
 namespace {
@@ -446,7 +447,7 @@ __device__ __forceinline__ void count_edges_row(const EmitArgs &e, int64_t i) {
     if (e.kept && lane == 0) e.kept[i * kw + (q0 >> 5)] = m;
     cnt += __popc(m);
   }
-  if (lane == 0) e.row_edges[i] = cnt;
+  if (lane == 0) e.row_cnt[i] = cnt;
 }
 
 __global__ void k_count_edges(EmitArgs e) {
@@ -464,27 +465,6 @@ __global__ void k_count_edges_batch(const BatchAsm *B, const int64_t *row0s, int
 // First edge of every assembly after the batch-wide scan of row_edges.
 __global__ void k_edge0s(const int64_t *row0s, int nb, const int32_t *row_edges, int64_t *edge0s) {
   for (int a = threadIdx.x; a <= nb; a += blockDim.x) edge0s[a] = row_edges[row0s[a]];
-}
-
-__global__ void k_scan(int32_t *v, int64_t n) {
-  // exclusive scan of n counts into v[0..n], one CTA of 1024 threads
-  __shared__ int64_t part[1024];
-  const int t = threadIdx.x;
-  const int64_t per = (n + 1023) / 1024;
-  const int64_t a = t * per, b = (a + per < n) ? a + per : n;
-  int64_t s = 0;
-  for (int64_t q = a; q < b; ++q) s += v[q];
-  part[t] = s;
-  __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {
-    const int64_t add = (t >= off) ? part[t - off] : 0;
-    __syncthreads();
-    part[t] += add;
-    __syncthreads();
-  }
-  int64_t run = (t > 0) ? part[t - 1] : 0;
-  for (int64_t q = a; q < b; ++q) { const int32_t x = v[q]; v[q] = (int32_t)run; run += x; }
-  if (t == 1023) v[n] = (int32_t)part[1023];
 }
 
 __device__ __forceinline__ void write_edges_row(const EmitArgs &e, int64_t i) {
@@ -673,7 +653,7 @@ void launch_count_edges(const EmitArgs &e, cudaStream_t s) {
   const int64_t rows = (e.row_hi < 0 ? e.n : e.row_hi) - e.row_lo;
   if (rows <= 0) return;
   k_count_edges<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(e);   // warp per row
-  k_scan<<<1, 1024, 0, s>>>(e.row_edges + e.row_lo, rows);
+  launch_exclusive_scan(e.row_cnt + e.row_lo, e.row_edges + e.row_lo, rows, s);
 }
 
 void launch_write_edges(const EmitArgs &e, cudaStream_t s) {
@@ -717,7 +697,8 @@ void launch_b0_batch_range(const BatchAsm *B, const int64_t *pair0s, int nb, int
 }
 
 void launch_emit_batch(const BatchAsm *B, const int64_t *row0s, int nb, int64_t rows, int max_k,
-                       int32_t *row_edges, int64_t *edge0s, cudaStream_t s) {
+                       const int32_t *row_cnt, int32_t *row_edges, int64_t *edge0s,
+                       cudaStream_t s) {
   if (rows > 0) {
     const int len = pow2_at_least(max_k > 32 ? max_k : 32);
     const int warps = 4;
@@ -725,7 +706,7 @@ void launch_emit_batch(const BatchAsm *B, const int64_t *row0s, int nb, int64_t 
                         (size_t)warps * len * 8, s>>>(B, row0s, nb, rows, len);
     k_count_edges_batch<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(B, row0s, nb, rows);
   }
-  k_scan<<<1, 1024, 0, s>>>(row_edges, rows);
+  launch_exclusive_scan(row_cnt, row_edges, rows, s);
   k_edge0s<<<1, 256, 0, s>>>(row0s, nb, row_edges, edge0s);
 }
 

@@ -311,7 +311,8 @@ struct EmitArgs {
   uint32_t *nbr_sorted = nullptr;      // [n][K] ids of kept neighbours, ascending
   float *nbr_sv = nullptr;             // [n][K]
   int32_t *nbr_cnt = nullptr;          // [n]
-  int32_t *row_edges = nullptr;        // [n+1] edges per row, then exclusive scan
+  int32_t *row_cnt = nullptr;          // [n] edges per row
+  int32_t *row_edges = nullptr;        // [n+1] their exclusive scan
   uint32_t *from = nullptr, *to = nullptr;
   float *scomp = nullptr;
   // optional [n][ceil(K/32)] bit masks: the edge count records which of a
@@ -405,7 +406,8 @@ void launch_merge_batch(const BatchAsm *B, const int64_t *row0s, int nb, int64_t
 void launch_rows_topk_batch(const BatchAsm *B, const int64_t *row0s, int nb, int64_t rows,
                             const SymOut &o, int64_t *rowoff, uint64_t *keys, cudaStream_t s);
 void launch_emit_batch(const BatchAsm *B, const int64_t *row0s, int nb, int64_t rows, int max_k,
-                       int32_t *row_edges, int64_t *edge0s, cudaStream_t s);
+                       const int32_t *row_cnt, int32_t *row_edges, int64_t *edge0s,
+                       cudaStream_t s);
 void launch_write_edges_batch(const BatchAsm *B, const int64_t *row0s, int nb, int64_t rows,
                               cudaStream_t s);
 void launch_edge_weights_batch(const BatchAsm *B, const int64_t *edge0s, int nb, int64_t edges,

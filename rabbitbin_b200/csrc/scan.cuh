@@ -1,0 +1,74 @@
+// Exclusive prefix sums of n 32-bit counts over many blocks in one launch, without
+// scratch: block b adds up everything before its tile itself (the counts are in
+// L2) and scans its tile.  Latency-bound at these sizes: one block walking the
+// counts took 50 us at 50,000 rows and 0.2 ms at 200,000; 13 us here at 50,000.
+#pragma once
+#include <algorithm>
+#include <cstdint>
+
+namespace rbg {
+
+constexpr int kScanThreads = 512;
+
+// Sum of v over the block (every thread gets it); sh: 33 values.
+__device__ __forceinline__ int64_t scan_block_sum(int64_t v, int64_t *sh) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+  __syncthreads();                       // the previous use of sh is over
+  if (lane == 0) sh[w] = v;
+  __syncthreads();
+  int64_t t = 0;
+#pragma unroll
+  for (int k = 0; k < kScanThreads / 32; ++k) t += sh[k];
+  return t;
+}
+
+// out[0 .. n] = exclusive prefix sums of in[0 .. n-1] (out[n] the total); out does
+// not overlap in.  tile: a multiple of kScanThreads; block b scans tile b.
+template <class T>
+__global__ void __launch_bounds__(kScanThreads) k_exclusive_scan(const int32_t *__restrict__ in,
+                                                                 T *__restrict__ out, int64_t n,
+                                                                 int64_t tile) {
+  __shared__ int64_t sh[kScanThreads / 32 + 1];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int64_t lo = (int64_t)blockIdx.x * tile, hi = min(n, lo + tile);
+  int64_t before = 0;
+#pragma unroll 8
+  for (int64_t q = t; q < lo; q += kScanThreads) before += in[q];
+  int64_t run = scan_block_sum(before, sh);
+  for (int64_t q0 = lo; q0 < hi; q0 += kScanThreads) {
+    const int64_t q = q0 + t;
+    const int32_t x = q < hi ? in[q] : 0;
+    int64_t incl = x;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int64_t y = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += y;
+    }
+    __syncthreads();
+    if (lane == 31) sh[w] = incl;
+    __syncthreads();
+    int64_t base = run, all = 0;
+#pragma unroll
+    for (int k = 0; k < kScanThreads / 32; ++k) {
+      if (k < w) base += sh[k];
+      all += sh[k];
+    }
+    if (q < hi) out[q] = (T)(base + incl - x);
+    run += all;
+  }
+  if (hi == n && t == 0) out[n] = (T)run;
+}
+
+// Tiles of 2,048 counts, and at most 512 of them: every block reads all counts
+// before its own.
+template <class T>
+inline void launch_exclusive_scan(const int32_t *in, T *out, int64_t n, cudaStream_t s) {
+  int64_t tile = std::max<int64_t>(2048, (n + 511) / 512);
+  tile = (tile + kScanThreads - 1) / kScanThreads * kScanThreads;
+  const int64_t blocks = std::max<int64_t>(1, (n + tile - 1) / tile);
+  k_exclusive_scan<T><<<(unsigned)blocks, kScanThreads, 0, s>>>(in, out, n, tile);
+}
+
+}  // namespace rbg
