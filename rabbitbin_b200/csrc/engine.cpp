@@ -971,7 +971,12 @@ void run_graph(rbg_ctx *c, const rbg_params *p, const ShardCtx *sc = nullptr) {
       if (*hnp <= c->sym_cap) break;
       CK(cudaStreamSynchronize(c->stream));
       if (streamed) {
-        c->no_stream_S |= 1ull << (S & 63);  // survivors outgrow the list at this S
+        // The streamed pass lists every survivor, not only the admitted ones: a
+        // larger list next time while that stays within four times the first one
+        // (256 pairs a contig), the resident pass at this S from now on otherwise.
+        // 200,003 contigs at S = 30 (67 M survivors) stay on the streamed pass.
+        if (*hnp <= (unsigned long long)n1 * 1024) c->sym_cap = *hnp + *hnp / 4;
+        else c->no_stream_S |= 1ull << (S & 63);
         streamed = false;
       } else {
         c->sym_cap = *hnp + *hnp / 4;
