@@ -105,6 +105,10 @@ __device__ __forceinline__ uint32_t spread16(uint32_t x) {
 // each of which stands for two 4-mers (its first and its last four bases):
 // half the shared-memory atomics; the 1,024 5-mer counts are folded into the
 // 4-mer histogram once per contig.
+// Bound by instruction issue (71% of the slots) around the shared atomics.  Words
+// are indexed in 32 bits from the contig's first one, only the first and last take
+// an end mask, and k = 4 is compiled on its own: 450 -> 343 us at 50,000 contigs of
+// 8 kb (330 -> 249 us at 30,000).
 constexpr int kCountWarps = 8;
 constexpr int kH5 = 1024;               // 5-mer counters of a group
 
@@ -120,7 +124,8 @@ struct CountGroup {
   uint32_t pad;
 };
 
-template <bool GC2, int W>              // GC2: GC-norm mode 2 (dinucleotide model)
+// GC2: GC-norm mode 2 (dinucleotide model); K4: k = 4.
+template <bool GC2, int W, bool K4>
 __global__ void __launch_bounds__(kCountWarps * 32) k_count(SketchArgs a) {
   extern __shared__ __align__(16) unsigned char sh_count[];
   __shared__ uint8_t code_of[kMaxElems];
@@ -135,7 +140,7 @@ __global__ void __launch_bounds__(kCountWarps * 32) k_count(SketchArgs a) {
     if constexpr (W == 1) __syncwarp();
     else __syncthreads();
   };
-  const int k = a.k;
+  const int k = K4 ? 4 : a.k;
   const int nb = 1 << (2 * k);
   const uint32_t kmask = (uint32_t)nb - 1u;
   for (int v = threadIdx.x; v < nb; v += blockDim.x) {
@@ -171,29 +176,41 @@ __global__ void __launch_bounds__(kCountWarps * 32) k_count(SketchArgs a) {
   uint32_t dn[GC2 ? 16 : 1] = {};      // mode 2: dinucleotides (prev, next) = dn[4 prev + next]
   gsync();
   if (e - s >= k) {
-    const int64_t w0 = s >> 4, w1 = (e + 15) >> 4;
-    // word wi of the contig and the word before the lane group's first one
-    auto fetch = [&](int64_t wi, uint32_t &cur, uint32_t &bad) {
+    // words of the contig by their index j from its first one (contigs are
+    // shorter than 2^31 words); only the first and last hold other contigs' bases
+    const int64_t w0 = s >> 4;
+    const int nw = (int)(((e + 15) >> 4) - w0);
+    const uint32_t *words = a.packed + w0;
+    const uint32_t *masks = a.nmask + (w0 >> 1);
+    const uint32_t odd = (uint32_t)w0 & 1u;
+    const uint32_t bad_first = 0xFFFFu & ~(0xFFFFu >> (int)(s & 15));
+    const uint32_t bad_last = (e & 15) ? 0xFFFFu >> (int)(e & 15) : 0u;
+    auto fetch = [&](int j, uint32_t &cur, uint32_t &bad) {
       cur = 0;
       bad = 0xFFFFu;
-      if (wi >= w0 && wi < w1) {
-        cur = __ldg(a.packed + wi);
-        bad = invalid16(a.nmask, wi, s, e);
+      if (j < nw) {
+        cur = __ldg(words + j);
+        const uint32_t q = (uint32_t)j + odd;
+        const uint32_t mw = __ldg(masks + (q >> 1));
+        bad = ((q & 1u) ? mw : mw >> 16) & 0xFFFFu;
+        if (j == 0) bad |= bad_first;
+        if (j == nw - 1) bad |= bad_last;
       }
     };
-    uint32_t ncur, nbad, npre = 0, nprebad = 0xFFFFu;   // the next step's words
-    int64_t base = w0 + 32 * wig;
-    fetch(base + lane, ncur, nbad);
-    if (lane == 0) fetch(base - 1, npre, nprebad);
-    for (; base < w1; base += 32 * W) {
-      const int64_t wi = base + lane;
+    // the next step's words, and for lane 0 the word before them
+    uint32_t ncur, nbad, npre = 0, nprebad = 0xFFFFu;
+    int j0 = 32 * wig;
+    fetch(j0 + lane, ncur, nbad);
+    if (lane == 0 && j0 > 0) fetch(j0 - 1, npre, nprebad);
+    for (; j0 < nw; j0 += 32 * W) {
       const uint32_t cur = ncur, bad = nbad;
       uint32_t prev = __shfl_up_sync(0xffffffffu, cur, 1);
       uint32_t prevbad = __shfl_up_sync(0xffffffffu, bad, 1);
       if (lane == 0) { prev = npre; prevbad = nprebad; }
-      fetch(wi + 32 * W, ncur, nbad);
-      if (lane == 0) fetch(wi + 32 * W - 1, npre, nprebad);
-      if (wi < w1) {
+      const int jn = j0 + 32 * W;
+      fetch(jn + lane, ncur, nbad);
+      if (lane == 0) fetch(jn - 1, npre, nprebad);
+      if (j0 + lane < nw) {
         // base counts of the valid bases (base t occupies bits 31-2t .. 30-2t)
         const uint32_t vs = spread16(~bad & 0xFFFFu);
         const uint32_t hi = (cur >> 1) & 0x55555555u, lo = cur & 0x55555555u;
@@ -218,10 +235,12 @@ __global__ void __launch_bounds__(kCountWarps * 32) k_count(SketchArgs a) {
         // codes are counted and folded onto canonical codes per contig
         const uint32_t winbad = (prevbad << 16) | bad;
         uint32_t any = winbad;
-        for (int q = 1; q < k; ++q) any |= winbad >> q;
+        if constexpr (K4) any |= winbad >> 1 | winbad >> 2 | winbad >> 3;
+        else
+          for (int q = 1; q < k; ++q) any |= winbad >> q;
         uint32_t kv = ~any & 0xFFFFu;                   // bit 15-t: k-mer ending at t
         const uint64_t win = ((uint64_t)prev << 32) | cur;
-        if (kv == 0xFFFFu && k == 4) {
+        if (K4 && kv == 0xFFFFu) {
           // bases -3 .. 15 are valid: the 5-mers ending at t = 1, 3, .., 15
 #pragma unroll
           for (int bp = 14; bp >= 0; bp -= 2)
@@ -254,7 +273,7 @@ __global__ void __launch_bounds__(kCountWarps * 32) k_count(SketchArgs a) {
     }
   }
   gsync();
-  if (k == 4) {
+  if constexpr (K4) {
     // 5-mer (first four = x, or last four = x) -> 4-mer x
     for (int x = gt; x < 256; x += GT) {
       const uint4 f = *reinterpret_cast<const uint4 *>(&G.h5[4 * x]);
@@ -269,6 +288,7 @@ __global__ void __launch_bounds__(kCountWarps * 32) k_count(SketchArgs a) {
   uint32_t tot = 0;
   for (int v = gt; v < nb; v += GT) {
     uint32_t rev = 0, x = (uint32_t)v;
+#pragma unroll
     for (int q = 0; q < k; ++q) { rev = (rev << 2) | (3u - (x & 3u)); x >>= 2; }
     if ((uint32_t)v > rev) continue;
     uint32_t cnt = G.hist[v];
@@ -376,16 +396,24 @@ __global__ void __launch_bounds__(kCountWarps * 32) k_count(SketchArgs a) {
 // equal to a finite best.
 //
 // A CTA holds 32 contigs (lane = contig) with their 1/w rows transposed in shared
-// memory ([E][32]: the per-step gather is conflict-free).  Each warp takes one
+// memory ([E][33]: the per-step gather is conflict-free, and so are the stores that
+// transpose the rows).  Each warp takes one
 // register at a time: the first 32 entries of its visiting order and its U row
 // (by element, table UT) are loaded into registers one register ahead, stored in
 // the warp's shared slot, and walked in lock step until every lane's bound has
-// passed (entries past 32 come straight from the table).  Winners go to a shared
-// tile and leave as 4-byte code words, padding columns included.
+// passed (entries past 32 come straight from the table), two entries a vote and no
+// branch on a lane's own bound: with one entry a vote the loop waited on each
+// vote and branch.  Winners go to a shared tile and leave as 4-byte code words,
+// padding columns included.
+//
+// Bound by the shared-memory reads of the walk (L1 wavefronts 79%, issue 63% of
+// peak); 50,000 contigs, m = 500: 790 -> 491 us (30,000: 600 -> 444 with 8 heavy
+// elements; 4 leave half of the direct products out for less than one more step).
 constexpr int kMC = 32;          // contigs per CTA, one per lane
 constexpr int kMThreads = 256;
 constexpr int kMWarps = kMThreads / 32;
-constexpr int kMHeavy = 8;       // smallest-1/w elements evaluated directly
+constexpr int kMHeavy = 4;       // smallest-1/w elements evaluated directly
+constexpr int kMRow = kMC + 1;   // row stride of sW: the transposing stores hit every bank
 constexpr int kMChunk = 256;     // registers per pass; a multiple of 16
 constexpr int kMWinStride = kMChunk + 4;
 constexpr int kMRec = 32;        // visiting-order entries staged per register (one per lane)
@@ -393,7 +421,7 @@ constexpr int kMUcPerLane = (kMaxElems / 2 + 31) / 32;   // 16-byte chunks of a 
 static_assert(kMaxElems % 2 == 0 && kMaxElems <= 5 * 32, "U rows in 16-byte chunks, 5 values per lane");
 
 __host__ __device__ constexpr size_t minreduce_smem(int E) {
-  return (size_t)E * kMC * sizeof(double)            // sW   [E][kMC]
+  return (size_t)E * kMRow * sizeof(double)          // sW   [E][kMRow]
          + (size_t)kMHeavy * kMC * sizeof(double)     // sHw  [kMHeavy][kMC]
          + (size_t)kMC * sizeof(double)               // sWb  [kMC]
          + (size_t)kMWarps * kMRec * 16               // sRec [kMWarps][kMRec]
@@ -403,9 +431,9 @@ __host__ __device__ constexpr size_t minreduce_smem(int E) {
 }
 
 __device__ __forceinline__ void lex_min(double h, int e, double &best, int &win) {
-  if (h < best || (h == best && e < win)) {
+  if (h <= best) {                       // false for NaN
+    if (h < best || e < win) win = e;
     best = h;
-    win = e;
   }
 }
 
@@ -439,7 +467,7 @@ __global__ void __launch_bounds__(kMThreads, 3) k_minreduce(SketchArgs a) {
   const int E = a.n_elems, m = a.m, mpad = a.mpad;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double *sW = reinterpret_cast<double *>(msh);
-  double *sHw = sW + (size_t)E * kMC;
+  double *sHw = sW + (size_t)E * kMRow;
   double *sWb = sHw + kMHeavy * kMC;
   double2 *sRec = reinterpret_cast<double2 *>(sWb + kMC);
   double *sUc = reinterpret_cast<double *>(sRec + kMWarps * kMRec);
@@ -453,7 +481,7 @@ __global__ void __launch_bounds__(kMThreads, 3) k_minreduce(SketchArgs a) {
   const uint64_t kNone = ~0ull;                      // key of a slot that is no element
   for (int i = threadIdx.x; i < kMC * E; i += kMThreads) {
     const int c = i / E, e = i - c * E;
-    sW[e * kMC + c] = c < nc ? __ldg(a.elem_winv + c0 * E + i) : inf;
+    sW[e * kMRow + c] = c < nc ? __ldg(a.elem_winv + c0 * E + i) : inf;
   }
   // Heavy sets.  A non-negative double orders as its bit pattern, so 1/w values
   // are compared as 64-bit keys.  Each lane sorts its (up to 5) values; kMHeavy + 1
@@ -512,6 +540,7 @@ __global__ void __launch_bounds__(kMThreads, 3) k_minreduce(SketchArgs a) {
   const double2 *ord = reinterpret_cast<const double2 *>(a.order);
   const double2 *ut = reinterpret_cast<const double2 *>(a.UT);
   const int half = E >> 1;
+  const int staged = E < kMRec ? E : kMRec;            // both even
   // this CTA's registers (gridDim.y ranges of whole 16-column groups)
   const int groups = mpad >> 4;
   const int r_lo = 16 * (int)((int64_t)blockIdx.y * groups / gridDim.y);
@@ -532,21 +561,30 @@ __global__ void __launch_bounds__(kMThreads, 3) k_minreduce(SketchArgs a) {
       if (rl + kMWarps < rn) min_fetch(st, ord, ut, r + kMWarps, E, lane);
       double best = inf;
       int win = -1;
-      bool done = empty;
-      if (!done) {
+      // an empty lane's products are all infinite and leave win at -1
 #pragma unroll
-        for (int i = 0; i < kMHeavy; ++i) lex_min(__dmul_rn(hw[i], myUc[he[i]]), he[i], best, win);
-      }
-      for (int k = 0; k < E; ++k) {
+      for (int i = 0; i < kMHeavy; ++i) lex_min(__dmul_rn(hw[i], myUc[he[i]]), he[i], best, win);
+      // Two entries a vote.  A lane whose bound has passed keeps evaluating with
+      // the others: its products are above its best and change nothing.
+      bool done = empty;
+      int k = 0;
+      for (; k < staged; k += 2) {
+        const double2 v0 = myRec[k], v1 = myRec[k + 1];
+        done |= __dmul_rn(wb, v0.x) > best;
         if (__all_sync(0xffffffffu, done)) break;
-        const double2 v = k < kMRec ? myRec[k] : __ldg(ord + (size_t)r * E + k);
-        if (!done) {
-          if (__dmul_rn(wb, v.x) > best) {
-            done = true;
-          } else {
-            const int e = (int)__double_as_longlong(v.y);
-            lex_min(__dmul_rn(sW[e * kMC + lane], v.x), e, best, win);
-          }
+        const int e0 = __double2loint(v0.y), e1 = __double2loint(v1.y);
+        const double h0 = __dmul_rn(sW[e0 * kMRow + lane], v0.x);
+        const double h1 = __dmul_rn(sW[e1 * kMRow + lane], v1.x);
+        lex_min(h0, e0, best, win);
+        lex_min(h1, e1, best, win);
+      }
+      if (k >= staged) {
+        for (; k < E; ++k) {                             // past the staged entries
+          const double2 v = __ldg(ord + (size_t)r * E + k);
+          done |= __dmul_rn(wb, v.x) > best;
+          if (__all_sync(0xffffffffu, done)) break;
+          const int e = __double2loint(v.y);
+          lex_min(__dmul_rn(sW[e * kMRow + lane], v.x), e, best, win);
         }
       }
       if (lane < nc) sWin[lane * kMWinStride + rl] = win < 0 ? (uint8_t)0xFF : (uint8_t)win;
@@ -633,8 +671,13 @@ namespace {
 template <bool GC2, int W>
 void launch_count_w(const SketchArgs &a, int64_t grid, cudaStream_t s) {
   const size_t smem = (size_t)(kCountWarps / W) * sizeof(CountGroup);
-  smem_cap_max((const void *)k_count<GC2, W>);
-  k_count<GC2, W><<<(unsigned)grid, kCountWarps * 32, smem, s>>>(a);
+  if (a.k == 4) {
+    smem_cap_max((const void *)k_count<GC2, W, true>);
+    k_count<GC2, W, true><<<(unsigned)grid, kCountWarps * 32, smem, s>>>(a);
+  } else {
+    smem_cap_max((const void *)k_count<GC2, W, false>);
+    k_count<GC2, W, false><<<(unsigned)grid, kCountWarps * 32, smem, s>>>(a);
+  }
 }
 }  // namespace
 
@@ -684,8 +727,8 @@ void smem_cap_max(const void *func) {
 // set-up (the heavy sets, about as long as three registers of a warp) plus
 // kMWarps registers at a time; few contigs leave SMs idle without a split,
 // many fill them alone.  The smallest cost over the waves of three CTAs per SM
-// (97 contigs: 163 -> 24 us, 2,000: 170 -> 61 us, 16,000: 330 us; from 25,000
-// contigs on unsplit, 50,000: 0.82 ms).
+// (97 contigs: 163 -> 24 us, 2,000: 170 -> 61 us; from 25,000 contigs on
+// unsplit).
 static int minreduce_split(int64_t gx, int mpad, int sms) {
   const int groups = mpad / 16;
   const int64_t slots = 3 * (int64_t)sms;
