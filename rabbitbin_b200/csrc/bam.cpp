@@ -51,8 +51,8 @@ void launch_depth_reads(const uint8_t *buf, const uint32_t *rec_off, int64_t nre
 void launch_depth_means(const unsigned long long *sums, int64_t n_targets, const int32_t *kept_tid,
                         int64_t n_kept, const uint32_t *target_len, const int32_t *edge_of_col,
                         int ncols, float *out, cudaStream_t s);
-void launch_depth_device(const uint8_t *comp, const DevBlk *blk, int nb, const uint64_t *ubound,
-                         uint64_t hdr_end, uint8_t *out, uint32_t *counts, uint32_t *scan,
+void launch_depth_device(const uint8_t *comp, const DevBlk *blk, int nb, uint64_t hdr_end,
+                         uint8_t *out, uint32_t *counts, uint32_t *scan, uint32_t *raw,
                          uint32_t *offs, uint32_t *flags, unsigned long long *rec_total,
                          const uint32_t *target_len, const depth::Params &P,
                          unsigned long long *sum, unsigned long long *sum_u, int sms,
@@ -414,6 +414,8 @@ Prefix host_prefix(const FileView &f, const std::vector<Blk> &B, const std::vect
   return r;
 }
 
+constexpr size_t kCopyPiece = 8 << 20;     // bytes of a pinned piece (device route)
+
 // One BAM through the device route: chunks of compressed blocks are copied in
 // and inflated, walked and summed on the device.  Returns false when a block
 // did not start on a record (a writer that lets records cross blocks): the
@@ -422,18 +424,20 @@ Prefix host_prefix(const FileView &f, const std::vector<Blk> &B, const std::vect
 // record count; zeroed by the caller): bit 0 a block that does not inflate or
 // fails its CRC32, bit 1 a block that does not start on a record.  Nothing
 // waits for the device here, so the next BAM's host work overlaps this one's
-// kernels; `timed` (per slot: its launch times are not read yet) and
-// `kernel_ms` carry over from BAM to BAM.
+// kernels; `timed` (per slot: its launch times are not read yet),
+// `kernel_ms` and the next slot carry over from BAM to BAM.  Each slot has its own
+// stream: a chunk of a small file leaves most of the SMs idle (its blocks are one
+// warp each), so two chunks, of one file or of two, run side by side.
 void run_sample_device(rbg_ctx *c, const FileView &f, const std::vector<Blk> &B,
                        const std::vector<uint64_t> &uoff, int64_t hdr_end, const depth::Params &P,
                        const rbg_depth_params *p, const uint32_t *d_tlen, unsigned long long *sum,
                        unsigned long long *sum_u, int threads, uint8_t *slot_dev, bool timed[2],
-                       double &kernel_ms) {
+                       double &kernel_ms, int &slot) {
   DepthBufs &D = *c->depthb;
-  cudaStream_t s = c->stream;
   for (int i = 0; i < 2; ++i) {
     if (!D.ev[i]) CK(cudaEventCreateWithFlags(&D.ev[i], cudaEventDisableTiming));
     if (!D.evc[i]) CK(cudaEventCreateWithFlags(&D.evc[i], cudaEventDisableTiming));
+    if (!D.evp[i]) CK(cudaEventCreateWithFlags(&D.evp[i], cudaEventDisableTiming));
     if (!D.k0[i]) CK(cudaEventCreate(&D.k0[i]));
     if (!D.k1[i]) CK(cudaEventCreate(&D.k1[i]));
   }
@@ -443,8 +447,8 @@ void run_sample_device(rbg_ctx *c, const FileView &f, const std::vector<Blk> &B,
   uint32_t *flags = (uint32_t *)slot_dev;
   unsigned long long *rec_total = (unsigned long long *)(slot_dev + 8);
   size_t b0 = 0;
-  int slot = 0;
   while (b0 < B.size()) {
+    cudaStream_t s = slot ? c->aux : c->stream;
     size_t b1 = b0;
     uint64_t bytes = 0;
     while (b1 < B.size() && (b1 == b0 || bytes + B[b1].isize <= budget)) bytes += B[b1++].isize;
@@ -460,12 +464,9 @@ void run_sample_device(rbg_ctx *c, const FileView &f, const std::vector<Blk> &B,
       kernel_ms += ms;
       timed[slot] = false;
     }
-    D.cpin[slot].ensure(cbytes + 16);
-    const size_t tab_bytes = (size_t)nb * sizeof(DevBlk) + (size_t)(nb + 1) * 8;
+    const size_t tab_bytes = (size_t)nb * sizeof(DevBlk);
     D.tpin[slot].ensure(tab_bytes);
-    par_copy(D.cpin[slot].as<uint8_t>(), f.p + cstart, cbytes, threads);
     DevBlk *tb = D.tpin[slot].as<DevBlk>();
-    uint64_t *ub = (uint64_t *)(D.tpin[slot].as<uint8_t>() + (size_t)nb * sizeof(DevBlk));
     for (int i = 0; i < nb; ++i) {
       const Blk &x = B[b0 + i];
       tb[i].cofs = (uint32_t)(x.cdata - cstart);
@@ -473,18 +474,27 @@ void run_sample_device(rbg_ctx *c, const FileView &f, const std::vector<Blk> &B,
       tb[i].isize = x.isize;
       tb[i].crc = x.crc;
       tb[i].uofs = uoff[b0 + i] - uoff[b0];
-      ub[i] = tb[i].uofs;
     }
-    ub[nb] = bytes;
     D.cdev[slot].ensure(cbytes + 16);
     D.tdev[slot].ensure(tab_bytes);
     D.outd[slot].ensure(bytes + 64);
     D.cntd[slot].ensure((size_t)(2 * nb + 2) * 4);
     D.offd[slot].ensure((size_t)(bytes / 36 + nb + 16) * 4);
+    D.rawd[slot].ensure((size_t)(bytes / 36 + nb + 16) * 4);
     // copies on the context's copy stream, so that chunk c + 1 arrives while
-    // chunk c is inflated
+    // chunk c is inflated; through two pinned pieces, since pinning takes longer
+    // (1 ms for about 2 MB) than a small file's decode
     CK(cudaStreamWaitEvent(c->copy, D.ev[slot], 0));
-    CK(cudaMemcpyAsync(D.cdev[slot].p, D.cpin[slot].p, cbytes, cudaMemcpyHostToDevice, c->copy));
+    int piece = 0;
+    for (size_t o = 0; o < cbytes; o += kCopyPiece, piece ^= 1) {
+      const size_t len = std::min(kCopyPiece, cbytes - o);
+      CK(cudaEventSynchronize(D.evp[piece]));              // the piece's last copy
+      D.cpin[piece].ensure(len);
+      par_copy(D.cpin[piece].as<uint8_t>(), f.p + cstart + o, len, threads);
+      CK(cudaMemcpyAsync(D.cdev[slot].as<uint8_t>() + o, D.cpin[piece].p, len,
+                         cudaMemcpyHostToDevice, c->copy));
+      CK(cudaEventRecord(D.evp[piece], c->copy));
+    }
     CK(cudaMemcpyAsync(D.tdev[slot].p, D.tpin[slot].p, tab_bytes, cudaMemcpyHostToDevice, c->copy));
     CK(cudaEventRecord(D.evc[slot], c->copy));
     CK(cudaStreamWaitEvent(s, D.evc[slot], 0));
@@ -493,15 +503,14 @@ void run_sample_device(rbg_ctx *c, const FileView &f, const std::vector<Blk> &B,
     uint32_t *cnt = D.cntd[slot].as<uint32_t>();
     CK(cudaEventRecord(D.k0[slot], s));
     launch_depth_device(D.cdev[slot].as<uint8_t>(), D.tdev[slot].as<DevBlk>(), nb,
-                        (const uint64_t *)(D.tdev[slot].as<uint8_t>() + (size_t)nb * sizeof(DevBlk)),
                         hdr_chunk, D.outd[slot].as<uint8_t>(), cnt, cnt + nb + 1,
-                        D.offd[slot].as<uint32_t>(), flags, rec_total, d_tlen, P, sum,
+                        D.rawd[slot].as<uint32_t>(), D.offd[slot].as<uint32_t>(), flags, rec_total, d_tlen, P, sum,
                         p->dual_map_qual > 0 ? sum_u : nullptr, sms, s);
     CK(cudaGetLastError());
     CK(cudaEventRecord(D.k1[slot], s));
     CK(cudaEventRecord(D.ev[slot], s));
     timed[slot] = true;
-    c->launches += 5;
+    c->launches += 4;
     b0 = b1;
     slot ^= 1;
   }
@@ -550,8 +559,11 @@ void bam_depth(rbg_ctx *c, const std::vector<FileView> &files, const rbg_depth_p
     // every BAM through the device route without waiting in between, then one
     // read-back of all their status slots
     D.flags.ensure((size_t)16 * nb);
+    // (a call that ended early may have left a chunk on the other slot's stream)
+    if (D.ev[1]) CK(cudaStreamWaitEvent(s, D.ev[1], 0));
     CK(cudaMemsetAsync(D.flags.p, 0, (size_t)16 * nb, s));
     bool timed[2] = {false, false};
+    int next_slot = 0;
     std::vector<int32_t> pre_avg(nb, 0);
     for (int b = 0; b < nb; ++b) {
       std::vector<Blk> B;
@@ -562,8 +574,15 @@ void bam_depth(rbg_ctx *c, const std::vector<FileView> &files, const rbg_depth_p
       const auto t0 = Clock::now();
       Prefix pre = host_prefix(files[b], B, uoff, threads);
       walk_ms += ms_since(t0);
-      if (!have_h0) set_h0(pre.h);
-      else if (pre.h.tlen != h0.tlen) throw Error(RBG_ERR_ARG, "BAM files carry different contigs");
+      if (!have_h0) {
+        set_h0(pre.h);
+        // the other slot's stream starts after the cleared sums and flags
+        if (!D.ev_set) CK(cudaEventCreateWithFlags(&D.ev_set, cudaEventDisableTiming));
+        CK(cudaEventRecord(D.ev_set, s));
+        CK(cudaStreamWaitEvent(c->aux, D.ev_set, 0));
+      } else if (pre.h.tlen != h0.tlen) {
+        throw Error(RBG_ERR_ARG, "BAM files carry different contigs");
+      }
       const int32_t nt = (int32_t)h0.tlen.size();
       unsigned long long *sums_all = D.sums.as<unsigned long long>();
       depth::Params P{p->percent_identity,
@@ -571,10 +590,11 @@ void bam_depth(rbg_ctx *c, const std::vector<FileView> &files, const rbg_depth_p
                       p->min_map_qual, p->dual_map_qual, nt};
       run_sample_device(c, files[b], B, uoff, pre.hdr_end, P, p, D.tlen.as<uint32_t>(),
                         sums_all + (size_t)b * nt, sums_all + (size_t)(nb + b) * nt, threads,
-                        D.flags.as<uint8_t>() + (size_t)16 * b, timed, kernel_ms);
+                        D.flags.as<uint8_t>() + (size_t)16 * b, timed, kernel_ms, next_slot);
       pre_avg[b] = pre.avg;
     }
     D.hflag.ensure((size_t)16 * nb);
+    if (D.ev[1]) CK(cudaStreamWaitEvent(s, D.ev[1], 0));     // the other slot's last chunk
     CK(cudaMemcpyAsync(D.hflag.p, D.flags.p, (size_t)16 * nb, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     for (int i = 0; i < 2; ++i)

@@ -3,6 +3,7 @@
 // per-configuration table cache, the context, and the host steps of the
 // calibration.
 #pragma once
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <list>
@@ -66,17 +67,19 @@ struct DBuf {
   }
 };
 
-// Pinned host staging buffer.
+// Pinned host staging buffer; grows by at least half its size, as DBuf (pinning
+// costs milliseconds).
 struct HBuf {
   void *p = nullptr;
   size_t cap = 0;
   template <typename T> T *as() const { return (T *)p; }
   void ensure(size_t bytes) {
     if (bytes <= cap) return;
+    const size_t grown = cap + cap / 2;
     if (p) cudaFreeHost(p);
     p = nullptr;
     cap = 0;
-    const size_t want = bytes < 256 ? 256 : bytes;
+    const size_t want = std::max<size_t>(std::max<size_t>(bytes, grown), 256);
     CK(cudaMallocHost(&p, want));
     cap = want;
   }
@@ -259,17 +262,21 @@ struct DepthBufs {
   HBuf slot[2], offp[2];
   // device route: compressed chunk, block table, inflated chunk, counts and
   // scan, record offsets; the route's flags and record count
-  DBuf cdev[2], tdev[2], outd[2], cntd[2], offd[2], flags;
+  DBuf cdev[2], tdev[2], outd[2], cntd[2], rawd[2], offd[2], flags;
   HBuf cpin[2], tpin[2], hflag;
   cudaEvent_t ev[2] = {nullptr, nullptr};
   cudaEvent_t k0[2] = {nullptr, nullptr}, k1[2] = {nullptr, nullptr};   // per-record launch times
   cudaEvent_t evc[2] = {nullptr, nullptr};                             // device route: chunk copied
+  cudaEvent_t evp[2] = {nullptr, nullptr};                             // device route: piece copied
+  cudaEvent_t ev_set = nullptr;                                        // sums and flags cleared
   void release() {
     DBuf *all[] = {&buf[0], &buf[1], &off[0], &off[1], &sums, &tlen, &kept, &edge, &means,
                    &cdev[0], &cdev[1], &tdev[0], &tdev[1], &outd[0], &outd[1], &cntd[0],
-                   &cntd[1], &offd[0], &offd[1], &flags};
+                   &cntd[1], &offd[0], &offd[1], &rawd[0], &rawd[1], &flags};
     for (DBuf *b : all) b->release();
     hflag.release();
+    if (ev_set) cudaEventDestroy(ev_set);
+    ev_set = nullptr;
     for (int i = 0; i < 2; ++i) {
       slot[i].release();
       offp[i].release();
@@ -279,7 +286,8 @@ struct DepthBufs {
       if (k0[i]) cudaEventDestroy(k0[i]);
       if (k1[i]) cudaEventDestroy(k1[i]);
       if (evc[i]) cudaEventDestroy(evc[i]);
-      ev[i] = k0[i] = k1[i] = evc[i] = nullptr;
+      if (evp[i]) cudaEventDestroy(evp[i]);
+      ev[i] = k0[i] = k1[i] = evc[i] = evp[i] = nullptr;
     }
   }
 };

@@ -4,13 +4,13 @@
 // only to bytes of the same member, so every block decodes on its own: the
 // device runs one warp per block.  All lanes of the warp decode the same
 // symbols in lockstep (same bits, same tables: no divergence, broadcast loads);
-// the leader lane stores literals, and the lanes copy matches and stored
-// blocks together, in rounds no longer than the match distance so that every
-// byte read was written in an earlier round.  The same code runs on the host
-// with one lane (the CPU tests).  Symbols are decoded with a 9-bit (literal /
+// the lanes store literals and copy matches and stored blocks together (a match
+// that overlaps itself repeats its first `distance` bytes, all of them written
+// before it).  The same code runs on the host
+// with one lane (the CPU tests).  Symbols are decoded with a 10-bit (literal /
 // length) and 8-bit (distance) lookup table of 32-bit entries that carry each
-// symbol's meaning (literal byte, length or distance base, extra bits), with
-// the canonical code walk for longer codes.  Every read stays inside [in, in + inlen),
+// symbol's meaning (one or two literal bytes, length or distance base, extra
+// bits), with the canonical code walk for longer codes.  Every read stays inside [in, in + inlen),
 // every write inside [out, out + outlen), and every match must point into
 // bytes already written: a stream that breaks a rule ends with a status, never
 // with an access out of bounds.
@@ -38,7 +38,7 @@ enum Status : int32_t {
   kErrShort = 8         // less output than the block's ISIZE
 };
 
-constexpr int kLitBits = 9, kDistBits = 8;
+constexpr int kLitBits = 10, kDistBits = 8;
 
 // The lanes that decode one block: one host thread, or one device warp.
 struct SerialLanes {
@@ -63,13 +63,14 @@ struct WarpLanes {
 //   bits 0-3   code length (0: longer code, or no code)
 //   bits 4-5   kind: 0 literal / distance / code-length symbol, 1 length,
 //              2 end of block, 3 invalid symbol
-//   bits 6-9   extra bits that follow the code
-//   bits 16-31 value: the literal byte, the length or distance base, or the
-//              code-length symbol
+//   bits 6-9   extra bits that follow the code; 1 for a literal: two of them
+//   bits 16-31 value: the literal byte (then the second one's), the length or
+//              distance base, or the code-length symbol
 template <int kBits, int kSyms>
 struct Code {
   uint32_t lut[1 << kBits];
   uint16_t count[16];
+  uint16_t next[16], offs[16];         // while the code is built
   uint16_t sym[kSyms];
 };
 constexpr uint32_t kEndOfInput = 0xFFFFFFFFu, kNoCode = 0xFFFFFFFEu;
@@ -78,6 +79,7 @@ struct Tables {
   Code<kLitBits, 288> lit;
   Code<kDistBits, 32> dist;
   uint8_t lens[320];          // code lengths being read (litlen then distance)
+  uint8_t clens[20];          // code-length code lengths
 };
 
 struct Bits {
@@ -127,12 +129,16 @@ struct Bits {
 };
 
 RBG_IHD uint32_t reverse_bits(uint32_t v, int n) {
+#ifdef __CUDA_ARCH__
+  return __brev(v) >> (32 - n);        // n >= 1
+#else
   uint32_t r = 0;
   for (int i = 0; i < n; ++i) {
     r = (r << 1) | (v & 1);
     v >>= 1;
   }
   return r;
+#endif
 }
 
 // Length symbols 257 + i: i < 8 give 3 + i with no extra bits; then groups of
@@ -149,6 +155,7 @@ RBG_IHD uint32_t dist_base(int d) { return d < 4 ? 1u + d : ((2u + (d & 1)) << d
 
 // Table entries of the three codes.
 struct LitEntry {
+  static constexpr bool kPairs = true;
   RBG_IHD static uint32_t make(int s, int l) {
     if (s < 256) return (uint32_t)s << 16 | (uint32_t)l;
     if (s == 256) return 2u << 4 | (uint32_t)l;
@@ -158,48 +165,106 @@ struct LitEntry {
   }
 };
 struct DistEntry {
+  static constexpr bool kPairs = false;
   RBG_IHD static uint32_t make(int s, int l) {
     if (s >= 30) return 3u << 4 | (uint32_t)l;
     return dist_base(s) << 16 | (uint32_t)dist_extra(s) << 6 | (uint32_t)l;
   }
 };
 struct PlainEntry {
+  static constexpr bool kPairs = false;
   RBG_IHD static uint32_t make(int s, int l) { return (uint32_t)s << 16 | (uint32_t)l; }
 };
 
+// Table entry of two literals in a row, when e1 at index idx is a literal and the
+// bits after it hold another whole one; 0 otherwise.
+template <int kBits>
+RBG_IHD uint32_t literal_pair(uint32_t e1, uint32_t e2) {
+  const uint32_t l1 = e1 & 0x3F, l2 = e2 & 0x3F;       // length and kind: 1..15 for a literal
+  if (l1 - 1u >= 15u || l2 - 1u >= 15u || l1 + l2 > (uint32_t)kBits) return 0;
+  return (e2 >> 16) << 24 | (e1 >> 16) << 16 | 1u << 6 | (l1 + l2);
+}
+
 // Builds a code from `n` code lengths.  Incomplete codes are accepted (a code
-// of one distance symbol is legal); over-subscribed ones are not.
-template <class Entry, int kBits, int kSyms>
-RBG_IHD int build(Code<kBits, kSyms> &c, const uint8_t *len, int n) {
-  for (int i = 0; i < 16; ++i) c.count[i] = 0;
-  for (int s = 0; s < n; ++s) c.count[len[s]]++;
-  c.count[0] = 0;
+// of one distance symbol is legal); over-subscribed ones are not.  The lanes take
+// 32 symbols at a time: a symbol's canonical code follows from the symbols of its
+// length before it (the lanes below with the same length).
+template <class Entry, int kBits, int kSyms, class Lanes>
+RBG_IHD int build(Code<kBits, kSyms> &c, const uint8_t *len, int n, const Lanes &L) {
+  const int lane = L.lane(), W = L.width();
+  L.sync();
+  for (int i = lane; i < 16; i += W) c.count[i] = 0;
+  for (int i = lane; i < (1 << kBits); i += W) c.lut[i] = 0;
+  L.sync();
+#ifdef __CUDA_ARCH__
+  for (int s0 = 0; s0 < n; s0 += 32) {
+    const int l = s0 + lane < n ? len[s0 + lane] : 0;
+    const unsigned same = __match_any_sync(0xffffffffu, l);
+    if (l && lane == __ffs(same) - 1) c.count[l] = (uint16_t)(c.count[l] + __popc(same));
+    L.sync();
+  }
+#else
+  for (int s = 0; s < n; ++s)
+    if (len[s]) c.count[len[s]]++;
+#endif
   int left = 1;
   for (int l = 1; l < 16; ++l) {
     left <<= 1;
     left -= c.count[l];
     if (left < 0) return kErrCodes;
   }
-  uint16_t offs[16];
-  offs[1] = 0;
-  for (int l = 1; l < 15; ++l) offs[l + 1] = (uint16_t)(offs[l] + c.count[l]);
-  for (int s = 0; s < n; ++s)
-    if (len[s]) c.sym[offs[len[s]]++] = (uint16_t)s;
-  for (int i = 0; i < (1 << kBits); ++i) c.lut[i] = 0;
-  // canonical codes in symbol order, entered bit-reversed into the table
-  uint32_t code = 0, next[16];
-  for (int l = 1; l < 16; ++l) {
-    code = (code + c.count[l - 1]) << 1;
-    next[l] = code;
+  // canonical codes in symbol order
+  if (L.leader()) {
+    uint32_t code = 0, at = 0;
+    for (int l = 1; l < 16; ++l) {
+      code = (code + c.count[l - 1]) << 1;             // count[0] is 0
+      c.next[l] = (uint16_t)code;
+      c.offs[l] = (uint16_t)at;
+      at += c.count[l];
+    }
   }
-  for (int s = 0; s < n; ++s) {
-    const int l = len[s];
-    if (!l) continue;
-    const uint32_t cd = next[l]++;
-    if (l > kBits) continue;
-    const uint32_t r = reverse_bits(cd, l);
-    const uint32_t e = Entry::make(s, l);
-    for (uint32_t f = r; f < (1u << kBits); f += (1u << l)) c.lut[f] = e;
+  L.sync();
+  for (int s0 = 0; s0 < n; s0 += W) {
+    const int s = s0 + lane;
+    const int l = s < n ? len[s] : 0;
+    uint32_t cd = 0, at = 0;
+#ifdef __CUDA_ARCH__
+    const unsigned same = __match_any_sync(0xffffffffu, l);
+    const uint32_t rank = (uint32_t)__popc(same & ((1u << lane) - 1u));
+    if (l) {
+      cd = c.next[l] + rank;
+      at = c.offs[l] + rank;
+    }
+    L.sync();
+    if (l && rank == 0) {
+      c.next[l] = (uint16_t)(c.next[l] + __popc(same));
+      c.offs[l] = (uint16_t)(c.offs[l] + __popc(same));
+    }
+#else
+    if (l) {
+      cd = c.next[l]++;
+      at = c.offs[l]++;
+    }
+#endif
+    if (l) {
+      c.sym[at] = (uint16_t)s;
+      if (l <= kBits) {                                // entered bit-reversed into the table
+        const uint32_t r = reverse_bits(cd, l), e = Entry::make(s, l);
+        for (uint32_t f = r; f < (1u << kBits); f += (1u << l)) c.lut[f] = e;
+      }
+    }
+    L.sync();
+  }
+  if (Entry::kPairs) {
+    // from the last entry down: the bits after a literal index an entry at half
+    // the index or below, which still holds its single symbol
+    for (int i0 = (1 << kBits) - W; i0 >= 0; i0 -= W) {
+      const uint32_t e1 = c.lut[i0 + lane];
+      const uint32_t e = literal_pair<kBits>(e1, c.lut[(uint32_t)(i0 + lane) >> (e1 & 15)]);
+      L.sync();
+      if (e) c.lut[i0 + lane] = e;
+      L.sync();
+    }
   }
   return kOk;
 }
@@ -240,6 +305,10 @@ RBG_IHD int inflate_block(const uint8_t *in, uint32_t inlen, uint8_t *out, uint3
   const int lane = L.lane(), W = L.width();
   Bits b{in, inlen, 0, 0, 0};
   uint32_t o = 0;
+#ifdef __CUDA_ARCH__
+  uint32_t held = 0, held_at = 0;      // a copy read but not stored: lane k's byte of `held`
+  uint8_t held_v = 0;
+#endif
   for (;;) {
     uint32_t hdr;
     if (!b.get(3, hdr)) return kErrInput;
@@ -281,7 +350,7 @@ RBG_IHD int inflate_block(const uint8_t *in, uint32_t inlen, uint8_t *out, uint3
         if (nlen > 286 || ndist > 30) return kErrCodes;
         // code-length code: lengths in the fixed permuted order
         const uint8_t ord[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11, 4, 12, 3, 13, 2, 14, 1, 15};
-        uint8_t cl[19];
+        uint8_t *cl = T.clens;                         // the lanes write the same values
         for (int i = 0; i < 19; ++i) cl[i] = 0;
         for (uint32_t i = 0; i < hclen + 4; ++i) {
           uint32_t v;
@@ -291,8 +360,7 @@ RBG_IHD int inflate_block(const uint8_t *in, uint32_t inlen, uint8_t *out, uint3
         // the code-length code decodes through the distance table's storage
         // (it has 19 symbols and codes of at most 7 bits)
         Code<kDistBits, 32> &cc = T.dist;
-        if (build<PlainEntry>(cc, cl, 19) != kOk) return kErrCodes;
-        L.sync();
+        if (build<PlainEntry>(cc, T.clens, 19, L) != kOk) return kErrCodes;
         int i = 0;
         while (i < nlen + ndist) {
           const uint32_t ce = decode<PlainEntry>(cc, b);
@@ -324,10 +392,26 @@ RBG_IHD int inflate_block(const uint8_t *in, uint32_t inlen, uint8_t *out, uint3
         if (T.lens[256] == 0) return kErrCodes;       // no end-of-block code
       }
       L.sync();
-      if (build<LitEntry>(T.lit, T.lens, nlen) != kOk) return kErrCodes;
-      if (build<DistEntry>(T.dist, T.lens + 288, ndist) != kOk) return kErrCodes;
+      if (build<LitEntry>(T.lit, T.lens, nlen, L) != kOk) return kErrCodes;
+      if (build<DistEntry>(T.dist, T.lens + 288, ndist, L) != kOk) return kErrCodes;
       L.sync();
       for (;;) {
+        // one or two literals from the table, the common case
+        if (b.cnt < 15) b.refill();
+        const uint32_t q = T.lit.lut[b.peek(kLitBits)];
+        if ((q & 0x3F) - 1u < 15u && (int)(q & 15) <= b.cnt) {
+          const uint32_t two = (q >> 6) & 1;
+          b.drop(q & 15);
+          if (o + two >= outlen) return kErrOutput;
+#ifdef __CUDA_ARCH__
+          if ((uint32_t)lane <= two) out[o + lane] = (uint8_t)(q >> (16 + 8 * lane));
+#else
+          out[o] = (uint8_t)(q >> 16);
+          if (two) out[o + 1] = (uint8_t)(q >> 24);
+#endif
+          o += 1 + two;
+          continue;
+        }
         const uint32_t e = decode<LitEntry>(T.lit, b);
         if (e >= kNoCode) return e == kEndOfInput ? kErrInput : kErrSymbol;
         const uint32_t kind = (e >> 4) & 3;
@@ -337,7 +421,13 @@ RBG_IHD int inflate_block(const uint8_t *in, uint32_t inlen, uint8_t *out, uint3
           ++o;
           continue;
         }
-        if (kind == 2) break;
+        if (kind == 2) {
+#ifdef __CUDA_ARCH__
+          if ((uint32_t)lane < held) out[held_at + lane] = held_v;
+          held = 0;
+#endif
+          break;
+        }
         if (kind == 3) return kErrSymbol;
         uint32_t len = e >> 16, ex;
         const int le = (int)((e >> 6) & 15);
@@ -356,16 +446,28 @@ RBG_IHD int inflate_block(const uint8_t *in, uint32_t inlen, uint8_t *out, uint3
         }
         if (dist > o) return kErrDistance;
         if (len > outlen - o) return kErrOutput;
-        // rounds of at most `dist` bytes: each round reads only bytes written
-        // before it (the leader's literals included, after the barrier)
-        L.sync();
+        // the bytes read are all written before the match: a match longer than its
+        // distance repeats the first `dist` of them
         const uint8_t *src = out + (o - dist);
         uint8_t *dst = out + o;
-        for (uint32_t base = 0; base < len; base += dist) {
-          const uint32_t step = len - base < dist ? len - base : dist;
-          for (uint32_t k = lane; k < step; k += W) dst[base + k] = src[base + k];
-          if (base + step < len) L.sync();
+#ifdef __CUDA_ARCH__
+        // The copy of up to 32 bytes is stored at the next one: the loads' latency
+        // passes under the symbols decoded in between.
+        if ((uint32_t)lane < held) out[held_at + lane] = held_v;
+        held = 0;
+        L.sync();
+        if (len <= 32) {
+          if ((uint32_t)lane < len) held_v = src[dist >= len ? lane : lane % dist];
+          held = len;
+          held_at = o;
+        } else if (dist >= len) {
+          for (uint32_t k = lane; k < len; k += W) dst[k] = src[k];
+        } else {
+          for (uint32_t k = lane; k < len; k += W) dst[k] = src[k % dist];
         }
+#else
+        for (uint32_t k = 0; k < len; ++k) dst[k] = src[dist >= len ? k : k % dist];
+#endif
         o += len;
       }
     } else {

@@ -1,6 +1,7 @@
 // BAM -> depth summariser, device side: BGZF inflation, the record walk,
 // per-record depth sums and the means matrix.  Two routes feed the sums:
-// the device route (k_inflate, k_walk, k_scan_counts, k_depth_reads_dev) takes
+// the device route (k_inflate, k_scan_counts, k_gather_offsets,
+// k_depth_reads_dev) takes
 // a chunk of compressed blocks; the host route (bam.cpp inflates and walks)
 // hands over decompressed records with one offset per record (k_depth_reads).
 //
@@ -17,7 +18,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cstdlib>
 
 #include "depth_record.cuh"
 #include "inflate.cuh"
@@ -82,11 +82,22 @@ __global__ void k_depth_means(const unsigned long long *__restrict__ sums, int64
 // (inflate.cuh: the lanes decode in lockstep and copy together; the warp's
 // Huffman tables in shared memory) and checks its CRC32 (lane segments joined
 // over GF(2)).  Failures set bit 0 of *flags.
-template <int kMinCtas>
-__global__ void __launch_bounds__(kInflateWarps * 32, kMinCtas) k_inflate(const uint8_t *__restrict__ comp,
-                                                               const DevBlk *__restrict__ blk,
-                                                               int nb, uint8_t *__restrict__ out,
-                                                               uint32_t *__restrict__ flags) {
+//
+// Then the block's record chain, while its bytes are near, assuming every block
+// starts on a record (as htslib writes BGZF: a record that would not fit starts
+// the next block): from the block's start (or the header's end) records are
+// followed to the block's end, their offsets listed from raw[uofs / 36] on (a
+// record has at least 36 bytes).  A record that does not fit, or a chain that does
+// not end exactly at the block's end, sets bit 1 of *flags (the file then goes
+// through the host walk).
+//
+// Bound by each block's serial decode chain; few warps a CTA spread the blocks of
+// a small file evenly.  3,100 blocks (200 MB inflated): 7.3 ms a launch -> 5.65 ms,
+// the chains (0.64 ms in a kernel of their own) included.
+__global__ void __launch_bounds__(kInflateWarps * 32, 32 / kInflateWarps)
+k_inflate(const uint8_t *__restrict__ comp, const DevBlk *__restrict__ blk, int nb,
+          uint64_t hdr_end, uint8_t *__restrict__ out, uint32_t *__restrict__ counts,
+          uint32_t *__restrict__ raw, uint32_t *__restrict__ flags) {
   __shared__ uint32_t crc_t[256];
   __shared__ inflate::Tables tabs[kInflateWarps];
   for (int i = threadIdx.x; i < 256; i += blockDim.x) {
@@ -102,44 +113,41 @@ __global__ void __launch_bounds__(kInflateWarps * 32, kMinCtas) k_inflate(const 
     int st = inflate::inflate_block(comp + b.cofs, b.clen, out + b.uofs, b.isize, tabs[w], L);
     __syncwarp();
     if (st == inflate::kOk && inflate::crc32(crc_t, out + b.uofs, b.isize, L) != b.crc) st = 9;
-    if (st != inflate::kOk && L.leader()) atomicOr(flags, 1u);
+    if (L.leader()) {
+      uint32_t n = 0;
+      if (st != inflate::kOk) {
+        atomicOr(flags, 1u);
+      } else {
+        const uint64_t hi = b.uofs + b.isize;
+        uint64_t p = b.uofs < hdr_end ? hdr_end : b.uofs;
+        uint32_t *list = raw + b.uofs / 36;
+        while (p < hi) {
+          const uint32_t rb = depth::record_bytes(out + p, hi - p);
+          if (!rb) {
+            atomicOr(flags, 2u);
+            break;
+          }
+          list[n++] = (uint32_t)p;
+          p += rb;
+        }
+      }
+      counts[i] = n;
+    }
     __syncwarp();
   }
 }
 
-// Record chain of each block, assuming every block starts on a record (as
-// htslib writes BGZF: a record that would not fit starts the next block):
-// from the block's start (or the header's end) records are followed to the
-// block's end.  A record that does not fit the chunk, or a chain that does not
-// end exactly at the block's end, sets bit 1 of *flags (the file then goes
-// through the host walk).  Pass 0 counts, pass 1 writes the records' offsets
-// at the block's place in the scan.
-__global__ void k_walk(const uint8_t *__restrict__ out, const uint64_t *__restrict__ ubound, int nb,
-                       uint64_t hdr_end, uint32_t *__restrict__ counts,
-                       const uint32_t *__restrict__ scan, uint32_t *__restrict__ offs,
-                       uint32_t *__restrict__ flags, int pass) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// The blocks' record offsets in file order, back to back (warp per block).
+__global__ void __launch_bounds__(256) k_gather_offsets(const DevBlk *__restrict__ blk, int nb,
+                                                        const uint32_t *__restrict__ counts,
+                                                        const uint32_t *__restrict__ scan,
+                                                        const uint32_t *__restrict__ raw,
+                                                        uint32_t *__restrict__ offs) {
+  const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i >= nb) return;
-  const uint64_t end = ubound[nb];
-  uint64_t p = ubound[i] < hdr_end ? hdr_end : ubound[i];
-  const uint64_t hi = ubound[i + 1];
-  uint32_t n = 0, base = pass ? scan[i] : 0;
-  bool bad = false;
-  while (p < hi) {
-    const uint32_t rb = depth::record_bytes(out + p, end - p);
-    if (!rb) {
-      bad = true;
-      break;
-    }
-    if (pass) offs[base + n] = (uint32_t)p;
-    ++n;
-    p += rb;
-  }
-  if (!pass) {
-    counts[i] = n;
-    const uint64_t start = ubound[i] < hdr_end ? hdr_end : ubound[i];
-    if (bad || (start < hi && p != hi)) atomicOr(flags, 2u);
-  }
+  const uint32_t n = counts[i], to = scan[i];
+  const uint32_t *from = raw + blk[i].uofs / 36;
+  for (uint32_t k = threadIdx.x & 31; k < n; k += 32) offs[to + k] = from[k];
 }
 
 // Exclusive scan of the per-block counts (one CTA); scan[nb] = total, also
@@ -229,29 +237,19 @@ void launch_depth_means(const unsigned long long *sums, int64_t n_targets, const
                                                               target_len, edge_of_col, ncols, out);
 }
 
-void launch_depth_device(const uint8_t *comp, const DevBlk *blk, int nb, const uint64_t *ubound,
-                         uint64_t hdr_end, uint8_t *out, uint32_t *counts, uint32_t *scan,
+void launch_depth_device(const uint8_t *comp, const DevBlk *blk, int nb, uint64_t hdr_end,
+                         uint8_t *out, uint32_t *counts, uint32_t *scan, uint32_t *raw,
                          uint32_t *offs, uint32_t *flags, unsigned long long *rec_total,
                          const uint32_t *target_len, const depth::Params &P,
                          unsigned long long *sum, unsigned long long *sum_u, int sms,
                          cudaStream_t s) {
   if (nb <= 0) return;
-  // four CTAs per SM (64 registers, a few spilled: 40 ms against 46 ms for the
-  // 80-register build on the 5.6 M-read benchmark BAM); RBG_INFLATE_CTAS=3
-  // takes the 80-register build
-  static const int per_sm = [] {
-    const char *e = getenv("RBG_INFLATE_CTAS");
-    return (e && atoi(e) == 3) ? 3 : 4;
-  }();
-  const int ctas = std::min((nb + kInflateWarps - 1) / kInflateWarps, sms * per_sm);
-  if (per_sm == 4)
-    k_inflate<4><<<ctas, kInflateWarps * 32, 0, s>>>(comp, blk, nb, out, flags);
-  else
-    k_inflate<3><<<ctas, kInflateWarps * 32, 0, s>>>(comp, blk, nb, out, flags);
-  const unsigned g = (unsigned)((nb + 127) / 128);
-  k_walk<<<g, 128, 0, s>>>(out, ubound, nb, hdr_end, counts, scan, offs, flags, 0);
+  // up to 32 warps a SM (64 registers, a few spilled: 40 ms against 46 ms at 24
+  // warps of 80 registers on a 5.6 M-read BAM)
+  const int ctas = std::min((nb + kInflateWarps - 1) / kInflateWarps, sms * (32 / kInflateWarps));
+  k_inflate<<<ctas, kInflateWarps * 32, 0, s>>>(comp, blk, nb, hdr_end, out, counts, raw, flags);
   k_scan_counts<<<1, 1024, 0, s>>>(counts, nb, scan, rec_total);
-  k_walk<<<g, 128, 0, s>>>(out, ubound, nb, hdr_end, counts, scan, offs, flags, 1);
+  k_gather_offsets<<<(unsigned)((nb + 7) / 8), 256, 0, s>>>(blk, nb, counts, scan, raw, offs);
   k_depth_reads_dev<<<(unsigned)(sms * 8), 256, 0, s>>>(out, offs, scan + nb, flags, target_len, P,
                                                         sum, sum_u);
 }

@@ -64,7 +64,7 @@ struct DevBlk {
   uint32_t cofs, clen, isize, crc;
   uint64_t uofs;
 };
-constexpr int kInflateWarps = 8;        // BGZF blocks in flight per CTA of the inflate kernel
+constexpr int kInflateWarps = 2;        // BGZF blocks in flight per CTA of the inflate kernel
 
 // ── kernel launchers (kernels_*.cu) ─────────────────────────────────────────
 struct SketchArgs {
@@ -445,14 +445,14 @@ void launch_fasta_scatter(const uint8_t *in, int64_t F, const int64_t *nl_base,
                           cudaStream_t s);
 // flag[0..ngt] becomes the exclusive scan of record-start flags; rs the starts.
 void launch_fasta_starts(const int64_t *gt_pos, int64_t ngt, const int64_t *nl_pos, int64_t nnl,
-                         int64_t *flag, int64_t *rs, cudaStream_t s);
+                         int32_t *flag, int64_t *rank, int64_t *rs, cudaStream_t s);
 void launch_fasta_records(const uint8_t *in, int64_t F, const int64_t *rs, int64_t nrs,
                           const int64_t *nl_pos, int64_t nnl, int64_t min_contig,
                           int64_t min_small, FastaRec *rec, cudaStream_t s);
 // Exclusive scans of class-c membership (output index) and length (byte
 // offset) over the records, totals at [nrs].
-void launch_fasta_class(const FastaRec *rec, int64_t nrs, int c, int64_t *flag, int64_t *bytes,
-                        cudaStream_t s);
+void launch_fasta_class(const FastaRec *rec, int64_t nrs, int c, int32_t *flag, int64_t *bytes,
+                        int64_t *idx, int64_t *off, cudaStream_t s);
 void launch_fasta_copy(const uint8_t *in, const FastaRec *rec, int64_t nrs, const int64_t *nl_pos,
                        int c, const int64_t *idx, const int64_t *off, uint8_t *out,
                        int64_t *out_off, int64_t *name_start, int32_t *name_len, cudaStream_t s);
@@ -478,7 +478,7 @@ void launch_lpa_scatter(const uint32_t *from, const uint32_t *to, const float *s
                         int64_t n, const int64_t *off, uint32_t *fill, uint64_t *key,
                         cudaStream_t s);
 void launch_lpa_sort(const int64_t *off, int64_t n, uint64_t *key, const float *q, uint32_t *nbr,
-                     float *w, cudaStream_t s);
+                     float *w, uint32_t *big, cudaStream_t s);
 void launch_lpa_init(const uint32_t *order, int64_t n, uint32_t *pos, uint32_t *label,
                      uint8_t *active, uint8_t *next_active, uint8_t *frozen, uint64_t *state,
                      uint32_t *vcnt, uint32_t *vnext, cudaStream_t s);
