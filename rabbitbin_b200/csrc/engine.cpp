@@ -91,7 +91,7 @@ void stage(rbg_ctx *c, const char *seqcat, const int64_t *offsets, int64_t n,
            const float *depth, int S) {
   stage_meta(c, seqcat, offsets, n, depth, S);
   const size_t abytes = (size_t)((c->nbases + 15) / 16) * 16 + 16;
-  CK(cudaMemsetAsync(c->ascii.p, 0, abytes, c->stream));
+  CK(cudaMemsetAsync(c->ascii.as<char>() + c->nbases, 0, abytes - (size_t)c->nbases, c->stream));
   if (c->nbases)
     CK(cudaMemcpyAsync(c->ascii.p, seqcat, (size_t)c->nbases, cudaMemcpyHostToDevice, c->stream));
 }
@@ -113,7 +113,7 @@ void stage_device(rbg_ctx *c, const char *dseq, const int64_t *doffsets, int64_t
   c->ascii.ensure(abytes);
   c->offsets.ensure((n + 1) * sizeof(int64_t));
   c->depth.ensure(std::max<size_t>(1, (size_t)n * S) * sizeof(float));
-  CK(cudaMemsetAsync(c->ascii.p, 0, abytes, c->stream));
+  CK(cudaMemsetAsync(c->ascii.as<char>() + nbases, 0, abytes - (size_t)nbases, c->stream));
   if (nbases)
     CK(cudaMemcpyAsync(c->ascii.p, dseq, (size_t)nbases, cudaMemcpyDeviceToDevice, c->stream));
   CK(cudaMemcpyAsync(c->offsets.p, doffsets, (n + 1) * sizeof(int64_t), cudaMemcpyDeviceToDevice,

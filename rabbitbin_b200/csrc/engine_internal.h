@@ -228,10 +228,10 @@ struct BatchBufs {
 
 // Buffers of the device FASTA parser.
 struct FastaBufs {
-  DBuf in, tile_nl, tile_gt, nl_base, gt_base, nl_pos, gt_pos, flag, rs, rec;
+  DBuf in, tile_nl, tile_gt, nl_base, gt_base, nl_pos, gt_pos, flag, rank, bytes, rs, rec;
   DBuf idx[2], off[2], seq[2], seq_off[2], name_start[2], name_len[2];
   void release() {
-    DBuf *all[] = {&in, &tile_nl, &tile_gt, &nl_base, &gt_base, &nl_pos, &gt_pos, &flag, &rs,
+    DBuf *all[] = {&in, &tile_nl, &tile_gt, &nl_base, &gt_base, &nl_pos, &gt_pos, &flag, &rank, &bytes, &rs,
                    &rec, &idx[0], &idx[1], &off[0], &off[1], &seq[0], &seq[1], &seq_off[0],
                    &seq_off[1], &name_start[0], &name_start[1], &name_len[0], &name_len[1]};
     for (DBuf *b : all) b->release();

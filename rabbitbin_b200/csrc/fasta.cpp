@@ -20,7 +20,8 @@ FastaCounts fasta_parse(rbg_ctx *c, const char *data, int64_t F, int64_t min_con
   const int64_t words = (F + 15) / 16;
   const int64_t tiles = (words + 255) / 256;
   B.in.ensure((size_t)words * 16 + 16);
-  CK(cudaMemsetAsync(B.in.p, 0, (size_t)words * 16 + 16, s));
+  const size_t tail = (size_t)F & ~(size_t)15;            // the last word and the padding
+  CK(cudaMemsetAsync(B.in.as<char>() + tail, 0, (size_t)words * 16 + 16 - tail, s));
   if (F) CK(cudaMemcpyAsync(B.in.p, data, (size_t)F, cudaMemcpyHostToDevice, s));
   const uint8_t *in = B.in.as<uint8_t>();
   B.tile_nl.ensure(std::max<int64_t>(tiles, 1) * sizeof(int));
@@ -39,49 +40,53 @@ FastaCounts fasta_parse(rbg_ctx *c, const char *data, int64_t F, int64_t min_con
   B.gt_pos.ensure(std::max<int64_t>(ngt, 1) * sizeof(int64_t));
   launch_fasta_scatter(in, F, B.nl_base.as<int64_t>(), B.gt_base.as<int64_t>(),
                        B.nl_pos.as<int64_t>(), B.gt_pos.as<int64_t>(), s);
-  B.flag.ensure((ngt + 1) * sizeof(int64_t));
+  B.flag.ensure((ngt + 1) * sizeof(int32_t));
+  B.rank.ensure((ngt + 1) * sizeof(int64_t));
   B.rs.ensure(std::max<int64_t>(ngt, 1) * sizeof(int64_t));
-  CK(cudaMemsetAsync(B.flag.p, 0, (ngt + 1) * sizeof(int64_t), s));
+  CK(cudaMemsetAsync(B.rank.p, 0, (ngt + 1) * sizeof(int64_t), s));
   launch_fasta_starts(B.gt_pos.as<int64_t>(), ngt, B.nl_pos.as<int64_t>(), nnl,
-                      B.flag.as<int64_t>(), B.rs.as<int64_t>(), s);
+                      B.flag.as<int32_t>(), B.rank.as<int64_t>(), B.rs.as<int64_t>(), s);
   int64_t nrs = 0;
-  CK(cudaMemcpyAsync(&nrs, B.flag.as<int64_t>() + ngt, 8, cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(&nrs, B.rank.as<int64_t>() + ngt, 8, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   B.rec.ensure(std::max<int64_t>(nrs, 1) * sizeof(FastaRec));
   launch_fasta_records(in, F, B.rs.as<int64_t>(), nrs, B.nl_pos.as<int64_t>(), nnl, min_contig,
                        min_small, B.rec.as<FastaRec>(), s);
-  // records without a header newline (a suffix of the records) are not counted
-  int64_t dropped = 0;
-  {
-    B.idx[0].ensure((nrs + 1) * sizeof(int64_t));
-    B.off[0].ensure((nrs + 1) * sizeof(int64_t));
-    CK(cudaMemsetAsync(B.idx[0].p, 0, (nrs + 1) * sizeof(int64_t), s));
-    launch_fasta_class(B.rec.as<FastaRec>(), nrs, 3, B.idx[0].as<int64_t>(), B.off[0].as<int64_t>(), s);
-    CK(cudaMemcpyAsync(&dropped, B.idx[0].as<int64_t>() + nrs, 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-  }
-  out.num_seqs = nrs - dropped;
-  for (int slot = 0; slot < 2; ++slot) {
-    const int cls = slot == 0 ? 2 : 1;
+  // Index and byte offset of every record among the large (slot 0) and small
+  // (slot 1) ones, and the count of records without a header newline (a suffix of
+  // the records; not counted), read back together.
+  int64_t cnt[2][2] = {{0, 0}, {0, 0}}, dropped = 0;
+  B.flag.ensure(std::max<int64_t>(nrs, 1) * sizeof(int32_t));
+  B.bytes.ensure(std::max<int64_t>(nrs, 1) * sizeof(int64_t));
+  for (int k = 2; k >= 0; --k) {                           // dropped first, in slot 0's arrays
+    const int slot = k & 1;
     B.idx[slot].ensure((nrs + 1) * sizeof(int64_t));
     B.off[slot].ensure((nrs + 1) * sizeof(int64_t));
     CK(cudaMemsetAsync(B.idx[slot].p, 0, (nrs + 1) * sizeof(int64_t), s));
     CK(cudaMemsetAsync(B.off[slot].p, 0, (nrs + 1) * sizeof(int64_t), s));
-    launch_fasta_class(B.rec.as<FastaRec>(), nrs, cls, B.idx[slot].as<int64_t>(),
+    launch_fasta_class(B.rec.as<FastaRec>(), nrs, k == 2 ? 3 : (slot == 0 ? 2 : 1),
+                       B.flag.as<int32_t>(), B.bytes.as<int64_t>(), B.idx[slot].as<int64_t>(),
                        B.off[slot].as<int64_t>(), s);
-    int64_t cnt[2] = {0, 0};
-    CK(cudaMemcpyAsync(&cnt[0], B.idx[slot].as<int64_t>() + nrs, 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&cnt[1], B.off[slot].as<int64_t>() + nrs, 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    out.n[slot] = cnt[0];
-    out.bytes[slot] = cnt[1];
-    const size_t sb = (size_t)((cnt[1] + 15) / 16) * 16 + 16;
+    CK(cudaMemcpyAsync(k == 2 ? &dropped : &cnt[slot][0], B.idx[slot].as<int64_t>() + nrs, 8,
+                       cudaMemcpyDeviceToHost, s));
+    if (k < 2)
+      CK(cudaMemcpyAsync(&cnt[slot][1], B.off[slot].as<int64_t>() + nrs, 8,
+                         cudaMemcpyDeviceToHost, s));
+  }
+  CK(cudaStreamSynchronize(s));
+  out.num_seqs = nrs - dropped;
+  for (int slot = 0; slot < 2; ++slot) {
+    const int cls = slot == 0 ? 2 : 1;
+    const int64_t n = cnt[slot][0], bytes = cnt[slot][1];
+    out.n[slot] = n;
+    out.bytes[slot] = bytes;
+    const size_t sb = (size_t)((bytes + 15) / 16) * 16 + 16;
     B.seq[slot].ensure(sb);
-    B.seq_off[slot].ensure((cnt[0] + 1) * sizeof(int64_t));
-    B.name_start[slot].ensure(std::max<int64_t>(cnt[0], 1) * sizeof(int64_t));
-    B.name_len[slot].ensure(std::max<int64_t>(cnt[0], 1) * sizeof(int32_t));
-    CK(cudaMemsetAsync(B.seq[slot].p, 0, sb, s));
-    CK(cudaMemsetAsync(B.seq_off[slot].p, 0, (cnt[0] + 1) * sizeof(int64_t), s));
+    B.seq_off[slot].ensure((n + 1) * sizeof(int64_t));
+    B.name_start[slot].ensure(std::max<int64_t>(n, 1) * sizeof(int64_t));
+    B.name_len[slot].ensure(std::max<int64_t>(n, 1) * sizeof(int32_t));
+    CK(cudaMemsetAsync(B.seq[slot].as<char>() + bytes, 0, sb - (size_t)bytes, s));
+    CK(cudaMemsetAsync(B.seq_off[slot].p, 0, (n + 1) * sizeof(int64_t), s));
     launch_fasta_copy(in, B.rec.as<FastaRec>(), nrs, B.nl_pos.as<int64_t>(), cls,
                       B.idx[slot].as<int64_t>(), B.off[slot].as<int64_t>(),
                       B.seq[slot].as<uint8_t>(), B.seq_off[slot].as<int64_t>(),

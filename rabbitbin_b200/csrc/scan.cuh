@@ -1,4 +1,4 @@
-// Exclusive prefix sums of n 32-bit counts over many blocks in one launch, without
+// Exclusive prefix sums of n counts over many blocks in one launch, without
 // scratch: block b adds up everything before its tile itself (the counts are in
 // L2) and scans its tile.  Latency-bound at these sizes: one block walking the
 // counts took 50 us at 50,000 rows and 0.2 ms at 200,000; 13 us here at 50,000.
@@ -26,8 +26,8 @@ __device__ __forceinline__ int64_t scan_block_sum(int64_t v, int64_t *sh) {
 
 // out[0 .. n] = exclusive prefix sums of in[0 .. n-1] (out[n] the total); out does
 // not overlap in.  tile: a multiple of kScanThreads; block b scans tile b.
-template <class T>
-__global__ void __launch_bounds__(kScanThreads) k_exclusive_scan(const int32_t *__restrict__ in,
+template <class I, class T>
+__global__ void __launch_bounds__(kScanThreads) k_exclusive_scan(const I *__restrict__ in,
                                                                  T *__restrict__ out, int64_t n,
                                                                  int64_t tile) {
   __shared__ int64_t sh[kScanThreads / 32 + 1];
@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(kScanThreads) k_exclusive_scan(const int32_t *
   int64_t run = scan_block_sum(before, sh);
   for (int64_t q0 = lo; q0 < hi; q0 += kScanThreads) {
     const int64_t q = q0 + t;
-    const int32_t x = q < hi ? in[q] : 0;
+    const I x = q < hi ? in[q] : (I)0;
     int64_t incl = x;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -63,12 +63,12 @@ __global__ void __launch_bounds__(kScanThreads) k_exclusive_scan(const int32_t *
 
 // Tiles of 2,048 counts, and at most 512 of them: every block reads all counts
 // before its own.
-template <class T>
-inline void launch_exclusive_scan(const int32_t *in, T *out, int64_t n, cudaStream_t s) {
+template <class I, class T>
+inline void launch_exclusive_scan(const I *in, T *out, int64_t n, cudaStream_t s) {
   int64_t tile = std::max<int64_t>(2048, (n + 511) / 512);
   tile = (tile + kScanThreads - 1) / kScanThreads * kScanThreads;
   const int64_t blocks = std::max<int64_t>(1, (n + tile - 1) / tile);
-  k_exclusive_scan<T><<<(unsigned)blocks, kScanThreads, 0, s>>>(in, out, n, tile);
+  k_exclusive_scan<I, T><<<(unsigned)blocks, kScanThreads, 0, s>>>(in, out, n, tile);
 }
 
 }  // namespace rbg
