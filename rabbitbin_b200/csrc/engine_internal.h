@@ -242,12 +242,12 @@ struct FastaBufs {
 // incidence lists and the sweep state.
 struct LpaBufs {
   DBuf from, to, score, q, deg, off, fill, key, nbr, w, early, rec, order, pos, label, act0,
-      act1, frozen, done, prop, vlab, vcnt, vnext, misc, gtab;
+      act1, frozen, done, prop, vlab, vcnt, vnext, misc, gtab, big;
   HBuf pin, order_pin;
   void release() {
     DBuf *all[] = {&from, &to, &score, &q, &deg, &off, &fill, &key, &nbr, &w, &early, &rec, &order, &pos,
                    &label, &act0, &act1, &frozen, &done, &prop, &vlab, &vcnt, &vnext, &misc,
-                   &gtab};
+                   &gtab, &big};
     for (DBuf *b : all) b->release();
     pin.release();
     order_pin.release();

@@ -11,6 +11,7 @@
 
 #include "rbg_internal.h"
 #include "scan.cuh"
+#include "warp_sort.cuh"
 
 namespace rbg {
 namespace {
@@ -308,39 +309,6 @@ __host__ __device__ __forceinline__ int pow2_at_least(int x) {
   int p = 1;
   while (p < x) p <<= 1;
   return p;
-}
-
-// Ascending bitonic sort of 32 R keys held in registers, element r * 32 + lane
-// in v[r]: strides of 32 and more pair registers of the same lane, shorter
-// strides pair lanes through shuffles.
-template <int R>
-__device__ __forceinline__ void warp_bitonic_asc(uint64_t (&v)[R]) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int size = 2; size <= 32 * R; size <<= 1) {
-#pragma unroll
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      if (stride >= 32) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int p = r ^ (stride >> 5);
-          if (p > r) {
-            const bool up = (((r * 32 + lane) & size) == 0);
-            const uint64_t x = v[r], y = v[p];
-            if ((x > y) == up) { v[r] = y; v[p] = x; }
-          }
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const uint64_t o = __shfl_xor_sync(FULL, v[r], stride);
-          const bool up = (((r * 32 + lane) & size) == 0);
-          const bool lower = (lane & stride) == 0;
-          v[r] = (lower == up) ? (v[r] < o ? v[r] : o) : (v[r] < o ? o : v[r]);
-        }
-      }
-    }
-  }
 }
 
 // The first `len` (= 32 R) keys of buf, ascending, written out as ids and

@@ -112,11 +112,12 @@ void propagate(rbg_ctx *c, const rbg_lpa_params *lp, int64_t n, const EdgeView &
   B.nbr.ensure(a1 * 4);
   B.w.ensure(a1 * 4);
   B.fill.ensure((size_t)std::max<int64_t>(n, 1) * 4);
+  B.big.ensure((size_t)(n + 1) * 4);
   CK(cudaMemsetAsync(B.fill.p, 0, (size_t)n * 4, s));
   launch_lpa_scatter(ev.from, ev.to, ev.score, E, n, B.off.as<int64_t>(), B.fill.as<uint32_t>(),
                      B.key.as<uint64_t>(), s);
   launch_lpa_sort(B.off.as<int64_t>(), n, B.key.as<uint64_t>(), B.q.as<float>(),
-                  B.nbr.as<uint32_t>(), B.w.as<float>(), s);
+                  B.nbr.as<uint32_t>(), B.w.as<float>(), B.big.as<uint32_t>(), s);
   CK(cudaEventRecord(e1, s));
 
   // ── sweep state ──
