@@ -182,7 +182,9 @@ int64_t batch_request_bytes(const rbg_params *p, int64_t n, int64_t nbases, int 
     int GR = 1, GC = 1;
     onehot_mma_grid((int)((n + 255) / 256), (int)((n + 255) / 256), 148, &GR, &GC);
     b += n * (int64_t)std::max(128, 136 * m / 8) +
-         ((n + 31) / 32) * 32 * 2 * GC * ((int64_t)onehot_mma_cap(n, GC, K, 0) * 4 + 4);
+         (onehot_sym_fits(n, m)                                  // or the count matrix
+              ? n * onehot_sym_ldc(n) * 2
+              : ((n + 31) / 32) * 32 * 2 * GC * ((int64_t)onehot_mma_cap(n, GC, K, 0) * 4 + 4));
   }
   else
     b += ((n + 31) / 32) * P * 32 * (cap * 8 + 4);               // slice candidate buffers

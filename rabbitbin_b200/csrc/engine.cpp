@@ -557,9 +557,11 @@ void index_graph(rbg_ctx *c, const rbg_params *p, const GraphArgs &g, double cut
 
 // Dense regime (no abundance prune): the counts of rows [g.row_lo, row_hi)
 // against every contig as the product of one-hot int8 rows on the tensor
-// cores (k_onehot_mma, int32 accumulation in TMEM: exact), consumed in the
+// cores (int32 accumulation in TMEM: exact).  A whole assembly of up to 32,768
+// contigs: each pair once (k_onehot_sym), the counts in a matrix of 2 n^2 bytes,
+// each row's top-K and maxima from its row.  Else k_onehot_mma, consumed in the
 // kernel into per-(row, column group) candidate lists, the row maxima and the
-// compared-pair count; k_merge_topk then gives each row its top-K keys.
+// compared-pair count; k_merge_onehot then gives each row its top-K keys.
 }  // namespace
 
 namespace rbg {
@@ -585,23 +587,31 @@ void dense_allpairs_onehot(rbg_ctx *c, const GraphArgs &g) {
   int dev = 0, sms = 148;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  int GR = 1, GC = 1;
-  onehot_mma_grid((int)((rows + 255) / 256), (int)((n + 255) / 256), sms, &GR, &GC);
-  // RBG_ONEHOT_CAP: shorter lists, to exercise the cut inside the kernel
+  // RBG_ONEHOT_CAP: shorter lists, to exercise the cut inside the list kernel
   const char *cap_env = getenv("RBG_ONEHOT_CAP");
-  const int cap = onehot_mma_cap(n, GC, g.K, cap_env ? atoi(cap_env) : 0);
-  const size_t lists = (size_t)((rows + 31) / 32) * 32 * 2 * GC;
-  c->oh_cand.ensure(lists * cap * sizeof(uint32_t));
-  c->oh_cnt.ensure(lists * sizeof(int32_t));
+  const bool sym = rows == n && onehot_sym_fits(n, m) && !cap_env;
+  int GR = 1, GC = 1, cap = 0;
+  if (sym) {
+    c->oh_cand.ensure((size_t)n * onehot_sym_ldc(n) * sizeof(uint16_t));
+  } else {
+    onehot_mma_grid((int)((rows + 255) / 256), (int)((n + 255) / 256), sms, &GR, &GC);
+    cap = onehot_mma_cap(n, GC, g.K, cap_env ? atoi(cap_env) : 0);
+    const size_t lists = (size_t)((rows + 31) / 32) * 32 * 2 * GC;
+    c->oh_cand.ensure(lists * cap * sizeof(uint32_t));
+    c->oh_cnt.ensure(lists * sizeof(int32_t));
+  }
   c->oh_tab.ensure((size_t)(2 * m + 4) * sizeof(uint32_t));
   c->oh_err.ensure(sizeof(int));
   c->oh_errpin.ensure(sizeof(int));
   // the status accumulates over the calls before the caller's next check
   if (!c->oh_pending) CK(cudaMemsetAsync(c->oh_err.p, 0, sizeof(int), s));
   const char *why = "";
-  const int rc = launch_onehot_mma(g, c->oh_X.as<int8_t>(), ldx, rows, c->oh_cand.as<uint32_t>(),
-                                   cap, c->oh_cnt.as<int32_t>(), c->oh_tab.as<uint32_t>(),
-                                   c->oh_err.as<int>(), GR, GC, s, &why);
+  const int rc =
+      sym ? launch_onehot_sym(g, c->oh_X.as<int8_t>(), ldx, c->oh_cand.as<uint16_t>(),
+                              c->oh_tab.as<uint32_t>(), c->oh_err.as<int>(), sms, s, &why)
+          : launch_onehot_mma(g, c->oh_X.as<int8_t>(), ldx, rows, c->oh_cand.as<uint32_t>(), cap,
+                              c->oh_cnt.as<int32_t>(), c->oh_tab.as<uint32_t>(),
+                              c->oh_err.as<int>(), GR, GC, s, &why);
   if (rc != RBG_OK) throw Error(rc, std::string("one-hot tensor-core pass: ") + why);
   // the kernel's wait status comes back with the caller's next synchronisation
   CK(cudaMemcpyAsync(c->oh_errpin.p, c->oh_err.p, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -41,6 +41,10 @@
 // candidates above the admission floor, maxima over all other contigs and
 // over the candidates).
 //
+// That form scores every ordered pair.  It takes the rows of a rank of a sharded
+// assembly and assemblies above 32,768 contigs; up to there a whole assembly goes
+// through k_onehot_sym below, which computes each pair once.
+//
 // Every wait on an mbarrier is bounded (2 s of %globaltimer); a wait that
 // runs out records an error code for the host and the CTA stops issuing work,
 // waits (bounded) for its own copies and MMAs in flight, frees its TMEM and
@@ -91,12 +95,17 @@ struct OhArgs {
   int *err;              // set when a bounded wait runs out
 };
 
-__device__ __forceinline__ void mma_i8(uint32_t dt, uint64_t ad, uint64_t bd, uint32_t acc) {
+__device__ __forceinline__ void mma_i8_id(uint32_t dt, uint64_t ad, uint64_t bd, uint32_t idesc,
+                                          uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(dt), "l"(ad), "l"(bd), "r"(kIdesc), "r"(acc));
+      ::"r"(dt), "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+}
+
+__device__ __forceinline__ void mma_i8(uint32_t dt, uint64_t ad, uint64_t bd, uint32_t acc) {
+  mma_i8_id(dt, ad, bd, kIdesc, acc);
 }
 
 // 128 consecutive TMEM columns of this warp's 32 lanes as 16-bit values, two
@@ -552,6 +561,634 @@ k_merge_onehot(GraphArgs g, const uint32_t *__restrict__ cand, const int32_t *__
   if (lane == 0) g.topk_cnt[row] = fill;
 }
 
+// ── whole assemblies: every pair once, counts to memory ─────────────────────
+// The count of (i, j) is that of (j, i), so the tiles on and above the diagonal
+// hold every count: half the contraction, which bounds the kernel above.  A tile
+// cannot feed the lists of its columns' rows, though (a row's list belongs to one
+// thread), so each tile leaves its 16-bit counts in a matrix C, in both
+// orientations (a 32 x 32 block is transposed in registers), and
+// k_select_counts takes every row's top-K from its row of C.  A tile on the
+// diagonal loads its rows once.  20,011 contigs, m = 500 (rows of 5,760 bytes):
+// 1.37 ms + 0.50 ms for the lists' merge -> 0.72 ms + 0.35 ms; of that the tensor
+// pipe needs about 0.5 ms at 4.5 PFLOP/s and the 0.8 GB of counts 0.25 ms, written
+// and read.
+//
+// MB 128-row blocks a side: tiles of 256 x 256 read each operand byte for 256
+// counts and run at the tensor rate; with few contigs 128 x 128 tiles occupy
+// more SMs.  Tiles are walked in bands of kBandRows row blocks, down each
+// column: the CTAs of a wave share about 12 + 12 blocks' rows in L2.
+constexpr int kBandRows = 12;
+
+template <int MB>
+struct SymCfg {
+  static constexpr int T = 128 * MB;                       // rows and columns of a tile
+  static constexpr int kStageB = 2 * T * kKC;
+  static constexpr int kSt = 3 * 65536 / kStageB;          // 192 KB of stages
+  static constexpr int kBlk = MB == 2 ? 4 : 1;             // 32-column blocks of an epilogue warp
+  static constexpr uint32_t kId =
+      (2u << 4) | ((uint32_t)(T >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+};
+
+struct SymArgs {
+  int n, NB;             // contigs, tile blocks a side
+  int nkc;               // one-hot chunks of 128 bytes
+  int tiles;             // NB (NB + 1) / 2
+  uint16_t *C;           // [n][ldc] counts
+  int64_t ldc;
+  int *err;
+};
+
+// Tile t: row block I and column block J >= I.
+__device__ __forceinline__ void sym_tile(int t, int NB, int &I, int &J) {
+  int s0 = 0, h = 0;
+  for (;; s0 += h) {
+    h = min(kBandRows, NB - s0);
+    const int cnt = h * (h + 1) / 2 + h * (NB - s0 - h);
+    if (t < cnt) break;
+    t -= cnt;
+  }
+  const int tri = h * (h + 1) / 2;
+  if (t < tri) {
+    int c = 0;
+    while ((c + 1) * (c + 2) / 2 <= t) ++c;
+    I = s0 + t - c * (c + 1) / 2;
+    J = s0 + c;
+  } else {
+    const int u = t - tri;
+    J = s0 + h + u / h;
+    I = s0 + u % h;
+  }
+}
+
+// 32 consecutive TMEM columns as 16-bit values, two per register (no wait).
+__device__ __forceinline__ void tmem_ld32_pack16(uint32_t taddr, uint32_t *v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.pack::16b.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+        "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr));
+}
+
+// 64 bytes (16-byte aligned pointer, 64-byte aligned here) in two 32-byte stores.
+__device__ __forceinline__ void store64(uint16_t *p, const uint32_t *v) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p + 16 * h),
+                 "r"(v[8 * h]), "r"(v[8 * h + 1]), "r"(v[8 * h + 2]), "r"(v[8 * h + 3]),
+                 "r"(v[8 * h + 4]), "r"(v[8 * h + 5]), "r"(v[8 * h + 6]), "r"(v[8 * h + 7])
+                 : "memory");
+}
+
+// 32 x 32 16-bit values, lane = row, columns 2k and 2k + 1 in v[k]; afterwards
+// lane = column, rows 2k and 2k + 1 in v[k].  Bit b of the row (lane) and column
+// (register, half) indices are exchanged one b at a time.
+__device__ __forceinline__ void transpose32(uint32_t *v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int b = 4; b >= 1; --b) {
+    const bool up = (lane >> b) & 1;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      if (k & (1 << (b - 1))) continue;
+      const int k1 = k | (1 << (b - 1));
+      const uint32_t got = __shfl_xor_sync(FULL, up ? v[k] : v[k1], 1 << b);
+      v[k] = up ? got : v[k];
+      v[k1] = up ? v[k1] : got;
+    }
+  }
+  const uint32_t sel = (lane & 1) ? 0x3276u : 0x5410u;     // odd: (partner's, my) high halves
+#pragma unroll
+  for (int k = 0; k < 16; ++k) v[k] = __byte_perm(v[k], __shfl_xor_sync(FULL, v[k], 1), sel);
+}
+
+template <int MB>
+__global__ void __launch_bounds__(kThreads, 1)
+k_onehot_sym(const __grid_constant__ CUtensorMap tmap, const SymArgs A) {
+  using F = SymCfg<MB>;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t *ring = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t *bars = (uint64_t *)(ring + F::kSt * F::kStageB);
+  // bars: full[kSt], empty[kSt], tmem_full, tmem_empty, mma_done
+  uint32_t *tmem_slot = (uint32_t *)(bars + 2 * F::kSt + 3);
+  int *abort_flag = (int *)(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t bar0 = smem_u32(bars);
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };
+  auto empty_bar = [&](int s) { return bar0 + 8u * (F::kSt + s); };
+  const uint32_t tfull = bar0 + 8u * (2 * F::kSt), tempty = tfull + 8u, mdone = tfull + 16u;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < F::kSt; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    mbar_init(tfull, 1);
+    mbar_init(tempty, kEpiWarps * 32);
+    mbar_init(mdone, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;"
+                 ::"r"(smem_u32(tmem_slot)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tbase = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int s = 0;
+      uint32_t ph = 0, issued = 0, last_ph = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < A.tiles && ok; t += gridDim.x) {
+        int I, J;
+        sym_tile(t, A.NB, I, J);
+        for (int kc = 0; kc < A.nkc; ++kc) {
+          if (!mbar_wait(empty_bar(s), ph ^ 1u, A.err, 11) || *(volatile int *)abort_flag) {
+            ok = false;
+            *(volatile int *)abort_flag = 1;
+            break;
+          }
+          const uint32_t dst = smem_u32(ring + (size_t)s * F::kStageB);
+          mbar_expect_tx(full_bar(s), I == J ? F::kStageB / 2 : F::kStageB);
+          tma_load(dst, &tmap, kc * kKC, I * F::T, full_bar(s));
+          if (I != J) tma_load(dst + F::T * kKC, &tmap, kc * kKC, J * F::T, full_bar(s));
+          issued |= 1u << s;
+          last_ph = (last_ph & ~(1u << s)) | (ph << s);
+          if (++s == F::kSt) { s = 0; ph ^= 1u; }
+        }
+      }
+      // copies in flight land before the CTA leaves
+      for (int t = 0; t < F::kSt; ++t)
+        if ((issued >> t) & 1u) mbar_wait(full_bar(t), (last_ph >> t) & 1u, A.err, 12);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int s = 0;
+      uint32_t ph = 0, tph = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < A.tiles && ok; t += gridDim.x) {
+        int I, J;
+        sym_tile(t, A.NB, I, J);
+        if (!mbar_wait(tempty, tph ^ 1u, A.err, 13) || *(volatile int *)abort_flag) {
+          *(volatile int *)abort_flag = 1;
+          break;
+        }
+        fence_after();
+        for (int kc = 0; kc < A.nkc; ++kc) {
+          if (!mbar_wait(full_bar(s), ph, A.err, 14) || *(volatile int *)abort_flag) {
+            ok = false;
+            *(volatile int *)abort_flag = 1;
+            break;
+          }
+          fence_after();
+          const uint32_t st = smem_u32(ring + (size_t)s * F::kStageB);
+          const uint64_t db = sdesc128(I == J ? st : st + F::T * kKC);
+#pragma unroll
+          for (int k = 0; k < kKC / 32; ++k) {
+            const uint32_t acc = (kc | k) ? 1u : 0u;
+#pragma unroll
+            for (int h = 0; h < MB; ++h)
+              mma_i8_id(tbase + h * F::T, sdesc128(st + h * kHalfBytes) + 2 * k, db + 2 * k, F::kId,
+                        acc);
+          }
+          mma_commit(empty_bar(s));
+          if (++s == F::kSt) { s = 0; ph ^= 1u; }
+        }
+        if (!ok) break;
+        mma_commit(tfull);
+        tph ^= 1u;
+      }
+      mma_commit(mdone);                         // every MMA issued has finished
+      mbar_wait(mdone, 0, A.err, 15);
+    }
+  } else {
+    const int grp = (warp - 2) >> 2, q = warp & 3;   // four warps of a group: the TMEM lane quarters
+    const int half = MB == 2 ? grp & 1 : 0;
+    const int col = MB == 2 ? (grp >> 1) * 128 : grp * 32;
+    uint32_t tph = 0;
+    for (int t = blockIdx.x; t < A.tiles; t += gridDim.x) {
+      int I, J;
+      sym_tile(t, A.NB, I, J);
+      const bool bad = !mbar_wait(tfull, tph, A.err, 16) || *(volatile int *)abort_flag;
+      if (__any_sync(FULL, bad)) {
+        *(volatile int *)abort_flag = 1;
+        break;
+      }
+      fence_after();
+      uint32_t v[16 * F::kBlk];                  // 32 columns (16 registers) a block
+#pragma unroll
+      for (int c = 0; c < F::kBlk; ++c)
+        tmem_ld32_pack16(tbase + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * F::T + col + 32 * c),
+                         v + 16 * c);
+      tmem_wait_ld();
+      fence_before();
+      mbar_arrive(tempty);                       // TMEM is free for the next tile's MMAs
+      const int i0 = I * F::T + half * 128 + q * 32, j0 = J * F::T + col;
+#pragma unroll
+      for (int c = 0; c < F::kBlk; ++c) {
+        const int jc = j0 + 32 * c;
+        if (i0 + lane < A.n) store64(A.C + (int64_t)(i0 + lane) * A.ldc + jc, v + 16 * c);
+        if (I != J) {                            // warp-uniform
+          transpose32(v + 16 * c);
+          if (jc + lane < A.n) store64(A.C + (int64_t)(jc + lane) * A.ldc + i0, v + 16 * c);
+        }
+      }
+      tph ^= 1u;
+    }
+  }
+  __syncthreads();
+  fence_after();
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tbase) : "memory");
+}
+
+template <int MB>
+size_t sym_smem() {
+  using F = SymCfg<MB>;
+  return 1024 + (size_t)F::kSt * F::kStageB + (2 * F::kSt + 3) * 8 + 16;
+}
+
+constexpr uint32_t kTop = 0x80008000u;
+
+// Largest of a lane's counts, and how many (with bit 15 set) are at least T.
+template <int R>
+__device__ __forceinline__ uint32_t largest(const uint32_t (&x)[R]) {
+  uint32_t m2 = 0;
+#pragma unroll
+  for (int k = 0; k < R; ++k) m2 = __vmaxu2(m2, x[k]);
+  return max(m2 & 0xFFFFu, m2 >> 16);
+}
+
+template <int R>
+__device__ __forceinline__ uint32_t at_least(const uint32_t (&x)[R], uint32_t T) {
+  const uint32_t t2 = T * 0x10001u;
+  uint32_t acc = 0;
+#pragma unroll
+  for (int k = 0; k < R; ++k) acc += ((x[k] - t2) & kTop) >> 15;
+  return (acc & 0xFFFFu) + (acc >> 16);
+}
+
+// A lane's 16-byte words w0, w0 + 32, ... of a row of counts (the row's own and
+// those past the row's end 0); the two halves of word r of a 16-byte word are
+// columns 8 q + 2 r and 8 q + 2 r + 1.
+template <int NV>
+__device__ __forceinline__ void load_counts(const uint16_t *C, int64_t ldc, int row, int w0,
+                                            uint32_t (&x)[4 * NV]) {
+  const uint4 *src = reinterpret_cast<const uint4 *>(C + (int64_t)row * ldc);
+  const int words = (int)(ldc >> 3);
+  const uint32_t keep = (row & 1) ? 0x0000FFFFu : 0xFFFF0000u;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int q = w0 + 32 * k;
+    const uint4 v = q < words ? __ldg(src + q) : make_uint4(0u, 0u, 0u, 0u);
+    const int self = q == (row >> 3) ? (row >> 1) & 3 : 4;
+    x[4 * k] = self == 0 ? v.x & keep : v.x;
+    x[4 * k + 1] = self == 1 ? v.y & keep : v.y;
+    x[4 * k + 2] = self == 2 ? v.z & keep : v.z;
+    x[4 * k + 3] = self == 3 ? v.w & keep : v.w;
+  }
+}
+
+// Abundance bits of the columns, eight a byte, when one of the block's rows has
+// none (its candidates are then the columns with abundance only).
+__device__ __forceinline__ void abundance_bits(const GraphArgs &g, int row0, int rows,
+                                               uint8_t *nzb) {
+  const int n = (int)g.n;
+  if (!__syncthreads_or((int)threadIdx.x < rows && !g.anynz[row0 + threadIdx.x])) return;
+  for (int q = threadIdx.x; 8 * q < n; q += blockDim.x) {
+    uint32_t b = 0;
+    for (int u = 0; u < 8 && 8 * q + u < n; ++u) b |= (g.anynz[8 * q + u] ? 1u : 0u) << u;
+    nzb[q] = (uint8_t)b;
+  }
+  __syncthreads();
+}
+
+template <int NV>
+__device__ __forceinline__ void mask_counts(const uint8_t *nzb, int n, int w0,
+                                            uint32_t (&x)[4 * NV]) {
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int q = w0 + 32 * k;
+    const uint32_t b = 8 * q < n ? nzb[q] : 0u;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      x[4 * k + r] &= ((b >> 2 * r & 1u) * 0xFFFFu) | ((b >> (2 * r + 1) & 1u) * 0xFFFF0000u);
+  }
+}
+
+// Top-K of a row from its counts: W warps a row hold it in registers (NV
+// 16-byte words a lane; warp w a contiguous range of columns), find the K-th
+// count by halving the range of counts, and write the keys above it, then those
+// of its similarity in ascending column order until there are K: the set the
+// list kernels keep.  Counts carry bit 15, so that (x - T) keeps bit 15 exactly
+// where the count is at least T, two counts a subtraction.
+template <int NV, int W>
+__device__ __forceinline__ void select_row(const GraphArgs &g, const uint16_t *__restrict__ C,
+                                           int64_t ldc, const uint32_t *__restrict__ tab, int row,
+                                           uint32_t (&red)[2][8], int (&s_pos)[8],
+                                           const uint8_t *nzb) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wr = warp & (W - 1);
+  const int n = (int)g.n, m = g.m, K = g.K;
+  int turn = 0;
+  // sum or maximum over the row's warps
+  auto combine = [&](uint32_t x, bool mx) -> uint32_t {
+    x = mx ? __reduce_max_sync(FULL, x) : __reduce_add_sync(FULL, x);
+    if constexpr (W > 1) {
+      if (lane == 0) red[turn][warp] = x;
+      __syncthreads();
+      x = red[turn][0];
+#pragma unroll
+      for (int w = 1; w < W; ++w) x = mx ? max(x, red[turn][w]) : x + red[turn][w];
+      turn ^= 1;
+    }
+    return x;
+  };
+  const int w0 = wr * NV * 32 + lane;
+  uint32_t x[4 * NV];
+  load_counts<NV>(C, ldc, row, w0, x);
+  const uint32_t mx_a = combine(largest(x), true);
+  uint32_t mx_c = mx_a;
+  if (!g.anynz[row]) {
+    mask_counts<NV>(nzb, n, w0, x);
+    mx_c = combine(largest(x), true);
+  }
+#pragma unroll
+  for (int k = 0; k < 4 * NV; ++k) x[k] |= kTop;
+  const uint32_t cf = max(tab[2 * (m + 1)], 1u);       // counts above the floor
+  const bool ident = tab[2 * (m + 1) + 1] != 0u;
+  uint32_t t_lo = cf, t_hi = cf;                 // [t_lo, t_hi): the K-th similarity's counts
+  uint32_t c_hi = 0, total = 0;
+  if (mx_c >= cf) total = combine(at_least(x, cf), false);
+  if (total > (uint32_t)K) {
+    uint32_t lo = cf, hi = mx_c + 1;             // at least K from lo on, fewer from hi on
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (combine(at_least(x, mid), false) >= (uint32_t)K) lo = mid; else hi = mid;
+    }
+    t_lo = lo;
+    t_hi = lo + 1;
+    if (!ident) {                                // counts of one similarity
+      const uint32_t R = tab[lo];
+      while (t_lo > cf && tab[t_lo - 1] == R) --t_lo;
+      while (t_hi <= (uint32_t)m && tab[t_hi] == R) ++t_hi;
+    }
+    c_hi = t_hi <= mx_c ? combine(at_least(x, t_hi), false) : 0u;
+  } else {
+    c_hi = total;                                // all of them
+  }
+  if (W == 1 ? lane == 0 : threadIdx.x == 0) {
+    s_pos[warp] = 0;
+    if (mx_a) atomicMax(g.maxcnt_all + row, mx_a);
+    if (mx_c) atomicMax(g.maxcnt_cand + row, mx_c);
+    g.topk_cnt[row] = (int)min(total, (uint32_t)K);
+  }
+  const uint32_t need = total > (uint32_t)K ? (uint32_t)K - c_hi : 0u;   // keys of the K-th similarity
+  // candidates of that similarity in the lower columns' warps
+  uint32_t eq_before = 0;
+  {
+    uint32_t eq = 0;
+    if (need) {
+      const uint32_t lo2 = t_lo * 0x10001u, hi2 = t_hi * 0x10001u;
+      uint32_t acc = 0;
+#pragma unroll
+      for (int k = 0; k < 4 * NV; ++k) acc += (((x[k] - lo2) & ~(x[k] - hi2)) & kTop) >> 15;
+      eq = __reduce_add_sync(FULL, (acc & 0xFFFFu) + (acc >> 16));
+    }
+    if constexpr (W > 1) {
+      if (lane == 0) red[turn][warp] = eq;
+      __syncthreads();                           // (s_pos, too)
+      for (int w = 0; w < wr; ++w) eq_before += red[turn][w];
+    } else {
+      __syncwarp();
+    }
+  }
+  const uint32_t *value = tab + m + 1;
+  uint64_t *out = g.topk + (int64_t)row * K;
+  int *pos = &s_pos[W == 1 ? warp : 0];
+  const uint32_t lo2 = t_lo * 0x10001u, hi2 = t_hi * 0x10001u;
+  const uint16_t *src16 = C + (int64_t)row * ldc;
+  auto put = [&](uint32_t at, uint32_t j) {
+    const uint32_t cnt = __ldg(src16 + j);
+    out[at] = ((uint64_t)__ldg(value + (ident ? cnt : tab[cnt])) << 32) | (uint64_t)(~j);
+  };
+  if (total == 0) return;
+  // a byte of hits for each 16-byte word, four words at a time
+  constexpr int KG = NV < 4 ? NV : 4;
+#pragma unroll
+  for (int k0 = 0; k0 < NV; k0 += KG) {
+    uint32_t h4 = 0, e4 = 0;                     // above the K-th similarity, of it
+#pragma unroll
+    for (int r = 0; r < 4 * KG; ++r) {
+      const uint32_t above = (x[4 * k0 + r] - hi2) & kTop;
+      const uint32_t tie = (x[4 * k0 + r] - lo2) & ~above & kTop;
+      h4 |= ((above >> 15 & 1u) | (above >> 30)) << (2 * r);
+      e4 |= ((tie >> 15 & 1u) | (tie >> 30)) << (2 * r);
+    }
+    if (!need) e4 = 0;
+    if (!__any_sync(FULL, (h4 | e4) != 0u)) continue;
+#pragma unroll 1
+    for (int k = 0; k < KG; ++k, h4 >>= 8, e4 >>= 8) {
+      const uint32_t j = 8u * (uint32_t)(w0 + 32 * (k0 + k));
+      const uint32_t h = h4 & 0xFFu, e = e4 & 0xFFu;
+      if (h) {
+        uint32_t at = (uint32_t)atomicAdd(pos, __popc(h));
+        for (uint32_t b = h; b; b &= b - 1) put(at++, j + (uint32_t)(__ffs(b) - 1));
+      }
+      if (!__any_sync(FULL, e != 0u)) continue;
+      uint32_t incl = (uint32_t)__popc(e);
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t o = __shfl_up_sync(FULL, incl, d);
+        if (lane >= d) incl += o;
+      }
+      uint32_t at = eq_before + incl - (uint32_t)__popc(e);
+      for (uint32_t b = e; b && at < need; b &= b - 1, ++at)
+        put(c_hi + at, j + (uint32_t)(__ffs(b) - 1));
+      eq_before += __shfl_sync(FULL, incl, 31);
+    }
+  }
+}
+
+__device__ __forceinline__ void count_pairs(const GraphArgs &g) {
+  if (g.stats && blockIdx.x == 0 && threadIdx.x == 0)    // every other contig, once per row
+    atomicAdd(g.stats + 1, (unsigned long long)g.n * (unsigned long long)(g.n - 1));
+}
+
+// A warp a row.
+template <int NV>
+__global__ void __launch_bounds__(256, NV <= 8 ? 4 : 2)
+k_select_counts(GraphArgs g, const uint16_t *__restrict__ C, int64_t ldc,
+                const uint32_t *__restrict__ tab) {
+  __shared__ uint32_t red[2][8];
+  __shared__ int s_pos[8];
+  __shared__ uint8_t nzb[NV * 32];
+  count_pairs(g);
+  const int row0 = (int)blockIdx.x * 8, row = row0 + (threadIdx.x >> 5);
+  abundance_bits(g, row0, min(8, (int)g.n - row0), nzb);
+  if (row < (int)g.n) select_row<NV, 1>(g, C, ldc, tab, row, red, s_pos, nzb);
+}
+
+// Eight warps a row, R <= 8 rows in turn.  Each thread's even and odd columns
+// give 512 disjoint groups; K of their maxima reach the K-th largest maximum, so
+// at least K counts do: one value a thread is searched instead of the whole row,
+// and few counts pass (about 1.2 K of 20,000).  These are listed, and each warp
+// selects one row's K best from its list.  A row whose list overflows (ties) is
+// selected from registers, as above.
+template <int NV>
+__global__ void __launch_bounds__(256, NV <= 12 ? 3 : 2)
+k_select_counts_rows(GraphArgs g, const uint16_t *__restrict__ C, int64_t ldc,
+                     const uint32_t *__restrict__ tab, int R) {
+  __shared__ uint32_t list[8][kOmBuf];
+  __shared__ uint32_t mx[2][256];
+  __shared__ unsigned cnt[8];
+  __shared__ uint32_t red[2][8];
+  __shared__ int s_pos[8];
+  __shared__ uint8_t nzb[NV * 32 * 8];
+  count_pairs(g);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n = (int)g.n, m = g.m, K = g.K;
+  const int row0 = (int)blockIdx.x * R, rows = min(R, n - row0);
+  const uint32_t cf = max(tab[2 * (m + 1)], 1u);
+  const bool ident = tab[2 * (m + 1) + 1] != 0u;
+  const int w0 = warp * NV * 32 + lane;
+  if (threadIdx.x < 8) cnt[threadIdx.x] = 0;
+  abundance_bits(g, row0, rows, nzb);
+  for (int r = 0; r < rows; ++r) {
+    const int row = row0 + r;
+    uint32_t x[4 * NV];
+    load_counts<NV>(C, ldc, row, w0, x);
+    const bool nz = g.anynz[row] != 0;
+    if (!nz) {
+      const uint32_t all = __reduce_max_sync(FULL, largest(x));
+      if (lane == 0 && all) atomicMax(g.maxcnt_all + row, all);
+      mask_counts<NV>(nzb, n, w0, x);
+    }
+    uint32_t m2 = 0;
+#pragma unroll
+    for (int k = 0; k < 4 * NV; ++k) m2 = __vmaxu2(m2, x[k]);
+    mx[r & 1][threadIdx.x] = m2;
+    __syncthreads();
+    uint32_t y[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) y[k] = mx[r & 1][32 * k + lane];
+    const uint32_t top = __reduce_max_sync(FULL, largest(y));
+    if (threadIdx.x == 0 && top) {
+      if (nz) atomicMax(g.maxcnt_all + row, top);
+      atomicMax(g.maxcnt_cand + row, top);
+    }
+    if (top < cf) continue;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) y[k] |= kTop;
+    uint32_t T = cf, hi = top + 1;               // K maxima reach T, or T = cf
+    while (hi - T > 1) {
+      const uint32_t mid = (T + hi) >> 1;
+      if (__reduce_add_sync(FULL, at_least(y, mid)) >= (uint32_t)K) T = mid; else hi = mid;
+    }
+    const uint32_t t2 = T * 0x10001u;
+    uint32_t hit[(4 * NV + 31) / 32] = {};
+#pragma unroll
+    for (int k = 0; k < 4 * NV; ++k)
+      if (((x[k] | kTop) - t2) & kTop) hit[k >> 5] |= 1u << (k & 31);
+#pragma unroll
+    for (int h = 0; h < (4 * NV + 31) / 32; ++h)
+      for (uint32_t b = hit[h]; b; b &= b - 1) {
+        const int k = 32 * h + __ffs(b) - 1;
+        const int j = 8 * (w0 + 32 * (k >> 2)) + 2 * (k & 3);
+        // (the same masks as the registers had)
+        const uint32_t v = __ldg(reinterpret_cast<const uint32_t *>(C + (int64_t)row * ldc + j));
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const uint32_t c = u ? v >> 16 : v & 0xFFFFu;
+          if (c >= T && j + u != row && (nz || g.anynz[j + u])) {
+            const unsigned at = atomicAdd(&cnt[r], 1u);
+            if (at < kOmBuf)
+              list[r][at] = ((ident ? c : tab[c]) << 20) | (0xFFFFFu - (uint32_t)(j + u));
+          }
+        }
+      }
+  }
+  __syncthreads();
+  if (warp < rows && cnt[warp] <= kOmBuf) {
+    const int row = row0 + warp;
+    uint32_t *keys = list[warp];
+    int fill = (int)cnt[warp];
+    if (fill > K) {
+      if (fill <= 16 * 32) select_topk32<16>(keys, fill, K);
+      else select_topk32<kCapW32>(keys, fill, K);
+      fill = K;
+    }
+    const uint32_t *value = tab + m + 1;
+    for (int i = lane; i < fill; i += 32) {
+      const uint32_t key = keys[i], j = 0xFFFFFu - (key & 0xFFFFFu);
+      g.topk[(int64_t)row * K + i] = ((uint64_t)__ldg(value + (key >> 20)) << 32) | (uint64_t)(~j);
+    }
+    if (lane == 0) g.topk_cnt[row] = fill;
+  }
+  for (int r = 0; r < rows; ++r)
+    if (cnt[r] > kOmBuf) {                       // block-uniform
+      select_row<NV, 8>(g, C, ldc, tab, row0 + r, red, s_pos, nzb);
+      __syncthreads();
+    }
+}
+
+template <int NV>
+void launch_select_rows_nv(const GraphArgs &g, const uint16_t *C, int64_t ldc, const uint32_t *tab,
+                           cudaStream_t s) {
+  const int R = g.n > 8192 ? 8 : 4;              // rows a block: fewer with few rows
+  k_select_counts_rows<NV><<<(unsigned)((g.n + R - 1) / R), 256, 0, s>>>(g, C, ldc, tab, R);
+}
+
+// A warp a row up to 4,096 columns (16 words a lane), a block above.  (20,011
+// contigs: 0.89 ms searching the whole row's registers, 0.35 ms with the lists.)
+void launch_select_counts(const GraphArgs &g, const uint16_t *C, int64_t ldc, const uint32_t *tab,
+                          cudaStream_t s) {
+  const unsigned blocks = (unsigned)((g.n + 7) / 8);
+  if (ldc <= 512) k_select_counts<2><<<blocks, 256, 0, s>>>(g, C, ldc, tab);
+  else if (ldc <= 1024) k_select_counts<4><<<blocks, 256, 0, s>>>(g, C, ldc, tab);
+  else if (ldc <= 2048) k_select_counts<8><<<blocks, 256, 0, s>>>(g, C, ldc, tab);
+  else if (ldc <= 4096) k_select_counts<16><<<blocks, 256, 0, s>>>(g, C, ldc, tab);
+  else if (ldc <= 8192) launch_select_rows_nv<4>(g, C, ldc, tab, s);
+  else if (ldc <= 16384) launch_select_rows_nv<8>(g, C, ldc, tab, s);
+  else if (ldc <= 24576) launch_select_rows_nv<12>(g, C, ldc, tab, s);
+  else launch_select_rows_nv<16>(g, C, ldc, tab, s);
+}
+
+// Tensor map of the one-hot rows: boxes of one 128-byte chunk of `rows` rows.
+bool onehot_map(CUtensorMap *map, const int8_t *X, int64_t ldx, int64_t n, int rows) {
+  auto enc = encode_fn();
+  if (!enc) return false;
+  std::memset(map, 0, sizeof(*map));
+  const cuuint64_t dims[2] = {(cuuint64_t)ldx, (cuuint64_t)n};
+  const cuuint64_t strides[1] = {(cuuint64_t)ldx};
+  const cuuint32_t box[2] = {(cuuint32_t)kKC, (cuuint32_t)rows};
+  const cuuint32_t estr[2] = {1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void *)X, dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int MB>
+cudaError_t launch_sym_mb(const CUtensorMap &map, const SymArgs &A, int sms, cudaStream_t s) {
+  cudaError_t e;
+  {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    e = cudaFuncSetAttribute(k_onehot_sym<MB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sym_smem<MB>());
+  }
+  if (e != cudaSuccess) return e;
+  k_onehot_sym<MB><<<(unsigned)std::min(A.tiles, sms), kThreads, sym_smem<MB>(), s>>>(map, A);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 bool onehot_mma_fits(int64_t n, int m) { return n < ((int64_t)1 << 20) && m < 4096; }
@@ -596,26 +1233,13 @@ void onehot_mma_grid(int RB, int NT, int sms, int *GR, int *GC) {
 int launch_onehot_mma(const GraphArgs &g, const int8_t *X, int64_t ldx, int64_t rows,
                       uint32_t *cand, int cap, int32_t *cand_cnt, uint32_t *tab, int *err, int GR,
                       int GC, cudaStream_t s, const char **why) {
-  auto enc = encode_fn();
-  if (!enc) {
-    *why = "cuTensorMapEncodeTiled is not available";
-    return RBG_ERR_CUDA;
-  }
   if (ldx % kKC != 0 || ((uintptr_t)X & 15u) != 0 || !onehot_mma_fits(g.n, g.m) || GC > 16 ||
       g.K < 1 || g.K > 448 || cap > 32 * kCapW32 || cap < g.K + 136 || cap % 32 != 0) {
     *why = "one-hot operand layout";
     return RBG_ERR_ARG;
   }
   CUtensorMap map;
-  std::memset(&map, 0, sizeof(map));
-  const cuuint64_t dims[2] = {(cuuint64_t)ldx, (cuuint64_t)g.n};
-  const cuuint64_t strides[1] = {(cuuint64_t)ldx};
-  const cuuint32_t box[2] = {(cuuint32_t)kKC, (cuuint32_t)kTM};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void *)X, dims, strides, box,
-                         estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
+  if (!onehot_map(&map, X, ldx, g.n, kTM)) {
     *why = "cuTensorMapEncodeTiled failed";
     return RBG_ERR_CUDA;
   }
@@ -646,6 +1270,56 @@ int launch_onehot_mma(const GraphArgs &g, const int8_t *X, int64_t ldx, int64_t 
     if (rows > 0)
       k_merge_onehot<<<(unsigned)((rows + kOmWarps - 1) / kOmWarps), kOmWarps * 32, 0, s>>>(
           g, cand, cand_cnt, cap, 2 * GC, tab, rows);
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) {
+    *why = cudaGetErrorString(e);
+    return RBG_ERR_CUDA;
+  }
+  return RBG_OK;
+}
+
+// Whole assemblies whose count matrix (2 n^2 bytes) and rows (registers of
+// k_select_counts) fit.
+bool onehot_sym_fits(int64_t n, int m) { return n <= 32768 && m < 4096; }
+
+int64_t onehot_sym_ldc(int64_t n) { return (n + 255) / 256 * 256; }
+
+// X as launch_onehot_mma takes it; C: [n][onehot_sym_ldc(n)] 16-bit counts; tab
+// [2m + 4].  The three launches: ranks, counts, top-K and maxima per row.
+//
+// 128 x 128 tiles while all of them run at once (up to 2,048 contigs on 148 SMs):
+// the whole dense pass takes 108 us at 2,000 contigs, 117 with 256 x 256; 144 and
+// 134 us at 3,000, where they take a third round.
+int launch_onehot_sym(const GraphArgs &g, const int8_t *X, int64_t ldx, uint16_t *C, uint32_t *tab,
+                      int *err, int sms, cudaStream_t s, const char **why) {
+  if (ldx % kKC != 0 || ((uintptr_t)X & 15u) != 0 || ((uintptr_t)C & 31u) != 0 ||
+      !onehot_sym_fits(g.n, g.m) || g.K < 1 || g.row_lo != 0 ||
+      (g.row_hi >= 0 && g.row_hi != g.n)) {
+    *why = "one-hot operand layout";
+    return RBG_ERR_ARG;
+  }
+  SymArgs A;
+  A.n = (int)g.n;
+  A.nkc = (int)(ldx / kKC);
+  A.C = C;
+  A.ldc = onehot_sym_ldc(g.n);
+  A.err = err;
+  const int nb2 = (int)((g.n + 255) / 256);
+  const bool small = nb2 * (2 * nb2 + 1) <= sms;
+  const int T = small ? 128 : 256;
+  // (columns up to ldc are written with 128-row blocks, too)
+  A.NB = small ? 2 * nb2 : nb2;
+  A.tiles = A.NB * (A.NB + 1) / 2;
+  CUtensorMap map;
+  if (!onehot_map(&map, X, ldx, g.n, T)) {
+    *why = "cuTensorMapEncodeTiled failed";
+    return RBG_ERR_CUDA;
+  }
+  k_sv_rank<<<1, 32, 0, s>>>(g.sv_bits, g.m, (uint32_t)(g.key_floor >> 32), tab);
+  cudaError_t e = small ? launch_sym_mb<1>(map, A, sms, s) : launch_sym_mb<2>(map, A, sms, s);
+  if (e == cudaSuccess) {
+    launch_select_counts(g, C, A.ldc, tab, s);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {

@@ -215,6 +215,12 @@ void launch_merge_topk(const GraphArgs &g, const uint64_t *gbuf, const int32_t *
 // keys per row) and the row maxima, then merged into g.topk / g.topk_cnt; tab [2m + 4]
 // is scratch for the similarity-rank tables; *err != 0 after it ran when a
 // bounded wait gave up.  Needs onehot_mma_fits(n, m) and 1 <= K <= 448.
+// launch_onehot_sym: the same results for a whole assembly from each pair's count
+// once, by way of the count matrix C [n][onehot_sym_ldc(n)].
+bool onehot_sym_fits(int64_t n, int m);
+int64_t onehot_sym_ldc(int64_t n);
+int launch_onehot_sym(const GraphArgs &g, const int8_t *X, int64_t ldx, uint16_t *C, uint32_t *tab,
+                      int *err, int sms, cudaStream_t s, const char **why);
 bool onehot_mma_fits(int64_t n, int m);
 int onehot_mma_cap(int64_t n, int GC, int K, int cap_max);
 void onehot_mma_grid(int RB, int NT, int sms, int *GR, int *GC);
@@ -382,7 +388,7 @@ void smem_cap_max(const void *func);
 void launch_unit_rows_batch(const BatchAsm *B, const int64_t *row0s, int nb, int64_t rows,
                             cudaStream_t s, int64_t r_begin = 0);
 // Column norms of the assemblies B[0..nb) (pass B + first for a range).
-void launch_colnorm_batch(const BatchAsm *B, int nb, int max_s, cudaStream_t s);
+void launch_colnorm_batch(const BatchAsm *B, int nb, cudaStream_t s);
 void launch_b0_batch(const BatchAsm *B, const int64_t *pair0s, int nb, int64_t npairs,
                      const int32_t *pairs, uint32_t *counts, int max_m, cudaStream_t s);
 // b0 and similarity tables of assemblies [b_begin, b_end), whose sampled
