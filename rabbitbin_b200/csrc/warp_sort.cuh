@@ -1,4 +1,4 @@
-// Sort of up to a few hundred 64-bit keys in a warp's registers, shared by the
+// Sort of up to a few hundred keys in a warp's registers, shared by the
 // neighbour lists and the incidence lists.
 #pragma once
 #include <cstdint>
@@ -7,9 +7,10 @@ namespace rbg {
 
 // Ascending bitonic sort of 32 R keys held in registers, element r * 32 + lane
 // in v[r]: strides of 32 and more pair registers of the same lane, shorter
-// strides pair lanes through shuffles.
-template <int R>
-__device__ __forceinline__ void warp_bitonic_asc(uint64_t (&v)[R]) {
+// strides pair lanes through shuffles.  32-bit keys take a third of the
+// instructions of 64-bit ones (one shuffle and one minimum or maximum a step).
+template <int R, class T>
+__device__ __forceinline__ void warp_bitonic_asc(T (&v)[R]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int size = 2; size <= 32 * R; size <<= 1) {
@@ -21,14 +22,16 @@ __device__ __forceinline__ void warp_bitonic_asc(uint64_t (&v)[R]) {
           const int p = r ^ (stride >> 5);
           if (p > r) {
             const bool up = (((r * 32 + lane) & size) == 0);
-            const uint64_t x = v[r], y = v[p];
-            if ((x > y) == up) { v[r] = y; v[p] = x; }
+            const T x = v[r], y = v[p];
+            const T lo = x < y ? x : y, hi = x < y ? y : x;
+            v[r] = up ? lo : hi;
+            v[p] = up ? hi : lo;
           }
         }
       } else {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          const uint64_t o = __shfl_xor_sync(0xffffffffu, v[r], stride);
+          const T o = __shfl_xor_sync(0xffffffffu, v[r], stride);
           const bool up = (((r * 32 + lane) & size) == 0);
           const bool lower = (lane & stride) == 0;
           v[r] = (lower == up) ? (v[r] < o ? v[r] : o) : (v[r] < o ? o : v[r]);
