@@ -388,7 +388,7 @@ void smem_cap_max(const void *func);
 void launch_unit_rows_batch(const BatchAsm *B, const int64_t *row0s, int nb, int64_t rows,
                             cudaStream_t s, int64_t r_begin = 0);
 // Column norms of the assemblies B[0..nb) (pass B + first for a range).
-void launch_colnorm_batch(const BatchAsm *B, int nb, cudaStream_t s);
+void launch_colnorm_batch(const BatchAsm *B, int nb, int max_s, cudaStream_t s);
 void launch_b0_batch(const BatchAsm *B, const int64_t *pair0s, int nb, int64_t npairs,
                      const int32_t *pairs, uint32_t *counts, int max_m, cudaStream_t s);
 // b0 and similarity tables of assemblies [b_begin, b_end), whose sampled
