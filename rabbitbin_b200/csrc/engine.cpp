@@ -271,14 +271,25 @@ void stage_sketch_chunked(rbg_ctx *c, const rbg_params *p, const char *seqcat,
       sym_tc5_setup(c, ga, G);
     }
   }
+  // First words of the chunks: equal ones, or, where the pairs stream, each 0.83 of
+  // the one before.  A late chunk's pairs (against all rows so far) take about that
+  // share of its copy's time, so each is done when the next one has arrived, and
+  // less is left behind the last one (200,003 contigs x 30, 1.6 GB: 42.8 ms a call in
+  // equal chunks, 41.0 ms).
+  const double shrink = 0.83;
+  auto cut = [&](int g) -> int64_t {
+    if (g == G) return nwords;
+    const double f = stream_pairs ? (1.0 - std::pow(shrink, g)) / (1.0 - std::pow(shrink, G))
+                                  : (double)g / G;
+    return (int64_t)(f * (double)nwords) & ~(int64_t)1;
+  };
   // Packing on the host sends 3/8 of a byte per base instead of the ASCII
   // byte: while chunk g's words copy, the host packs chunk g + 1 into the
   // other pinned slot.
   const bool hpack = pack_on_host();
   int64_t c0 = 0;
   for (int g = 0; g < G; ++g) {
-    const int64_t w0 = (int64_t)g * nwords / G & ~(int64_t)1;
-    const int64_t w1 = g + 1 == G ? nwords : ((int64_t)(g + 1) * nwords / G & ~(int64_t)1);
+    const int64_t w0 = cut(g), w1 = cut(g + 1);
     const int64_t b0 = 16 * w0, b1 = std::min<int64_t>(16 * w1, nb);
     if (hpack) {
       const int sl = g & 1;
