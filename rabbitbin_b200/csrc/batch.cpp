@@ -1031,7 +1031,7 @@ void run_batch(rbg_ctx *c, const rbg_params *defaults, const rbg_assembly *asms,
   captured(c, 2, use_graph, stats.graph_launches, [&] {
     CK(cudaMemcpyAsync(B.desc.p, h_desc, desc_bytes, cudaMemcpyHostToDevice, c->stream));
     launch_write_edges_batch(dD, B.row0s.as<int64_t>(), nb, rows, c->stream);
-    launch_edge_weights_batch(dD, B.edge0s.as<int64_t>(), nb, E, c->stream);
+    launch_edge_weights_batch(dD, B.edge0s.as<int64_t>(), nb, E, L.max_s, c->stream);
     launches += (rows ? 1 : 0) + (E ? 1 : 0);
     if (E) {
       CK(cudaMemcpyAsync(h_from, B.e_from.p, E * 4, cudaMemcpyDeviceToHost, c->stream));

@@ -417,7 +417,7 @@ void launch_emit_batch(const BatchAsm *B, const int64_t *row0s, int nb, int64_t 
 void launch_write_edges_batch(const BatchAsm *B, const int64_t *row0s, int nb, int64_t rows,
                               cudaStream_t s);
 void launch_edge_weights_batch(const BatchAsm *B, const int64_t *edge0s, int nb, int64_t edges,
-                               cudaStream_t s);
+                               int max_s, cudaStream_t s);
 // ── dense regime on the tensor cores (kernels_onehot.cu) ───────────────────
 // Codes occurring per register column of rows [0, n): pres[m][8] (256 bits).
 void launch_code_presence(const uint8_t *codesA, int64_t n, int m, int mpad, uint32_t *pres,
