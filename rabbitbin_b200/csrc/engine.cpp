@@ -1889,10 +1889,37 @@ int rbg_pmh_compare(rbg_ctx *c, int32_t metric, int32_t m, int32_t kmer_size, co
       const int64_t ra = std::min(blk, na - a0);
       CK(cudaMemcpyAsync(c->qa.p, (const char *)A + (size_t)a0 * rowb, (size_t)ra * rowb,
                          cudaMemcpyHostToDevice, c->stream));
-      launch_pmh_compare(c->qa.as<uint64_t>(), ra, c->qb.as<uint64_t>(), nb, m, regs,
-                         c->qt.as<double>(), c->qo.as<double>(), c->stream);
-      CK(cudaGetLastError());
-      copy_out(c, out + (size_t)a0 * nb, c->qo.p, (size_t)ra * nb * sizeof(double), c->stream);
+      // A pinned result leaves in parts of 8 MB or more (and of 256 tiles of 64 x 64
+      // pairs), each behind the comparisons of the next; two streams take turns, so
+      // that a part starts in the last wave of the one before.
+      double *dst = out + (size_t)a0 * nb;
+      const size_t bytes = (size_t)ra * nb * sizeof(double);
+      const int64_t tiles = (ra + 63) / 64 * ((nb + 63) / 64);
+      const int parts = bounced(dst, bytes)
+                            ? 1
+                            : (int)std::max<int64_t>(1, std::min<int64_t>({kChunks, (int64_t)(bytes >> 23),
+                                                                           tiles / 256}));
+      if (parts > 1) {
+        CK(cudaEventRecord(c->ev_cin, c->stream));             // the rows are on the device
+        CK(cudaStreamWaitEvent(c->aux, c->ev_cin, 0));
+      }
+      for (int k = 0; k < parts; ++k) {
+        cudaStream_t s = k & 1 ? c->aux : c->stream;
+        const int64_t r0 = ra * k / parts, r1 = ra * (k + 1) / parts;
+        double *o = c->qo.as<double>() + (size_t)r0 * nb;
+        launch_pmh_compare(c->qa.as<uint64_t>() + (size_t)r0 * m, r1 - r0, c->qb.as<uint64_t>(), nb, m,
+                           regs, c->qt.as<double>(), o, s);
+        CK(cudaGetLastError());
+        if (parts == 1) {
+          copy_out(c, dst, o, bytes, s);
+        } else {
+          CK(cudaEventRecord(c->ev_chunk[k], s));
+          CK(cudaStreamWaitEvent(c->copy, c->ev_chunk[k], 0));
+          CK(cudaMemcpyAsync(dst + (size_t)r0 * nb, o, (size_t)(r1 - r0) * nb * sizeof(double),
+                             cudaMemcpyDeviceToHost, c->copy));
+        }
+      }
+      if (parts > 1) CK(cudaStreamSynchronize(c->copy));
     }
   });
 }
