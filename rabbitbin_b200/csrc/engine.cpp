@@ -1013,7 +1013,7 @@ void run_graph(rbg_ctx *c, const rbg_params *p, const ShardCtx *sc = nullptr) {
     const int64_t rows = sc ? sc->row_hi - sc->row_lo : n;
     CK(cudaMemsetAsync(c->maxc_cand.p, 0, n1 * sizeof(uint32_t), c->stream));
     CK(cudaMemsetAsync(c->maxc_all.p, 0, n1 * sizeof(uint32_t), c->stream));
-    if (!g.prefilter && dense_on_gemm() && onehot_mma_fits(n, m)) {
+    if (!g.prefilter && dense_on_gemm(n) && onehot_mma_fits(n, m)) {
       dense_allpairs_onehot(c, g);                      // tensor cores, exact counts
     } else {
       const size_t slots = (size_t)((rows + 31) / 32) * allpairs_slices_rows(rows, n, K) * 32;

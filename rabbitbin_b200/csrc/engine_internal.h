@@ -160,10 +160,15 @@ void sym_tc5_pass(rbg_ctx *c, const GraphArgs &g, const SymOut &o, int64_t cb, i
                   int slot);
 void sym_tc5_readback(rbg_ctx *c, int64_t n);
 bool sym_tc5_settle(rbg_ctx *c, int64_t n, int S);
-// The dense regime runs on the one-hot tensor-core kernel unless RBG_DENSE_ALU
-// is set (then the integer-ALU register compare, kept for the measured
-// comparison).
-inline bool dense_on_gemm() { return getenv("RBG_DENSE_ALU") == nullptr; }
+// The dense regime runs on the one-hot tensor-core kernels, unless RBG_DENSE_ALU is
+// set (for measurement) or the contigs are few: the integer-ALU register compare
+// then, without the one-hot rows' four launches and the read-back of their width.
+// A resident call with ALU / tensor cores at m = 500: 97 contigs 267 / 300 us, 200
+// 292 / 303, 300 321 / 309, 500 316 / 326, 1,000 363 / 339, 2,000 518 / 390.
+constexpr int64_t kDenseAlu = 256;
+inline bool dense_on_gemm(int64_t n) {
+  return n > kDenseAlu && getenv("RBG_DENSE_ALU") == nullptr;
+}
 
 // 2-bit packing on the host (host_pack.cpp): words [w0, w1) of the packed
 // bases (w0 even; rounded up to whole word pairs: 2 * ceil((w1 - w0) / 2)
