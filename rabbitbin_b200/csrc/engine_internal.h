@@ -163,9 +163,9 @@ bool sym_tc5_settle(rbg_ctx *c, int64_t n, int S);
 // The dense regime runs on the one-hot tensor-core kernels, unless RBG_DENSE_ALU is
 // set (for measurement) or the contigs are few: the integer-ALU register compare
 // then, without the one-hot rows' four launches and the read-back of their width.
-// A resident call with ALU / tensor cores at m = 500: 97 contigs 267 / 300 us, 200
-// 292 / 303, 300 321 / 309, 500 316 / 326, 1,000 363 / 339, 2,000 518 / 390.
-constexpr int64_t kDenseAlu = 256;
+// A resident call with ALU / tensor cores at m = 500: 97 contigs 251 / 300 us, 300
+// 279 / 313, 500 295 / 332, 700 330 / 343 (m = 1,000: 368 / 368), 1,000 363 / 351.
+constexpr int64_t kDenseAlu = 512;
 inline bool dense_on_gemm(int64_t n) {
   return n > kDenseAlu && getenv("RBG_DENSE_ALU") == nullptr;
 }

@@ -1368,7 +1368,7 @@ int allpairs_slices_rows(int64_t rows, int64_t n, int K) {
   int64_t P = (4 * 148 * 48 + blocks - 1) / std::max<int64_t>(blocks, 1);
   // at least 64 columns a slice (fewer lists to merge); 8 with few contigs, whose row
   // blocks leave most SMs idle
-  P = std::min<int64_t>(P, std::max<int64_t>(n / (n <= 256 ? 8 : 64), 1));
+  P = std::min<int64_t>(P, std::max<int64_t>(n / (n <= 512 ? 8 : 64), 1));
   P = std::max<int64_t>(P, 1);
   const int pmax = std::max(kWarps, std::min(32, (6400 / std::max(K, 1)) / kWarps * kWarps));
   P = std::min<int64_t>(P, pmax);
