@@ -1150,8 +1150,7 @@ void launch_select_rows_nv(const GraphArgs &g, const uint16_t *C, int64_t ldc, c
 void launch_select_counts(const GraphArgs &g, const uint16_t *C, int64_t ldc, const uint32_t *tab,
                           cudaStream_t s) {
   const unsigned blocks = (unsigned)((g.n + 7) / 8);
-  if (ldc <= 512) k_select_counts<2><<<blocks, 256, 0, s>>>(g, C, ldc, tab);
-  else if (ldc <= 1024) k_select_counts<4><<<blocks, 256, 0, s>>>(g, C, ldc, tab);
+  if (ldc <= 1024) k_select_counts<4><<<blocks, 256, 0, s>>>(g, C, ldc, tab);
   else if (ldc <= 2048) k_select_counts<8><<<blocks, 256, 0, s>>>(g, C, ldc, tab);
   else if (ldc <= 4096) k_select_counts<16><<<blocks, 256, 0, s>>>(g, C, ldc, tab);
   else if (ldc <= 8192) launch_select_rows_nv<4>(g, C, ldc, tab, s);
