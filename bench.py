@@ -53,12 +53,12 @@ INT32_LANES_PER_SM = 128
 #     gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum,
 #     sm__pipe_alu_cycles_active.avg.pct_of_peak_sustained_active
 #     python bench.py --steps 1 --warmup 1 --no-cpu-baseline --no-e2e
-# (prefilter 0.627 ms, 6.50 + 4.74 MB, ALU 53.8%; check 1.051 ms, 132.0 + 155.7 MB,
-# ALU 50.7%; the ALU share below is their time-weighted mean).  Reported only
+# (prefilter 0.298 ms, 12.9 + 2.7 MB, ALU 64.5%; check 0.893 ms, 93.9 + 147.9 MB,
+# ALU 40.5%; the ALU share below is their time-weighted mean).  Reported only
 # when the timed workload is that one.
 ALLPAIRS_NCU = {"contigs": 50000, "samples": 20,
-                "dram_bytes": 12854016 + 4613632 + 131647232 + 155896576,
-                "alu_pipe_frac": (0.460032 * 0.4908 + 1.020576 * 0.5053) / (0.460032 + 1.020576)}
+                "dram_bytes": 12857344 + 2669568 + 93880064 + 147903744,
+                "alu_pipe_frac": (0.297952 * 0.6447 + 0.892512 * 0.4046) / (0.297952 + 0.892512)}
 
 
 class ClockSampler:
@@ -837,25 +837,26 @@ def run_depth_form(args):
                       "call_ms": float(out["total_ms"]), "total_ms": ms},
         "decompressed_gbs": ub / (ms / 1000.0) / 1e9,
         "device_route": bool(out["device_bams"] == nbam),
-        "kernels": {"names": "k_inflate + k_walk (2 passes) + k_scan_counts + k_depth_reads_dev "
-                             "per chunk, k_depth_means per call",
+        "kernels": {"names": "k_inflate + k_scan_counts + k_gather_offsets + k_depth_reads_dev "
+                             "per chunk, k_depth_means per call; chunks run two at a time, so "
+                             "device_ms counts the time two of them share twice",
                     "device_ms": kms, "records_per_s": recs / (kms / 1000.0),
                     "inflated_gbs": ub / (kms / 1000.0) / 1e9},
-        # k_inflate is 96% of the route's device time (launch list of this
+        # k_inflate is 98% of the route's device time (launch list of this
         # workload); its algorithmic bytes are the compressed blocks read and
         # the inflated bytes written
-        "roofline": {"bound": "hbm", "kernel": "k_inflate (with walk and rule: 96% inflate)",
+        "roofline": {"bound": "hbm", "kernel": "k_inflate (with gather and rule: 98% inflate)",
                      "achieved": (bam_bytes + ub) / (kms / 1000.0) / 1e9,
                      "peak": pk.get("hbm_gbs") if pk else 6650.0, "unit": "GB/s",
                      "frac": (bam_bytes + ub) / (kms / 1000.0) / 1e9 /
                              (pk.get("hbm_gbs") if pk else 6650.0),
                      "peak_source": "hbm_gbs of MEASURED_PEAKS.json" if pk else "fallback",
-                     "traffic": 1.85 * (bam_bytes + ub),
+                     "traffic": 2.0 * (bam_bytes + ub),
                      "traffic_source": "ncu dram__bytes_read+write of k_inflate on the 8,000-contig "
-                                       "case (1.85x its algorithmic bytes: the CRC pass re-reads "
-                                       "the output), scaled by bytes",
+                                       "case (2.0x its algorithmic bytes: matches, the CRC "
+                                       "and the record walk re-read the output), scaled by bytes",
                      "note": "latency-bound Huffman decode chain, not bandwidth"},
-        "gpu_launches": 5 * sum(max(1, -(-(ub // nbam) // (1024 << 20))) for _ in range(nbam)) + 1,
+        "gpu_launches": 4 * sum(max(1, -(-(ub // nbam) // (1024 << 20))) for _ in range(nbam)) + 1,
         "clocks": clk.summary(),
     }
     if not args.no_cpu_baseline:
