@@ -628,17 +628,15 @@ Lists sub_lists(const Lists &W, int bb, int be) {
   return R;
 }
 
-// The passes' flags after their synchronisation: a kept fraction per S with room
-// to spare for the next lists; false when a list overflowed.
+// The passes' flags after their synchronisation: the kept fractions, for the next
+// lists; false when a list overflowed.
 bool tc5_batch_settle(rbg_ctx *c) {
   const int *fl = c->tc5_host.as<int>();
-  if (fl[1] != 0)
-    throw Error(RBG_ERR_TIMEOUT, "tensor-core prefilter: a bounded device wait gave up (stage " +
-                                     std::to_string(fl[1]) + ")");
-  for (size_t S = 0; S < c->tc5_frac.size(); ++S) {
+  tc5_check_wait(fl[1]);
+  for (int key = 0; key < kTc5Keys; ++key) {
     float need;
-    std::memcpy(&need, fl + 2 + S, sizeof(need));
-    c->tc5_frac[S] = std::max(c->tc5_frac[S], 1.25 * (double)need);
+    std::memcpy(&need, fl + 2 + key, sizeof(need));
+    tc5_raise_frac(c, key, (double)need);
   }
   return fl[0] == 0;
 }

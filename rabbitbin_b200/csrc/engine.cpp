@@ -255,7 +255,7 @@ void stage_sketch_chunked(rbg_ctx *c, const rbg_params *p, const char *seqcat,
   // samples the prune passes a large share of the pairs, so it streams from
   // S >= 10, and never again at an S whose survivors outgrew the list.
   const bool stream_pairs = G > 1 && S >= 10 && !want_winners && sym_regime(p, n, S) &&
-                            !((c->no_stream_S >> (S & 63)) & 1u);
+                            !((c->no_stream_S >> (S & 63)) & 1u) && !tc5_lists_large(c, S, n);
   GraphArgs ga;
   SymOut o;
   bool tc5 = false;
@@ -650,37 +650,93 @@ void sym_tc5_clear(rbg_ctx *c) {
   CK(cudaMemsetAsync(c->tc5_flags.p, 0, kTc5Flags * sizeof(int), c->stream));
 }
 
+void tc5_check_wait(int stage) {
+  if (stage != 0)
+    throw Error(RBG_ERR_TIMEOUT, "tensor-core prefilter: a bounded device wait gave up (stage " +
+                                     std::to_string(stage) + ")");
+}
+
+// A pass kept the fraction `need`: lists with a quarter to spare from now on (at 1
+// every pair of a block has a place).
+void tc5_raise_frac(rbg_ctx *c, int key, double need) {
+  c->tc5_frac[key] = std::min(1.0, std::max(c->tc5_frac[key], 1.25 * need));
+}
+
+// The next setup's capacities: room for the counts cnt of every block.
+void tc5_exact_caps(rbg_ctx *c, int64_t n, const int32_t *cnt) {
+  c->tc5_cap.resize((size_t)((n + 31) / 32));
+  for (size_t b = 0; b < c->tc5_cap.size(); ++b)
+    c->tc5_cap[b] = ((int64_t)cnt[b] + 256 + 31) & ~(int64_t)31;
+  c->tc5_exact = true;
+}
+
+// The fraction at which an assembly's lists (4 bytes an entry) take c->list_bytes.
+double tc5_most(const rbg_ctx *c, int64_t n) {
+  return (double)c->list_bytes / (2.0 * (double)n * (double)n);
+}
+
+bool tc5_lists_large(const rbg_ctx *c, int S, int64_t n) {
+  return c->tc5_frac[tc5_key(S, n)] > tc5_most(c, n);
+}
+
+// The fraction that sizes an assembly's lists: the remembered one, at least kTc5First
+// as far as list_bytes allows.
+double tc5_list_frac(const rbg_ctx *c, int S, int64_t n) {
+  return std::max(c->tc5_frac[tc5_key(S, n)], std::min(kTc5First, tc5_most(c, n)));
+}
+
+int sym_tc5_prefilter(rbg_ctx *c, const GraphArgs &g, int64_t cb, int64_t ce, int slot);
+
 // Buffers, list capacities (for the whole assembly) and the padded FP16 rows
 // for the passes over one assembly; `slots` item tables (one per
 // pass in flight).  The capacities come from the kept fraction, or exact ones
 // right after a pass whose lists overflowed (the one host copy here, on a
 // rerun only); offsets and item tables are made on the device, so nothing is
-// copied in while input chunks stream in.
+// copied in while input chunks stream in.  Lists that the fraction would make too
+// large are sized by counting first (tc5_lists_large).
 void sym_tc5_setup(rbg_ctx *c, const GraphArgs &g, int slots) {
   const int64_t n = g.n, B32 = (n + 31) / 32, RBmax = (n + 127) / 128;
   cudaStream_t s = c->stream;
   int64_t total = 0;
-  c->tc5_coff.ensure((size_t)(B32 + 1) * sizeof(int64_t));
-  if (c->tc5_exact && c->tc5_n == n && c->tc5_cap.size() == (size_t)B32) {
-    for (int64_t b = 0; b < B32; ++b) total += c->tc5_cap[b];
-    c->tc5_pin.ensure((size_t)B32 * sizeof(int64_t));
-    std::memcpy(c->tc5_pin.p, c->tc5_cap.data(), (size_t)B32 * sizeof(int64_t));
-    c->tc5_caps.ensure((size_t)B32 * sizeof(int64_t));
-    CK(cudaMemcpyAsync(c->tc5_caps.p, c->tc5_pin.p, (size_t)B32 * sizeof(int64_t),
-                       cudaMemcpyHostToDevice, s));
-    launch_tc5_coff(n, 0.0, c->tc5_caps.as<int64_t>(), c->tc5_coff.as<int64_t>(), s);
-  } else {
-    total = tc5_capacity(n, c->tc5_frac[g.S]);
-    launch_tc5_coff(n, c->tc5_frac[g.S], nullptr, c->tc5_coff.as<int64_t>(), s);
-  }
+  auto lists = [&](double frac) {             // frac < 0: the capacities tc5_cap
+    c->tc5_coff.ensure((size_t)(B32 + 1) * sizeof(int64_t));
+    total = 0;
+    if (frac < 0.0) {
+      for (int64_t b = 0; b < B32; ++b) total += c->tc5_cap[b];
+      c->tc5_pin.ensure((size_t)B32 * sizeof(int64_t));
+      std::memcpy(c->tc5_pin.p, c->tc5_cap.data(), (size_t)B32 * sizeof(int64_t));
+      c->tc5_caps.ensure((size_t)B32 * sizeof(int64_t));
+      CK(cudaMemcpyAsync(c->tc5_caps.p, c->tc5_pin.p, (size_t)B32 * sizeof(int64_t),
+                         cudaMemcpyHostToDevice, s));
+      launch_tc5_coff(n, 0.0, c->tc5_caps.as<int64_t>(), c->tc5_coff.as<int64_t>(), s);
+    } else {
+      total = tc5_capacity(n, frac);
+      launch_tc5_coff(n, frac, nullptr, c->tc5_coff.as<int64_t>(), s);
+    }
+    c->tc5_cand.ensure((size_t)std::max<int64_t>(total, 1) * sizeof(uint32_t));
+  };
+  const bool exact = c->tc5_exact && c->tc5_n == n && c->tc5_cap.size() == (size_t)B32;
+  const bool count = !exact && tc5_lists_large(c, g.S, n);
+  lists(exact ? -1.0 : (count ? 0.0 : tc5_list_frac(c, g.S, n)));
   c->tc5_exact = false;
   c->tc5_n = n;
   c->tc5_rbmax = RBmax;
   c->tc5_items.ensure((size_t)slots * (RBmax + 1) * sizeof(int32_t));
-  c->tc5_cand.ensure((size_t)std::max<int64_t>(total, 1) * sizeof(uint32_t));
   c->tc5_cnt.ensure((size_t)(B32 + 1) * sizeof(int32_t));   // the counts, then the item counter
   c->tc5_u16p.ensure((size_t)n * 256);         // row and column copies
   launch_pad_unit16(g, prefilter_lo16(g.S, g.prefilter_eps), c->tc5_u16p.as<uint16_t>(), s);
+  if (count) {
+    GraphArgs gc = g;
+    gc.stats = nullptr;
+    sym_tc5_prefilter(c, gc, 0, n, 0);
+    sym_tc5_readback(c, n);
+    CK(cudaMemsetAsync(c->tc5_flags.p, 0, sizeof(int), s));    // (lists without room overflow)
+    CK(cudaStreamSynchronize(s));
+    tc5_check_wait(c->tc5_host.as<int>()[1]);
+    tc5_exact_caps(c, n, c->tc5_host.as<int>() + 2);
+    c->tc5_exact = false;
+    lists(-1.0);
+  }
   const int pg = (g.mpad + 31) / 32;
   c->planesA.ensure((size_t)n * pg * 32);
   c->planesB.ensure((size_t)n * pg * 32);
@@ -691,21 +747,12 @@ void sym_tc5_setup(rbg_ctx *c, const GraphArgs &g, int slots) {
   c->launches += 2;
 }
 
-// The pass over the pairs i < j with j in [cb, ce) (item table in `slot`), the
-// rows below cb being in earlier passes' windows; makes the register planes of
-// the rows [cb, ce).
-void sym_tc5_pass(rbg_ctx *c, const GraphArgs &g0, const SymOut &o, int64_t cb, int64_t ce,
-                  int slot) {
-  GraphArgs g = g0;
-  g.pg = (g.mpad + 31) / 32;
-  g.planesA = c->planesA.as<uint32_t>();
-  g.planesB = c->planesB.as<uint32_t>();
-  g.lowA = c->lowA.as<uint32_t>();
-  g.lowB = c->lowB.as<uint32_t>();
-  g.pflag = c->pflag.as<uint8_t>();
+// The prefilter over the pairs i < j with j in [cb, ce) (item table in `slot`);
+// the number of SMs, or 0 when there is no such pair.
+int sym_tc5_prefilter(rbg_ctx *c, const GraphArgs &g, int64_t cb, int64_t ce, int slot) {
   int RB = 0, NT = 0;
   const int items = sym_tc5_items(cb, ce, &RB, &NT);
-  if (items == 0) return;
+  if (items == 0) return 0;
   const int64_t blocks = (ce + 31) / 32;
   int32_t *di0 = c->tc5_items.as<int32_t>() + (size_t)slot * (c->tc5_rbmax + 1);
   cudaStream_t s = c->stream;
@@ -719,44 +766,49 @@ void sym_tc5_pass(rbg_ctx *c, const GraphArgs &g0, const SymOut &o, int64_t cb, 
       g, c->tc5_u16p.as<uint16_t>(), cb, ce, di0, RB, NT, items, c->tc5_cand.as<uint32_t>(), c->tc5_coff.as<int64_t>(), c->tc5_cnt.as<int32_t>(),
       c->tc5_flags.as<int>(), c->tc5_flags.as<int>() + 1, sms, s, &why);
   if (rc != RBG_OK) throw Error(rc, std::string("tensor-core prefilter: ") + why);
+  c->launches += 2;
+  return sms;
+}
+
+// The pass over the pairs i < j with j in [cb, ce), the rows below cb being in
+// earlier passes' windows; makes the register planes of the rows [cb, ce).
+void sym_tc5_pass(rbg_ctx *c, const GraphArgs &g0, const SymOut &o, int64_t cb, int64_t ce,
+                  int slot) {
+  GraphArgs g = g0;
+  g.pg = (g.mpad + 31) / 32;
+  g.planesA = c->planesA.as<uint32_t>();
+  g.planesB = c->planesB.as<uint32_t>();
+  g.lowA = c->lowA.as<uint32_t>();
+  g.lowB = c->lowB.as<uint32_t>();
+  g.pflag = c->pflag.as<uint8_t>();
+  const int sms = sym_tc5_prefilter(c, g, cb, ce, slot);
+  if (sms == 0) return;
+  const int64_t blocks = (ce + 31) / 32;
+  cudaStream_t s = c->stream;
   launch_code_planes(g, cb, ce, c->planesA.as<uint32_t>(), c->planesB.as<uint32_t>(),
                      c->lowA.as<uint32_t>(), c->lowB.as<uint32_t>(), c->pflag.as<uint8_t>(), s);
   launch_sym_check(g, o, c->tc5_cand.as<uint32_t>(), c->tc5_coff.as<int64_t>(),
                    c->tc5_cnt.as<int32_t>(), blocks, c->tc5_seg.as<int32_t>(),
                    (unsigned *)c->tc5_cnt.as<int32_t>() + blocks,
-                   c->tc5_flags.as<float>() + 2 + g.S, sms, s);
-  c->launches += 5;
+                   c->tc5_flags.as<float>() + 2 + tc5_key(g.S, g.n), sms, s);
+  c->launches += 3;
 }
 
 // After the pass's synchronisation (the flags and counts read back into
 // c->tc5_host): false when a list overflowed (capacities now exact: rerun).
 bool sym_tc5_settle(rbg_ctx *c, int64_t n, int S) {
   const int64_t B32 = (n + 31) / 32;
-  double &frac_S = c->tc5_frac[S];
   const int *fl = c->tc5_host.as<int>();
   const int32_t *cnt = fl + 2;
-  if (fl[1] != 0)
-    throw Error(RBG_ERR_TIMEOUT, "tensor-core prefilter: a bounded device wait gave up (stage " +
-                                     std::to_string(fl[1]) + ")");
+  tc5_check_wait(fl[1]);
   double frac = 0.0;
-  for (int64_t b = 0; b < B32; ++b) {
-    const double pairs = 32.0 * (double)std::max<int64_t>(n - 32 * b, 0);
+  for (int64_t b = 0; b < B32 && n - 32 * b > kTc5Tail; ++b)
     // past the 256 entries every list has room for
-    if (pairs > 0) frac = std::max(frac, (cnt[b] - 256) / pairs);
-  }
-  if (fl[0] != 0) {                          // rerun with room for every block's count
-    c->tc5_cap.assign((size_t)B32, 0);
-    for (int64_t b = 0; b < B32; ++b) {
-      const double pairs = 32.0 * (double)std::max<int64_t>(n - 32 * b, 0);
-      const int64_t fc = ((int64_t)(pairs * frac_S) + 256 + 31) & ~(int64_t)31;
-      c->tc5_cap[b] = std::max<int64_t>(fc, ((int64_t)cnt[b] + 256 + 31) & ~(int64_t)31);
-    }
-    c->tc5_exact = true;
-    frac_S = std::max(frac_S, frac * 1.25);
-    return false;
-  }
-  if (frac * 1.25 > frac_S) frac_S = frac * 1.25;   // room to spare next time
-  return true;
+    frac = std::max(frac, (cnt[b] - 256) / (32.0 * (double)(n - 32 * b)));
+  tc5_raise_frac(c, tc5_key(S, n), frac);    // room to spare next time
+  if (fl[0] == 0) return true;
+  tc5_exact_caps(c, n, cnt);                 // rerun with room for every block's count
+  return false;
 }
 
 // The flags and per-block counts to the host on the stream (read after its sync).
@@ -975,12 +1027,10 @@ void run_graph(rbg_ctx *c, const rbg_params *p, const ShardCtx *sc = nullptr) {
       CK(cudaEventSynchronize(c->ev[10]));
       if (streamed && c->streamed_tc5) {
         const int *fl = c->tc5_host.as<int>();
-        if (fl[1] != 0)
-          throw Error(RBG_ERR_TIMEOUT, "tensor-core prefilter: a bounded device wait gave up "
-                                       "(stage " + std::to_string(fl[1]) + ")");
+        tc5_check_wait(fl[1]);
         if (fl[0] != 0) {                            // a window's list overflowed: rescore
           CK(cudaStreamSynchronize(c->stream));
-          c->tc5_frac[S] *= 2.0;
+          tc5_raise_frac(c, tc5_key(S, n), 1.6 * tc5_list_frac(c, S, n));   // twice as much
           streamed = false;
           continue;
         }
@@ -1531,6 +1581,15 @@ int rbg_create(int device, rbg_ctx **out) {
     delete c;
     return RBG_ERR_CUDA;
   }
+  size_t free_bytes = 0, total_bytes = 0;
+  if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) {
+    cudaStreamDestroy(c->stream);
+    delete c;
+    return RBG_ERR_CUDA;
+  }
+  // RBG_LIST_BYTES: a smaller bound, to exercise the count of the candidates
+  const char *lb = getenv("RBG_LIST_BYTES");
+  c->list_bytes = lb ? std::max<int64_t>(1 << 20, strtoll(lb, nullptr, 10)) : (int64_t)(total_bytes / 4);
   for (auto &e : c->ev) cudaEventCreate(&e);
   if (cudaStreamCreateWithFlags(&c->aux, cudaStreamNonBlocking) != cudaSuccess) {
     cudaStreamDestroy(c->stream);

@@ -153,13 +153,32 @@ void check_onehot_status(rbg_ctx *c);
 bool sym_tc5_fits(const GraphArgs &g);
 void sym_tc5_setup(rbg_ctx *c, const GraphArgs &g, int slots);
 void sym_tc5_clear(rbg_ctx *c);
-// Flags read back: [0] a list overflowed, [1] wait error, [2 + S] float bits of
-// the largest kept fraction of the passes at S samples.
-constexpr int kTc5Flags = 2 + 65;
+// The kept fractions that size the lists are remembered by S and by the power of
+// two below n, so that a small assembly of one genome, nearly all of whose pairs
+// pass the prune, does not size the lists of a large one.
+constexpr int kTc5Keys = 65 * 27;      // S <= 64, n <= 2^26
+inline int tc5_key(int S, int64_t n) {
+  int lg = 0;
+  while (lg < 26 && ((int64_t)2 << lg) <= n) ++lg;
+  return S * 27 + lg;
+}
+// Flags read back: [0] a list overflowed, [1] wait error, [2 + key] float bits of
+// the largest kept fraction of the passes of that key.
+constexpr int kTc5Flags = 2 + kTc5Keys;
 void sym_tc5_pass(rbg_ctx *c, const GraphArgs &g, const SymOut &o, int64_t cb, int64_t ce,
                   int slot);
+// Before a pass has been seen: 3% of the pairs.
+constexpr double kTc5First = 0.03;
+// Whether the lists of the remembered fraction would take more than
+// rbg_ctx::list_bytes (one block of 32 rows sets it for all: a single dense block
+// among 300,000 contigs would ask for 180 GB).  sym_tc5_setup then counts the
+// candidates first, by the prefilter alone over the whole assembly, and waits for
+// them; such an assembly's pairs do not stream behind its input.
+bool tc5_lists_large(const rbg_ctx *c, int S, int64_t n);
 void sym_tc5_readback(rbg_ctx *c, int64_t n);
 bool sym_tc5_settle(rbg_ctx *c, int64_t n, int S);
+void tc5_check_wait(int stage);
+void tc5_raise_frac(rbg_ctx *c, int key, double need);
 // The dense regime runs on the one-hot tensor-core kernels, unless RBG_DENSE_ALU is
 // set (for measurement) or the contigs are few: the integer-ALU register compare
 // then, without the one-hot rows' four launches and the read-back of their width.
@@ -398,7 +417,9 @@ struct rbg_ctx {
   rbg::HBuf tc5_pin, tc5_host;
   std::vector<int64_t> tc5_cap;
   int64_t tc5_n = -1;
-  std::vector<double> tc5_frac = std::vector<double>(65, 0.03);   // by S
+  std::vector<double> tc5_frac = std::vector<double>(rbg::kTc5Keys, 0.0);   // by tc5_key, <= 1
+  int64_t list_bytes = 0;               // most that lists sized from a fraction take: a
+                                        // quarter of the device's memory
   bool tc5_exact = false;               // tc5_cap holds exact capacities for the next setup
   int64_t tc5_rbmax = 0;                // item-table slot length - 1
   bool streamed_tc5 = false;            // the pairs behind the copy went through that pass

@@ -819,7 +819,8 @@ __global__ void __launch_bounds__(1024) k_check_items(const int64_t *coff, const
   for (int64_t b = lo; b < hi; ++b) {
     sum += (unsigned)listed(b);
     // (past the 256 entries every list has room for)
-    kept = fmaxf(kept, (float)(ccnt[b] - 256) / (32.f * (float)(n - 32 * b)));
+    if (n - 32 * b > kTc5Tail)
+      kept = fmaxf(kept, (float)(ccnt[b] - 256) / (32.f * (float)(n - 32 * b)));
   }
   // non-negative floats order as their bits
   kept = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(kept)));

@@ -435,13 +435,11 @@ __device__ void block_scan_into(int64_t count, F v, T *out) {
 }
 
 // List offsets of the 32-row blocks: capacities from the kept fraction
-// (32 (n - 32 b) pairs x frac + 256, rounded up to 32) or given ones.
+// (tc5_block_cap) or given ones.
 __global__ void k_tc5_coff(int64_t n, double frac, const int64_t *caps, int64_t *coff) {
   const int64_t B32 = (n + 31) / 32;
   block_scan_into(B32, [&](int64_t b) -> int64_t {
-    if (caps) return caps[b];
-    const double pairs = 32.0 * (double)max((int64_t)0, n - 32 * b);
-    return (((int64_t)(pairs * frac) + 256 + 31) & ~(int64_t)31);
+    return caps ? caps[b] : tc5_block_cap(n, b, frac);
   }, coff);
 }
 
@@ -470,10 +468,7 @@ int sym_tc5_items(int64_t cb, int64_t ce, int *RB, int *NT) {
 // Total list capacity of the frac-based capacities (the arithmetic of k_tc5_coff).
 int64_t tc5_capacity(int64_t n, double frac) {
   int64_t tot = 0;
-  for (int64_t b = 0; b < (n + 31) / 32; ++b) {
-    const double pairs = 32.0 * (double)std::max<int64_t>(0, n - 32 * b);
-    tot += ((int64_t)(pairs * frac) + 256 + 31) & ~(int64_t)31;
-  }
+  for (int64_t b = 0; b < (n + 31) / 32; ++b) tot += tc5_block_cap(n, b, frac);
   return tot;
 }
 

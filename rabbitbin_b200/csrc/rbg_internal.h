@@ -259,8 +259,19 @@ void launch_allpairs_sym(const GraphArgs &g, const SymOut &o, cudaStream_t s, in
 // in the last half (2 x n x 128 bytes, 16-byte aligned).  Needs g.S < 64 and
 // n < 2^27.  The offsets and item tables are made on the device, so nothing
 // crosses PCIe while input chunks stream in; tc5_capacity is the total of the
-// frac-based capacities of launch_tc5_coff (caps null).
+// frac-based capacities (tc5_block_cap) of launch_tc5_coff (caps null).
 int sym_tc5_items(int64_t cb, int64_t ce, int *RB, int *NT);
+// Entries of 32-row block b's candidate list for a kept fraction of its pairs (32
+// rows against the columns from its first on), with 256 to spare.  The blocks with
+// at most kTc5Tail columns left have room for every pair (all of them together 2 MB):
+// they say little about the fraction, and one of few columns often keeps most of
+// its pairs.
+constexpr int64_t kTc5Tail = 1024;
+__host__ __device__ inline int64_t tc5_block_cap(int64_t n, int64_t b, double frac) {
+  const int64_t cols = n > 32 * b ? n - 32 * b : 0;
+  const double pairs = 32.0 * (double)cols * (cols <= kTc5Tail ? 1.0 : frac);
+  return ((int64_t)pairs + 256 + 31) & ~(int64_t)31;
+}
 int64_t tc5_capacity(int64_t n, double frac);
 void launch_tc5_coff(int64_t n, double frac, const int64_t *caps, int64_t *coff, cudaStream_t s);
 void launch_tc5_items(int64_t cb, int64_t ce, int32_t *item0, cudaStream_t s);
@@ -277,7 +288,8 @@ void launch_code_planes(const GraphArgs &g, int64_t r_lo, int64_t r_hi, uint32_t
                         cudaStream_t s);
 // Exact check and register compare of the candidate lists of blocks [0, B)
 // (seg: B + 2 words of scratch; next: a counter zeroed before the launch).
-// need: raised to the largest fraction of a block's pairs that were candidates.
+// need: raised to the largest fraction of a block's pairs that were candidates
+// (blocks of more than kTc5Tail columns).
 void launch_sym_check(const GraphArgs &g, const SymOut &o, const uint32_t *cand,
                       const int64_t *coff, const int32_t *ccnt, int64_t B, int32_t *seg,
                       unsigned *next, float *need, int sms, cudaStream_t s);
