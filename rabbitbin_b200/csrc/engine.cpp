@@ -1044,10 +1044,14 @@ void run_graph(rbg_ctx *c, const rbg_params *p, const ShardCtx *sc = nullptr) {
       if (streamed) {
         // The streamed pass lists every survivor, not only the admitted ones: a
         // larger list next time while that stays within four times the first one
-        // (256 pairs a contig), the resident pass at this S from now on otherwise.
-        // 200,003 contigs at S = 30 (67 M survivors) stay on the streamed pass.
-        if (*hnp <= (unsigned long long)n1 * 1024) c->sym_cap = *hnp + *hnp / 4;
-        else c->no_stream_S |= 1ull << (S & 63);
+        // (256 pairs a contig) and list_bytes, the resident pass at this S from now
+        // on otherwise.  200,003 contigs at S = 30 (67 M survivors) stay on the
+        // streamed pass.
+        const unsigned long long more = *hnp + *hnp / 4;
+        if (*hnp <= (unsigned long long)n1 * 1024 && more * kPairBytes <= (uint64_t)c->list_bytes)
+          c->sym_cap = more;
+        else
+          c->no_stream_S |= 1ull << (S & 63);
         streamed = false;
       } else {
         c->sym_cap = *hnp + *hnp / 4;

@@ -210,6 +210,9 @@ inline bool pack_on_host() {
 void *pinned_take(size_t bytes);
 void pinned_share(void *blk, const std::vector<void *> &firsts);
 
+// Device bytes of an admitted pair: its record and its two keys.
+constexpr int kPairBytes = 16 + 2 * 8;
+
 // Buffers of the batch engine (many assemblies per launch).
 struct BatchBufs {
   DBuf ascii, offsets, depth, packed, nmask, winv, ecnt, codesA, codesB;

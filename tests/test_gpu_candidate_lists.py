@@ -83,3 +83,38 @@ def test_dense_assembly_graph(orc, monkeypatch, S, list_bytes):
                     assert np.array_equal(g[k], x), k
     finally:
         ctx.close()
+
+
+def test_streamed_pair_list_within_its_bound(monkeypatch):
+    """A streamed pass lists every survivor of the prune.  Where they outgrow the
+    list, it grows only within the bound of the lists; the pairs are scored after
+    the copy from then on otherwise, with a list of the admitted pairs alone."""
+    a = make_assembly(40, 3000, 12, seed=74, median_len=4000.0, max_len=6000)
+    depth = a.depth.copy()
+    rows = [a.depth[a.genome_of == g] for g in range(4)]         # 40 genomes, 4 coverages
+    for i in range(a.n):
+        r = rows[a.genome_of[i] & 3]
+        depth[i] = r[i % len(r)]
+    buf, offs = a.concat()
+    case = (buf, offs, depth, api.default_params(force_path=2))
+    monkeypatch.setenv("RBG_PAIR_CAP", "1024")
+
+    def taken():
+        gc.collect()
+        before = _free()
+        ctx = api.Context(0)
+        try:
+            got = [ctx.bin_graph(*case) for _ in range(2)]
+            return before - _free(), got
+        finally:
+            ctx.close()
+
+    taken()                                                      # modules load
+    most, want = taken()
+    monkeypatch.setenv("RBG_LIST_BYTES", str(16 << 20))
+    least, got = taken()
+    for g in got:
+        for k in ("src", "dst", "scomp", "score"):
+            assert np.array_equal(g[k], want[0][k]), k
+    # about 1.1 M survivors: 45 MB with a quarter to spare
+    assert least <= most - (12 << 20)
