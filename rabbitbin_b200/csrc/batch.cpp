@@ -164,7 +164,8 @@ void validate_assembly(const rbg_assembly &x, const rbg_params *p, const std::st
     throw Error(RBG_ERR_ARG, who + "the fused path samples 2500 contigs; need n > 2500");
 }
 
-int64_t batch_request_bytes(const rbg_params *p, int64_t n, int64_t nbases, int S) {
+int64_t batch_request_bytes(const rbg_params *p, int64_t n, int64_t nbases, int S,
+                            int64_t list_bytes, bool most) {
   const int m = p->m, mpad = mpad_of(m), K = p->max_edges;
   const int Su = (std::max(S, 1) + 3) & ~3, Kp = unit16_stride(S);
   const int E = p->k == 4 ? 136 : (p->k == 3 ? 32 : (p->k == 2 ? 10 : 2));
@@ -176,9 +177,15 @@ int64_t batch_request_bytes(const rbg_params *p, int64_t n, int64_t nbases, int 
   int64_t b = nbases + nbases / 4 + nbases / 8 + 64;             // ASCII, 2-bit words, mask
   b += n * (int64_t)(S * 4 + 8 + E * 8 + 4 + 2 * mpad + Su * 4 + Kp * 2 + 1);
   b += n * (int64_t)K * (8 + 4 + 4) + n * 32;                    // top-K, neighbour lists
-  if (abd)
-    b += n * 256 * (16 + 2 * 8) + n * 12;                        // admitted pairs, keys, rows
-  else if (dense_on_gemm(n) && onehot_mma_fits(n, m)) {           // one-hot rows, candidate lists
+  if (abd) {
+    // admitted pairs and keys (a streamed pass lists up to 1,280 survivors a contig),
+    // rows; the two-kernel pass's buffers, with candidate lists of every pair at most
+    const int64_t pairs = std::max<int64_t>(1 << 20, n * 256);
+    b += std::max<int64_t>(pairs * kPairBytes,
+                           most && S >= 10 ? std::min(n * 1280 * kPairBytes, list_bytes) : 0) + n * 12;
+    const int64_t entries = tc5_capacity(n, most ? 1.0 : kTc5First);
+    b += tc5_sizes(n, mpad, std::min<int64_t>(entries, list_bytes / 4), kChunks).bytes();
+  } else if (dense_on_gemm(n) && onehot_mma_fits(n, m)) {           // one-hot rows, candidate lists
     int GR = 1, GC = 1;
     onehot_mma_grid((int)((n + 255) / 256), (int)((n + 255) / 256), 148, &GR, &GC);
     b += n * (int64_t)std::max(128, 136 * m / 8) +

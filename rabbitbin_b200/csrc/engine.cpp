@@ -697,10 +697,8 @@ int sym_tc5_prefilter(rbg_ctx *c, const GraphArgs &g, int64_t cb, int64_t ce, in
 void sym_tc5_setup(rbg_ctx *c, const GraphArgs &g, int slots) {
   const int64_t n = g.n, B32 = (n + 31) / 32, RBmax = (n + 127) / 128;
   cudaStream_t s = c->stream;
-  int64_t total = 0;
   auto lists = [&](double frac) {             // frac < 0: the capacities tc5_cap
-    c->tc5_coff.ensure((size_t)(B32 + 1) * sizeof(int64_t));
-    total = 0;
+    int64_t total = 0;
     if (frac < 0.0) {
       for (int64_t b = 0; b < B32; ++b) total += c->tc5_cap[b];
       c->tc5_pin.ensure((size_t)B32 * sizeof(int64_t));
@@ -713,17 +711,19 @@ void sym_tc5_setup(rbg_ctx *c, const GraphArgs &g, int slots) {
       total = tc5_capacity(n, frac);
       launch_tc5_coff(n, frac, nullptr, c->tc5_coff.as<int64_t>(), s);
     }
-    c->tc5_cand.ensure((size_t)std::max<int64_t>(total, 1) * sizeof(uint32_t));
+    c->tc5_cand.ensure(tc5_sizes(n, g.mpad, total, slots).cand);
   };
+  const Tc5Sizes z = tc5_sizes(n, g.mpad, 0, slots);
+  c->tc5_coff.ensure(z.coff);
   const bool exact = c->tc5_exact && c->tc5_n == n && c->tc5_cap.size() == (size_t)B32;
   const bool count = !exact && tc5_lists_large(c, g.S, n);
   lists(exact ? -1.0 : (count ? 0.0 : tc5_list_frac(c, g.S, n)));
   c->tc5_exact = false;
   c->tc5_n = n;
   c->tc5_rbmax = RBmax;
-  c->tc5_items.ensure((size_t)slots * (RBmax + 1) * sizeof(int32_t));
-  c->tc5_cnt.ensure((size_t)(B32 + 1) * sizeof(int32_t));   // the counts, then the item counter
-  c->tc5_u16p.ensure((size_t)n * 256);         // row and column copies
+  c->tc5_items.ensure(z.items);
+  c->tc5_cnt.ensure(z.cnt);
+  c->tc5_u16p.ensure(z.u16p);
   launch_pad_unit16(g, prefilter_lo16(g.S, g.prefilter_eps), c->tc5_u16p.as<uint16_t>(), s);
   if (count) {
     GraphArgs gc = g;
@@ -737,13 +737,12 @@ void sym_tc5_setup(rbg_ctx *c, const GraphArgs &g, int slots) {
     c->tc5_exact = false;
     lists(-1.0);
   }
-  const int pg = (g.mpad + 31) / 32;
-  c->planesA.ensure((size_t)n * pg * 32);
-  c->planesB.ensure((size_t)n * pg * 32);
-  c->lowA.ensure((size_t)n * low_plane_words(pg) * 4);
-  c->lowB.ensure((size_t)n * low_plane_words(pg) * 4);
-  c->pflag.ensure((size_t)n);
-  c->tc5_seg.ensure((size_t)(B32 + 2) * sizeof(int32_t));
+  c->planesA.ensure(z.planes);
+  c->planesB.ensure(z.planes);
+  c->lowA.ensure(z.low);
+  c->lowB.ensure(z.low);
+  c->pflag.ensure(z.flag);
+  c->tc5_seg.ensure(z.seg);
   c->launches += 2;
 }
 

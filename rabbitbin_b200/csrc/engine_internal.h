@@ -177,6 +177,28 @@ constexpr double kTc5First = 0.03;
 bool tc5_lists_large(const rbg_ctx *c, int S, int64_t n);
 void sym_tc5_readback(rbg_ctx *c, int64_t n);
 bool sym_tc5_settle(rbg_ctx *c, int64_t n, int S);
+// Bytes of the pass's device buffers for an assembly whose lists hold `entries`
+// (sym_tc5_setup allocates these).
+struct Tc5Sizes {
+  size_t coff, items, cand, cnt, u16p, planes, low, flag, seg;   // planes, low: one side
+  int64_t bytes() const {
+    return (int64_t)(coff + items + cand + cnt + u16p + 2 * planes + 2 * low + flag + seg);
+  }
+};
+inline Tc5Sizes tc5_sizes(int64_t n, int mpad, int64_t entries, int slots) {
+  const size_t n1 = (size_t)n, B32 = (n1 + 31) / 32, pg = ((size_t)mpad + 31) / 32;
+  Tc5Sizes z;
+  z.coff = (B32 + 1) * sizeof(int64_t);
+  z.items = (size_t)slots * ((n1 + 127) / 128 + 1) * sizeof(int32_t);
+  z.cand = (size_t)std::max<int64_t>(entries, 1) * sizeof(uint32_t);
+  z.cnt = (B32 + 1) * sizeof(int32_t);           // the counts, then the item counter
+  z.u16p = n1 * 256;                             // row and column copies
+  z.planes = n1 * pg * 32;
+  z.low = n1 * low_plane_words((int)pg) * 4;
+  z.flag = n1;
+  z.seg = (B32 + 2) * sizeof(int32_t);
+  return z;
+}
 void tc5_check_wait(int stage);
 void tc5_raise_frac(rbg_ctx *c, int key, double need);
 // The dense regime runs on the one-hot tensor-core kernels, unless RBG_DENSE_ALU is
@@ -372,9 +394,12 @@ FastaCounts fasta_parse(rbg_ctx *c, const char *data, int64_t F, int64_t min_con
 // Frees the CUDA graphs the batch engine keeps for a context.
 void release_batch_graphs(rbg_ctx *c);
 
-// Device bytes the batch engine needs for one assembly (its share of every
-// batch buffer; a bound on the edge arrays).
-int64_t batch_request_bytes(const rbg_params *p, int64_t n, int64_t nbases, int S);
+// Device bytes one assembly needs (its share of every batch buffer, or those of the
+// single-assembly path; a bound on the edge arrays).  most: with the pair and
+// candidate lists at the largest they grow to (list_bytes: rbg_ctx::list_bytes),
+// else as a first call sizes them.
+int64_t batch_request_bytes(const rbg_params *p, int64_t n, int64_t nbases, int S,
+                            int64_t list_bytes, bool most);
 
 // Validation of one assembly's arguments (the checks rbg_bin_batch makes).
 void validate_assembly(const rbg_assembly &x, const rbg_params *p, const std::string &who);

@@ -214,10 +214,13 @@ int rbg_server_submit(rbg_server *s, const rbg_assembly *a, int64_t *request_id)
   r->a = *a;
   r->p = a->params ? *a->params : s->defaults;
   r->a.params = nullptr;
+  int64_t need = 0;                     // with the lists as a first call sizes them
   try {
     rbg::validate_assembly(r->a, &r->p, "");
     const int64_t nbases = r->a.n > 0 ? r->a.offsets[r->a.n] : 0;
-    r->est_bytes = rbg::batch_request_bytes(&r->p, r->a.n, nbases, r->a.S);
+    const int64_t list_bytes = s->ctxs[0]->list_bytes;
+    r->est_bytes = rbg::batch_request_bytes(&r->p, r->a.n, nbases, r->a.S, list_bytes, true);
+    need = rbg::batch_request_bytes(&r->p, r->a.n, nbases, r->a.S, list_bytes, false);
     r->pairs = r->a.n * (r->a.n - 1) / 2;
   } catch (const rbg::Error &e) {
     std::lock_guard<std::mutex> lk(s->mu);
@@ -229,8 +232,8 @@ int rbg_server_submit(rbg_server *s, const rbg_assembly *a, int64_t *request_id)
     s->err = "the server is shutting down";
     return RBG_ERR_ARG;
   }
-  if (r->est_bytes > s->cfg.hbm_budget) {
-    s->err = "the request needs " + std::to_string(r->est_bytes) +
+  if (need > s->cfg.hbm_budget) {
+    s->err = "the request needs " + std::to_string(need) +
              " bytes of device memory, more than the HBM budget (" +
              std::to_string(s->cfg.hbm_budget) + ")";
     return RBG_ERR_NOMEM;
