@@ -79,7 +79,16 @@ struct HBuf {
     if (p) cudaFreeHost(p);
     p = nullptr;
     cap = 0;
-    const size_t want = std::max<size_t>(std::max<size_t>(bytes, grown), 256);
+    const size_t want = bytes < 256 ? 256 : bytes;
+    if (grown > want) {
+      // fall back to the exact size when the grown one cannot be pinned
+      if (cudaMallocHost(&p, grown) == cudaSuccess) {
+        cap = grown;
+        return;
+      }
+      cudaGetLastError();
+      p = nullptr;
+    }
     CK(cudaMallocHost(&p, want));
     cap = want;
   }
