@@ -305,6 +305,7 @@ def lib():
         "rbg_fetch_graph": ([vp, P(Graph)], C.c_int),
         "rbg_free_graph": ([P(Graph)], C.c_int),
         "rbg_result_alloc": ([C.c_size_t], vp),
+        "rbg_result_alloc_on": ([vp, C.c_size_t], vp),
         "rbg_result_free": ([vp], None),
         "rbg_pmh_stream_tables": ([C.c_int32, C.c_int32, C.c_uint64, C.c_int32,
                                    P(C.c_int32), P(C.c_int32), P(C.c_double),
@@ -420,7 +421,7 @@ class _View:
 
 
 class _ResultMem:
-    """Owns one block of rbg_result_alloc and describes it as an array."""
+    """Owns one block of rbg_result_alloc_on and describes it as an array."""
 
     def __init__(self, L, addr, shape, typestr):
         self._L, self._addr = L, addr
@@ -434,13 +435,14 @@ class _ResultMem:
             pass
 
 
-def _result(L, shape, dtype):
+def _result(ctx, shape, dtype):
     """An output array that the call fills completely: pinned memory of the
     library's pool from 1 MB on (the device writes it at bus speed)."""
+    L = ctx._L
     dt = np.dtype(dtype)
     nbytes = int(np.prod(shape, dtype=np.int64)) * dt.itemsize
     if nbytes >= 1 << 20:
-        addr = L.rbg_result_alloc(nbytes)
+        addr = L.rbg_result_alloc_on(ctx._h, nbytes)
         if addr:
             return np.asarray(_ResultMem(L, addr, tuple(shape), dt.str))
     return np.zeros(shape, dt)
@@ -497,7 +499,7 @@ class Context:
         p = params or default_params()
         offs = np.ascontiguousarray(offsets, np.int64)
         n = len(offs) - 1
-        out = _result(self._L, (n, p.m), np.uint32)
+        out = _result(self, (n, p.m), np.uint32)
         self._check(self._L.rbg_build_pmh_winners(self._h, C.byref(p), seqcat, _p(offs, C.c_int64),
                                                   n, _p(out, C.c_uint32)), "build_pmh_winners")
         return out
@@ -508,8 +510,8 @@ class Context:
         p = params or default_params()
         offs = np.ascontiguousarray(offsets, np.int64)
         n = len(offs) - 1
-        w = _result(self._L, (n, p.m), np.uint64)
-        r = _result(self._L, (n, p.m), np.float64)
+        w = _result(self, (n, p.m), np.uint64)
+        r = _result(self, (n, p.m), np.float64)
         self._check(self._L.rbg_build_pmh_sketches(self._h, C.byref(p), seqcat,
                                                    _p(offs, C.c_int64), n, _p(w, C.c_uint64),
                                                    _p(r, C.c_double)), "build_pmh_sketches")
@@ -524,7 +526,7 @@ class Context:
         dt = np.uint64 if code == 0 else np.float64
         A = np.ascontiguousarray(A, dt)
         B = np.ascontiguousarray(B, dt)
-        out = _result(self._L, (A.shape[0], B.shape[0]), np.float64)
+        out = _result(self, (A.shape[0], B.shape[0]), np.float64)
         self._check(self._L.rbg_pmh_compare(self._h, code, A.shape[1], kmer_size,
                                             A.ctypes.data, A.shape[0], B.ctypes.data,
                                             B.shape[0], _p(out, C.c_double)), "pmh_compare")
@@ -533,7 +535,7 @@ class Context:
     def pmh_merge_registers(self, A, B):
         A = np.ascontiguousarray(A, np.float64)
         B = np.ascontiguousarray(B, np.float64)
-        out = _result(self._L, A.shape, np.float64)
+        out = _result(self, A.shape, np.float64)
         self._check(self._L.rbg_pmh_merge_registers(self._h, _p(A, C.c_double), _p(B, C.c_double),
                                                     A.shape[0], A.shape[1], _p(out, C.c_double)),
                     "pmh_merge_registers")

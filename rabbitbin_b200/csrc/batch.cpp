@@ -1022,7 +1022,7 @@ void run_batch(rbg_ctx *c, const rbg_params *defaults, const rbg_assembly *asms,
   // the edge arrays land in one pinned block that the graphs share (no host
   // copy per graph); the staging buffer and copies are the fallback
   const size_t eb = up256(E1 * 4);
-  char *shared = (char *)pinned_take(4 * eb);
+  char *shared = (char *)pinned_take(c, 4 * eb);
   struct Back {                         // an error before the graphs own it: back to the pool
     void *p;
     ~Back() { if (p) pinned_share(p, {}); }

@@ -16,6 +16,8 @@
 #include <numeric>
 #include <random>
 #include <stdexcept>
+#include <system_error>
+#include <thread>
 #include <unordered_map>
 #include <string>
 #include <vector>
@@ -1190,16 +1192,39 @@ void run_graph(rbg_ctx *c, const rbg_params *p, const ShardCtx *sc = nullptr) {
 // kept, the longest idle freed first.  A batch's graphs share one block (each
 // graph's arrays are ranges of the batch-wide arrays): it returns to the pool
 // when the last of them is freed.
+//
+// Blocks are pinned and unpinned with their device current (on a thread of its own
+// where the caller's is another one: setting it back would bring up a context
+// there).
 struct PinnedPool {
+  static constexpr size_t kKeep = (size_t)4 << 30;
   struct Shared {
     void *blk;
     int refs;
   };
+  struct Block {
+    size_t cls;
+    int dev;
+  };
   std::mutex mu;
-  std::unordered_map<void *, size_t> live;
+  std::unordered_map<void *, Block> live;
   std::unordered_map<void *, Shared *> part;   // a graph's first array -> its shared block
-  std::deque<std::pair<size_t, void *>> idle;  // oldest first
+  std::deque<std::pair<Block, void *>> idle;   // oldest first
   size_t idle_bytes = 0;
+
+  template <class F>
+  static void on_device(int dev, F &&f) {
+    int cur = dev;
+    if (cudaGetDevice(&cur) != cudaSuccess) cudaGetLastError();
+    if (cur == dev) {
+      f();
+      return;
+    }
+    try {
+      std::thread([&] { if (cudaSetDevice(dev) == cudaSuccess) f(); }).join();
+    } catch (const std::system_error &) {       // no thread: no block, or one kept for good
+    }
+  }
 
   // 1, 1.5, 2, 3, 4, 6, ... MB: at most a third of a block unused
   static size_t size_class(size_t bytes) {
@@ -1208,23 +1233,27 @@ struct PinnedPool {
     return c;
   }
 
-  void *take(size_t bytes) {
+  void *take(size_t bytes, int dev) {
     const size_t cls = size_class(bytes);
     std::lock_guard<std::mutex> lk(mu);
+    void *p = nullptr;
     for (auto it = idle.rbegin(); it != idle.rend(); ++it)
-      if (it->first == cls) {
-        void *p = it->second;
+      if (it->first.cls == cls) {
+        p = it->second;
+        dev = it->first.dev;
         idle_bytes -= cls;
         idle.erase(std::next(it).base());
-        live[p] = cls;
-        return p;
+        break;
       }
-    void *p = nullptr;
-    if (cudaHostAlloc(&p, cls, cudaHostAllocPortable) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    live[p] = cls;
+    if (!p)
+      on_device(dev, [&] {
+        if (cudaHostAlloc(&p, cls, cudaHostAllocPortable) != cudaSuccess) {
+          cudaGetLastError();
+          p = nullptr;
+        }
+      });
+    if (!p) return nullptr;
+    live[p] = Block{cls, dev};
     return p;
   }
 
@@ -1253,12 +1282,13 @@ struct PinnedPool {
     auto it = live.find(p);
     if (it == live.end()) return false;
     idle.emplace_back(it->second, p);
-    idle_bytes += it->second;
+    idle_bytes += it->second.cls;
     live.erase(it);
-    while (idle.size() > 16 || idle_bytes > ((size_t)4 << 30)) {
-      idle_bytes -= idle.front().first;
-      cudaFreeHost(idle.front().second);
+    while (idle.size() > 16 || idle_bytes > kKeep) {
+      const std::pair<Block, void *> old = idle.front();
+      idle_bytes -= old.first.cls;
       idle.pop_front();
+      on_device(old.first.dev, [&] { cudaFreeHost(old.second); });
     }
     return true;
   }
@@ -1318,7 +1348,7 @@ void copy_out(rbg_ctx *c, void *dst, const void *src, size_t bytes, cudaStream_t
   }
 }
 
-void *pinned_take(size_t bytes) { return pinned_pool().take(bytes); }
+void *pinned_take(rbg_ctx *c, size_t bytes) { return pinned_pool().take(bytes, c->device); }
 void pinned_share(void *blk, const std::vector<void *> &firsts) {
   pinned_pool().share(blk, firsts);
 }
@@ -1338,7 +1368,7 @@ void fetch(rbg_ctx *c, rbg_graph *out) {
   out->path = c->path;
   const size_t n1 = std::max<size_t>(ne, 1);
   const size_t nb = n1 * 4;
-  if (void *blk = pinned_pool().take(4 * nb)) {
+  if (void *blk = pinned_take(c, 4 * nb)) {
     out->from = (uint32_t *)blk;
     out->to = out->from + n1;
     out->scomp = (float *)(out->to + n1);
@@ -1521,9 +1551,22 @@ void bin_graph_one(rbg_ctx *c, const rbg_params *p, const rbg_assembly &x, rbg_g
 
 extern "C" {
 
-void *rbg_result_alloc(size_t bytes) {
+void *rbg_result_alloc_on(rbg_ctx *c, size_t bytes) {
   try {
-    return bytes ? pinned_pool().take(bytes) : nullptr;
+    return c && bytes ? pinned_pool().take(bytes, c->device) : nullptr;
+  } catch (...) {
+    return nullptr;
+  }
+}
+
+void *rbg_result_alloc(size_t bytes) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  try {
+    return bytes ? pinned_pool().take(bytes, dev) : nullptr;
   } catch (...) {
     return nullptr;
   }

@@ -234,11 +234,12 @@ inline bool pack_on_host() {
   return getenv("RBG_HOST_PACK") != nullptr && host_pack_threads() >= 4;
 }
 
-// Pinned result blocks (pooled).  pinned_take: a block of `bytes` or null;
+// Pinned result blocks (pooled).  pinned_take: a block of `bytes`, pinned on the
+// context's device, or null;
 // pinned_share: the block now backs graphs whose first edge arrays are
 // `firsts` (distinct), and returns to the pool when rbg_free_graph has been
 // called on each of them.
-void *pinned_take(size_t bytes);
+void *pinned_take(rbg_ctx *c, size_t bytes);
 void pinned_share(void *blk, const std::vector<void *> &firsts);
 
 // Device bytes of an admitted pair: its record and its two keys.
