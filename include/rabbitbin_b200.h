@@ -415,8 +415,9 @@ int rbg_free_graph(rbg_graph *g);
 /* Pinned host memory for results, from the pool that the graphs' arrays come
  * from: a call that writes its output there skips the driver's staging of
  * pageable memory and a fresh array's page faults.  NULL when it cannot be had
- * (use any memory then); release with rbg_result_free.  Pinned on the context's
- * device, or on the calling thread's current one. */
+ * (use any memory then), above 4 GB, and while the results not yet released hold
+ * that much; release with rbg_result_free.  Pinned on the context's device, or on
+ * the calling thread's current one. */
 void *rbg_result_alloc_on(rbg_ctx *ctx, size_t bytes);
 void *rbg_result_alloc(size_t bytes);
 void rbg_result_free(void *p);

@@ -437,7 +437,8 @@ class _ResultMem:
 
 def _result(ctx, shape, dtype):
     """An output array that the call fills completely: pinned memory of the
-    library's pool from 1 MB on (the device writes it at bus speed)."""
+    library's pool from 1 MB on (the device writes it at bus speed), as far as the
+    pool goes (4 GB of results held)."""
     L = ctx._L
     dt = np.dtype(dtype)
     nbytes = int(np.prod(shape, dtype=np.int64)) * dt.itemsize

@@ -1193,6 +1193,11 @@ void run_graph(rbg_ctx *c, const rbg_params *p, const ShardCtx *sc = nullptr) {
 // graph's arrays are ranges of the batch-wide arrays): it returns to the pool
 // when the last of them is freed.
 //
+// Results that callers hold (rbg_result_alloc) take at most as much as the pool
+// keeps: a larger one would be pinned and unpinned in every call (1 ms per 2 MB,
+// more than the staging it saves), and many small ones would pin the host's memory
+// for as long as they live.
+//
 // Blocks are pinned and unpinned with their device current (on a thread of its own
 // where the caller's is another one: setting it back would bring up a context
 // there).
@@ -1205,12 +1210,13 @@ struct PinnedPool {
   struct Block {
     size_t cls;
     int dev;
+    bool result;
   };
   std::mutex mu;
   std::unordered_map<void *, Block> live;
   std::unordered_map<void *, Shared *> part;   // a graph's first array -> its shared block
   std::deque<std::pair<Block, void *>> idle;   // oldest first
-  size_t idle_bytes = 0;
+  size_t idle_bytes = 0, result_bytes = 0;
 
   template <class F>
   static void on_device(int dev, F &&f) {
@@ -1233,9 +1239,11 @@ struct PinnedPool {
     return c;
   }
 
-  void *take(size_t bytes, int dev) {
+  void *take(size_t bytes, int dev, bool result = false) {
+    if (result && bytes > kKeep) return nullptr;
     const size_t cls = size_class(bytes);
     std::lock_guard<std::mutex> lk(mu);
+    if (result && result_bytes + cls > kKeep) return nullptr;
     void *p = nullptr;
     for (auto it = idle.rbegin(); it != idle.rend(); ++it)
       if (it->first.cls == cls) {
@@ -1253,7 +1261,8 @@ struct PinnedPool {
         }
       });
     if (!p) return nullptr;
-    live[p] = Block{cls, dev};
+    live[p] = Block{cls, dev, result};
+    if (result) result_bytes += cls;
     return p;
   }
 
@@ -1281,6 +1290,7 @@ struct PinnedPool {
     }
     auto it = live.find(p);
     if (it == live.end()) return false;
+    if (it->second.result) result_bytes -= it->second.cls;
     idle.emplace_back(it->second, p);
     idle_bytes += it->second.cls;
     live.erase(it);
@@ -1553,7 +1563,7 @@ extern "C" {
 
 void *rbg_result_alloc_on(rbg_ctx *c, size_t bytes) {
   try {
-    return c && bytes ? pinned_pool().take(bytes, c->device) : nullptr;
+    return c && bytes ? pinned_pool().take(bytes, c->device, true) : nullptr;
   } catch (...) {
     return nullptr;
   }
@@ -1566,7 +1576,7 @@ void *rbg_result_alloc(size_t bytes) {
     return nullptr;
   }
   try {
-    return bytes ? pinned_pool().take(bytes, dev) : nullptr;
+    return bytes ? pinned_pool().take(bytes, dev, true) : nullptr;
   } catch (...) {
     return nullptr;
   }
