@@ -6,8 +6,10 @@
 // symbols in lockstep (same bits, same tables: no divergence, broadcast loads);
 // the lanes store literals and copy matches and stored blocks together (a match
 // that overlaps itself repeats its first `distance` bytes, all of them written
-// before it).  The same code runs on the host
-// with one lane (the CPU tests).  Symbols are decoded with a 10-bit (literal /
+// before it).  The code is written against a Lanes type: one lane on the host
+// (SerialLanes), the warp on the device (WarpLanes), and in the tests 32 lanes that
+// take turns on the host, which run the warp's branches (Lanes::kWarp) on plain
+// memory.  Symbols are decoded with a 10-bit (literal /
 // length) and 8-bit (distance) lookup table of 32-bit entries that carry each
 // symbol's meaning (one or two literal bytes, length or distance base, extra
 // bits), with the canonical code walk for longer codes.  Every read stays inside [in, in + inlen),
@@ -40,22 +42,46 @@ enum Status : int32_t {
 
 constexpr int kLitBits = 10, kDistBits = 8;
 
-// The lanes that decode one block: one host thread, or one device warp.
+// The lanes that decode one block: one host thread, or one device warp.  A warp's
+// match(v) is the set of lanes with the same v, from(v, i) lane i's v.
 struct SerialLanes {
+  static constexpr bool kWarp = false;
   RBG_IHD int lane() const { return 0; }
   RBG_IHD int width() const { return 1; }
   RBG_IHD bool leader() const { return true; }
   RBG_IHD void sync() const {}
+  RBG_IHD uint32_t match(int) const { return 1; }
+  RBG_IHD uint32_t from(uint32_t v, int) const { return v; }
 };
 #ifdef __CUDACC__
 struct WarpLanes {
+  static constexpr bool kWarp = true;
   int l;
   __device__ __forceinline__ int lane() const { return l; }
   __device__ __forceinline__ int width() const { return 32; }
   __device__ __forceinline__ bool leader() const { return l == 0; }
   __device__ __forceinline__ void sync() const { __syncwarp(); }
+  __device__ __forceinline__ uint32_t match(int v) const { return __match_any_sync(0xffffffffu, v); }
+  __device__ __forceinline__ uint32_t from(uint32_t v, int i) const {
+    return __shfl_sync(0xffffffffu, v, i);
+  }
 };
 #endif
+
+RBG_IHD int bits_set(uint32_t v) {
+#ifdef __CUDA_ARCH__
+  return __popc(v);
+#else
+  return __builtin_popcount(v);
+#endif
+}
+RBG_IHD uint64_t load8(const uint64_t *p) {
+#ifdef __CUDA_ARCH__
+  return __ldg(p);
+#else
+  return *p;
+#endif
+}
 
 // One Huffman code: lookup table for codes up to kBits bits and the canonical
 // tables for the rest.  A table entry carries what the symbol means, so the
@@ -82,34 +108,35 @@ struct Tables {
   uint8_t clens[20];          // code-length code lengths
 };
 
+template <bool kWarp>
 struct Bits {
   const uint8_t *p;
   uint32_t n, pos;
   uint64_t buf;
   int cnt;
   RBG_IHD void refill() {
-#ifdef __CUDA_ARCH__
-    // two aligned 8-byte loads and a funnel shift; the device buffers hold the
-    // input from a 256-byte aligned start with 16 bytes of slack after its end,
-    // and bytes past the stream's end are masked off
-    if (pos >= n || cnt > 56) return;
-    const uintptr_t a = (uintptr_t)(p + pos);
-    const uint64_t *q = (const uint64_t *)(a & ~(uintptr_t)7);
-    const uint32_t sh = (uint32_t)(a & 7) * 8;
-    uint64_t w = __ldg(q) >> sh;
-    if (sh) w |= __ldg(q + 1) << (64 - sh);
-    uint32_t take = (uint32_t)(63 - cnt) >> 3;
-    if (take > n - pos) take = n - pos;
-    w &= take >= 8 ? ~0ull : ((1ull << (8 * take)) - 1);
-    buf |= w << cnt;
-    pos += take;
-    cnt += 8 * (int)take;
-#else
-    while (cnt <= 56 && pos < n) {
-      buf |= (uint64_t)p[pos++] << cnt;
-      cnt += 8;
+    if constexpr (kWarp) {
+      // two aligned 8-byte loads and a funnel shift; the device buffers hold the
+      // input from a 256-byte aligned start with 16 bytes of slack after its end,
+      // and bytes past the stream's end are masked off
+      if (pos >= n || cnt > 56) return;
+      const uintptr_t a = (uintptr_t)(p + pos);
+      const uint64_t *q = (const uint64_t *)(a & ~(uintptr_t)7);
+      const uint32_t sh = (uint32_t)(a & 7) * 8;
+      uint64_t w = load8(q) >> sh;
+      if (sh) w |= load8(q + 1) << (64 - sh);
+      uint32_t take = (uint32_t)(63 - cnt) >> 3;
+      if (take > n - pos) take = n - pos;
+      w &= take >= 8 ? ~0ull : ((1ull << (8 * take)) - 1);
+      buf |= w << cnt;
+      pos += take;
+      cnt += 8 * (int)take;
+    } else {
+      while (cnt <= 56 && pos < n) {
+        buf |= (uint64_t)p[pos++] << cnt;
+        cnt += 8;
+      }
     }
-#endif
   }
   RBG_IHD bool need(int k) {
     if (cnt < k) refill();
@@ -196,17 +223,13 @@ RBG_IHD int build(Code<kBits, kSyms> &c, const uint8_t *len, int n, const Lanes 
   for (int i = lane; i < 16; i += W) c.count[i] = 0;
   for (int i = lane; i < (1 << kBits); i += W) c.lut[i] = 0;
   L.sync();
-#ifdef __CUDA_ARCH__
-  for (int s0 = 0; s0 < n; s0 += 32) {
+  for (int s0 = 0; s0 < n; s0 += W) {
     const int l = s0 + lane < n ? len[s0 + lane] : 0;
-    const unsigned same = __match_any_sync(0xffffffffu, l);
-    if (l && lane == __ffs(same) - 1) c.count[l] = (uint16_t)(c.count[l] + __popc(same));
+    const uint32_t same = L.match(l);
+    if (l && (same & ((1u << lane) - 1u)) == 0)          // the lowest lane of the length
+      c.count[l] = (uint16_t)(c.count[l] + bits_set(same));
     L.sync();
   }
-#else
-  for (int s = 0; s < n; ++s)
-    if (len[s]) c.count[len[s]]++;
-#endif
   int left = 1;
   for (int l = 1; l < 16; ++l) {
     left <<= 1;
@@ -228,24 +251,17 @@ RBG_IHD int build(Code<kBits, kSyms> &c, const uint8_t *len, int n, const Lanes 
     const int s = s0 + lane;
     const int l = s < n ? len[s] : 0;
     uint32_t cd = 0, at = 0;
-#ifdef __CUDA_ARCH__
-    const unsigned same = __match_any_sync(0xffffffffu, l);
-    const uint32_t rank = (uint32_t)__popc(same & ((1u << lane) - 1u));
+    const uint32_t same = L.match(l);
+    const uint32_t rank = (uint32_t)bits_set(same & ((1u << lane) - 1u));
     if (l) {
       cd = c.next[l] + rank;
       at = c.offs[l] + rank;
     }
     L.sync();
     if (l && rank == 0) {
-      c.next[l] = (uint16_t)(c.next[l] + __popc(same));
-      c.offs[l] = (uint16_t)(c.offs[l] + __popc(same));
+      c.next[l] = (uint16_t)(c.next[l] + bits_set(same));
+      c.offs[l] = (uint16_t)(c.offs[l] + bits_set(same));
     }
-#else
-    if (l) {
-      cd = c.next[l]++;
-      at = c.offs[l]++;
-    }
-#endif
     if (l) {
       c.sym[at] = (uint16_t)s;
       if (l <= kBits) {                                // entered bit-reversed into the table
@@ -271,8 +287,8 @@ RBG_IHD int build(Code<kBits, kSyms> &c, const uint8_t *len, int n, const Lanes 
 
 // Decodes one symbol and returns its table entry; kEndOfInput when the stream
 // ends, kNoCode for a code that is not in the table.
-template <class Entry, int kBits, int kSyms>
-RBG_IHD uint32_t decode(const Code<kBits, kSyms> &c, Bits &b) {
+template <class Entry, int kBits, int kSyms, bool kWarp>
+RBG_IHD uint32_t decode(const Code<kBits, kSyms> &c, Bits<kWarp> &b) {
   if (b.cnt < 15) b.refill();
   // bits above cnt are zero, so the table index is defined near the end too;
   // an entry counts only when its whole code is in the buffer
@@ -303,12 +319,11 @@ template <class Lanes>
 RBG_IHD int inflate_block(const uint8_t *in, uint32_t inlen, uint8_t *out, uint32_t outlen,
                           Tables &T, const Lanes &L) {
   const int lane = L.lane(), W = L.width();
-  Bits b{in, inlen, 0, 0, 0};
+  constexpr bool kWarp = Lanes::kWarp;
+  Bits<kWarp> b{in, inlen, 0, 0, 0};
   uint32_t o = 0;
-#ifdef __CUDA_ARCH__
-  uint32_t held = 0, held_at = 0;      // a copy read but not stored: lane k's byte of `held`
+  uint32_t held = 0, held_at = 0;      // (warp) a copy read but not stored: lane k's byte of `held`
   uint8_t held_v = 0;
-#endif
   for (;;) {
     uint32_t hdr;
     if (!b.get(3, hdr)) return kErrInput;
@@ -403,12 +418,12 @@ RBG_IHD int inflate_block(const uint8_t *in, uint32_t inlen, uint8_t *out, uint3
           const uint32_t two = (q >> 6) & 1;
           b.drop(q & 15);
           if (o + two >= outlen) return kErrOutput;
-#ifdef __CUDA_ARCH__
-          if ((uint32_t)lane <= two) out[o + lane] = (uint8_t)(q >> (16 + 8 * lane));
-#else
-          out[o] = (uint8_t)(q >> 16);
-          if (two) out[o + 1] = (uint8_t)(q >> 24);
-#endif
+          if constexpr (kWarp) {
+            if ((uint32_t)lane <= two) out[o + lane] = (uint8_t)(q >> (16 + 8 * lane));
+          } else {
+            out[o] = (uint8_t)(q >> 16);
+            if (two) out[o + 1] = (uint8_t)(q >> 24);
+          }
           o += 1 + two;
           continue;
         }
@@ -422,10 +437,8 @@ RBG_IHD int inflate_block(const uint8_t *in, uint32_t inlen, uint8_t *out, uint3
           continue;
         }
         if (kind == 2) {
-#ifdef __CUDA_ARCH__
-          if ((uint32_t)lane < held) out[held_at + lane] = held_v;
+          if (kWarp && (uint32_t)lane < held) out[held_at + lane] = held_v;
           held = 0;
-#endif
           break;
         }
         if (kind == 3) return kErrSymbol;
@@ -450,24 +463,24 @@ RBG_IHD int inflate_block(const uint8_t *in, uint32_t inlen, uint8_t *out, uint3
         // distance repeats the first `dist` of them
         const uint8_t *src = out + (o - dist);
         uint8_t *dst = out + o;
-#ifdef __CUDA_ARCH__
-        // The copy of up to 32 bytes is stored at the next one: the loads' latency
-        // passes under the symbols decoded in between.
-        if ((uint32_t)lane < held) out[held_at + lane] = held_v;
-        held = 0;
-        L.sync();
-        if (len <= 32) {
-          if ((uint32_t)lane < len) held_v = src[dist >= len ? lane : lane % dist];
-          held = len;
-          held_at = o;
-        } else if (dist >= len) {
-          for (uint32_t k = lane; k < len; k += W) dst[k] = src[k];
+        if constexpr (kWarp) {
+          // The copy of up to 32 bytes is stored at the next one: the loads' latency
+          // passes under the symbols decoded in between.
+          if ((uint32_t)lane < held) out[held_at + lane] = held_v;
+          held = 0;
+          L.sync();
+          if (len <= 32) {
+            if ((uint32_t)lane < len) held_v = src[dist >= len ? lane : lane % dist];
+            held = len;
+            held_at = o;
+          } else if (dist >= len) {
+            for (uint32_t k = lane; k < len; k += W) dst[k] = src[k];
+          } else {
+            for (uint32_t k = lane; k < len; k += W) dst[k] = src[k % dist];
+          }
         } else {
-          for (uint32_t k = lane; k < len; k += W) dst[k] = src[k % dist];
+          for (uint32_t k = 0; k < len; ++k) dst[k] = src[dist >= len ? k : k % dist];
         }
-#else
-        for (uint32_t k = 0; k < len; ++k) dst[k] = src[dist >= len ? k : k % dist];
-#endif
         o += len;
       }
     } else {
@@ -521,23 +534,20 @@ RBG_IHD uint32_t crc32(const uint32_t *t, const uint8_t *p, uint32_t n, const La
   const uint32_t W = (uint32_t)L.width();
   const uint32_t seg = (n + W - 1) / W;
   uint32_t acc = 0;
-#ifdef __CUDA_ARCH__
-  if (W > 1) {
+  if constexpr (Lanes::kWarp) {
     const uint32_t a = (uint32_t)L.lane() * seg;
     const uint32_t e = a + seg < n ? a + seg : n;
     const uint32_t c = a < n ? crc_raw(t, 0u, p + a, e - a) : 0u;
     const uint32_t xs = x_pow8(seg);
     // Horner over the lanes: acc = acc * x^(8 len_i) + c_i
     for (uint32_t i = 0; i < W; ++i) {
-      const uint32_t ci = __shfl_sync(0xffffffffu, c, (int)i);
+      const uint32_t ci = L.from(c, (int)i);
       const uint32_t ai = i * seg;
       const uint32_t li = ai >= n ? 0u : (ai + seg < n ? seg : n - ai);
       if (li == seg) acc = gf2_mul(acc, xs) ^ ci;
       else if (li) acc = gf2_mul(acc, x_pow8(li)) ^ ci;
     }
-  } else
-#endif
-  {
+  } else {
     // one lane: the same joining, over W = 32 virtual segments
     const uint32_t vs = (n + 31) / 32;
     const uint32_t xs = x_pow8(vs);
