@@ -12,7 +12,7 @@
 // memory.  Symbols are decoded with a 10-bit (literal /
 // length) and 8-bit (distance) lookup table of 32-bit entries that carry each
 // symbol's meaning (one or two literal bytes, length or distance base, extra
-// bits), with the canonical code walk for longer codes.  Every read stays inside [in, in + inlen),
+// bits), with a search over the code lengths for longer codes.  Every read stays inside [in, in + inlen),
 // every write inside [out, out + outlen), and every match must point into
 // bytes already written: a stream that breaks a rule ends with a status, never
 // with an access out of bounds.
@@ -230,12 +230,10 @@ RBG_IHD int build(Code<kBits, kSyms> &c, const uint8_t *len, int n, const Lanes 
       c.count[l] = (uint16_t)(c.count[l] + bits_set(same));
     L.sync();
   }
-  int left = 1;
-  for (int l = 1; l < 16; ++l) {
-    left <<= 1;
-    left -= c.count[l];
-    if (left < 0) return kErrCodes;
-  }
+  // a code of l bits takes 2^(15 - l) of the 2^15 values of 15 bits
+  uint32_t taken = 0;
+  for (int l = 1; l < 16; ++l) taken += (uint32_t)c.count[l] << (15 - l);
+  if (taken > 1u << 15) return kErrCodes;
   // canonical codes in symbol order
   if (L.leader()) {
     uint32_t code = 0, at = 0;
@@ -297,20 +295,22 @@ RBG_IHD uint32_t decode(const Code<kBits, kSyms> &c, Bits<kWarp> &b) {
     b.drop(e & 15);
     return e;
   }
-  // canonical walk, one bit at a time (codes longer than the table)
-  int code = 0, first = 0, index = 0;
+  // Codes longer than the table.  Read as 15-bit numbers, first bit highest, the
+  // canonical codes of each length fill the range that follows the shorter ones', a
+  // code of l bits 2^(15 - l) numbers of it: the next 15 bits (zeros past the end of
+  // the stream) lie in the range of their length.
+  uint32_t at = reverse_bits(b.peek(15), 15), sym = 0;   // place past the shorter lengths' ranges
   for (int l = 1; l < 16; ++l) {
-    if (!b.need(1)) return kEndOfInput;
-    code |= (int)b.peek(1);
-    b.drop(1);
-    const int cnt = c.count[l];
-    if (code - cnt < first) return Entry::make(c.sym[index + (code - first)], l);
-    index += cnt;
-    first += cnt;
-    first <<= 1;
-    code <<= 1;
+    const uint32_t cnt = c.count[l];
+    if (at < cnt << (15 - l)) {
+      if (l > b.cnt) return kEndOfInput;
+      b.drop(l);
+      return Entry::make(c.sym[sym + (at >> (15 - l))], l);
+    }
+    at -= cnt << (15 - l);
+    sym += cnt;
   }
-  return kNoCode;
+  return b.cnt < 15 ? kEndOfInput : kNoCode;
 }
 
 // Inflates one raw deflate stream into out[0, outlen).  Returns kOk when the
