@@ -96,7 +96,6 @@ template <int kBits, int kSyms>
 struct Code {
   uint32_t lut[1 << kBits];
   uint16_t count[16];
-  uint16_t next[16], offs[16];         // while the code is built
   uint16_t sym[kSyms];
 };
 constexpr uint32_t kEndOfInput = 0xFFFFFFFFu, kNoCode = 0xFFFFFFFEu;
@@ -104,6 +103,7 @@ constexpr uint32_t kEndOfInput = 0xFFFFFFFFu, kNoCode = 0xFFFFFFFEu;
 struct Tables {
   Code<kLitBits, 288> lit;
   Code<kDistBits, 32> dist;
+  uint16_t next[16], offs[16];   // while a code is built
   uint8_t lens[320];          // code lengths being read (litlen then distance)
   uint8_t clens[20];          // code-length code lengths
 };
@@ -217,7 +217,7 @@ RBG_IHD uint32_t literal_pair(uint32_t e1, uint32_t e2) {
 // 32 symbols at a time: a symbol's canonical code follows from the symbols of its
 // length before it (the lanes below with the same length).
 template <class Entry, int kBits, int kSyms, class Lanes>
-RBG_IHD int build(Code<kBits, kSyms> &c, const uint8_t *len, int n, const Lanes &L) {
+RBG_IHD int build(Code<kBits, kSyms> &c, Tables &T, const uint8_t *len, int n, const Lanes &L) {
   const int lane = L.lane(), W = L.width();
   L.sync();
   for (int i = lane; i < 16; i += W) c.count[i] = 0;
@@ -239,8 +239,8 @@ RBG_IHD int build(Code<kBits, kSyms> &c, const uint8_t *len, int n, const Lanes 
     uint32_t code = 0, at = 0;
     for (int l = 1; l < 16; ++l) {
       code = (code + c.count[l - 1]) << 1;             // count[0] is 0
-      c.next[l] = (uint16_t)code;
-      c.offs[l] = (uint16_t)at;
+      T.next[l] = (uint16_t)code;
+      T.offs[l] = (uint16_t)at;
       at += c.count[l];
     }
   }
@@ -252,13 +252,13 @@ RBG_IHD int build(Code<kBits, kSyms> &c, const uint8_t *len, int n, const Lanes 
     const uint32_t same = L.match(l);
     const uint32_t rank = (uint32_t)bits_set(same & ((1u << lane) - 1u));
     if (l) {
-      cd = c.next[l] + rank;
-      at = c.offs[l] + rank;
+      cd = T.next[l] + rank;
+      at = T.offs[l] + rank;
     }
     L.sync();
     if (l && rank == 0) {
-      c.next[l] = (uint16_t)(c.next[l] + bits_set(same));
-      c.offs[l] = (uint16_t)(c.offs[l] + bits_set(same));
+      T.next[l] = (uint16_t)(T.next[l] + bits_set(same));
+      T.offs[l] = (uint16_t)(T.offs[l] + bits_set(same));
     }
     if (l) {
       c.sym[at] = (uint16_t)s;
@@ -375,7 +375,7 @@ RBG_IHD int inflate_block(const uint8_t *in, uint32_t inlen, uint8_t *out, uint3
         // the code-length code decodes through the distance table's storage
         // (it has 19 symbols and codes of at most 7 bits)
         Code<kDistBits, 32> &cc = T.dist;
-        if (build<PlainEntry>(cc, T.clens, 19, L) != kOk) return kErrCodes;
+        if (build<PlainEntry>(cc, T, T.clens, 19, L) != kOk) return kErrCodes;
         int i = 0;
         while (i < nlen + ndist) {
           const uint32_t ce = decode<PlainEntry>(cc, b);
@@ -407,8 +407,8 @@ RBG_IHD int inflate_block(const uint8_t *in, uint32_t inlen, uint8_t *out, uint3
         if (T.lens[256] == 0) return kErrCodes;       // no end-of-block code
       }
       L.sync();
-      if (build<LitEntry>(T.lit, T.lens, nlen, L) != kOk) return kErrCodes;
-      if (build<DistEntry>(T.dist, T.lens + 288, ndist, L) != kOk) return kErrCodes;
+      if (build<LitEntry>(T.lit, T, T.lens, nlen, L) != kOk) return kErrCodes;
+      if (build<DistEntry>(T.dist, T, T.lens + 288, ndist, L) != kOk) return kErrCodes;
       L.sync();
       for (;;) {
         // one or two literals from the table, the common case

@@ -94,7 +94,15 @@ __global__ void k_depth_means(const unsigned long long *__restrict__ sums, int64
 // Bound by each block's serial decode chain; few warps a CTA spread the blocks of
 // a small file evenly.  3,100 blocks (200 MB inflated): 7.3 ms a launch -> 5.65 ms,
 // the chains (0.64 ms in a kernel of their own) included.
-__global__ void __launch_bounds__(kInflateWarps * 32, 32 / kInflateWarps)
+//
+// 32 warps a SM: 62 registers a thread and the tables' 13.5 KB a CTA leave room for
+// them (13.6 KB, with the arrays of the table build kept twice, were room for 30
+// where the grid had 32: a second wave of one CTA a SM.  32,700 blocks in two chunks
+// 75 -> 64 ms a call, 7,100 blocks 11.8 -> 11.7 ms of kernels, 380 blocks 4.48 both).
+constexpr int kInflateCtas = 32 / kInflateWarps;       // a SM's
+static_assert(kInflateCtas * (kInflateWarps * sizeof(inflate::Tables) + 256 * 4 + 1024) <= 228 * 1024,
+              "the CTAs of a SM: tables, CRC table and the 1 KB that the system takes of each");
+__global__ void __launch_bounds__(kInflateWarps * 32, kInflateCtas)
 k_inflate(const uint8_t *__restrict__ comp, const DevBlk *__restrict__ blk, int nb,
           uint64_t hdr_end, uint8_t *__restrict__ out, uint32_t *__restrict__ counts,
           uint32_t *__restrict__ raw, uint32_t *__restrict__ flags) {
@@ -244,9 +252,13 @@ void launch_depth_device(const uint8_t *comp, const DevBlk *blk, int nb, uint64_
                          unsigned long long *sum, unsigned long long *sum_u, int sms,
                          cudaStream_t s) {
   if (nb <= 0) return;
-  // up to 32 warps a SM (64 registers, a few spilled: 40 ms against 46 ms at 24
-  // warps of 80 registers on a 5.6 M-read BAM)
-  const int ctas = std::min((nb + kInflateWarps - 1) / kInflateWarps, sms * (32 / kInflateWarps));
+  // As many CTAs as are resident at once (blocks are dealt out by a fixed stride, so a
+  // CTA that starts late ends late).
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_inflate, kInflateWarps * 32, 0) !=
+      cudaSuccess)
+    return;                                              // (the caller reads the error)
+  const int ctas = std::min((nb + kInflateWarps - 1) / kInflateWarps, sms * std::max(per_sm, 1));
   k_inflate<<<ctas, kInflateWarps * 32, 0, s>>>(comp, blk, nb, hdr_end, out, counts, raw, flags);
   k_scan_counts<<<1, 1024, 0, s>>>(counts, nb, scan, rec_total);
   k_gather_offsets<<<(unsigned)((nb + 7) / 8), 256, 0, s>>>(blk, nb, counts, scan, raw, offs);
