@@ -25,8 +25,7 @@ CU_SRCS = ["kernels_sketch.cu", "kernels_graph.cu", "kernels_allpairs.cu", "kern
 CPP_SRCS = ["pmh_streams.cpp", "calib.cpp", "engine.cpp", "batch.cpp", "server.cpp", "fasta.cpp",
             "cache.cpp", "host_pack.cpp", "lpa.cpp", "bam.cpp"]
 HEADERS = ["rbg_internal.h", "engine_internal.h", "select_topk.cuh", "scan.cuh", "warp_sort.cuh",
-           "tc05.cuh", "ddmath.cuh",
-           "depth_record.cuh", "inflate.cuh",
+           "sim_bins.cuh", "tc05.cuh", "ddmath.cuh", "depth_record.cuh", "inflate.cuh",
            "../../include/rabbitbin_b200.h", "gen_zig_tables.py"]
 
 

@@ -29,6 +29,7 @@
 #include "rbg_internal.h"
 #include "scan.cuh"
 #include "select_topk.cuh"
+#include "sim_bins.cuh"
 
 namespace rbg {
 namespace {
@@ -1201,19 +1202,11 @@ __global__ void k_scatter_pairs(SymOut o, const int64_t *off, uint64_t *keys,
   }
 }
 
-// Keys of a row ranked by a histogram of their similarity.  Bins of 2^15 steps of
-// the similarity's float bits above 1/32 (admitted similarities lie in
-// (0.039, 1)): one register count a bin at m = 500, finer below 0.5.
-constexpr uint32_t kBinBase = 0x3D000000u;          // 0.03125f
-constexpr int kBins = 1280;                         // through 1.0f
-constexpr int kBinShift = 15;
+// Keys of a row ranked by a histogram of their similarity (sim_bins.cuh).
 constexpr int kSelWords = kBins;                    // 32-bit words of a warp's buffer
 static_assert(kMergeBuf * 2 <= kSelWords, "the tie buffer lies over the histogram");
 
-__device__ __forceinline__ int key_bin(uint64_t key) {
-  const uint32_t b = ((uint32_t)(key >> 32) - kBinBase) >> kBinShift;
-  return (int)(b < (uint32_t)kBins ? b : 0u);       // below the base: the lowest bin
-}
+__device__ __forceinline__ int key_bin(uint64_t key) { return sim_bin((uint32_t)(key >> 32)); }
 
 // Keeps the R largest of the cnt unique keys in buf, in place.  Up to 96 keys by
 // their ranks (each lane counts the keys above its own), else by select_topk.
