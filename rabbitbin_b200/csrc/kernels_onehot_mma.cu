@@ -1091,6 +1091,8 @@ k_select_counts_rows(GraphArgs g, const uint16_t *__restrict__ C, int64_t ldc,
       const uint32_t mid = (T + hi) >> 1;
       if (__reduce_add_sync(FULL, at_least(y, mid)) >= (uint32_t)K) T = mid; else hi = mid;
     }
+    if (!ident)                                  // with every count of T's similarity
+      while (T > cf && tab[T - 1] == tab[T]) --T;
     const uint32_t t2 = T * 0x10001u;
     uint32_t hit[(4 * NV + 31) / 32] = {};
 #pragma unroll
