@@ -440,10 +440,6 @@ void launch_onehot_map(const uint32_t *pres, int m, int32_t *map, int32_t *koff,
 // X [n][ldx] int8: 1 at (i, map[r][code_i(r)]) for every set register, else 0.
 void launch_onehot_fill(const uint8_t *codesA, int64_t n, int m, int mpad, const int32_t *map,
                         int8_t *X, int64_t ldx, cudaStream_t s);
-// Rows [r0, r0 + nr) from their counts D[(i - r0) * ldd + j]: per-row top-K
-// keys, row maxima and compared pairs, as the dense all-pairs kernel gives.
-void launch_dense_select(const GraphArgs &g, const int32_t *D, int64_t ldd, int64_t r0, int64_t nr,
-                         cudaStream_t s);
 
 // ── FASTA ingest (kernels_fasta.cu) ────────────────────────────────────────
 // One record of a FASTA file on the device: its name range in the input, its
