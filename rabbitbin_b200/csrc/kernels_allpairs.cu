@@ -1353,8 +1353,8 @@ size_t tc_smem(int KS, int mpad, int Su) {
 
 int allpairs_cap(int K) { return (K + 64 + 31) & ~31; }
 
-// Column slices per 32-row block: enough warps for several waves of the GPU,
-// each slice at least 64 columns; a multiple of the CTA's warp count.
+// Column slices per 32-row block: enough warps for several waves of the GPU, a
+// multiple of the CTA's warp count.
 int allpairs_slices(int64_t n, int K) { return allpairs_slices_rows(n, n, K); }
 
 int allpairs_slices_rows(int64_t rows, int64_t n, int K) {

@@ -180,8 +180,6 @@ void launch_b0(const uint32_t *counts, int np, int m, float *b0_out, uint32_t *s
 void launch_pair_counts(const uint8_t *codesA, const uint8_t *codesB, int mpad, int m,
                         const int64_t *pairs, int npairs, uint32_t *out, cudaStream_t s);
 void launch_allpairs(const GraphArgs &g, uint64_t *gbuf, int32_t *gcnt, cudaStream_t s);
-// Warp per row of [g.row_lo, row_hi): its top-K from P partial lists of up to
-// cap keys (list of row r, part s at ((r/32 * P + s) * 32 + r%32) * cap).
 // ProbMinHash4 rows of n contigs from their winning elements (win_elem [n][m])
 // and 1/w rows (elem_winv [n][E]): winners_ (W64 [E][m]; 0 unset) and the
 // register values (1/w_e) * U_e(r) (U [E][m]; +inf unset).  Either output may be null.
@@ -206,6 +204,8 @@ void launch_index_rows(const GraphArgs &g, const uint64_t *row_keys, const uint6
                        const int32_t *ucount, const int64_t *uoff, const uint32_t *post,
                        const int32_t *nk, int64_t pl_cap, int min_common, double cutoff, int sms,
                        cudaStream_t s);
+// Warp per row of [g.row_lo, row_hi): its top-K from P partial lists of up to
+// cap keys (list of row r, part s at ((r/32 * P + s) * 32 + r%32) * cap).
 void launch_merge_topk(const GraphArgs &g, const uint64_t *gbuf, const int32_t *gcnt, int cap,
                        int P, cudaStream_t s);
 // Dense regime on tcgen05 (kernels_onehot_mma.cu): counts of the rows
@@ -457,7 +457,8 @@ void launch_fasta_positions(const uint8_t *in, int64_t F, int *tile_nl, int *til
 void launch_fasta_scatter(const uint8_t *in, int64_t F, const int64_t *nl_base,
                           const int64_t *gt_base, int64_t *nl_pos, int64_t *gt_pos,
                           cudaStream_t s);
-// flag[0..ngt] becomes the exclusive scan of record-start flags; rs the starts.
+// flag[0..ngt): whether a '>' starts a record; rank[0..ngt] their exclusive scan; rs
+// the starts.
 void launch_fasta_starts(const int64_t *gt_pos, int64_t ngt, const int64_t *nl_pos, int64_t nnl,
                          int32_t *flag, int64_t *rank, int64_t *rs, cudaStream_t s);
 void launch_fasta_records(const uint8_t *in, int64_t F, const int64_t *rs, int64_t nrs,
