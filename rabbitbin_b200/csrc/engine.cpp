@@ -2014,6 +2014,11 @@ int rbg_pmh_compare(rbg_ctx *c, int32_t metric, int32_t m, int32_t kmer_size, co
                             ? 1
                             : (int)std::max<int64_t>(1, std::min<int64_t>({kChunks, (int64_t)(bytes >> 23),
                                                                            tiles / 256}));
+      // also when an error ends the call: the result goes back to its owner then
+      struct Drain {
+        cudaStream_t s;
+        ~Drain() { if (s) cudaStreamSynchronize(s); }
+      } drain{parts > 1 ? c->copy : nullptr};
       if (parts > 1) {
         CK(cudaEventRecord(c->ev_cin, c->stream));             // the rows are on the device
         CK(cudaStreamWaitEvent(c->aux, c->ev_cin, 0));
