@@ -274,14 +274,19 @@ void stage_sketch_chunked(rbg_ctx *c, const rbg_params *p, const char *seqcat,
     }
   }
   // First words of the chunks: equal ones, or, where the pairs stream, each 0.83 of
-  // the one before.  A late chunk's pairs (against all rows so far) take about that
-  // share of its copy's time, so each is done when the next one has arrived, and
-  // less is left behind the last one (200,003 contigs x 30, 1.6 GB: 42.8 ms a call in
-  // equal chunks, 41.0 ms).
+  // the one before: a late chunk's pairs (against all rows so far) are more work, and
+  // less is left behind the last one.  Milliseconds a call in equal chunks / so
+  // (m = 500): 26,000 contigs x 12 samples 5.36 / 5.36, 40,000 x 10 (m = 250) 8.22 /
+  // 8.05, 60,000 x 20 11.76 / 11.52, 100,003 x 20 19.6 / 19.1, 150,000 x 10 43.8 /
+  // 43.8, 200,003 x 30 39.8 / 38.4, 300,000 x 30 62.1 / 60.2; 0.75 and 0.92 within 1%.
+  // Below 12 samples at more registers the pairs take longer than the copy from the
+  // first chunk on, and a large first chunk only delays them (m = 1,000: 60,000 x 10
+  // 13.44 / 13.61, 100,000 x 10 24.4 / 24.8; x 14 20.7 / 20.0): equal ones there.
+  const bool shrinking = stream_pairs && (S >= 12 || p->m <= 500);
   const double shrink = 0.83;
   auto cut = [&](int g) -> int64_t {
     if (g == G) return nwords;
-    const double f = stream_pairs ? (1.0 - std::pow(shrink, g)) / (1.0 - std::pow(shrink, G))
+    const double f = shrinking ? (1.0 - std::pow(shrink, g)) / (1.0 - std::pow(shrink, G))
                                   : (double)g / G;
     return (int64_t)(f * (double)nwords) & ~(int64_t)1;
   };
