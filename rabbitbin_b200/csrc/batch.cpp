@@ -185,7 +185,7 @@ int64_t batch_request_bytes(const rbg_params *p, int64_t n, int64_t nbases, int 
                            most && S >= 10 ? std::min(n * 1280 * kPairBytes, list_bytes) : 0) + n * 12;
     const int64_t entries = tc5_capacity(n, most ? 1.0 : kTc5First);
     b += tc5_sizes(n, mpad, std::min<int64_t>(entries, list_bytes / 4), kChunks).bytes();
-  } else if (dense_on_gemm(n) && onehot_mma_fits(n, m)) {           // one-hot rows, candidate lists
+  } else if (dense_on_gemm(n, m)) {           // one-hot rows, candidate lists
     int GR = 1, GC = 1;
     onehot_mma_grid((int)((n + 255) / 256), (int)((n + 255) / 256), 148, &GR, &GC);
     b += n * (int64_t)std::max(128, 136 * m / 8) +
@@ -260,7 +260,7 @@ void plan_batch(const rbg_params *defaults, const rbg_assembly *asms, int nb, Ba
     a.fused = (a.p->force_path == 2) || (a.p->force_path == 0 && a.n > 25000);
     a.abdfirst = a.fused && a.p->abdfirst && a.S > 1 && a.w_comp < 1.0 && a.w_comp < a.p->min_edge;
     a.variant = a.abdfirst ? a.Kp / 16 : 0;
-    a.gemm = !a.abdfirst && dense_on_gemm(a.n) && onehot_mma_fits(a.n, a.m);
+    a.gemm = !a.abdfirst && dense_on_gemm(a.n, a.m);
     double mult = untuned;
     if (tune) {
       const auto it = tune->find(tune_key(a));

@@ -529,7 +529,7 @@ void index_graph(rbg_ctx *c, const rbg_params *p, const GraphArgs &g, double cut
   const int64_t n = c->n;
   if (n == 0) return;
   const int m = p->m, K = p->max_edges;
-  if (index_rows_smem(n, K) > (size_t)227 * 1024)
+  if (index_rows_smem(n, K) > kMaxSmem)
     throw Error(RBG_ERR_UNSUPPORTED, "graph_index: at most about 37,000 contigs");
   const double Md = (double)m;
   size_t min_common = (size_t)std::floor(cutoff * Md * 0.7);
@@ -1073,7 +1073,7 @@ void run_graph(rbg_ctx *c, const rbg_params *p, const ShardCtx *sc = nullptr) {
     const int64_t rows = sc ? sc->row_hi - sc->row_lo : n;
     CK(cudaMemsetAsync(c->maxc_cand.p, 0, n1 * sizeof(uint32_t), c->stream));
     CK(cudaMemsetAsync(c->maxc_all.p, 0, n1 * sizeof(uint32_t), c->stream));
-    if (!g.prefilter && dense_on_gemm(n) && onehot_mma_fits(n, m)) {
+    if (!g.prefilter && dense_on_gemm(n, m)) {
       dense_allpairs_onehot(c, g);                      // tensor cores, exact counts
     } else {
       const size_t slots = (size_t)((rows + 31) / 32) * allpairs_slices_rows(rows, n, K) * 32;

@@ -114,6 +114,8 @@ void copy_out(rbg_ctx *c, void *dst, const void *src, size_t bytes, cudaStream_t
 
 inline int mpad_of(int m) { return (m + 15) & ~15; }
 
+constexpr size_t kMaxSmem = 227 * 1024;        // shared memory a CTA can have
+
 // Chunks of the host-to-device copy that rbg_bin_graph overlaps with the sketch.
 constexpr int kChunks = 8;
 
@@ -212,12 +214,15 @@ void tc5_check_wait(int stage);
 void tc5_raise_frac(rbg_ctx *c, int key, double need);
 // The dense regime runs on the one-hot tensor-core kernels, unless RBG_DENSE_ALU is
 // set (for measurement) or the contigs are few: the integer-ALU register compare
-// then, without the one-hot rows' four launches and the read-back of their width.
+// then, without the one-hot rows' four launches and the read-back of their width
+// (as far as its rows fit the shared memory: up to 3,520 registers).
 // A resident call with ALU / tensor cores at m = 500: 97 contigs 251 / 300 us, 300
 // 279 / 313, 500 295 / 332, 700 330 / 343 (m = 1,000: 368 / 368), 1,000 363 / 351.
 constexpr int64_t kDenseAlu = 512;
-inline bool dense_on_gemm(int64_t n) {
-  return n > kDenseAlu && getenv("RBG_DENSE_ALU") == nullptr;
+inline bool dense_on_gemm(int64_t n, int m) {
+  // (64 bytes: the batch kernel's variables beside the rows)
+  if (n <= kDenseAlu && allpairs_batch_smem(0, mpad_of(m), 0) + 64 <= kMaxSmem) return false;
+  return onehot_mma_fits(n, m) && getenv("RBG_DENSE_ALU") == nullptr;
 }
 
 // 2-bit packing on the host (host_pack.cpp): words [w0, w1) of the packed
