@@ -1026,7 +1026,15 @@ void launch_lpa_sort(const int64_t *off, int64_t n, uint64_t *key, const float *
   if (n == 0) return;
   cudaMemsetAsync(big, 0, sizeof(uint32_t), s);
   k_lpa_sort<<<(unsigned)((n + 3) / 4), 128, 0, s>>>(off, n, key, q, nbr, w, big);
-  k_lpa_sort_big<<<296, 256, 0, s>>>(off, key, q, nbr, w, big);
+  // as many CTAs as the shared keys let be resident: a graph may list every node
+  // (incidence of 20,000 nodes of 560 arcs 2.68 ms with two CTAs a SM, 1.98 so;
+  // 3,000 of 2,000 arcs 1.47 / 1.13)
+  int dev = 0, sms = 148, per_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lpa_sort_big, 256, 0);
+  const int64_t grid = std::min<int64_t>(n, (int64_t)sms * std::max(per_sm, 1));
+  k_lpa_sort_big<<<(unsigned)grid, 256, 0, s>>>(off, key, q, nbr, w, big);
 }
 
 void launch_lpa_init(const uint32_t *order, int64_t n, uint32_t *pos, uint32_t *label,
