@@ -5,6 +5,7 @@ The product is the CUDA library ``librabbitbin_b200.so`` built in-tree by
 CPU fallback: without a CUDA device every compute call raises ``RbgError``.
 """
 import ctypes as C
+import math
 import os
 
 import numpy as np
@@ -441,7 +442,7 @@ def _result(ctx, shape, dtype):
     pool goes (4 GB of results held)."""
     L = ctx._L
     dt = np.dtype(dtype)
-    nbytes = int(np.prod(shape, dtype=np.int64)) * dt.itemsize
+    nbytes = math.prod(shape) * dt.itemsize
     if nbytes >= 1 << 20:
         addr = L.rbg_result_alloc_on(ctx._h, nbytes)
         if addr:

@@ -41,10 +41,6 @@ __global__ void k_pmh_rows(const uint8_t *__restrict__ win_elem,
   }
 }
 
-constexpr int kQT = 64;       // rows of A and of B per CTA
-constexpr int kQC = 16;       // registers per staged chunk
-constexpr int kQS = kQC + 2;  // words of a staged row: 16-byte reads of 8 rows hit every bank
-
 // A word as compared: register values that are not numbers never match (they take
 // the pattern of an unset register), and zeros have one sign, so that equal
 // doubles are equal bits.
@@ -58,54 +54,62 @@ __device__ __forceinline__ uint64_t canonical(uint64_t w) {
   return w;
 }
 
-// CTA: a 64 x 64 tile of (A row, B row) pairs; thread (tx, ty) owns the 16 pairs
-// (ty + 16 u, tx + 16 v).  Register chunks of A and B rows are staged in shared
-// memory, the next chunk's words loading meanwhile.  Bound by the integer pipe
-// (76% busy, issue 82%): two half-word comparisons and a count a pair and
-// register.  1,000 x 4,999 rows, m = 1,000: 1.16 ms with 4 pairs a thread and
-// both words tested for every pair, 1.00 ms now.
-template <bool REGS>
+// CTA: a T x T tile of (A row, B row) pairs; thread (tx, ty) owns the pairs (ty + 16 u,
+// tx + 16 v), u, v < T / 16.  Chunks of QC registers of A and B rows are staged in
+// shared memory, the next chunk's words loading meanwhile.
+//
+// T = 64, QC = 16: bound by the integer pipe (76% busy, issue 82%): two half-word
+// comparisons and a count a pair and register.  1,000 x 4,999 rows, m = 1,000: 1.16 ms
+// with 4 pairs a thread and both words tested for every pair, 1.00 ms now.  Few rows
+// leave most SMs idle and are bound by the chain of chunks, so they take smaller
+// tiles of longer chunks (launch_pmh_compare).
+template <bool REGS, int T, int QC>
 __global__ void __launch_bounds__(256)
 k_pmh_compare(const uint64_t *__restrict__ A, int64_t na, const uint64_t *__restrict__ B,
               int64_t nb, int m, const double *__restrict__ table, double *__restrict__ out) {
-  __shared__ __align__(16) uint64_t sa[2][kQT][kQS], sb[2][kQT][kQS];
-  constexpr int kPer = kQT * kQC / 256;          // words of A and of B a thread stages
+  constexpr int QS = QC + 2;                     // words of a staged row: 16-byte reads of 8
+                                                 // rows hit every bank
+  constexpr int P = T / 16;                      // pairs of a thread, a side
+  constexpr int kPer = T * QC / 256;             // words of A and of B a thread stages
+  constexpr int kRows = 256 / QC;                // rows that the threads stage at a time
+  static_assert(kPer * kRows == T, "a thread stages one column of rows kRows apart");
+  __shared__ __align__(16) uint64_t sa[2][T][QS], sb[2][T][QS];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t a0 = (int64_t)blockIdx.y * kQT, b0 = (int64_t)blockIdx.x * kQT;
-  int cnt[4][4] = {};
+  const int sc = threadIdx.x % QC, sr = threadIdx.x / QC;
+  const int64_t a0 = (int64_t)blockIdx.y * T, b0 = (int64_t)blockIdx.x * T;
+  int cnt[P][P] = {};
   const uint64_t unset = REGS ? 0x7ff0000000000000ull : 0ull;
   uint64_t ra[kPer], rb[kPer];
   // the next chunk's words load while a chunk is compared
   auto fetch = [&](int k0) {
 #pragma unroll
     for (int t = 0; t < kPer; ++t) {
-      const int row = ty + 16 * t, col = k0 + tx;
+      const int row = sr + kRows * t, col = k0 + sc;
       ra[t] = (col < m && a0 + row < na) ? __ldg(A + (a0 + row) * m + col) : unset;
       rb[t] = (col < m && b0 + row < nb) ? __ldg(B + (b0 + row) * m + col) : unset;
     }
   };
-  static_assert(kQC == 16 && kPer * 16 == kQT, "a thread stages column tx of rows ty, ty + 16, ..");
   fetch(0);
   int s = 0;
-  for (int k0 = 0; k0 < m; k0 += kQC, s ^= 1) {
+  for (int k0 = 0; k0 < m; k0 += QC, s ^= 1) {
 #pragma unroll
     for (int t = 0; t < kPer; ++t) {
-      sa[s][ty + 16 * t][tx] = canonical<REGS>(ra[t]);
-      sb[s][ty + 16 * t][tx] = canonical<REGS>(rb[t]);
+      sa[s][sr + kRows * t][sc] = canonical<REGS>(ra[t]);
+      sb[s][sr + kRows * t][sc] = canonical<REGS>(rb[t]);
     }
     __syncthreads();
-    if (k0 + kQC < m) fetch(k0 + kQC);
+    if (k0 + QC < m) fetch(k0 + QC);
 #pragma unroll 2
-    for (int k = 0; k < kQC; k += 2) {
-      ulonglong2 b[4];
+    for (int k = 0; k < QC; k += 2) {
+      ulonglong2 b[P];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) b[v] = *reinterpret_cast<const ulonglong2 *>(&sb[s][tx + 16 * v][k]);
+      for (int v = 0; v < P; ++v) b[v] = *reinterpret_cast<const ulonglong2 *>(&sb[s][tx + 16 * v][k]);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < P; ++u) {
         const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(&sa[s][ty + 16 * u][k]);
         const bool set0 = a.x != unset, set1 = a.y != unset;
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
+        for (int v = 0; v < P; ++v) {
           if (set0 && a.x == b[v].x) ++cnt[u][v];
           if (set1 && a.y == b[v].y) ++cnt[u][v];
         }
@@ -113,12 +117,20 @@ k_pmh_compare(const uint64_t *__restrict__ A, int64_t na, const uint64_t *__rest
     }
   }
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+  for (int u = 0; u < P; ++u)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
+    for (int v = 0; v < P; ++v) {
       const int64_t i = a0 + ty + 16 * u, j = b0 + tx + 16 * v;
       if (i < na && j < nb) out[i * nb + j] = __ldg(table + cnt[u][v]);
     }
+}
+
+template <int T, int QC>
+void launch_compare_tiles(const uint64_t *A, int64_t na, const uint64_t *B, int64_t nb, int m,
+                          bool regs, const double *table, double *out, cudaStream_t s) {
+  const dim3 grid((unsigned)((nb + T - 1) / T), (unsigned)((na + T - 1) / T));
+  if (regs) k_pmh_compare<true, T, QC><<<grid, 256, 0, s>>>(A, na, B, nb, m, table, out);
+  else k_pmh_compare<false, T, QC><<<grid, 256, 0, s>>>(A, na, B, nb, m, table, out);
 }
 
 __global__ void k_pmh_merge(const double *__restrict__ a, const double *__restrict__ b,
@@ -145,9 +157,16 @@ void launch_pmh_rows(const uint8_t *win_elem, const double *elem_winv, int64_t n
 void launch_pmh_compare(const uint64_t *A, int64_t na, const uint64_t *B, int64_t nb, int m,
                         bool regs, const double *table, double *out, cudaStream_t s) {
   if (na == 0 || nb == 0) return;
-  const dim3 grid((unsigned)((nb + kQT - 1) / kQT), (unsigned)((na + kQT - 1) / kQT));
-  if (regs) k_pmh_compare<true><<<grid, 256, 0, s>>>(A, na, B, nb, m, table, out);
-  else k_pmh_compare<false><<<grid, 256, 0, s>>>(A, na, B, nb, m, table, out);
+  const int64_t c64 = (na + 63) / 64 * ((nb + 63) / 64), c32 = (na + 31) / 32 * ((nb + 31) / 32);
+  const int64_t few = std::min(na, nb);
+  // A call in tiles of 64 / 32 / 16 (winner rows, m registers, ms): 1 x 1 (m = 1,000) 0.164 /
+  // 0.092 / 0.074, 65 x 65 (4,000) 0.603 / 0.319 / 0.247, 10 x 300 (1,000) 0.219 / 0.143 /
+  // 0.125, 1 x 20,000 (500) 1.68 / 1.61 / 1.59, 300 x 300 (1,000) 0.395 / 0.320 / 0.322,
+  // 500 x 500 (1,000) 0.341 / 0.299 / 0.342, 700 x 700 (500) 0.277 / 0.289 / 0.325,
+  // 1,000 x 4,999 (1,000) 2.20 / 2.44 / 3.42
+  if (few > 32 && c64 >= 100) launch_compare_tiles<64, 16>(A, na, B, nb, m, regs, table, out, s);
+  else if (few > 16 && c32 > 100) launch_compare_tiles<32, 32>(A, na, B, nb, m, regs, table, out, s);
+  else launch_compare_tiles<16, 64>(A, na, B, nb, m, regs, table, out, s);
 }
 
 void launch_pmh_merge(const double *a, const double *b, int64_t count, double *out,
