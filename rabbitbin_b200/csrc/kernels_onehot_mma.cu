@@ -1037,18 +1037,19 @@ k_select_counts(GraphArgs g, const uint16_t *__restrict__ C, int64_t ldc,
   if (row < (int)g.n) select_row<NV, 1>(g, C, ldc, tab, row, red, s_pos, nzb);
 }
 
-// Eight warps a row, R <= 8 rows in turn.  Each thread's even and odd columns
-// give 512 disjoint groups; K of their maxima reach the K-th largest maximum, so
-// at least K counts do: one value a thread is searched instead of the whole row,
-// and few counts pass (about 1.2 K of 20,000).  These are listed, and each warp
-// selects one row's K best from its list.  A row whose list overflows (ties) is
-// selected from registers, as above.
-template <int NV>
+// Eight warps a row, R <= 8 rows in turn.  Each thread's even and odd columns, of
+// each of H parts of them, give 512 H disjoint groups; K of their maxima reach the
+// K-th largest maximum, so at least K counts do: H values a thread are searched
+// instead of the whole row, and few counts pass (about 1.2 K of 20,000 at K = 200,
+// but -512 H ln(1 - K / 512 H) as K nears the groups: over 1,024 at K = 448 of 512).
+// These are listed, and each warp selects one row's K best from its list.  A row
+// whose list overflows (ties) is selected from registers, as above.
+template <int NV, int H>
 __global__ void __launch_bounds__(256, NV <= 12 ? 3 : 2)
 k_select_counts_rows(GraphArgs g, const uint16_t *__restrict__ C, int64_t ldc,
                      const uint32_t *__restrict__ tab, int R) {
   __shared__ uint32_t list[8][kOmBuf];
-  __shared__ uint32_t mx[2][256];
+  __shared__ uint32_t mx[2][H][256];
   __shared__ unsigned cnt[8];
   __shared__ uint32_t red[2][8];
   __shared__ int s_pos[8];
@@ -1072,14 +1073,17 @@ k_select_counts_rows(GraphArgs g, const uint16_t *__restrict__ C, int64_t ldc,
       if (lane == 0 && all) atomicMax(g.maxcnt_all + row, all);
       mask_counts<NV>(nzb, n, w0, x);
     }
-    uint32_t m2 = 0;
 #pragma unroll
-    for (int k = 0; k < 4 * NV; ++k) m2 = __vmaxu2(m2, x[k]);
-    mx[r & 1][threadIdx.x] = m2;
+    for (int h = 0; h < H; ++h) {
+      uint32_t m2 = 0;
+#pragma unroll
+      for (int k = 4 * NV / H * h; k < 4 * NV / H * (h + 1); ++k) m2 = __vmaxu2(m2, x[k]);
+      mx[r & 1][h][threadIdx.x] = m2;
+    }
     __syncthreads();
-    uint32_t y[8];
+    uint32_t y[8 * H];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) y[k] = mx[r & 1][32 * k + lane];
+    for (int k = 0; k < 8 * H; ++k) y[k] = mx[r & 1][k >> 3][32 * (k & 7) + lane];
     const uint32_t top = __reduce_max_sync(FULL, largest(y));
     if (threadIdx.x == 0 && top) {
       if (nz) atomicMax(g.maxcnt_all + row, top);
@@ -1087,7 +1091,7 @@ k_select_counts_rows(GraphArgs g, const uint16_t *__restrict__ C, int64_t ldc,
     }
     if (top < cf) continue;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) y[k] |= kTop;
+    for (int k = 0; k < 8 * H; ++k) y[k] |= kTop;
     uint32_t T = cf, hi = top + 1;               // K maxima reach T, or T = cf
     while (hi - T > 1) {
       const uint32_t mid = (T + hi) >> 1;
@@ -1149,7 +1153,12 @@ void launch_select_rows_nv(const GraphArgs &g, const uint16_t *C, int64_t ldc, c
   // 0.609 ms, 8,000 0.783 / 0.786, 20,011 2.170 / 2.163, 32,000 4.06 / 4.03; 1 row
   // 3 to 8% more).
   const int R = g.n > 8192 ? 8 : 4;
-  k_select_counts_rows<NV><<<(unsigned)((g.n + R - 1) / R), 256, 0, s>>>(g, C, ldc, tab, R);
+  const unsigned blocks = (unsigned)((g.n + R - 1) / R);
+  // A staged call with 512 / 1,024 groups, 25,000 contigs: K = 200 2.87 / 2.90 ms, 300
+  // 3.10 / 3.04, 350 3.20 / 3.11, 400 5.04 / 3.17, 448 5.87 / 3.21; 8,000: 350 0.838 /
+  // 0.842, 448 0.955 / 0.855
+  if (g.K <= 320) k_select_counts_rows<NV, 1><<<blocks, 256, 0, s>>>(g, C, ldc, tab, R);
+  else k_select_counts_rows<NV, 2><<<blocks, 256, 0, s>>>(g, C, ldc, tab, R);
 }
 
 // A warp a row up to 4,096 columns (16 words a lane), a block above.  (20,011

@@ -26,9 +26,7 @@ def _assembly(n, seed):
     return buf.tobytes(), np.arange(n + 1, dtype=np.int64) * 400, depth
 
 
-@pytest.mark.parametrize("n", [513, 641, 767, 768, 769, 1024, 8192, 16384, 24576, 24577, 32768, 32769])
-@pytest.mark.parametrize("m,K", [(24, 448), (250, 200)])
-def test_counts_equal_register_compare(gpu_ctx, monkeypatch, n, m, K):
+def _check(gpu_ctx, monkeypatch, n, m, K):
     seqcat, offs, depth = _assembly(n, n + m)
     p = api.default_params(m=m, max_edges=K, force_path=1)
     for env in ("RBG_ONEHOT_CAP", "RBG_DENSE_ALU"):
@@ -40,3 +38,16 @@ def test_counts_equal_register_compare(gpu_ctx, monkeypatch, n, m, K):
     assert got["sim_cutoff"] == want["sim_cutoff"] and got["b0"] == want["b0"]
     for k in ("src", "dst", "scomp", "score"):
         assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("n", [513, 641, 767, 768, 769, 1024, 8192, 16384, 24576, 24577, 32768, 32769])
+@pytest.mark.parametrize("m,K", [(24, 448), (250, 200)])
+def test_counts_equal_register_compare(gpu_ctx, monkeypatch, n, m, K):
+    _check(gpu_ctx, monkeypatch, n, m, K)
+
+
+@pytest.mark.parametrize("n", [4097, 8193, 16385, 24577])
+@pytest.mark.parametrize("K", [320, 321, 400, 448])
+def test_many_neighbours(gpu_ctx, monkeypatch, n, K):
+    """512 and 1,024 groups of columns a row (K up to 320, and above)."""
+    _check(gpu_ctx, monkeypatch, n, 120, K)
