@@ -22,6 +22,7 @@
 #include <cstdint>
 #include <cstring>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -108,54 +109,62 @@ class Pool {
     for (auto &t : threads_) t.join();
   }
   int size() const { return nthreads_; }
+  // fn(0) .. fn(parts - 1), each once, on the calling thread and the pool's.
   void run(const std::function<void(int)> &fn, int parts) {
     std::lock_guard<std::mutex> one(run_mu_);         // one job at a time
+    const auto job = std::make_shared<Job>(fn, parts);
     {
       std::lock_guard<std::mutex> lk(mu_);
-      fn_ = &fn;
-      parts_ = parts;
-      next_.store(0);
-      done_ = 0;
+      job_ = job;
       ++gen_;
     }
     cv_.notify_all();
-    work();
+    work(*job);
     std::unique_lock<std::mutex> lk(mu_);
-    done_cv_.wait(lk, [&] { return done_ == parts_; });
-    fn_ = nullptr;
+    done_cv_.wait(lk, [&] { return job->done == parts; });
+    job_.reset();
   }
 
  private:
-  void work() {
+  // A thread works on the job that it took under the lock: one that comes late finds
+  // that job's parts all taken, and never counts a part of the next job for it.
+  struct Job {
+    Job(const std::function<void(int)> &f, int n) : fn(f), parts(n) {}
+    const std::function<void(int)> &fn;               // the caller's, until every part is done
+    const int parts;
+    std::atomic<int> next{0};
+    int done = 0;                                     // under mu_
+  };
+  void work(Job &job) {
     for (;;) {
-      const int i = next_.fetch_add(1);
-      if (i >= parts_) return;
-      (*fn_)(i);
+      const int i = job.next.fetch_add(1);
+      if (i >= job.parts) return;
+      job.fn(i);
       std::lock_guard<std::mutex> lk(mu_);
-      if (++done_ == parts_) done_cv_.notify_all();
+      if (++job.done == job.parts) done_cv_.notify_all();
     }
   }
   void loop() {
     uint64_t seen = 0;
     for (;;) {
+      std::shared_ptr<Job> job;
       {
         std::unique_lock<std::mutex> lk(mu_);
         cv_.wait(lk, [&] { return stop_ || gen_ != seen; });
         if (stop_) return;
         seen = gen_;
+        job = job_;
       }
-      work();
+      if (job) work(*job);
     }
   }
   int nthreads_ = 1;
   std::vector<std::thread> threads_;
   std::mutex mu_, run_mu_;
   std::condition_variable cv_, done_cv_;
-  const std::function<void(int)> *fn_ = nullptr;
-  int parts_ = 0, done_ = 0;
+  std::shared_ptr<Job> job_;
   uint64_t gen_ = 0;
   bool stop_ = false;
-  std::atomic<int> next_{0};
 };
 
 Pool &pool() {
