@@ -686,10 +686,20 @@ bool tc5_lists_large(const rbg_ctx *c, int S, int64_t n) {
   return c->tc5_frac[tc5_key(S, n)] > tc5_most(c, n);
 }
 
-// The fraction that sizes an assembly's lists: the remembered one, at least kTc5First
-// as far as list_bytes allows.
+// The fraction that sizes an assembly's lists: the remembered one, at least kTc5First;
+// for a size not seen yet that of the nearest one at these samples, up to four times
+// smaller or larger.  What is not this size's own stays within list_bytes.
 double tc5_list_frac(const rbg_ctx *c, int S, int64_t n) {
-  return std::max(c->tc5_frac[tc5_key(S, n)], std::min(kTc5First, tc5_most(c, n)));
+  const int key = tc5_key(S, n), lo = 27 * S, hi = lo + 26;
+  const double own = c->tc5_frac[key];
+  double guess = kTc5First;
+  if (own == 0.0) {
+    double near = 0.0;
+    for (int d = 1; d <= 2 && near == 0.0; ++d)
+      near = std::max(key - d >= lo ? c->tc5_frac[key - d] : 0.0, key + d <= hi ? c->tc5_frac[key + d] : 0.0);
+    guess = std::max(guess, near);
+  }
+  return std::max(own, std::min(guess, tc5_most(c, n)));
 }
 
 int sym_tc5_prefilter(rbg_ctx *c, const GraphArgs &g, int64_t cb, int64_t ce, int slot);

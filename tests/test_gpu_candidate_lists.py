@@ -118,3 +118,23 @@ def test_streamed_pair_list_within_its_bound(monkeypatch):
             assert np.array_equal(g[k], want[0][k]), k
     # about 1.1 M survivors: 45 MB with a quarter to spare
     assert least <= most - (12 << 20)
+
+
+def test_nearby_sizes_share_their_fraction():
+    """An assembly of twice the contigs of one seen before takes no second pass: its
+    first call launches what its second does."""
+    ctx = api.Context(0)
+    try:
+        def launches(n):
+            # 20 genomes: about 0.7 M pairs of one genome at 5,200 contigs, below the 1 M
+            # that the pair list holds at first
+            a = make_assembly(20, n, 5, seed=7, median_len=2600.0, max_len=3000)
+            ctx.stage(*a.concat(), a.depth)
+            p = api.default_params(force_path=2)
+            return [ctx.run_resident(p)["kernel_launches"] for _ in range(2)]
+        first, later = launches(2600)
+        assert first > later                                # lists overflowed, and the pass ran again
+        first, later = launches(5200)
+        assert first == later
+    finally:
+        ctx.close()
